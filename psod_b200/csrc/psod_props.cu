@@ -18,7 +18,7 @@
 //                     unwrapped member positions staged in member order;
 //   k_props_potential (halo, 256-member chunk) items over all CTAs: each
 //                     member's potential sum against the halo's members,
-//                     read through shared-memory tiles;
+//                     two members a thread, read through shared tiles;
 //   k_props_finish    a CTA per halo: total potential and its most bound
 //                     member, the two radial histograms, the R178
 //                     interpolation, the eigen solve and every output.
@@ -27,6 +27,7 @@
 // file is built with --fmad=false, so no product is fused into a sum.  The
 // sums run in another order than the sequential reference, so FP64 values
 // can differ in their last bits before the real(4) outputs are rounded.
+#include <algorithm>
 #include <cmath>
 
 #include "psod_internal.cuh"
@@ -233,45 +234,122 @@ __device__ __forceinline__ long long pot_member(long long k, long long np, long 
   return m == np ? k : (k * np) / m;
 }
 
-__global__ void __launch_bounds__(PR_TPB) k_props_potential(PropsConst K, const long long *ipref, long long nitem,
+// float -> double by its bits, for x >= 0 below 2^127: exact for normal x;
+// zero and denormals come out below 2^-125, far under half an ulp of the
+// softening they are added to.  Two integer operations, where the 64-bit
+// conversion unit (16 lanes a clock) would bound the pair loop.
+__device__ __forceinline__ double widen_pos(float x) {
+  const unsigned b = __float_as_uint(x);
+  return __hiloint2double((int)((b >> 3) + (896u << 20)), (int)(b << 29));
+}
+
+// 1/sqrt(x) in FP64 from the FP32 estimate y0 (relative error below 2^-21):
+// Halley's third-order step y0 + y0 e (1/2 + 3/8 e), e = 1 - x y0^2, whose
+// truncation error 5/16 e^3 is below 2^-61; with its roundings the result is
+// within one ulp, as the rounded square root and quotient it replaces.
+__device__ __forceinline__ double rsqrt_halley(double x, float y0f) {
+  const double y0 = widen_pos(y0f);
+  const double t = x * y0;
+  const double e = __fma_rn(-t, y0, 1.0);
+  return __fma_rn(__fma_rn(0.375, e, 0.5), y0 * e, y0);
+}
+
+// one MUFU operation; x is at least the softening, never denormal
+__device__ __forceinline__ float rsqrt_est(float x) {
+  float y;
+  asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+__device__ __forceinline__ unsigned long long pk2(float lo, float hi) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// A CTA of PP_TPB threads takes one (halo, PR_TPB members) item from a
+// counter, two members a thread: the real(4) differences and squares of the
+// two run as packed pairs (each half rounded as the scalar operation), the
+// staged members are read by broadcast.  Bound: FP64 pipe (7 operations a
+// pair) and instruction issue (about 17 a pair), against ~37 FP64
+// operations a pair with the square root and the division.  192^3 box, 3
+// million members, 1.5e10 ordered pairs: POTENTIAL_MS.
+constexpr int PP_TPB = PR_TPB / 2;
+
+__global__ void __launch_bounds__(PP_TPB) k_props_potential(PropsConst K, const long long *ipref, unsigned nitem,
                                                             const unsigned *ihalo, const long long *off,
-                                                            const HaloWork *W, const float *hpos, double *epi) {
-  __shared__ float tx[PR_TPB], ty[PR_TPB], tz[PR_TPB];
-  const double mp2 = K.mass_part * K.mass_part;
-  for (long long it = blockIdx.x; it < nitem; it += gridDim.x) {
+                                                            const HaloWork *W, const float *hpos, unsigned *next,
+                                                            double *epi) {
+  __shared__ ulonglong2 txy[PR_TPB];          // (-x, -x), (-y, -y)
+  __shared__ unsigned long long tz[PR_TPB];   // (-z, -z)
+  __shared__ unsigned s_item;
+  const double mp2 = K.mass_part * K.mass_part;  // a power of two: scales the finished sums exactly
+  const float dxf = (float)K.delta_x2;
+  const unsigned long long dxf2 = pk2(dxf, dxf);
+  while (true) {
+    __syncthreads();
+    if (threadIdx.x == 0) s_item = atomicAdd(next, 1u);
+    __syncthreads();
+    const unsigned it = s_item;
+    if (it >= nitem) break;
     const unsigned h = ihalo[it];
-    const long long chunk = it - ipref[h];
+    const long long i0 = ((long long)it - ipref[h]) * PR_TPB;
     const long long b = off[h], np = W[h].np, m = W[h].m;
-    const long long ii = chunk * PR_TPB + threadIdx.x;
-    const bool have = ii < m;
-    float xi = 0.f, yi = 0.f, zi = 0.f;
-    if (have) {
-      const long long k = b + pot_member(ii, np, m);
-      xi = hpos[3 * k];
-      yi = hpos[3 * k + 1];
-      zi = hpos[3 * k + 2];
-    }
-    double ei = 0.0;
+    const int ta = threadIdx.x, tb = threadIdx.x + PP_TPB;  // the members' places in the own tile
+    const bool ha = i0 + ta < m, hb = i0 + tb < m;
+    const float *pa = hpos + 3 * (b + (ha ? pot_member(i0 + ta, np, m) : 0));
+    const float *pb = hpos + 3 * (b + (hb ? pot_member(i0 + tb, np, m) : 0));
+    const unsigned long long xi = pk2(pa[0], pb[0]), yi = pk2(pa[1], pb[1]), zi = pk2(pa[2], pb[2]);
+    double ea = 0.0, eb = 0.0;
     for (long long j0 = 0; j0 < m; j0 += PR_TPB) {
-      const long long jj = j0 + threadIdx.x;
+      const int nt = (int)min((long long)PR_TPB, m - j0);
       __syncthreads();
-      if (jj < m) {
-        const long long k = b + pot_member(jj, np, m);
-        tx[threadIdx.x] = hpos[3 * k];
-        ty[threadIdx.x] = hpos[3 * k + 1];
-        tz[threadIdx.x] = hpos[3 * k + 2];
+      for (int t = threadIdx.x; t < nt; t += PP_TPB) {
+        const float *p = hpos + 3 * (b + pot_member(j0 + t, np, m));
+        const float x = -p[0], y = -p[1], z = -p[2];
+        txy[t] = make_ulonglong2(pk2(x, x), pk2(y, y));
+        tz[t] = pk2(z, z);
       }
       __syncthreads();
-      const int nt = (int)min((long long)PR_TPB, m - j0);
-      if (have)
+      if (!ha) continue;
+      auto pair = [&](int t, double &va, double &vb) {
+        const ulonglong2 q = txy[t];
+        const unsigned long long ax = add2(xi, q.x), ay = add2(yi, q.y), az = add2(zi, tz[t]);
+        const unsigned long long s3 = add2(add2(mul2(ax, ax), mul2(ay, ay)), mul2(az, az));
+        const unsigned long long x2 = add2(s3, dxf2);
+        const float sa = __uint_as_float((unsigned)s3), sb = __uint_as_float((unsigned)(s3 >> 32));
+        va = rsqrt_halley(widen_pos(sa) + K.delta_x2, rsqrt_est(__uint_as_float((unsigned)x2)));
+        vb = rsqrt_halley(widen_pos(sb) + K.delta_x2, rsqrt_est(__uint_as_float((unsigned)(x2 >> 32))));
+      };
+      if (j0 != i0) {
+#pragma unroll 4
         for (int t = 0; t < nt; t++) {
-          if (j0 + t == ii) continue;
-          const float ax = xi - tx[t], ay = yi - ty[t], az = zi - tz[t];
-          const float s3 = ax * ax + ay * ay + az * az;
-          ei = ei + mp2 / sqrt((double)s3 + K.delta_x2);
+          double va, vb;
+          pair(t, va, vb);
+          ea += va;
+          eb += vb;
         }
+      } else {  // the members' own tile: a member skips itself
+        for (int t = 0; t < nt; t++) {
+          double va, vb;
+          pair(t, va, vb);
+          if (t != ta) ea += va;
+          if (t != tb) eb += vb;
+        }
+      }
     }
-    if (have) epi[b + ii] = ei;
+    if (ha) epi[b + i0 + ta] = mp2 * ea;
+    if (hb) epi[b + i0 + tb] = mp2 * eb;
   }
 }
 
@@ -306,7 +384,7 @@ __global__ void __launch_bounds__(PR_TPB) k_props_finish(PropsConst K, long long
   __shared__ double red[PR_TPB / 32 + 1];
   __shared__ unsigned long long s_arg;
   __shared__ unsigned hist1[NB1 + 1], hist2[NB2 + 1];
-  __shared__ double s_r178;
+  __shared__ double s_r178, dint[NB1], s_vc[NB1], s_mass[NB1];
   for (long long h = blockIdx.x; h < nh; h += gridDim.x) {
     HaloWork &w = W[h];
     const long long b = off[h], np = w.np, m = w.m;
@@ -352,32 +430,44 @@ __global__ void __launch_bounds__(PR_TPB) k_props_finish(PropsConst K, long long
       if (j >= 0) atomicAdd(&hist1[j], 1u);  // bin 0: inside the first edge
     }
     __syncthreads();
+    // a thread per bin; their maximum and the R178 walk by thread 0, the
+    // scalar outputs by thread PR_TPB / 2 meanwhile
+    if (threadIdx.x < NB1) {
+      const int j = (int)threadIdx.x + 1;
+      double d = (double)hist1[j] * K.mass_part * K.unit_d * p3(K.unit_l) / MSUN * h100;
+      d = d / (K.f43 * K.pi * (p3(exp(K.lmin_r + j * DELTA_LR)) - p3(exp(K.lmin_r + (j - 1) * DELTA_LR))));
+      d = d * MSUN / h100 / p3(MPC / 1e3);
+      d = d / Rho_m;
+      long long cum = 0;
+      for (int q = 0; q <= j; q++) cum += hist1[q];
+      double di = (double)cum * K.mass_part * K.unit_d * p3(K.unit_l);
+      const double R_tmp = exp(K.lmin_r + j * DELTA_LR) * (MPC / 1e3);
+      const double vc = sqrt(K.g * di / R_tmp);
+      s_mass[j - 1] = di;
+      s_vc[j - 1] = vc;
+      di = di / (K.f43 * K.pi * p3(R_tmp));
+      di = di / Rho_m;
+      dint[j - 1] = di;
+      o.vcirc[NB1 * h + j - 1] = (float)(vc / 1e5);
+      o.dens[NB1 * h + j - 1] = (float)d;
+      o.dens_int[NB1 * h + j - 1] = (float)di;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
-      double dint[NB1];
       double V_circ_max = 0.0, M_circ_max = 0.0, R_circ_max = 0.0, Rho_circ_max = 0.0;
-      long long cum = hist1[0];
-      for (int j = 1; j <= NB1; j++) {
-        double d = (double)hist1[j] * K.mass_part * K.unit_d * p3(K.unit_l) / MSUN * h100;
-        d = d / (K.f43 * K.pi * (p3(exp(K.lmin_r + j * DELTA_LR)) - p3(exp(K.lmin_r + (j - 1) * DELTA_LR))));
-        d = d * MSUN / h100 / p3(MPC / 1e3);
-        d = d / Rho_m;
-        cum += hist1[j];
-        double di = (double)cum * K.mass_part * K.unit_d * p3(K.unit_l);
-        const double R_tmp = exp(K.lmin_r + j * DELTA_LR) * (MPC / 1e3);
-        const double vc = sqrt(K.g * di / R_tmp);
-        if (vc > V_circ_max) {
-          V_circ_max = vc;
-          M_circ_max = di / MSUN * h100;
-          R_circ_max = R_tmp / (MPC / 1e3) * h100;
-          Rho_circ_max = di / (K.f43 * K.pi * p3(R_tmp));
-          Rho_circ_max = Rho_circ_max / Rho_m;
+      int jmax = 0;
+      for (int j = 1; j <= NB1; j++)
+        if (s_vc[j - 1] > V_circ_max) {
+          V_circ_max = s_vc[j - 1];
+          jmax = j;
         }
-        di = di / (K.f43 * K.pi * p3(R_tmp));
-        di = di / Rho_m;
-        dint[j - 1] = di;
-        o.vcirc[NB1 * h + j - 1] = (float)(vc / 1e5);
-        o.dens[NB1 * h + j - 1] = (float)d;
-        o.dens_int[NB1 * h + j - 1] = (float)di;
+      if (jmax > 0) {
+        const double di = s_mass[jmax - 1];
+        const double R_tmp = exp(K.lmin_r + jmax * DELTA_LR) * (MPC / 1e3);
+        M_circ_max = di / MSUN * h100;
+        R_circ_max = R_tmp / (MPC / 1e3) * h100;
+        Rho_circ_max = di / (K.f43 * K.pi * p3(R_tmp));
+        Rho_circ_max = Rho_circ_max / Rho_m;
       }
       // R178 interpolation (:567-602), Fortran's 1-based j
       int j = 1;
@@ -401,35 +491,7 @@ __global__ void __launch_bounds__(PR_TPB) k_props_finish(PropsConst K, long long
       o.circ[4 * h + 3] = (float)Rho_circ_max;
       o.delta_vals[2 * h + 0] = (float)M178;
       o.delta_vals[2 * h + 1] = (float)(R178 * K.h0 / 100.0);
-    }
-    __syncthreads();
-    const double R178 = s_r178;
-    for (long long k = b + threadIdx.x; k < b + np; k += PR_TPB) {
-      const double dx = (double)hpos[3 * k] - cen[0], dy = (double)hpos[3 * k + 1] - cen[1],
-                   dz = (double)hpos[3 * k + 2] - cen[2];
-      double r = sqrt(dx * dx + dy * dy + dz * dz);
-      r = r * K.unit_l / (MPC / 1e3);
-      r = r / R178;
-      const int j = log_bin(log(r), K.lmin_r178, DELTA_LR178, NB2);
-      if (j >= 0) atomicAdd(&hist2[j], 1u);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      long long cum = hist2[0];
-      for (int j = 1; j <= NB2; j++) {
-        double d = (double)hist2[j] * K.mass_part * K.unit_d * p3(K.unit_l) / MSUN * h100;
-        d = d / p3(R178) /
-            (K.f43 * K.pi * (p3(exp(K.lmin_r178 + j * DELTA_LR178)) - p3(exp(K.lmin_r178 + (j - 1) * DELTA_LR178))));
-        d = d * MSUN / h100 / p3(MPC / 1e3);
-        d = d / Rho_m;
-        cum += hist2[j];
-        double di = (double)cum * K.mass_part * K.unit_d * p3(K.unit_l);
-        const double Rt = exp(K.lmin_r178 + j * DELTA_LR178) * R178 * (MPC / 1e3);
-        di = di / (K.f43 * K.pi * p3(Rt));
-        di = di / Rho_m;
-        o.dens178[NB2 * h + j - 1] = (float)d;
-        o.dens_int178[NB2 * h + j - 1] = (float)di;
-      }
+    } else if (threadIdx.x == PR_TPB / 2) {
       // scalar outputs (:280-300, 312-313, 327-331, 350-354, 400-438, 672-720)
       const double conv = K.h0 / 100.0 / K.aexp;
       o.npart[h] = np;
@@ -480,6 +542,34 @@ __global__ void __launch_bounds__(PR_TPB) k_props_finish(PropsConst K, long long
       o.cos_alpha[h] = (v[0][2] * ang[0] + v[1][2] * ang[1] + v[2][2] * ang[2]) /
                        sqrt((v[0][2] * v[0][2] + v[1][2] * v[1][2] + v[2][2] * v[2][2]) *
                             (ang[0] * ang[0] + ang[1] * ang[1] + ang[2] * ang[2]));
+    }
+    __syncthreads();
+    const double R178 = s_r178;
+    for (long long k = b + threadIdx.x; k < b + np; k += PR_TPB) {
+      const double dx = (double)hpos[3 * k] - cen[0], dy = (double)hpos[3 * k + 1] - cen[1],
+                   dz = (double)hpos[3 * k + 2] - cen[2];
+      double r = sqrt(dx * dx + dy * dy + dz * dz);
+      r = r * K.unit_l / (MPC / 1e3);
+      r = r / R178;
+      const int j = log_bin(log(r), K.lmin_r178, DELTA_LR178, NB2);
+      if (j >= 0) atomicAdd(&hist2[j], 1u);
+    }
+    __syncthreads();
+    if (threadIdx.x < NB2) {
+      const int j = (int)threadIdx.x + 1;
+      double d = (double)hist2[j] * K.mass_part * K.unit_d * p3(K.unit_l) / MSUN * h100;
+      d = d / p3(R178) /
+          (K.f43 * K.pi * (p3(exp(K.lmin_r178 + j * DELTA_LR178)) - p3(exp(K.lmin_r178 + (j - 1) * DELTA_LR178))));
+      d = d * MSUN / h100 / p3(MPC / 1e3);
+      d = d / Rho_m;
+      long long cum = 0;
+      for (int q = 0; q <= j; q++) cum += hist2[q];
+      double di = (double)cum * K.mass_part * K.unit_d * p3(K.unit_l);
+      const double Rt = exp(K.lmin_r178 + j * DELTA_LR178) * R178 * (MPC / 1e3);
+      di = di / (K.f43 * K.pi * p3(Rt));
+      di = di / Rho_m;
+      o.dens178[NB2 * h + j - 1] = (float)d;
+      o.dens_int178[NB2 * h + j - 1] = (float)di;
     }
     __syncthreads();
   }
@@ -630,7 +720,10 @@ int psod_halo_properties(psod_ctx *c, const psod_props_params *p, psod_props_sta
     if ((st = scratch(c, SLOT_PR_IHALO, (size_t)nitem + 1, &ihalo))) return st;
     k_props_item_halo<<<grid_of(nh), PR_TPB, 0, c->stream>>>(cnt, nh, ihalo);
     k_props_pref64<<<grid_of(nh + 1), PR_TPB, 0, c->stream>>>(cnt, nh, ipref);
-    k_props_potential<<<148 * 8, PR_TPB, 0, c->stream>>>(K, ipref, nitem, ihalo, off, W, hpos, epi);
+    // cnt has been read: its first entry is the item counter
+    PSOD_CUDA(c, cudaMemsetAsync(cnt, 0, sizeof(unsigned), c->stream));
+    k_props_potential<<<(unsigned)std::min<long long>(nitem, 148 * 12), PP_TPB, 0, c->stream>>>(
+        K, ipref, nitem_u, ihalo, off, W, hpos, cnt, epi);
     k_props_finish<<<148 * 4, PR_TPB, 0, c->stream>>>(K, nh, off, W, hpos, epi, o);
     PSOD_CUDA(c, cudaGetLastError());
     S.potential_items = nitem;
