@@ -343,8 +343,8 @@ enum : int {
   SLOT_PR_POS,          // props: member positions after the periodic shifts
   SLOT_PR_EPI,          // props: per-member potential sums
   SLOT_PR_WORK,         // props: per-halo sums
-  SLOT_PR_CNT,          // props: potential items per halo, then their scan
-  SLOT_PR_PREF,         // props: the scan as int64
+  SLOT_PR_CNT,          // props: potential items per (size class, halo), then their scan
+  SLOT_PR_PREF,         // props: each halo's first item
   SLOT_PR_IHALO,        // props: halo of each potential item
   SLOT_PO_NPART,        // props outputs (kept until the next call)
   SLOT_PO_VIR,

@@ -283,7 +283,7 @@ __device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigne
 // staged members are read by broadcast.  Bound: FP64 pipe (7 operations a
 // pair) and instruction issue (about 17 a pair), against ~37 FP64
 // operations a pair with the square root and the division.  192^3 box, 3
-// million members, 1.5e10 ordered pairs: POTENTIAL_MS.
+// million members in halos of 100-50000: 31.5 -> 9.8 ms.
 constexpr int PP_TPB = PR_TPB / 2;
 
 __global__ void __launch_bounds__(PP_TPB) k_props_potential(PropsConst K, const long long *ipref, unsigned nitem,
@@ -575,21 +575,28 @@ __global__ void __launch_bounds__(PR_TPB) k_props_finish(PropsConst K, long long
   }
 }
 
-// potential work items: ceil(m / PR_TPB) per halo
+// Potential work items: ceil(m / PR_TPB) per halo, the longest ones first
+// (an item walks all m members, so a long one begun late would run alone):
+// the halos are listed by size class, PR_CLASSES passes over one count array.
+constexpr int PR_CLASSES = 3;
+__device__ __forceinline__ int size_class(long long m) { return m >= 8192 ? 0 : (m >= 2048 ? 1 : 2); }
+
 __global__ void k_props_items(const HaloWork *W, long long nh, unsigned *cnt) {
   const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (h < nh) cnt[h] = (unsigned)((W[h].m + PR_TPB - 1) / PR_TPB);
+  if (h >= nh) return;
+  const long long m = W[h].m;
+  for (int k = 0; k < PR_CLASSES; k++)
+    cnt[k * nh + h] = k == size_class(m) ? (unsigned)((m + PR_TPB - 1) / PR_TPB) : 0u;
 }
 
-__global__ void k_props_item_halo(const unsigned *pref, long long nh, unsigned *ihalo) {
+// the halo of each item and each halo's first item
+__global__ void k_props_item_halo(const HaloWork *W, const unsigned *pref, long long nh, unsigned *ihalo,
+                                  long long *first) {
   const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (h >= nh) return;
-  for (unsigned q = pref[h]; q < pref[h + 1]; q++) ihalo[q] = (unsigned)h;
-}
-
-__global__ void k_props_pref64(const unsigned *pref, long long nh, long long *out) {
-  const long long h = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (h <= nh) out[h] = pref[h];
+  const unsigned *p = pref + size_class(W[h].m) * nh + h;
+  first[h] = p[0];
+  for (unsigned q = p[0]; q < p[1]; q++) ihalo[q] = (unsigned)h;
 }
 
 unsigned grid_of(long long n, int tpb = PR_TPB) { return (unsigned)((n + tpb - 1) / tpb); }
@@ -666,7 +673,7 @@ int psod_halo_properties(psod_ctx *c, const psod_props_params *p, psod_props_sta
   if ((st = scratch(c, SLOT_PR_POS, (size_t)3 * nm + 3, &hpos))) return st;
   if ((st = scratch(c, SLOT_PR_EPI, (size_t)nm + 1, &epi))) return st;
   if ((st = scratch(c, SLOT_PR_WORK, (size_t)nh + 1, &W))) return st;
-  if ((st = scratch(c, SLOT_PR_CNT, (size_t)nh + 1, &cnt))) return st;
+  if ((st = scratch(c, SLOT_PR_CNT, (size_t)PR_CLASSES * nh + 1, &cnt))) return st;
   if ((st = scratch(c, SLOT_PR_PREF, (size_t)nh + 1, &ipref))) return st;
   // outputs
   PropsOut o;
@@ -712,14 +719,13 @@ int psod_halo_properties(psod_ctx *c, const psod_props_params *p, psod_props_sta
   if (nh > 0) {
     k_props_moments<<<148 * 4, PR_TPB, 0, c->stream>>>(K, nh, off, mem, c->d_cube, c->d_inv, c->d_vel, hpos, W);
     k_props_items<<<grid_of(nh), PR_TPB, 0, c->stream>>>(W, nh, cnt);
-    if ((st = scan_u32(c, cnt, cnt, nh, true))) return st;
+    if ((st = scan_u32(c, cnt, cnt, PR_CLASSES * nh, true))) return st;
     unsigned nitem_u = 0;
-    PSOD_CUDA(c, cudaMemcpyAsync(&nitem_u, cnt + nh, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+    PSOD_CUDA(c, cudaMemcpyAsync(&nitem_u, cnt + PR_CLASSES * nh, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
     PSOD_CUDA(c, cudaStreamSynchronize(c->stream));
     const long long nitem = nitem_u;
     if ((st = scratch(c, SLOT_PR_IHALO, (size_t)nitem + 1, &ihalo))) return st;
-    k_props_item_halo<<<grid_of(nh), PR_TPB, 0, c->stream>>>(cnt, nh, ihalo);
-    k_props_pref64<<<grid_of(nh + 1), PR_TPB, 0, c->stream>>>(cnt, nh, ipref);
+    k_props_item_halo<<<grid_of(nh), PR_TPB, 0, c->stream>>>(W, cnt, nh, ihalo, ipref);
     // cnt has been read: its first entry is the item counter
     PSOD_CUDA(c, cudaMemsetAsync(cnt, 0, sizeof(unsigned), c->stream));
     k_props_potential<<<(unsigned)std::min<long long>(nitem, 148 * 12), PP_TPB, 0, c->stream>>>(
