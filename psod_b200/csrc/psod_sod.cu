@@ -22,6 +22,7 @@
 //   4. profile counts (main:2103-2115) and claims (main:2148-2166).
 #include <algorithm>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstdlib>
 
@@ -31,9 +32,13 @@ namespace psod {
 
 namespace {
 
-constexpr int TPB = 256;          // threads per seed CTA
+constexpr int TPB = 256;          // threads per seed CTA of the host rounds' kernels
+constexpr int LOOP_TPB = 512;     // threads per seed CTA of the device round loop
 constexpr unsigned RN_CHUNK = 2048;  // neighbour records per refinement work item
-constexpr int NWARP = TPB / 32;
+constexpr int MAX_WARP = LOOP_TPB / 32;
+// the seed steps run in CTAs of either size
+__device__ __forceinline__ int tpb() { return (int)blockDim.x; }
+__device__ __forceinline__ int nwarp() { return (int)(blockDim.x >> 5); }
 constexpr unsigned SEL_SPLIT_MAX = 4;  // select: contenders summed by the whole CTA
 constexpr int NB = 4096;          // histogram buckets per level
 constexpr int MAXLEV = 4;         // histogram levels kept in shared memory
@@ -185,11 +190,11 @@ struct Smem {
   Level lev[MAXLEV];
   double edges[PSOD_MAX_BINS];
   unsigned phist[PSOD_MAX_BINS + 1];
-  unsigned long long red_u64[NWARP];
-  unsigned long long red_u64b[NWARP];
-  unsigned red_u32[NWARP];
-  int red_i[NWARP];
-  long long red_i64[NWARP];
+  unsigned long long red_u64[MAX_WARP];
+  unsigned long long red_u64b[MAX_WARP];
+  unsigned red_u32[MAX_WARP];
+  int red_i[MAX_WARP];
+  long long red_i64[MAX_WARP];
   // per-seed scalars
   unsigned na;
   unsigned cube_records;
@@ -240,7 +245,7 @@ __device__ __forceinline__ void for_cube(const SodConst &K, const SodBufs &B, in
   const int side = 2 * R + 1;
   const int nrow = side * side;
   const unsigned nx = (unsigned)K.nx;
-  for (int row = w; row < nrow; row += NWARP) {
+  for (int row = w; row < nrow; row += nwarp()) {
     const int dj = row % side - R, dk = row / side - R;
     const unsigned jj = (unsigned)wrapi(jc + dj, K.nx), kk = (unsigned)wrapi(kc + dk, K.nx);
     const unsigned long long base = (unsigned long long)nx * (jj + (unsigned long long)nx * kk);
@@ -276,6 +281,32 @@ __device__ __forceinline__ double cell_gap(double t0, int t, double nxd) {
   return fmax(d - 0.5, 0.0);
 }
 
+// the bounded window of cube rows (dj, dk) that can meet a ball of radius rm
+// around (ty, tz) (cell offsets relative to the seed cell centre)
+__device__ __forceinline__ void ball_rows(const SodConst &K, double ty, double tz, double rm, int &jlo, int &jhi,
+                                          int &klo, int &khi) {
+  const int R = K.ncut;
+  jlo = max(-R, (int)floor(ty - rm - 0.5));
+  jhi = min(R, (int)ceil(ty + rm + 0.5));
+  klo = max(-R, (int)floor(tz - rm - 0.5));
+  khi = min(R, (int)ceil(tz + rm + 0.5));
+}
+
+// The rows a region walk visits: the ball's window, or every row of the cube
+// where the cube nearly spans the box and a row can be near across the
+// periodic boundary.  At ncut = 11 a first ball of 1.5 cells meets about 25
+// of the cube's 529 rows, each a few FP64 operations to test.
+struct RowWin {
+  int jlo, klo, ny, nrow;
+  __device__ __forceinline__ RowWin(const SodConst &K, double ty, double tz, double rm) {
+    int jhi = K.ncut, khi = K.ncut;
+    jlo = klo = -K.ncut;
+    if (K.nx >= 2 * K.ncut + 4) ball_rows(K, ty, tz, rm, jlo, jhi, klo, khi);
+    ny = jhi - jlo + 1;
+    nrow = ny * (khi - klo + 1);
+  }
+};
+
 template <typename F>
 __device__ __forceinline__ void for_region(const SodConst &K, const SodBufs &B, const Region &G, F f) {
   if (G.rb2 < 0.0) {
@@ -283,7 +314,7 @@ __device__ __forceinline__ void for_region(const SodConst &K, const SodBufs &B, 
     return;
   }
   const int w = threadIdx.x >> 5;
-  const int R = K.ncut, side = 2 * R + 1, nrow = side * side;
+  const int R = K.ncut;
   const unsigned nx = (unsigned)K.nx;
   const double nxd = (double)K.nx;
   // ball centre relative to the seed cell centre (cell i spans [i+xs, i+xs+1))
@@ -295,8 +326,9 @@ __device__ __forceinline__ void for_region(const SodConst &K, const SodBufs &B, 
   const double tx = rel(G.xc, G.ic, 0), ty = rel(G.yc, G.jc, 1), tz = rel(G.zc, G.kc, 2);
   const double rm = G.rb + 1e-3;  // margin for rounding at cell edges
   const double rm2 = rm * rm;
-  for (int row = w; row < nrow; row += NWARP) {
-    const int dj = row % side - R, dk = row / side - R;
+  const RowWin W(K, ty, tz, rm);
+  for (int row = w; row < W.nrow; row += nwarp()) {
+    const int dj = W.jlo + row % W.ny, dk = W.klo + row / W.ny;
     const double gy = cell_gap(ty, dj, nxd), gz = cell_gap(tz, dk, nxd);
     const double rem = rm2 - gy * gy - gz * gz;
     if (rem < 0.0) continue;
@@ -326,7 +358,7 @@ __device__ __forceinline__ void for_region(const SodConst &K, const SodBufs &B, 
 // offsets alone (no record loads).  For the ball out to the stopping
 // particle this is the algorithmic read volume of the crossing search.
 __device__ __forceinline__ unsigned region_records(const SodConst &K, const SodBufs &B, const Region &G) {
-  const int R = K.ncut, side = 2 * R + 1, nrow = side * side;
+  const int R = K.ncut;
   const unsigned nx = (unsigned)K.nx;
   const double nxd = (double)K.nx;
   auto rel = [&](double x, int i, int a) {
@@ -336,9 +368,10 @@ __device__ __forceinline__ unsigned region_records(const SodConst &K, const SodB
   };
   const double tx = rel(G.xc, G.ic, 0), ty = rel(G.yc, G.jc, 1), tz = rel(G.zc, G.kc, 2);
   const double rm2 = G.rb * G.rb;
+  const RowWin W(K, ty, tz, G.rb);
   unsigned sum = 0;
-  for (int row = threadIdx.x; row < nrow; row += TPB) {
-    const int dj = row % side - R, dk = row / side - R;
+  for (int row = threadIdx.x; row < W.nrow; row += tpb()) {
+    const int dj = W.jlo + row % W.ny, dk = W.klo + row / W.ny;
     const double gy = cell_gap(ty, dj, nxd), gz = cell_gap(tz, dk, nxd);
     // each operation rounded on its own (no contraction): the count is
     // restated exactly by the oracle
@@ -372,8 +405,7 @@ __device__ __forceinline__ unsigned block_sum_u32(Smem &S, unsigned v) {
   if ((threadIdx.x & 31) == 0) S.red_u32[threadIdx.x >> 5] = v;
   __syncthreads();
   unsigned s = 0;
-#pragma unroll
-  for (int q = 0; q < NWARP; q++) s += S.red_u32[q];
+  for (int q = 0; q < nwarp(); q++) s += S.red_u32[q];
   return s;
 }
 
@@ -383,8 +415,7 @@ __device__ __forceinline__ int block_min_i(Smem &S, int v) {
   if ((threadIdx.x & 31) == 0) S.red_i[threadIdx.x >> 5] = v;
   __syncthreads();
   int s = S.red_i[0];
-#pragma unroll
-  for (int q = 1; q < NWARP; q++) s = min(s, S.red_i[q]);
+  for (int q = 1; q < nwarp(); q++) s = min(s, S.red_i[q]);
   return s;
 }
 
@@ -394,8 +425,7 @@ __device__ __forceinline__ int block_max_i(Smem &S, int v) {
   if ((threadIdx.x & 31) == 0) S.red_i[threadIdx.x >> 5] = v;
   __syncthreads();
   int s = S.red_i[0];
-#pragma unroll
-  for (int q = 1; q < NWARP; q++) s = max(s, S.red_i[q]);
+  for (int q = 1; q < nwarp(); q++) s = max(s, S.red_i[q]);
   return s;
 }
 
@@ -414,23 +444,17 @@ __device__ __forceinline__ void block_max_pair(Smem &S, unsigned long long &a, u
   __syncthreads();
   a = S.red_u64[0];
   b = S.red_u64b[0];
-#pragma unroll
-  for (int q = 1; q < NWARP; q++) {
+  for (int q = 1; q < nwarp(); q++) {
     unsigned long long ta = S.red_u64[q], tb = S.red_u64b[q];
     if (ta > a || (ta == a && tb > b)) { a = ta; b = tb; }
   }
 }
 
-// block exclusive scan over S.hist[l] into S.pref (NB = 16 per thread)
+// block exclusive scan over S.hist[l] into S.pref (NB / tpb() per thread)
 __device__ __forceinline__ void hist_prefix(Smem &S, int l) {
-  const int t = threadIdx.x;
-  unsigned v[NB / TPB];
+  const int t = threadIdx.x, per = NB / tpb();
   unsigned s = 0;
-#pragma unroll
-  for (int k = 0; k < NB / TPB; k++) {
-    v[k] = S.hist[l][t * (NB / TPB) + k];
-    s += v[k];
-  }
+  for (int k = 0; k < per; k++) s += S.hist[l][t * per + k];
   // warp inclusive scan
   const int lane = t & 31, w = t >> 5;
   unsigned inc = s;
@@ -445,10 +469,9 @@ __device__ __forceinline__ void hist_prefix(Smem &S, int l) {
   unsigned woff = 0;
   for (int q = 0; q < w; q++) woff += S.red_u32[q];
   unsigned off = woff + inc - s;
-#pragma unroll
-  for (int k = 0; k < NB / TPB; k++) {
-    S.pref[t * (NB / TPB) + k] = off;
-    off += v[k];
+  for (int k = 0; k < per; k++) {
+    S.pref[t * per + k] = off;
+    off += S.hist[l][t * per + k];
   }
   __syncthreads();
 }
@@ -511,7 +534,7 @@ struct BufSrc {
   unsigned long long lo, hi;  // entries [lo, hi) of the crossing buffer
   template <typename F>
   __device__ __forceinline__ void each(const SodConst &K, const SodBufs &B, F &&f) const {
-    for (unsigned long long e = lo + threadIdx.x; e < hi; e += TPB) f(B.xkey[e], B.xidx[e], B.xpos[e]);
+    for (unsigned long long e = lo + threadIdx.x; e < hi; e += tpb()) f(B.xkey[e], B.xidx[e], B.xpos[e]);
   }
 };
 
@@ -519,7 +542,7 @@ struct BufSrc {
 // bits lie in the level's range (level 0: all)
 template <class Src>
 __device__ __forceinline__ void build_hist(const SodConst &K, const SodBufs &B, Smem &S, int l, const Src &src) {
-  for (int k = threadIdx.x; k < NB; k += TPB) S.hist[l][k] = 0;
+  for (int k = threadIdx.x; k < NB; k += tpb()) S.hist[l][k] = 0;
   __syncthreads();
   const Level L = S.lev[l];
   src.each(K, B, [&](unsigned long long x, unsigned, unsigned) {
@@ -537,7 +560,7 @@ __device__ __forceinline__ unsigned ball_hist0(const SodConst &K, const SodBufs 
     S.lev[0].hi = 0x7fefffffffffffffull;
     S.lev[0].shift = L1_SHIFT;
   }
-  for (int k = threadIdx.x; k < NB; k += TPB) S.hist[0][k] = 0;
+  for (int k = threadIdx.x; k < NB; k += tpb()) S.hist[0][k] = 0;
   __syncthreads();
   unsigned inball = 0;
   RegionSrc{G}.each(K, B, [&](unsigned long long x, unsigned, unsigned) {
@@ -569,7 +592,7 @@ __device__ __forceinline__ unsigned extract_sorted(const SodConst &K, const SodB
   const unsigned n = min(S.nsorted, (unsigned)CAP);
   unsigned m = 1;
   while (m < n) m <<= 1;
-  for (unsigned k = n + threadIdx.x; k < m; k += TPB) {
+  for (unsigned k = n + threadIdx.x; k < m; k += tpb()) {
     S.skey[k] = ~0ull;
     S.sidx[k] = 0xffffffffu;
   }
@@ -577,7 +600,7 @@ __device__ __forceinline__ unsigned extract_sorted(const SodConst &K, const SodB
   // bitonic sort of m (power of two) pairs
   for (unsigned size = 2; size <= m; size <<= 1) {
     for (unsigned stride = size >> 1; stride > 0; stride >>= 1) {
-      for (unsigned k = threadIdx.x; k < m / 2; k += TPB) {
+      for (unsigned k = threadIdx.x; k < m / 2; k += tpb()) {
         unsigned a = 2 * k - (k & (stride - 1));
         unsigned bb = a + stride;
         bool up = ((a & size) == 0);
@@ -603,6 +626,39 @@ __device__ __forceinline__ unsigned extract_sorted(const SodConst &K, const SodB
 // uses.
 __device__ __forceinline__ unsigned *small_pos(Smem &S) { return S.hist[MAXLEV - 1]; }
 
+// bitonic sort of the n loaded entries (d2 bits, index, position)
+__device__ __forceinline__ void sort_ball(Smem &S, unsigned n) {
+  unsigned *spos = small_pos(S);
+  unsigned m = 1;
+  while (m < n) m <<= 1;
+  for (unsigned k = n + threadIdx.x; k < m; k += tpb()) {
+    S.skey[k] = ~0ull;
+    S.sidx[k] = 0xffffffffu;
+  }
+  __syncthreads();
+  for (unsigned size = 2; size <= m; size <<= 1) {
+    for (unsigned stride = size >> 1; stride > 0; stride >>= 1) {
+      for (unsigned k = threadIdx.x; k < m / 2; k += tpb()) {
+        const unsigned a = 2 * k - (k & (stride - 1)), bb = a + stride;
+        const bool up = ((a & size) == 0);
+        const unsigned long long ka = S.skey[a], kb = S.skey[bb];
+        const unsigned ia = S.sidx[a], ib = S.sidx[bb];
+        const bool gt = (ka > kb) || (ka == kb && ia > ib);
+        if (gt == up) {
+          S.skey[a] = kb;
+          S.skey[bb] = ka;
+          S.sidx[a] = ib;
+          S.sidx[bb] = ia;
+          const unsigned pa = spos[a];
+          spos[a] = spos[bb];
+          spos[bb] = pa;
+        }
+      }
+      bitonic_stage_sync(size, stride, m);
+    }
+  }
+}
+
 // every alive record of region G, sorted; returns the count, or CAP + 1 when
 // the region holds more than CAP (the list is then unusable)
 __device__ __forceinline__ unsigned load_ball_sorted(const SodConst &K, const SodBufs &B, Smem &S, const Region &G) {
@@ -624,34 +680,7 @@ __device__ __forceinline__ unsigned load_ball_sorted(const SodConst &K, const So
   if (threadIdx.x == 0) atomicAdd(B.cross_records, (unsigned long long)n);
   __syncthreads();
   if (n > CAP) return CAP + 1;
-  unsigned m = 1;
-  while (m < n) m <<= 1;
-  for (unsigned k = n + threadIdx.x; k < m; k += TPB) {
-    S.skey[k] = ~0ull;
-    S.sidx[k] = 0xffffffffu;
-  }
-  __syncthreads();
-  for (unsigned size = 2; size <= m; size <<= 1) {
-    for (unsigned stride = size >> 1; stride > 0; stride >>= 1) {
-      for (unsigned k = threadIdx.x; k < m / 2; k += TPB) {
-        const unsigned a = 2 * k - (k & (stride - 1)), bb = a + stride;
-        const bool up = ((a & size) == 0);
-        const unsigned long long ka = S.skey[a], kb = S.skey[bb];
-        const unsigned ia = S.sidx[a], ib = S.sidx[bb];
-        const bool gt = (ka > kb) || (ka == kb && ia > ib);
-        if (gt == up) {
-          S.skey[a] = kb;
-          S.skey[bb] = ka;
-          S.sidx[a] = ib;
-          S.sidx[bb] = ia;
-          const unsigned pa = spos[a];
-          spos[a] = spos[bb];
-          spos[bb] = pa;
-        }
-      }
-      bitonic_stage_sync(size, stride, m);
-    }
-  }
+  sort_ball(S, n);
   return n;
 }
 
@@ -659,7 +688,7 @@ __device__ __forceinline__ unsigned load_ball_sorted(const SodConst &K, const So
 // position i >= 10 where the reference's loop stops (main:2046); 0 if none
 __device__ __forceinline__ long long sorted_stop(const SodConst &K, Smem &S, unsigned n, long long na, double delta) {
   int best = 0x7fffffff;
-  for (unsigned k = 9 + threadIdx.x; k < n; k += TPB)
+  for (unsigned k = 9 + threadIdx.x; k < n; k += tpb())
     if (!keeps_going(K, (long long)k + 1, bitsd(S.skey[k]), na, delta)) best = min(best, (int)k);
   best = block_min_i(S, best);
   return best == 0x7fffffff ? 0 : (long long)best + 1;
@@ -690,8 +719,8 @@ __device__ __forceinline__ long long radial_search(const SodConst &K, const SodB
     const Level L = S.lev[l];
     // find the first (forward) / last (backward) bucket that may hold a hit
     int cand = (mode == 0) ? 0x7fffffff : -1;
-    for (int k = 0; k < NB / TPB; k++) {
-      int b = threadIdx.x * (NB / TPB) + k;
+    for (int k = 0; k < NB / tpb(); k++) {
+      int b = threadIdx.x * (NB / tpb()) + k;
       if (mode == 0 ? (b < L.next) : (b > L.next)) continue;
       unsigned nb = S.hist[l][b];
       if (nb == 0) continue;
@@ -747,7 +776,7 @@ __device__ __forceinline__ long long radial_search(const SodConst &K, const SodB
       long long hit;
       if (mode == 0) {
         int best = 0x7fffffff;
-        for (unsigned k = threadIdx.x; k < n; k += TPB) {
+        for (unsigned k = threadIdx.x; k < n; k += tpb()) {
           long long i = c0 + 1 + k;
           if (!keeps_going(K, i, bitsd(S.skey[k]), na, delta)) best = min(best, (int)k);
         }
@@ -755,7 +784,7 @@ __device__ __forceinline__ long long radial_search(const SodConst &K, const SodB
         hit = (best == 0x7fffffff) ? -1 : best;
       } else {
         int best = -1;
-        for (unsigned k = threadIdx.x; k < n; k += TPB) {
+        for (unsigned k = threadIdx.x; k < n; k += tpb()) {
           long long i = c0 + 1 + k;
           if (i >= 2 && i <= imax && overdens(K, i, bitsd(S.skey[k])) > delta) best = max(best, (int)k);
         }
@@ -840,7 +869,7 @@ __device__ __forceinline__ unsigned next_item(unsigned *ctr) {
 __device__ __forceinline__ unsigned cube_records(const SodConst &K, const SodBufs &B, Smem &S, int ic, int jc, int kc) {
   const int R = K.ncut, side = 2 * R + 1;
   unsigned sum = 0;
-  for (int row = threadIdx.x; row < side * side; row += TPB) {
+  for (int row = threadIdx.x; row < side * side; row += tpb()) {
     const int dj = row % side - R, dk = row / side - R;
     const unsigned jj = (unsigned)wrapi(jc + dj, K.nx), kk = (unsigned)wrapi(kc + dk, K.nx);
     const unsigned long long base = (unsigned long long)K.nx * (jj + (unsigned long long)K.nx * kk);
@@ -866,7 +895,7 @@ __device__ __forceinline__ unsigned alive_rows(const SodConst &K, const SodBufs 
   const int R = K.ncut, side = 2 * R + 1, nrow = side * side;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   unsigned total = 0;
-  for (int r0 = 0; r0 < nrow; r0 += NWARP) {
+  for (int r0 = 0; r0 < nrow; r0 += nwarp()) {
     const int row = r0 + w;
     unsigned part = 0;
     if (row < nrow) {
@@ -938,7 +967,7 @@ __device__ __forceinline__ void prep_seed(const SodConst &K, const SodBufs &B, S
   // grouped by cell in the reference's scan order (x outer, z inner)
   __shared__ unsigned s_cnt[27], s_coff[27], s_base;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int o = w; o < 27; o += NWARP) {
+  for (int o = w; o < 27; o += nwarp()) {
     const int di = o / 9 - 1, dj = (o / 3) % 3 - 1, dk = o % 3 - 1;
     const unsigned cell = (unsigned)wrapi(g.ic + di, K.nx) +
                           (unsigned)K.nx * ((unsigned)wrapi(g.jc + dj, K.nx) + (unsigned)K.nx * (unsigned)wrapi(g.kc + dk, K.nx));
@@ -1006,7 +1035,7 @@ __device__ __forceinline__ void prep_seed(const SodConst &K, const SodBufs &B, S
     B.cell_chunks[slot * 27 + o] = ((s_cnt[o] + 63u) / 64u) * nch;
     B.cell_groups[slot * 27 + o] = (s_cnt[o] + 63u) / 64u;
   }
-  for (int o = w; o < 27; o += NWARP) {
+  for (int o = w; o < 27; o += nwarp()) {
     const int di = o / 9 - 1, dj = (o / 3) % 3 - 1, dk = o % 3 - 1;
     const unsigned cell = (unsigned)wrapi(g.ic + di, K.nx) +
                           (unsigned)K.nx * ((unsigned)wrapi(g.jc + dj, K.nx) + (unsigned)K.nx * (unsigned)wrapi(g.kc + dk, K.nx));
@@ -1737,7 +1766,7 @@ __device__ __forceinline__ void select_seed(const SodConst &K, const SodBufs &B,
   // max of the finite approximate sums (non-negative doubles order as their
   // bits); an infinite entry marks a candidate that always goes exact
   unsigned long long mb = 0, dummy = 0;
-  for (unsigned k = threadIdx.x; k < n; k += TPB) {
+  for (unsigned k = threadIdx.x; k < n; k += tpb()) {
     const unsigned long long b = dbits(B.cand_s[off + k]);
     if (b < 0x7ff0000000000000ull) mb = b > mb ? b : mb;
   }
@@ -1752,7 +1781,7 @@ __device__ __forceinline__ void select_seed(const SodConst &K, const SodBufs &B,
   // so the split leaves it unchanged); with more, a warp sums a contender.
   if (threadIdx.x == 0) S.nsel = 0;
   __syncthreads();
-  for (unsigned k = threadIdx.x; k < n; k += TPB)
+  for (unsigned k = threadIdx.x; k < n; k += tpb())
     if (B.cand_s[off + k] >= thr) {
       const unsigned j = atomicAdd(&S.nsel, 1u);
       if (j < SEL_SPLIT_MAX) S.sel[j] = k;
@@ -1761,20 +1790,19 @@ __device__ __forceinline__ void select_seed(const SodConst &K, const SodBufs &B,
   const unsigned nsel = S.nsel;
   const bool split = nsel <= SEL_SPLIT_MAX;
   const unsigned nloop = split ? nsel : n;
-  for (unsigned k = split ? 0u : (unsigned)w; k < nloop; k += split ? 1u : (unsigned)NWARP) {
+  for (unsigned k = split ? 0u : (unsigned)w; k < nloop; k += split ? 1u : (unsigned)nwarp()) {
     const unsigned ck = split ? S.sel[k] : k;
     if (!split && !(B.cand_s[off + ck] >= thr)) continue;  // cannot reach the maximum
     const unsigned cp = B.cand_pos[off + ck];
     unsigned long long sq;
     double sf;
     if (split) {
-      refine_sum<true>(K, B, cp, g.ic, g.jc, g.kc, sq, sf, nullptr, (unsigned)w, NWARP);
+      refine_sum<true>(K, B, cp, g.ic, g.jc, g.kc, sq, sf, nullptr, (unsigned)w, nwarp());
       __syncthreads();
       if (lane == 0) S.red_u64[w] = sq;
       __syncthreads();
       sq = 0;
-#pragma unroll
-      for (int q = 0; q < NWARP; q++) sq += S.red_u64[q];
+      for (int q = 0; q < nwarp(); q++) sq += S.red_u64[q];
     } else {
       refine_sum<true>(K, B, cp, g.ic, g.jc, g.kc, sq, sf);
     }
@@ -1899,7 +1927,7 @@ __device__ __forceinline__ void seed_features(const SodConst &K, const SodBufs &
   const SeedGeo g = seed_geo(K, B, rank);
   unsigned s0 = 0, s1 = 0, s2 = 0, s3 = 0, s4 = 0;
   if (B.alive_cnt) {
-    for (int q = threadIdx.x; q < 729; q += TPB) {
+    for (int q = threadIdx.x; q < 729; q += tpb()) {
       const int dx = q % 9 - 4, dy = (q / 9) % 9 - 4, dz = q / 81 - 4;
       const int d = max(abs(dx), max(abs(dy), abs(dz)));
       const unsigned cell = (unsigned)wrapi(g.ic + dx, K.nx) +
@@ -2001,8 +2029,8 @@ __device__ __forceinline__ bool stop_may_lie_inside(const SodConst &K, Smem &S, 
   hist_prefix(S, 0);
   const Level L = S.lev[0];
   int any = 0;
-  for (int k = 0; k < NB / TPB; k++) {
-    const int b = threadIdx.x * (NB / TPB) + k;
+  for (int k = 0; k < NB / tpb(); k++) {
+    const int b = threadIdx.x * (NB / tpb()) + k;
     const unsigned nb = S.hist[0][b];
     if (nb == 0) continue;
     unsigned long long lo, hi;
@@ -2050,7 +2078,7 @@ __device__ __forceinline__ long long bucket_ball(const SodConst &K, const SodBuf
   // cursors: the level-0 bucket starts
   hist_prefix(S, 0);
   unsigned *cur = S.hist[1];
-  for (int k = threadIdx.x; k < NB; k += TPB) cur[k] = S.pref[k];
+  for (int k = threadIdx.x; k < NB; k += tpb()) cur[k] = S.pref[k];
   __syncthreads();
   const unsigned long long base = S.xbase;
   RegionSrc{G}.each(K, B, [&](unsigned long long x, unsigned ix, unsigned p) {
@@ -2063,12 +2091,58 @@ __device__ __forceinline__ long long bucket_ball(const SodConst &K, const SodBuf
   return (long long)nball;
 }
 
-__device__ __forceinline__ void cross_seed(const SodConst &K, const SodBufs &B, Smem &S, unsigned slot, unsigned rank) {
-  if (!B.st_active[slot]) return;
-  const SeedGeo g = seed_geo(K, B, rank);
-  unsigned na = B.st_na[slot];
+// Alive records of the cells around a seed, gathered by the device round loop
+// (small_seed): coordinates in one frame, cube slots, in the histograms' place
+struct SmallList {
+  float x[NB], y[NB], z[NB];
+  unsigned pos[NB];
+};
+static_assert(sizeof(SmallList) == sizeof(unsigned) * MAXLEV * NB, "the list takes the histograms' place");
+
+// The list's entries within LIST_R of list entry q (the refined centre), sorted
+// as load_ball_sorted sorts a region's records; the list's cells hold every
+// record within one cell of a centre in the 27 inner cells.
+constexpr double LIST_R = 0.999;
+
+__device__ __forceinline__ unsigned load_ball_list(const SodConst &K, const SodBufs &B, Smem &S, unsigned nlist,
+                                                   unsigned q) {
+  const SmallList &L = *reinterpret_cast<const SmallList *>(S.hist);
+  if (threadIdx.x == 0) S.nsorted = 0;
+  __syncthreads();
+  const double xc = (double)L.x[q], yc = (double)L.y[q], zc = (double)L.z[q];
+  for (unsigned j = threadIdx.x; j < nlist; j += tpb()) {
+    if (L.x[j] > 1e17f) continue;  // padding
+    const double d2 = min_image_d2((double)L.x[j], (double)L.y[j], (double)L.z[j], xc, yc, zc, K.tx);
+    if (!(d2 <= LIST_R * LIST_R)) continue;
+    const unsigned s = atomicAdd(&S.nsorted, 1u);
+    if (s < CAP) {
+      const unsigned p = L.pos[j];
+      S.skey[s] = dbits(d2);
+      S.sidx[s] = __float_as_uint(B.cube[p].w) & PSOD_IDX_MASK;
+      S.pref[s] = p;
+    }
+  }
+  __syncthreads();
+  const unsigned n = S.nsorted;
+  if (threadIdx.x == 0) atomicAdd(B.cross_records, (unsigned long long)n);
+  if (n <= CAP) {  // the list is read: its slots may be overwritten
+    unsigned *spos = small_pos(S);
+    for (unsigned k = threadIdx.x; k < n; k += tpb()) spos[k] = S.pref[k];
+  }
+  __syncthreads();
+  if (n > CAP) return CAP + 1;
+  sort_ball(S, n);
+  return n;
+}
+
+// na: alive particles of the preselect cube where that count is known (plain
+// mode); cpos: the refined centre's cube position; nlist > 0: the device
+// loop's record list is in shared memory, the centre its entry lq, and the
+// first ball is taken from it (any first ball gives the same stop)
+__device__ __forceinline__ void cross_seed(const SodConst &K, const SodBufs &B, Smem &S, unsigned slot, unsigned rank,
+                                           const SeedGeo &g, unsigned na, unsigned cpos, unsigned nlist = 0,
+                                           unsigned lq = 0) {
   bool na_known = (B.mode == PSOD_MODE_PLAIN);
-  const unsigned cpos = B.st_centre[slot];
   const float4 cvv = B.cube[cpos];
   Region G;
   G.ic = g.ic;
@@ -2100,7 +2174,22 @@ __device__ __forceinline__ void cross_seed(const SodConst &K, const SodBufs &B, 
   double d2stop = 0;
   long long istop = 0;
   unsigned nball = 0;
-  {
+  if (nlist > 0) {
+    const unsigned n = load_ball_list(K, B, S, nlist, lq);
+    if (threadIdx.x == 0) atomicAdd(B.cross_balls, 1ull);
+    if (n <= CAP) {
+      const long long i = sorted_stop(K, S, n, 0x7fffffffffffffffll, K.delta);
+      if (i != 0) {
+        G.rb = LIST_R;
+        G.rb2 = LIST_R * LIST_R;
+        istop = i;
+        d2stop = bitsd(S.skey[i - 1]);
+        form = SMALL;
+        nball = n;
+      }
+    }
+  }
+  if (form != SMALL) {
     double rb = rb0;
     while (true) {
       const bool full = !(rb > 0.0) || rb >= (double)K.ncut;
@@ -2187,7 +2276,7 @@ __device__ __forceinline__ void cross_seed(const SodConst &K, const SodBufs &B, 
   long long masse2 = 0;
   if (form == SMALL) {
     int best = -1;
-    for (unsigned k = 1 + threadIdx.x; k < (unsigned)istop; k += TPB)
+    for (unsigned k = 1 + threadIdx.x; k < (unsigned)istop; k += tpb())
       if (overdens(K, (long long)k + 1, bitsd(S.skey[k])) > K.delta2) best = max(best, (int)k);
     best = block_max_i(S, best);
     if (best >= 0) masse2 = best + 1;
@@ -2253,8 +2342,8 @@ __device__ __forceinline__ void cross_seed(const SodConst &K, const SodBufs &B, 
   // 4a. profile (main:2103-2115): cumulative counts below each edge; the
   // region must hold every particle closer than the last edge
   if (keep) {
-    for (int j = threadIdx.x; j < K.nbins; j += TPB) S.edges[j] = dmul(rayon, B.edge_fac[j]);
-    for (int j = threadIdx.x; j <= K.nbins; j += TPB) S.phist[j] = 0;
+    for (int j = threadIdx.x; j < K.nbins; j += tpb()) S.edges[j] = dmul(rayon, B.edge_fac[j]);
+    for (int j = threadIdx.x; j <= K.nbins; j += tpb()) S.phist[j] = 0;
     __syncthreads();
     const double emax = S.edges[K.nbins - 1];
     const bool ball_holds = G.rb2 < 0.0 || emax * (1.0 + 1e-9) < G.rb;
@@ -2272,7 +2361,7 @@ __device__ __forceinline__ void cross_seed(const SodConst &K, const SodBufs &B, 
     if (small && ball_holds) {
       // every particle closer than the last edge is in the sorted list:
       // cumulative counts by binary search, one bin per thread
-      for (int j = threadIdx.x; j < K.nbins; j += TPB) {
+      for (int j = threadIdx.x; j < K.nbins; j += tpb()) {
         unsigned lo = 0, hi = nball;  // first k with r_k >= edge
         while (lo < hi) {
           const unsigned mid = (lo + hi) >> 1;
@@ -2282,7 +2371,7 @@ __device__ __forceinline__ void cross_seed(const SodConst &K, const SodBufs &B, 
         S.pref[j] = lo;
       }
       __syncthreads();
-      for (int j = threadIdx.x; j < K.nbins; j += TPB) S.phist[j] = S.pref[j] - (j > 0 ? S.pref[j - 1] : 0u);
+      for (int j = threadIdx.x; j < K.nbins; j += tpb()) S.phist[j] = S.pref[j] - (j > 0 ? S.pref[j - 1] : 0u);
       __syncthreads();
     } else if (form == BUF && ball_holds) {
       ball_buf.each(K, B, [&](unsigned long long x, unsigned, unsigned) { bin_entry(x); });
@@ -2329,7 +2418,7 @@ __device__ __forceinline__ void cross_seed(const SodConst &K, const SodBufs &B, 
   if (small) {
     // the first masse entries of the sorted list
     const unsigned *spos = small_pos(S);
-    for (unsigned k = threadIdx.x; k < (unsigned)masse; k += TPB) {
+    for (unsigned k = threadIdx.x; k < (unsigned)masse; k += tpb()) {
       const unsigned p = spos[k];
       const float4 v = B.cube[p];
       B.cube[p].w = __uint_as_float(__float_as_uint(v.w) | PSOD_DEAD_BIT);
@@ -2405,17 +2494,6 @@ __device__ __forceinline__ int warp_max_i(int v) {
 __device__ __forceinline__ unsigned warp_sum_u(unsigned v) {
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
-}
-
-// the bounded window of cube rows (dj, dk) that can meet a ball of radius rm
-// around (ty, tz) (cell offsets relative to the seed cell centre)
-__device__ __forceinline__ void ball_rows(const SodConst &K, double ty, double tz, double rm, int &jlo, int &jhi,
-                                          int &klo, int &khi) {
-  const int R = K.ncut;
-  jlo = max(-R, (int)floor(ty - rm - 0.5));
-  jhi = min(R, (int)ceil(ty + rm + 0.5));
-  klo = max(-R, (int)floor(tz - rm - 0.5));
-  khi = min(R, (int)ceil(tz + rm + 0.5));
 }
 
 // x-ranges of cube row (dj, dk) meeting the ball (the row rule of
@@ -2739,7 +2817,9 @@ __global__ void __launch_bounds__(TPB) k_cross(SodConst K, SodBufs B) {
     const unsigned item = next_item(&B.work[3]);
     if (item >= min(*B.nready, B.cap_ready)) break;
     if (B.st_big && !B.st_big[item]) continue;  // done by the warp pass
-    cross_seed(K, B, S, item, B.ready[item]);
+    if (!B.st_active[item]) continue;
+    const unsigned rank = B.ready[item];
+    cross_seed(K, B, S, item, rank, seed_geo(K, B, rank), B.st_na[item], B.st_centre[item]);
   }
 }
 
@@ -3078,107 +3158,424 @@ __global__ void k_ready_direct(const unsigned *active, const unsigned *nactive, 
 // not depend on it).  Every barrier wait is bounded: a wait that runs out
 // records PSOD_ERR_TIMEOUT and every CTA leaves at its next barrier.
 // ---------------------------------------------------------------------------
-// Approximate refinement sums of the candidates of one candidate cell (o of
-// the 27 around the seed) by one warp (the device tail loop): 32 candidates
-// a pass, the alive records of the cell's 3x3x3 neighbourhood staged 32 at
-// a time in the warp's tile and summed by tile_terms, i.e. the same FP32
-// terms and partial sums as k_refine_warp and the same error bound.
-__device__ __forceinline__ void tail_refine_cell(const SodConst &K, const SodBufs &B, unsigned slot, int o,
-                                                 const SeedGeo &g, RecTile &T) {
-  const int lane = threadIdx.x & 31;
-  const unsigned lt = (1u << lane) - 1u;
-  auto clear = [&](int c, int a) {  // the 3-cell coordinate window stays clear of the box edge
-    double s0 = (double)(c - 1) + K.xs[a];
-    s0 -= K.tx * floor(s0 / K.tx);
-    return s0 >= 1.0 && s0 + 3.0 <= K.tx - 1.0;
+// One seed from the preselect to the claims in one CTA (the device round
+// loop).  The alive records filed under the 125 cells within +-2 of the seed
+// cell (the reference's x_sel2) are gathered once into shared memory, cell
+// after cell, so that the three cells of a neighbour row are one contiguous
+// range; the candidates are the records of the 27 inner cells.  Refinement
+// sums, exact sums and the argmax then read shared memory only, with block
+// barriers where separate steps over the whole grid needed grid barriers.
+//
+// Bound: latency of one CTA (late rounds hold a few seeds, each waiting for
+// the one before it).  Measured per round at 512^3 (1-50 seeds a round):
+// separate steps 200 us (preselect 20, refinement a warp per candidate cell
+// 120, select 12, crossing 30, seven grid barriers); one CTA ROUND_US.
+constexpr int SL_CELLS = 125;
+
+// the inner cell (listed offset o of the 27, x outer and z inner as the
+// reference scans) as an index of the 125
+__device__ __forceinline__ int sl_inner(int o) {
+  return (o / 9 + 1) + 5 * ((o / 3) % 3 + 1) + 25 * (o % 3 + 1);
+}
+
+// Sum of one candidate pair's terms (one candidate: TWO false) over list
+// entries [j0, j1), j0 and j1 multiples of 4: as tile_terms2, FP32 partials of
+// at most 16 terms each, a span with a pair near the inclusion edge redone
+// with the FP64 test.  WRAP: minimum-image differences (boxes too small for
+// the shifted coordinates of the list).
+template <bool WRAP, bool TWO>
+__device__ __forceinline__ void list_terms(const SmallList &L, unsigned j0, unsigned j1, float ax, float ay, float az,
+                                           float bx, float by, float bz, const SodConst &K, double &sa, double &sb) {
+  const float e2f = (float)K.eps2, limf = (float)(1.0 + K.eps2);
+  const unsigned long long e2 = f2_pack(e2f, e2f), nlim = f2_pack(-limf, -limf);
+  const unsigned long long nax = f2_pack(-ax, -ax), nay = f2_pack(-ay, -ay), naz = f2_pack(-az, -az);
+  const unsigned long long nbx = f2_pack(-bx, -bx), nby = f2_pack(-by, -by), nbz = f2_pack(-bz, -bz);
+  auto exact_span = [&](unsigned s0, unsigned s1, float cx, float cy, float cz) {
+    double sum = 0.0;
+    for (unsigned j = s0; j < s1; j++) {
+      const float rx = L.x[j], ry = L.y[j], rz = L.z[j];
+      if (rx > 1e17f) continue;  // padding
+      const float dx = WRAP ? mi_dx(rx, cx, K.nxf) : __fsub_rn(rx, cx), dy = WRAP ? mi_dx(ry, cy, K.nxf) : __fsub_rn(ry, cy),
+                  dz = WRAP ? mi_dx(rz, cz, K.nxf) : __fsub_rn(rz, cz);
+      const float d2e = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmaf_rn(dz, dz, e2f)));
+      if (min_image_d2((double)rx, (double)ry, (double)rz, (double)cx, (double)cy, (double)cz, K.tx) <= K.rmin2)
+        sum += (double)rsqrt_pos(d2e);
+    }
+    return sum;
   };
-  {
-    const unsigned ci = slot * 27u + (unsigned)o;
-    const unsigned cnt = B.cell_cnt[ci];
-    if (cnt == 0) return;
-    const unsigned coff = B.cell_off[ci];
-    const int cxc = wrapi(g.ic + o / 9 - 1, K.nx), cyc = wrapi(g.jc + (o / 3) % 3 - 1, K.nx),
-              czc = wrapi(g.kc + o % 3 - 1, K.nx);
-    const bool wf = clear(cxc, 0) && clear(cyc, 1) && clear(czc, 2);
-    const NbrList L = nbr_list(K, B, cxc, cyc, czc, g.ic, g.jc, g.kc);
-    for (unsigned c0 = 0; c0 < cnt; c0 += 32) {
-      const unsigned k = c0 + (unsigned)lane;
-      const bool have = k < cnt;
-      const unsigned cp = have ? B.cand_pos[coff + k] : 0u;
-      const bool active = have && !(K.has_quirk && cp == K.quirk_pos);  // that one goes exact
-      float cx = 1e18f, cy = 1e18f, cz = 1e18f;
-      if (active) {
-        const float4 cv = B.cube[cp];
-        cx = to_grid(cv.x, K.nxf);
-        cy = to_grid(cv.y, K.nxf);
-        cz = to_grid(cv.z, K.nxf);
-      }
-      double sum = 0.0;
-      unsigned fill = 0;
-      for (unsigned t0 = 0; t0 < L.total; t0 += 32) {
-        const unsigned t = t0 + (unsigned)lane;
-        const unsigned q = L.at(t < L.total ? t : L.total - 1);
-        bool keep = false;
-        float rx = 0.f, ry = 0.f, rz = 0.f;
-        if (t < L.total) {
-          const float4 v = B.cube[q];
-          keep = !(__float_as_uint(v.w) & PSOD_DEAD_BIT);
-          rx = to_grid(v.x, K.nxf);
-          ry = to_grid(v.y, K.nxf);
-          rz = to_grid(v.z, K.nxf);
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, keep);
-        if (keep) {  // fill < 32: index < 64
-          const unsigned at = fill + __popc(m & lt);
-          T.x[at] = rx;
-          T.y[at] = ry;
-          T.z[at] = rz;
-        }
-        fill += (unsigned)__popc(m);
-        __syncwarp();
-        if (fill >= 32u) {
-          if (active) sum += wf ? tile_terms<true>(T, 32u, cx, cy, cz, K) : tile_terms<false>(T, 32u, cx, cy, cz, K);
-          __syncwarp();
-          if ((unsigned)lane < fill - 32u) {
-            T.x[lane] = T.x[32 + lane];
-            T.y[lane] = T.y[32 + lane];
-            T.z[lane] = T.z[32 + lane];
-          }
-          __syncwarp();
-          fill -= 32u;
+  for (unsigned s0 = j0; s0 < j1; s0 += 32u) {
+    const unsigned s1 = min(s0 + 32u, j1);
+    float ea = 1.f, eb = 1.f, a0 = 0.f, a1 = 0.f, b0 = 0.f, b1 = 0.f;
+    if (!WRAP) {
+      unsigned long long acca = f2_pack(0.f, 0.f), accb = f2_pack(0.f, 0.f);
+#pragma unroll 2
+      for (unsigned j = s0; j < s1; j += 4u) {
+        const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(&L.x[j]), Y = *reinterpret_cast<const ulonglong2 *>(&L.y[j]),
+                         Z = *reinterpret_cast<const ulonglong2 *>(&L.z[j]);
+        pair_packed(X.x, Y.x, Z.x, nax, nay, naz, e2, nlim, acca, ea);
+        pair_packed(X.y, Y.y, Z.y, nax, nay, naz, e2, nlim, acca, ea);
+        if (TWO) {
+          pair_packed(X.x, Y.x, Z.x, nbx, nby, nbz, e2, nlim, accb, eb);
+          pair_packed(X.y, Y.y, Z.y, nbx, nby, nbz, e2, nlim, accb, eb);
         }
       }
-      if (fill > 0) {
-        // pad to a multiple of 8 with records far from every candidate
-        if ((unsigned)lane < ((8u - (fill & 7u)) & 7u)) {
-          T.x[fill + lane] = 1e18f;
-          T.y[fill + lane] = 1e18f;
-          T.z[fill + lane] = 1e18f;
-        }
-        __syncwarp();
-        if (active) sum += wf ? tile_terms<true>(T, fill, cx, cy, cz, K) : tile_terms<false>(T, fill, cx, cy, cz, K);
-        __syncwarp();
+      f2_unpack(acca, a0, a1);
+      f2_unpack(accb, b0, b1);
+    } else {
+      for (unsigned j = s0; j < s1; j += 2u) {
+        if (L.x[j] > 1e17f) break;  // padding ends a cell; spans of one cell in this form
+        pair_fast<false>(L.x[j], L.y[j], L.z[j], ax, ay, az, e2f, limf, K.nxf, a0, ea);
+        if (TWO) pair_fast<false>(L.x[j], L.y[j], L.z[j], bx, by, bz, e2f, limf, K.nxf, b0, eb);
+        if (L.x[j + 1] > 1e17f) break;
+        pair_fast<false>(L.x[j + 1], L.y[j + 1], L.z[j + 1], ax, ay, az, e2f, limf, K.nxf, a1, ea);
+        if (TWO) pair_fast<false>(L.x[j + 1], L.y[j + 1], L.z[j + 1], bx, by, bz, e2f, limf, K.nxf, b1, eb);
       }
-      if (active && K.has_quirk) {
-        // the particle the run scan files under another cell: counted if
-        // that cell is in x_sel2 but outside this candidate cell's 27
-        // neighbours (as k_refine_warp does)
-        const int ax = (int)(K.quirk_listed % K.nx), ay = (int)((K.quirk_listed / K.nx) % K.nx),
-                  az = (int)(K.quirk_listed / ((unsigned)K.nx * K.nx));
-        const bool listed_in_sel2 = in_sel2(K, ax, ay, az, g.ic, g.jc, g.kc);
-        const bool seen = abs(pdiff(ax, cxc, K.nx)) <= 1 && abs(pdiff(ay, cyc, K.nx)) <= 1 && abs(pdiff(az, czc, K.nx)) <= 1;
-        if (listed_in_sel2 && !seen) {
-          const float4 qv = B.cube[K.quirk_pos];
-          if (!(__float_as_uint(qv.w) & PSOD_DEAD_BIT)) {
-            const double d2 = min_image_d2((double)to_grid(qv.x, K.nxf), (double)to_grid(qv.y, K.nxf),
-                                           (double)to_grid(qv.z, K.nxf), (double)cx, (double)cy, (double)cz, K.tx);
-            if (d2 <= K.rmin2) sum += ddiv(1.0, dsqrt(dadd(d2, K.eps2)));
-          }
-        }
+    }
+    sa += ea < EDGE_MARGIN ? exact_span(s0, s1, ax, ay, az) : (double)a0 + (double)a1;
+    if (TWO) sb += eb < EDGE_MARGIN ? exact_span(s0, s1, bx, by, bz) : (double)b0 + (double)b1;
+  }
+}
+
+__device__ __forceinline__ void small_seed(const SodConst &K, const SodBufs &B, Smem &S, unsigned slot, unsigned rank) {
+  // per cell: first record, first flat record number, alive records, first
+  // list entry, fill cursor
+  __shared__ unsigned c_beg[SL_CELLS], c_flat[SL_CELLS + 1], c_al[SL_CELLS], c_off[SL_CELLS + 1], c_cur[SL_CELLS];
+  __shared__ unsigned i_pre[28];  // groups of 32 or 64 candidates before each inner cell
+  __shared__ unsigned s_ncand, s_work;
+  SmallList &L = *reinterpret_cast<SmallList *>(S.hist);
+  double *csum = reinterpret_cast<double *>(S.skey);  // per list entry: over skey, sidx and pref
+  static_assert(offsetof(Smem, lev) - offsetof(Smem, skey) >= sizeof(double) * NB, "room for the candidate sums");
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+  const unsigned bi = B.bidx_of_rank[rank];
+  if (t == 0) {
+    B.processed[rank] = 1;
+    mark_resolved(B, bi);
+  }
+  const SeedGeo g = seed_geo(K, B, rank);
+  const float4 sv = B.cube[g.sp];
+  if (__float_as_uint(sv.w) & PSOD_DEAD_BIT) return;  // claimed (main:1628)
+  auto put_back = [&]() {  // the seed waits: it is unresolved again
+    if (t == 0) {
+      B.processed[rank] = 0;
+      atomicAnd(&B.resolved[bi >> 5], ~(1u << (bi & 31)));
+    }
+  };
+  // ---- preselect (as prep_seed) and the cells' alive counts ----
+  unsigned na = 0;
+  if (B.mode == PSOD_MODE_PLAIN) {
+    unsigned cnt = 0, recs = 0;
+    for_cube(K, B, g.ic, g.jc, g.kc, K.ncut, [&](unsigned, float4 v) {
+      recs++;
+      if (!(__float_as_uint(v.w) & PSOD_DEAD_BIT)) cnt++;
+    });
+    na = block_sum_u32(S, cnt);
+    const unsigned nrec = block_sum_u32(S, recs);
+    if (t == 0) atomicAdd(B.touched, (unsigned long long)nrec);
+    if ((long long)na > K.nsel) {
+      if (t == 0) record_error(B, rank, PSOD_ERR_NSEL);
+      return;
+    }
+    if (!(dmul((double)na, K.munit) >= K.mmin)) return;  // main:1759
+  } else if (K.n_total > K.nsel) {
+    const unsigned recs = cube_records(K, B, S, g.ic, g.jc, g.kc);
+    if ((long long)recs > K.nsel) {
+      const unsigned exact = alive_rows(K, B, S, g.ic, g.jc, g.kc, ~0u);
+      if ((long long)exact > K.nsel) {
+        if (t == 0) record_error(B, rank, PSOD_ERR_NSEL);
+        return;
       }
-      if (active) B.cand_s[coff + k] = sum;
     }
   }
+  unsigned beg = 0, len = 0, al = 0;
+  if (t < SL_CELLS) {
+    const unsigned cell = (unsigned)wrapi(g.ic + t % 5 - 2, K.nx) +
+                          (unsigned)K.nx * ((unsigned)wrapi(g.jc + (t / 5) % 5 - 2, K.nx) +
+                                            (unsigned)K.nx * (unsigned)wrapi(g.kc + t / 25 - 2, K.nx));
+    beg = B.cs[cell];
+    len = B.cs[cell + 1] - beg;
+    if (B.alive_cnt) {
+      al = B.alive_cnt[cell];
+      if (al == 0) len = 0;  // nothing to gather
+    }
+    c_beg[t] = beg;
+  }
+  // exclusive scan of v over the threads (the first 128 hold the cells);
+  // returns the total
+  auto scan = [&](unsigned v, unsigned &excl) {
+    unsigned inc = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += y;
+    }
+    __syncthreads();
+    if (lane == 31) S.red_u32[w] = inc;
+    __syncthreads();
+    unsigned base = 0, tot = 0;
+    for (int q = 0; q < nwarp(); q++) {
+      if (q < w) base += S.red_u32[q];
+      tot += S.red_u32[q];
+    }
+    excl = base + inc - v;
+    return tot;
+  };
+  unsigned ex;
+  const unsigned nflat = scan(len, ex);
+  if (t < SL_CELLS) c_flat[t] = ex;
+  if (t == 0) c_flat[SL_CELLS] = nflat;
+  auto cell_of = [&](unsigned f) {  // the last cell whose first flat record is <= f
+    int lo = 0, hi = SL_CELLS - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (c_flat[mid] <= f) lo = mid;
+      else hi = mid - 1;
+    }
+    return lo;
+  };
+  if (!B.alive_cnt) {
+    if (t < SL_CELLS) c_al[t] = 0;
+    __syncthreads();
+    for (unsigned f = t; f < nflat; f += tpb()) {
+      const int c = cell_of(f);
+      if (!(__float_as_uint(B.cube[c_beg[c] + (f - c_flat[c])].w) & PSOD_DEAD_BIT)) atomicAdd(&c_al[c], 1u);
+    }
+    __syncthreads();
+    if (t < SL_CELLS) al = c_al[t];
+  }
+  const unsigned nlist = scan((al + 3u) & ~3u, ex);
+  if (t < SL_CELLS) {
+    c_al[t] = al;
+    c_off[t] = ex;
+    c_cur[t] = 0;
+  }
+  if (t == 0) {
+    c_off[SL_CELLS] = nlist;
+    s_work = 0;
+  }
+  // alive records of those of the cells that lie in the preselect cube
+  const int cheb = max(abs(t % 5 - 2), max(abs((t / 5) % 5 - 2), abs(t / 25 - 2)));
+  const unsigned near = block_sum_u32(S, cheb <= K.ncut ? al : 0u);
+  if (B.mode != PSOD_MODE_PLAIN) {
+    // Mmin: the cells at hand usually reach it
+    const unsigned need = K.mmin_count;
+    if (near < need && alive_rows(K, B, S, g.ic, g.jc, g.kc, need) < need) return;  // main:1759
+  }
+  if (w == 0) {
+    const int o = lane;
+    const unsigned cn = o < 27 ? c_al[sl_inner(o)] : 0u;
+    const unsigned ng = cn > 32u ? (cn + 63u) / 64u : (cn > 0u ? 1u : 0u);
+    unsigned ic = cn, ig = ng;
+    for (int sh = 1; sh < 32; sh <<= 1) {
+      const unsigned a = __shfl_up_sync(0xffffffffu, ic, sh), b = __shfl_up_sync(0xffffffffu, ig, sh);
+      if (lane >= sh) {
+        ic += a;
+        ig += b;
+      }
+    }
+    if (o < 28) i_pre[o] = ig - ng;
+    if (lane == 31) s_ncand = ic;
+  }
+  __syncthreads();
+  const unsigned ncand = s_ncand;
+  if (nlist > (unsigned)NB || ncand > B.max_cand) {
+    // more than shared memory holds (or the loop's limit): the host's rounds
+    put_back();
+    if (t == 0) atomicOr(B.deferred, 1u);
+    return;
+  }
+  if (t == 0) atomicAdd(B.nprocessed, 1ull);
+  // ---- gather: coordinates in grid units, padding far from every candidate.
+  // The cells reach at most 3 from the seed; where that crosses the box edge,
+  // the records beyond it are moved down by nx (exact, their coordinates are
+  // above nx/2), so plain differences are minimum-image ones.  Small boxes,
+  // and a list that may hold the particle filed under a foreign cell, keep
+  // their coordinates and take the minimum image pair by pair. ----
+  const bool wrap =
+      K.nx < 16 || (K.has_quirk && in_sel2(K, (int)(K.quirk_listed % K.nx), (int)((K.quirk_listed / K.nx) % K.nx),
+                                           (int)(K.quirk_listed / ((unsigned)K.nx * K.nx)), g.ic, g.jc, g.kc));
+  auto beyond = [&](float x) {  // coordinates above this move down
+    const float h = 0.5f * K.nxf;
+    return wrap ? 3e38f : (x < 3.5f ? x + h : (x > K.nxf - 3.5f ? x - h : 3e38f));
+  };
+  const float ox = beyond(to_grid(sv.x, K.nxf)), oy = beyond(to_grid(sv.y, K.nxf)), oz = beyond(to_grid(sv.z, K.nxf));
+  for (unsigned j = t; j < nlist; j += tpb()) L.x[j] = L.y[j] = L.z[j] = 1e18f;
+  __syncthreads();
+  for (unsigned f0 = t; f0 < nflat; f0 += 4u * tpb()) {
+    int cc[4];
+    float4 vv[4];
+#pragma unroll
+    for (int u = 0; u < 4; u++) {  // four records a thread in flight
+      const unsigned f = f0 + (unsigned)(u * tpb());
+      cc[u] = f < nflat ? cell_of(f) : -1;
+      if (cc[u] >= 0) vv[u] = B.cube[c_beg[cc[u]] + (f - c_flat[cc[u]])];
+    }
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int c = cc[u];
+      if (c < 0) break;
+      const float4 v = vv[u];
+      if (__float_as_uint(v.w) & PSOD_DEAD_BIT) continue;
+      const unsigned k = atomicAdd(&c_cur[c], 1u);
+      if (k >= c_al[c]) {  // the alive counts do not match the flags
+        record_error(B, rank, PSOD_ERR_STATE);
+        continue;
+      }
+      const unsigned at = c_off[c] + k;
+      const float x = to_grid(v.x, K.nxf), y = to_grid(v.y, K.nxf), z = to_grid(v.z, K.nxf);
+      L.x[at] = x > ox ? x - K.nxf : x;
+      L.y[at] = y > oy ? y - K.nxf : y;
+      L.z[at] = z > oz ? z - K.nxf : z;
+      L.pos[at] = c_beg[c] + (f0 + (unsigned)(u * tpb()) - c_flat[c]);
+    }
+  }
+  for (unsigned j = t; j < nlist; j += tpb()) csum[j] = 0.0;
+  __syncthreads();
+  // ---- approximate sums: a warp per (group of candidates, plane of
+  // neighbour rows) ----
+  {
+    const unsigned nitem = 3u * i_pre[27];
+    while (true) {
+      unsigned it = 0;
+      if (lane == 0) it = atomicAdd(&s_work, 1u);
+      it = __shfl_sync(0xffffffffu, it, 0);
+      if (it >= nitem) break;
+      const unsigned gi = it / 3u;
+      const int dz = (int)(it % 3u) - 1;
+      int o = 0;
+      while (i_pre[o + 1] <= gi) o++;  // i_pre[27] > gi
+      const int c = sl_inner(o);
+      const unsigned cn = c_al[c], k0 = (gi - i_pre[o]) * 64u + (unsigned)lane, k1 = k0 + 32u;
+      const bool two = cn > (gi - i_pre[o]) * 64u + 32u;
+      const unsigned q0 = c_off[c] + (k0 < cn ? k0 : 0u), q1 = c_off[c] + (k1 < cn ? k1 : 0u);
+      const float ax = L.x[q0], ay = L.y[q0], az = L.z[q0], bx = L.x[q1], by = L.y[q1], bz = L.z[q1];
+      double sa = 0.0, sb = 0.0;
+      for (int dy = -1; dy <= 1; dy++) {
+        const int row = c + 5 * dy + 25 * dz;  // the three cells row-1 .. row+1 are contiguous
+        if (!wrap) {
+          const unsigned j0 = c_off[row - 1], j1 = c_off[row + 2];
+          if (two) list_terms<false, true>(L, j0, j1, ax, ay, az, bx, by, bz, K, sa, sb);
+          else list_terms<false, false>(L, j0, j1, ax, ay, az, bx, by, bz, K, sa, sb);
+        } else {
+          for (int dx = -1; dx <= 1; dx++)
+            list_terms<true, true>(L, c_off[row + dx], c_off[row + dx + 1], ax, ay, az, bx, by, bz, K, sa, sb);
+        }
+      }
+      if (k0 < cn) atomicAdd(&csum[q0], sa);
+      if (two && k1 < cn) atomicAdd(&csum[q1], sb);
+    }
+  }
+  __syncthreads();
+  // ---- exact sums of the contenders and the argmax (as select_seed) ----
+  unsigned cpos = g.sp, lq = ~0u;  // no candidate: the seed stays the centre
+  unsigned long long sbest = 0;
+  if (ncand > 0) {
+    unsigned long long mb = 0, dummy = 0;
+    for (int o = w; o < 27; o += nwarp()) {
+      const int c = sl_inner(o);
+      for (unsigned k = lane; k < c_al[c]; k += 32u) {
+        const unsigned long long b = dbits(csum[c_off[c] + k]);
+        mb = b > mb ? b : mb;
+      }
+    }
+    block_max_pair(S, mb, dummy);
+    const double thr = dmul(bitsd(mb), 1.0 - 2.0 * REF_TOL);
+    unsigned long long best_sq = 0, best_key = ~0ull;
+    unsigned best_q = 0xffffffffu;
+    // exact sum of candidate q of inner cell c over this warp's share of the
+    // neighbour rows (part of nparts)
+    auto exact = [&](int c, unsigned q, int part, int nparts) {
+      const double cx = (double)L.x[q], cy = (double)L.y[q], cz = (double)L.z[q];
+      unsigned long long sq = 0;
+      for (int r = part; r < 9; r += nparts) {
+        const int row = c + 5 * (r % 3 - 1) + 25 * (r / 3 - 1);
+        for (unsigned j = c_off[row - 1] + lane; j < c_off[row + 2]; j += 32u) {
+          const float rx = L.x[j];
+          if (rx > 1e17f) continue;
+          const double d2 = min_image_d2((double)rx, (double)L.y[j], (double)L.z[j], cx, cy, cz, K.tx);
+          if (d2 <= K.rmin2) {
+            const double tt = ddiv(1.0, dsqrt(dadd(d2, K.eps2)));
+            sq += (unsigned long long)__double2ll_rn(dmul(tt, 1099511627776.0));
+          }
+        }
+      }
+      for (int sh = 16; sh > 0; sh >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, sh);
+      return sq;
+    };
+    auto better = [&](unsigned long long sq, int o, unsigned q) {
+      const unsigned long long key =
+          ((unsigned long long)o << 32) | (__float_as_uint(B.cube[L.pos[q]].w) & PSOD_IDX_MASK);
+      if (sq > best_sq || (sq == best_sq && key < best_key)) {
+        best_sq = sq;
+        best_key = key;
+        best_q = q;
+      }
+    };
+    if (t == 0) S.nsel = 0;
+    __syncthreads();
+    for (int o = w; o < 27; o += nwarp()) {
+      const int c = sl_inner(o);
+      for (unsigned k = lane; k < c_al[c]; k += 32u)
+        if (csum[c_off[c] + k] >= thr) {
+          const unsigned j = atomicAdd(&S.nsel, 1u);
+          if (j < SEL_SPLIT_MAX) S.sel[j] = ((unsigned)o << 16) | (c_off[c] + k);
+        }
+    }
+    __syncthreads();
+    const unsigned nsel = S.nsel;
+    if (nsel <= SEL_SPLIT_MAX) {  // the whole CTA on each contender
+      for (unsigned j = 0; j < nsel; j++) {
+        const int o = (int)(S.sel[j] >> 16);
+        const unsigned q = S.sel[j] & 0xffffu;
+        const unsigned long long part = exact(sl_inner(o), q, w, nwarp());
+        __syncthreads();
+        if (lane == 0) S.red_u64[w] = part;
+        __syncthreads();
+        unsigned long long sq = 0;
+        for (int e = 0; e < nwarp(); e++) sq += S.red_u64[e];
+        if (t == 0) better(sq, o, q);
+      }
+    } else {  // a warp per contender
+      for (int o = w; o < 27; o += nwarp()) {
+        const int c = sl_inner(o);
+        for (unsigned k = 0; k < c_al[c]; k++) {
+          const unsigned q = c_off[c] + k;
+          if (!(csum[q] >= thr)) continue;
+          const unsigned long long sq = exact(c, q, 0, 1);
+          if (lane == 0) better(sq, o, q);
+        }
+      }
+    }
+    unsigned long long a = best_sq, b = ~best_key;
+    const unsigned long long pa = a, pb = b;
+    block_max_pair(S, a, b);
+    if (t == 0) S.best_pos = 0xffffffffu;
+    __syncthreads();
+    if (lane == 0 && best_q != 0xffffffffu && pa == a && pb == b) S.best_pos = best_q;
+    __syncthreads();
+    lq = S.best_pos;
+    if (lq != ~0u) cpos = L.pos[lq];
+    sbest = a;
+  }
+  if (B.learn_collect) {
+    if (t == 0) {
+      B.st_active[slot] = 1;
+      B.st_cn[slot] = ncand;
+      B.st_centre[slot] = cpos;
+      B.st_sbest[slot] = sbest;
+    }
+    __syncthreads();
+    seed_features(K, B, S, slot, rank);
+    __syncthreads();
+  }
+  // The list holds the preselect cube's records around the centre when the
+  // cube has the list's cells.  The particle filed under a foreign cell may
+  // lie near the centre without being in them: then the region walk finds it.
+  bool use_list = lq != ~0u && K.ncut >= 2;
+  if (K.has_quirk && abs(pdiff((int)(K.quirk_listed % K.nx), g.ic, K.nx)) <= 4 &&
+      abs(pdiff((int)((K.quirk_listed / K.nx) % K.nx), g.jc, K.nx)) <= 4 &&
+      abs(pdiff((int)(K.quirk_listed / ((unsigned)K.nx * K.nx)), g.kc, K.nx)) <= 4)
+    use_list = false;
+  cross_seed(K, B, S, slot, rank, g, na, cpos, use_list ? nlist : 0u, lq);
 }
 
 enum : unsigned { TAIL_RUNNING = 0, TAIL_DONE = 1, TAIL_DEFERRED = 2, TAIL_STALLED = 3, TAIL_TIMEOUT = 4 };
@@ -3186,11 +3583,7 @@ enum : unsigned { TAIL_RUNNING = 0, TAIL_DONE = 1, TAIL_DEFERRED = 2, TAIL_STALL
 struct TailState {
   unsigned nact[2];       // active-block count of list act[p]
   unsigned nready[2];     // per round parity
-  unsigned work[2];       // work counters of the seed steps: preselect,
-  unsigned work_r[2];     // refinement (candidate cells), select, crossing
-  unsigned work_s[2];
-  unsigned work_c[2];
-  unsigned cand_used[2];
+  unsigned work[2];       // work counter of the seed step
   unsigned gmin[2];
   unsigned deferred;
   unsigned status;
@@ -3209,7 +3602,7 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-constexpr unsigned long long BARRIER_POLLS = 1ull << 24;  // about 2-4 s of polling
+constexpr unsigned long long BARRIER_POLLS = 1ull << 25;  // a few seconds of polling
 
 // Grid-wide barrier of the cooperative launch (generation counting).  The
 // fences make every write before the barrier visible to every read after
@@ -3234,7 +3627,7 @@ __device__ bool grid_barrier(TailState *ts) {
           ok = 0;
           break;
         }
-        __nanosleep(128);
+        __nanosleep(32);
       }
       if (!ok) atomicExch(&ts->status, TAIL_TIMEOUT);
     }
@@ -3249,14 +3642,13 @@ __device__ bool grid_barrier(TailState *ts) {
 // value written by another CTA before the last barrier
 __device__ __forceinline__ unsigned ld_shared_state(const unsigned *p) { return *(volatile const unsigned *)p; }
 
-__global__ void __launch_bounds__(TPB) k_tail_rounds(SodConst K, SodBufs B, TailState *ts, unsigned *act0,
+__global__ void __launch_bounds__(LOOP_TPB, 1) k_tail_rounds(SodConst K, SodBufs B, TailState *ts, unsigned *act0,
                                                     unsigned *act1, const unsigned *bbegin, unsigned *cursor,
                                                     const unsigned *blist, unsigned *head, int nb, int rb,
                                                     unsigned quirk_rank, unsigned *ready) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem &S = *reinterpret_cast<Smem *>(smem_raw);
   __shared__ unsigned s_cnt, s_next, s_nready;
-  __shared__ RecTile t_tiles[NWARP];
   const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
   const int lane = threadIdx.x & 31;
   // the round parity: every CTA flips its own copy once per round
@@ -3307,10 +3699,6 @@ __global__ void __launch_bounds__(TPB) k_tail_rounds(SodConst K, SodBufs B, Tail
       ts->gmin[q ^ 1u] = PSOD_INF_RANK;
       ts->nready[q ^ 1u] = 0;
       ts->work[q ^ 1u] = 0;
-      ts->work_r[q ^ 1u] = 0;
-      ts->work_s[q ^ 1u] = 0;
-      ts->work_c[q ^ 1u] = 0;
-      ts->cand_used[q ^ 1u] = 0;
       ts->xused[q ^ 1u] = 0;
     }
     if (threadIdx.x == 0) s_next = ld_shared_state(&ts->nact[q ^ 1u]);
@@ -3339,48 +3727,18 @@ __global__ void __launch_bounds__(TPB) k_tail_rounds(SodConst K, SodBufs B, Tail
       }
       return;
     }
-    // the round's seeds, a CTA each
+    // the round's seeds, a CTA each from the preselect to the claims: ready
+    // seeds share no particle, so nothing is waited for in between
     SodBufs Br = B;
     Br.nready = &ts->nready[q];
-    Br.cand_used = &ts->cand_used[q];
     Br.xused = &ts->xused[q];
     Br.deferred = &ts->deferred;
     Br.maxcand = nullptr;
     Br.learn_use = 0;
-    // preselect: a CTA per seed
     while (true) {
       const unsigned item = next_item(&ts->work[q]);
       if (item >= nready) break;
-      prep_seed(K, Br, S, item, B.ready[item]);
-    }
-    if (!grid_barrier(ts)) return;
-    // refinement: a warp per (seed, candidate cell) over the whole grid
-    {
-      const int w = threadIdx.x >> 5;
-      while (true) {
-        unsigned it = 0;
-        if (lane == 0) it = atomicAdd(&ts->work_r[q], 1u);
-        it = __shfl_sync(0xffffffffu, it, 0);
-        if (it >= nready * 27u) break;
-        const unsigned slot = it / 27u;
-        if (!Br.st_active[slot]) continue;
-        tail_refine_cell(K, Br, slot, (int)(it % 27u), seed_geo(K, Br, B.ready[slot]), t_tiles[w]);
-      }
-    }
-    if (!grid_barrier(ts)) return;
-    // exact sums of the contenders and the argmax: a CTA per seed
-    while (true) {
-      const unsigned item = next_item(&ts->work_s[q]);
-      if (item >= nready) break;
-      select_seed(K, Br, S, item, B.ready[item]);
-      if (Br.learn_collect) seed_features(K, Br, S, item, B.ready[item]);
-    }
-    if (!grid_barrier(ts)) return;
-    // crossing, profile and claims: a CTA per seed
-    while (true) {
-      const unsigned item = next_item(&ts->work_c[q]);
-      if (item >= nready) break;
-      cross_seed(K, Br, S, item, B.ready[item]);
+      small_seed(K, Br, S, item, B.ready[item]);
     }
     if (!grid_barrier(ts)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -3403,10 +3761,6 @@ __global__ void k_tail_init(TailState *ts, unsigned n_active) {
   ts->nact[1] = 0;
   ts->nready[0] = ts->nready[1] = 0;
   ts->work[0] = ts->work[1] = 0;
-  ts->work_r[0] = ts->work_r[1] = 0;
-  ts->work_s[0] = ts->work_s[1] = 0;
-  ts->work_c[0] = ts->work_c[1] = 0;
-  ts->cand_used[0] = ts->cand_used[1] = 0;
   ts->gmin[0] = ts->gmin[1] = PSOD_INF_RANK;
   ts->xused[0] = ts->xused[1] = 0;
   ts->deferred = 0;
@@ -3645,12 +3999,14 @@ enum {
 };
 static_assert((int)SC_BIGSEG < (int)SLOT_CELL_U32, "SOD scratch slots overlap the shared ones");
 
-// Rounds go to the device tail loop once the last host round had no seed
-// for the bound pass, no seed with more than tail_max_cand candidates, at
-// most tail_max_ready ready seeds (psod_tuning) and few enough active blocks
-// for the direct readiness test; after a launch that ended on a larger
-// seed, the host runs at least TAIL_REST rounds before the next launch.
-constexpr int TAIL_REST = 8;
+// Rounds go to the device round loop once the last host round had no seed for
+// the bound pass, none with more than LOOP_CAND x tail_max_cand candidates and
+// at most LOOP_READY x tail_max_ready ready seeds (psod_tuning), and few
+// enough active blocks for the direct readiness test inside the loop
+// (LOOP_TESTS heads read a round).  A launch that ended on a larger seed within
+// LOOP_SHORT rounds is followed by LOOP_REST host rounds before the next.
+constexpr long long LOOP_READY = 16, LOOP_CAND = 4, LOOP_TESTS = 1ll << 27;
+constexpr int LOOP_SHORT = 4, LOOP_REST = 8;
 
 struct PhaseTimer {
   cudaEvent_t a, b;
@@ -3984,7 +4340,7 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
   const long long direct_cost_per_block = window * window * window, filter_cost = 3 * nblocks * window;
   bool pending = false, pend_learn = false, pend_bound = false;
   // device tail loop: one CTA per seed slot resident on every SM
-  int tail_grid = 0, rest = 0;
+  int tail_grid = 0, rest = 0, rest_need = 1;
   long long tail_rounds = 0;
   TailState *tail = nullptr;
   {
@@ -3993,7 +4349,7 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
     int per_sm_tail = 0;
     if (coop && (rc = scratch(c, SC_TAIL, 1, &tail)) == PSOD_OK &&
         cudaFuncSetAttribute(k_tail_rounds, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_tail, k_tail_rounds, TPB, smem) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_tail, k_tail_rounds, LOOP_TPB, smem) == cudaSuccess &&
         per_sm_tail > 0)
       tail_grid = dev_sms * per_sm_tail;
     if (rc) return rc;
@@ -4126,13 +4482,13 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
     seed_launches += 4;
     kernels += 4;
     rest++;
-    if (tail_grid > 0 && nbig == 0 && maxcand <= (unsigned)c->tune.tail_max_cand &&
-        nready <= (unsigned)c->tune.tail_max_ready && rest >= TAIL_REST &&
-        n_active > 0 && (long long)n_active * direct_cost_per_block <= filter_cost) {
+    if (tail_grid > 0 && nbig == 0 && (long long)maxcand <= LOOP_CAND * c->tune.tail_max_cand &&
+        (long long)nready <= LOOP_READY * c->tune.tail_max_ready && rest >= rest_need && n_active > 0 &&
+        (long long)n_active * direct_cost_per_block <= LOOP_TESTS) {
       // the following rounds on the device, until a larger seed or the end
       k_tail_init<<<1, 1, 0, c->stream>>>(tail, n_active);
       SodBufs Bt = B;
-      Bt.max_cand = (unsigned)c->tune.tail_max_cand;
+      Bt.max_cand = (unsigned)std::min<long long>(LOOP_CAND * c->tune.tail_max_cand, NB);
       Bt.st_big = nullptr;
       Bt.touch = u64s + 19;  // the tail's crossings counted apart from k_cross
       Bt.kept_members = u64s + 20;
@@ -4140,7 +4496,7 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
                       (void *)&bbegin, (void *)&cursor, (void *)&blist, (void *)&head, (void *)&nb,
                       (void *)&rb,    (void *)&quirk_rank, (void *)&ready};
       t_tail.start(c->stream);
-      PSOD_CUDA(c, cudaLaunchCooperativeKernel((const void *)k_tail_rounds, dim3(tail_grid), dim3(TPB), args, smem,
+      PSOD_CUDA(c, cudaLaunchCooperativeKernel((const void *)k_tail_rounds, dim3(tail_grid), dim3(LOOP_TPB), args, smem,
                                                c->stream));
       t_tail.stop(c->stream);
       kernels += 2;
@@ -4164,6 +4520,7 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
       if (ts.parity) std::swap(act_a, act_b);
       n_active = ts.status == TAIL_DONE ? 0u : ts.nact[ts.parity];
       rest = 0;
+      rest_need = (int)ts.rounds < LOOP_SHORT ? LOOP_REST : 1;
     }
   }
   collect_pending();
