@@ -35,6 +35,8 @@ namespace {
 constexpr int TPB = 256;          // threads per seed CTA of the host rounds' kernels
 constexpr int LOOP_TPB = 512;     // threads per seed CTA of the device round loop
 constexpr unsigned RN_CHUNK = 2048;  // neighbour records per refinement work item
+constexpr unsigned LOOP_CHUNK = 512;  // in the device round loop: few seeds, all SMs for each
+constexpr unsigned LOOP_BIG = 64;     // seeds of a loop round whose refinement the whole grid shares
 constexpr int MAX_WARP = LOOP_TPB / 32;
 // the seed steps run in CTAs of either size
 __device__ __forceinline__ int tpb() { return (int)blockDim.x; }
@@ -95,6 +97,8 @@ struct SodBufs {
   unsigned *maxcand;    // largest candidate count of a seed this round (or null)
   unsigned max_cand;    // seeds with more candidates wait (device tail loop), else ~0u
   unsigned *deferred;   // set when a seed waited for that reason
+  unsigned rn_chunk;    // neighbour records per refinement work item
+  unsigned *bigq, *nbigq;  // device round loop: slots of the seeds refined by the whole grid
   unsigned *alive_cnt;  // alive records per cell (batched modes)
   unsigned long long *pairs;       // candidate-neighbour records visited
   unsigned long long *touch;       // records of the balls out to each stop
@@ -1028,7 +1032,7 @@ __device__ __forceinline__ void prep_seed(const SodConst &K, const SodBufs &B, S
         nbr += B.cs[base + (unsigned)x1 + 1] - B.cs[base + (unsigned)x0];
       }
     }
-    const unsigned nch = max(1u, (nbr + RN_CHUNK - 1) / RN_CHUNK);
+    const unsigned nch = max(1u, (nbr + B.rn_chunk - 1) / B.rn_chunk);
     B.cell_cnt[slot * 27 + o] = s_cnt[o];
     B.cell_off[slot * 27 + o] = s_base + s_coff[o];
     B.cell_nch[slot * 27 + o] = nch;
@@ -1431,22 +1435,292 @@ __device__ __forceinline__ void tile_terms2(const RecTile &tile, unsigned nt, fl
 constexpr unsigned ITEM_GRAB = 1;  // refinement items claimed per counter update
 constexpr float NEAR2 = 0.09f;
 
+// One warp's staging area and counters
+struct WarpRef {
+  RecTile tile;
+  unsigned rb[18], rp[19];
+  int nr, wf;
+  // pair, slot and staged-record counts and items taken: per item in 32 bits,
+  // per warp here (keeps 64-bit totals out of the registers)
+  unsigned long long count[4];
+};
+
+// item `rem` of candidate cell ci (phase2: over its surviving candidates)
+template <bool BOUND>
+__device__ __forceinline__ void refine_item(const SodConst &K, const SodBufs &B, unsigned ci, unsigned rem, bool phase2,
+                                            WarpRef &R) {
+  const int lane = threadIdx.x & 31;
+  const unsigned nch = B.cell_nch[ci];
+  const unsigned chunk = rem / nch, nchunk = rem % nch;
+  const unsigned slot = ci / 27, o = ci % 27;
+  const bool bounded = B.bound_on && B.st_cn[slot] >= B.bound_min;
+  if (BOUND && !bounded) return;
+  if (!BOUND && lane == 0) R.count[3]++;
+  const SeedGeo g = seed_geo(K, B, B.ready[slot]);
+  const int di = (int)(o / 9) - 1, dj = (int)((o / 3) % 3) - 1, dk = (int)(o % 3) - 1;
+  const int cxc = wrapi(g.ic + di, K.nx), cyc = wrapi(g.jc + dj, K.nx), czc = wrapi(g.kc + dk, K.nx);
+  const unsigned cnt = phase2 ? B.cnt2[ci] : B.cell_cnt[ci];
+  // candidates k0 = 64*chunk + lane and k1 = k0 + 32 of the cell (phase 2:
+  // of its surviving candidates); items of at most 32 candidates run one
+  // per lane
+  const unsigned k0 = chunk * 64u + (unsigned)lane, k1 = k0 + 32u;
+  const bool two = cnt > chunk * 64u + 32u;
+  const bool have = k0 < cnt, have1 = k1 < cnt;
+  const unsigned coff = B.cell_off[ci];
+  const unsigned q = phase2 ? (have ? B.cand_list[coff + k0] : 0u) : coff + k0;
+  const unsigned q1 = phase2 ? (have1 ? B.cand_list[coff + k1] : 0u) : coff + k1;
+  const unsigned cp = have ? B.cand_pos[q] : 0u, cp1 = have1 ? B.cand_pos[q1] : 0u;
+  const bool quirk = have && K.has_quirk && cp == K.quirk_pos;
+  const bool quirk1 = have1 && K.has_quirk && cp1 == K.quirk_pos;
+  float cx = 0.f, cy = 0.f, cz = 0.f, bx = 1e18f, by = 1e18f, bz = 1e18f;
+  if (have) {
+    const float4 cv = B.cube[cp];
+    cx = to_grid(cv.x, K.nxf);
+    cy = to_grid(cv.y, K.nxf);
+    cz = to_grid(cv.z, K.nxf);
+  }
+  if (have1) {
+    const float4 cv = B.cube[cp1];
+    bx = to_grid(cv.x, K.nxf);
+    by = to_grid(cv.y, K.nxf);
+    bz = to_grid(cv.z, K.nxf);
+  }
+  {
+    // record runs of the 3x3x3 cells around the candidate cell: 9 rows of a
+    // 3-cell x-run each (two runs when it wraps), lane r < 9 on row r; a
+    // warp scan of the run counts and lengths places them in row order
+    int np = 0;
+    unsigned b0 = 0, l0 = 0, b1 = 0, l1 = 0;
+    if (lane < 9) {
+      const unsigned yy = (unsigned)wrapi(cyc + lane % 3 - 1, K.nx), zz = (unsigned)wrapi(czc + lane / 3 - 1, K.nx);
+      const unsigned long long base = (unsigned long long)K.nx * (yy + (unsigned long long)K.nx * zz);
+      const int x0 = cxc - 1, x1 = cxc + 1;
+      int pa0, pb0, pa1 = 0, pb1 = -1;
+      if (x0 < 0) { pa0 = x0 + K.nx; pb0 = K.nx - 1; pa1 = 0; pb1 = x1; np = 2; }
+      else if (x1 >= K.nx) { pa0 = x0; pb0 = K.nx - 1; pa1 = 0; pb1 = x1 - K.nx; np = 2; }
+      else { pa0 = x0; pb0 = x1; np = 1; }
+      b0 = B.cs[base + (unsigned)pa0];
+      l0 = B.cs[base + (unsigned)pb0 + 1] - b0;
+      if (np == 2) {
+        b1 = B.cs[base + (unsigned)pa1];
+        l1 = B.cs[base + (unsigned)pb1 + 1] - b1;
+      }
+    }
+    unsigned pc = (unsigned)np, len = l0 + l1;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned tp = __shfl_up_sync(0xffffffffu, pc, o), tl = __shfl_up_sync(0xffffffffu, len, o);
+      if (lane >= o) {
+        pc += tp;
+        len += tl;
+      }
+    }
+    if (lane < 9) {
+      const unsigned pf = pc - (unsigned)np, lf = len - (l0 + l1);
+      R.rb[pf] = b0;
+      R.rp[pf] = lf;
+      if (np == 2) {
+        R.rb[pf + 1] = b1;
+        R.rp[pf + 1] = lf + l0;
+      }
+    }
+    if (lane == 8) {
+      R.rp[pc] = len;
+      R.nr = (int)pc;
+    }
+    if (lane == 0) {
+      // the 3-cell coordinate window of each axis stays clear of the box edge
+      auto clear = [&](int c, int a) {
+        double s0 = (double)(c - 1) + K.xs[a];
+        s0 -= K.tx * floor(s0 / K.tx);
+        return s0 >= 1.0 && s0 + 3.0 <= K.tx - 1.0;
+      };
+      R.wf = clear(cxc, 0) && clear(cyc, 1) && clear(czc, 2);
+    }
+  }
+  __syncwarp();
+  const int nr = R.nr;
+  const unsigned total = R.rp[nr];
+  const bool wf = R.wf;
+  const bool active = have && !quirk, active1 = have1 && !quirk1;
+  // bounding box of the item's candidates: records farther than 1 from it
+  // in every direction meet no candidate (wrap-free items only)
+  float lox = active ? cx : 3e38f, hix = active ? cx : -3e38f, loy = active ? cy : 3e38f,
+        hiy = active ? cy : -3e38f, loz = active ? cz : 3e38f, hiz = active ? cz : -3e38f;
+  if (active1) {
+    lox = fminf(lox, bx);
+    hix = fmaxf(hix, bx);
+    loy = fminf(loy, by);
+    hiy = fmaxf(hiy, by);
+    loz = fminf(loz, bz);
+    hiz = fmaxf(hiz, bz);
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    lox = fminf(lox, __shfl_xor_sync(0xffffffffu, lox, o));
+    hix = fmaxf(hix, __shfl_xor_sync(0xffffffffu, hix, o));
+    loy = fminf(loy, __shfl_xor_sync(0xffffffffu, loy, o));
+    hiy = fmaxf(hiy, __shfl_xor_sync(0xffffffffu, hiy, o));
+    loz = fminf(loz, __shfl_xor_sync(0xffffffffu, loz, o));
+    hiz = fmaxf(hiz, __shfl_xor_sync(0xffffffffu, hiz, o));
+  }
+  const bool any_active = lox <= hix;
+  const unsigned r0 = nchunk * B.rn_chunk, r1 = any_active ? min(total, r0 + B.rn_chunk) : r0;
+  const unsigned lt = (1u << lane) - 1u;
+  double sum = 0.0, sum1 = 0.0;
+  unsigned visits = 0, slots = 0, loaded = 0;
+  // tile of 32 kept records: the pair tests of every candidate lane
+  float uf = 0.f;  // BOUND: this lane's far records
+  const float e2b = (float)K.eps2;
+  auto consume = [&](unsigned nt) {
+    // pad to a multiple of 8 with records far from every candidate
+    if ((unsigned)lane < ((8u - (nt & 7u)) & 7u)) {
+      R.tile.x[nt + lane] = 1e18f;
+      R.tile.y[nt + lane] = 1e18f;
+      R.tile.z[nt + lane] = 1e18f;
+    }
+    __syncwarp();
+    if (two) {
+      if (active || active1) {
+        if (wf) tile_terms2<true>(R.tile, nt, cx, cy, cz, bx, by, bz, K, sum, sum1);
+        else tile_terms2<false>(R.tile, nt, cx, cy, cz, bx, by, bz, K, sum, sum1);
+      }
+    } else if (active) {
+      sum += wf ? tile_terms<true>(R.tile, nt, cx, cy, cz, K) : tile_terms<false>(R.tile, nt, cx, cy, cz, K);
+    }
+    if (lane == 0) {
+      visits += min(64u, cnt - chunk * 64u) * nt;
+      slots += (two ? 64u : 32u) * ((nt + 7u) & ~7u);
+    }
+    __syncwarp();
+  };
+  // Stage the chunk's records run by run, lanes on consecutive records of
+  // one run.  Only alive records within reach of the candidates' box are
+  // kept (warp-wide compaction into a 64-entry buffer); each full tile of
+  // 32 is consumed at once and the overflow moves to the front, so no
+  // record is loaded twice.
+  unsigned fill = 0;
+  int r = 0;
+  while (r + 1 < nr && R.rp[r + 1] <= r0) r++;
+  // (items near the periodic edge have no box filter: their bound is
+  // infinite and they are not staged by the bound pass)
+  for (unsigned pos = (BOUND && !wf) ? r1 : r0; pos < r1; r++) {
+    const unsigned run_end = min(R.rp[r + 1], r1);
+    const unsigned base = R.rb[r] - R.rp[r];  // cube slot = base + record number
+    // SD steps of 32 records per pass: each lane issues its SD loads
+    // before the first is used.  Both passes run best with one (measured
+    // at 1024^3: with its exact near-field tiles the bound pass needs the
+    // registers more than the loads in flight; four took it from 325 to
+    // 603 ms through spills).
+    constexpr int SD = 1;
+    for (unsigned xs0 = pos; xs0 < run_end; xs0 += 32u * SD) {
+      float4 vs[SD];
+#pragma unroll
+      for (int u = 0; u < SD; u++) {
+        const unsigned x = xs0 + 32u * (unsigned)u + (unsigned)lane;
+        vs[u] = x < run_end ? B.cube[base + x] : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < SD; u++) {
+        const unsigned x0 = xs0 + 32u * (unsigned)u;
+        if (x0 >= run_end) break;  // warp-uniform
+        const unsigned x = x0 + (unsigned)lane;
+        bool keep = false;
+        float4 rec = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (x < run_end) {
+          const float4 v = vs[u];
+          rec = make_float4(to_grid(v.x, K.nxf), to_grid(v.y, K.nxf), to_grid(v.z, K.nxf), 0.f);
+          keep = !(__float_as_uint(v.w) & PSOD_DEAD_BIT);
+          if (wf) {
+            const float ex = fmaxf(fmaxf(lox - rec.x, rec.x - hix), 0.f), ey = fmaxf(fmaxf(loy - rec.y, rec.y - hiy), 0.f),
+                        ez = fmaxf(fmaxf(loz - rec.z, rec.z - hiz), 0.f);
+            const float db2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+            if (BOUND) {
+              // far records add k(d to the group's box) to every
+              // candidate here; near ones go to the tile for exact sums
+              if (keep && db2 >= NEAR2 && db2 <= 1.0001f) uf += rsqrt_pos(db2 + e2b);
+              keep = keep && db2 < NEAR2;
+            } else {
+              keep = keep && db2 <= 1.0001f;
+            }
+          }
+        }
+        const unsigned m = __ballot_sync(0xffffffffu, keep);
+        if (keep) {  // fill < 32: index < 64
+          const unsigned at = fill + __popc(m & lt);
+          R.tile.x[at] = rec.x;
+          R.tile.y[at] = rec.y;
+          R.tile.z[at] = rec.z;
+        }
+        fill += (unsigned)__popc(m);
+        if (!BOUND) loaded += min(32u, run_end - x0);
+        if (fill >= 32u) {
+          consume(32u);
+          if ((unsigned)lane < fill - 32u) {
+            R.tile.x[lane] = R.tile.x[32 + lane];
+            R.tile.y[lane] = R.tile.y[32 + lane];
+            R.tile.z[lane] = R.tile.z[32 + lane];
+          }
+          __syncwarp();
+          fill -= 32u;
+        }
+      }
+    }
+    pos = run_end;
+  }
+  if (fill > 0) consume(fill);
+  if (BOUND) {
+    for (int sh = 16; sh > 0; sh >>= 1) uf += __shfl_xor_sync(0xffffffffu, uf, sh);
+    // the particle the run scan files under another cell may add up to
+    // 1/eps = 64 to any candidate's sum outside these runs; a candidate
+    // that is the run scan's own quirk particle gets no bound (it always
+    // stays in the exact pass), nor do items near the periodic edge
+    const float extra = (K.has_quirk && nchunk == 0) ? 64.f : 0.f;
+    const float inf = __int_as_float(0x7f800000);
+    if (have) atomicAdd(&B.cand_u[q], (wf && !quirk) ? (float)((sum + (double)uf) * 1.001) + extra : inf);
+    if (have1) atomicAdd(&B.cand_u[q1], (wf && !quirk1) ? (float)((sum1 + (double)uf) * 1.001) + extra : inf);
+  }
+  if (lane == 0) {
+    R.count[0] += visits;
+    R.count[1] += slots;
+    R.count[2] += loaded;
+  }
+  if (BOUND) return;
+  if (nchunk == 0 && K.has_quirk && (active || active1)) {
+    // the particle the run scan files under another cell: counted if that
+    // cell is in x_sel2 but outside this candidate cell's 27 neighbours
+    const int ax = (int)(K.quirk_listed % K.nx), ay = (int)((K.quirk_listed / K.nx) % K.nx),
+              az = (int)(K.quirk_listed / ((unsigned)K.nx * K.nx));
+    const bool listed_in_sel2 = in_sel2(K, ax, ay, az, g.ic, g.jc, g.kc);
+    const bool seen = abs(pdiff(ax, cxc, K.nx)) <= 1 && abs(pdiff(ay, cyc, K.nx)) <= 1 && abs(pdiff(az, czc, K.nx)) <= 1;
+    if (listed_in_sel2 && !seen) {
+      const float4 qv = B.cube[K.quirk_pos];
+      if (!(__float_as_uint(qv.w) & PSOD_DEAD_BIT)) {
+        const double qx = to_grid(qv.x, K.nxf), qy = to_grid(qv.y, K.nxf), qz = to_grid(qv.z, K.nxf);
+        if (active) {
+          const double d2 = min_image_d2(qx, qy, qz, (double)cx, (double)cy, (double)cz, K.tx);
+          if (d2 <= K.rmin2) sum += ddiv(1.0, dsqrt(dadd(d2, K.eps2)));
+        }
+        if (active1) {
+          const double d2 = min_image_d2(qx, qy, qz, (double)bx, (double)by, (double)bz, K.tx);
+          if (d2 <= K.rmin2) sum1 += ddiv(1.0, dsqrt(dadd(d2, K.eps2)));
+        }
+      }
+    }
+  }
+  if (active && sum != 0.0) atomicAdd(&B.cand_s[q], sum);
+  if (active1 && sum1 != 0.0) atomicAdd(&B.cand_s[q1], sum1);
+}
+
 template <bool BOUND>
 __global__ void __launch_bounds__(256, 3) k_refine_warp(SodConst K, SodBufs B) {
-  __shared__ RecTile s_tile[8];
-  __shared__ unsigned s_rb[8][18], s_rp[8][19];
-  __shared__ int s_nr[8], s_wf[8];
+  __shared__ WarpRef s_ref[8];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   const bool phase1 = !BOUND && B.ref_phase == 1;
   const unsigned nready = min(*B.nready, B.cap_ready);
   const bool phase2 = !BOUND && B.ref_phase == 2;
   const unsigned *cpref = phase2 ? B.chunk_pref2 : B.chunk_pref;
   const unsigned nitems = phase1 ? B.top_pref[nready] : cpref[B.nitems_cells];
-  // pair, slot and staged-record counts: per item in 32 bits, per warp in
-  // shared memory (keeps 64-bit totals out of the registers)
-  // (pair pass: also items taken)
-  __shared__ unsigned long long s_count[8][4];
-  if (lane < 4) s_count[w][lane] = 0;
+  WarpRef &R = s_ref[w];
+  if (lane < 4) R.count[lane] = 0;
   // items are claimed ITEM_GRAB at a time (one counter update per group of
   // consecutive items)
   unsigned grab = 0, grab_left = 0;
@@ -1483,270 +1757,13 @@ __global__ void __launch_bounds__(256, 3) k_refine_warp(SodConst K, SodBufs B) {
     if (item >= nitems) break;
     ci = __shfl_sync(0xffffffffu, ci, 0);
     rem = __shfl_sync(0xffffffffu, rem, 0);
-    const unsigned nch = B.cell_nch[ci];
-    const unsigned chunk = rem / nch, nchunk = rem % nch;
-    const unsigned slot = ci / 27, o = ci % 27;
-    const bool bounded = B.bound_on && B.st_cn[slot] >= B.bound_min;
-    if (BOUND && !bounded) continue;
-    if (!BOUND && lane == 0) s_count[w][3]++;
-    const SeedGeo g = seed_geo(K, B, B.ready[slot]);
-    const int di = (int)(o / 9) - 1, dj = (int)((o / 3) % 3) - 1, dk = (int)(o % 3) - 1;
-    const int cxc = wrapi(g.ic + di, K.nx), cyc = wrapi(g.jc + dj, K.nx), czc = wrapi(g.kc + dk, K.nx);
-    const unsigned cnt = phase2 ? B.cnt2[ci] : B.cell_cnt[ci];
-    // candidates k0 = 64*chunk + lane and k1 = k0 + 32 of the cell (phase 2:
-    // of its surviving candidates); items of at most 32 candidates run one
-    // per lane
-    const unsigned k0 = chunk * 64u + (unsigned)lane, k1 = k0 + 32u;
-    const bool two = cnt > chunk * 64u + 32u;
-    const bool have = k0 < cnt, have1 = k1 < cnt;
-    const unsigned coff = B.cell_off[ci];
-    const unsigned q = phase2 ? (have ? B.cand_list[coff + k0] : 0u) : coff + k0;
-    const unsigned q1 = phase2 ? (have1 ? B.cand_list[coff + k1] : 0u) : coff + k1;
-    const unsigned cp = have ? B.cand_pos[q] : 0u, cp1 = have1 ? B.cand_pos[q1] : 0u;
-    const bool quirk = have && K.has_quirk && cp == K.quirk_pos;
-    const bool quirk1 = have1 && K.has_quirk && cp1 == K.quirk_pos;
-    float cx = 0.f, cy = 0.f, cz = 0.f, bx = 1e18f, by = 1e18f, bz = 1e18f;
-    if (have) {
-      const float4 cv = B.cube[cp];
-      cx = to_grid(cv.x, K.nxf);
-      cy = to_grid(cv.y, K.nxf);
-      cz = to_grid(cv.z, K.nxf);
-    }
-    if (have1) {
-      const float4 cv = B.cube[cp1];
-      bx = to_grid(cv.x, K.nxf);
-      by = to_grid(cv.y, K.nxf);
-      bz = to_grid(cv.z, K.nxf);
-    }
-    {
-      // record runs of the 3x3x3 cells around the candidate cell: 9 rows of a
-      // 3-cell x-run each (two runs when it wraps), lane r < 9 on row r; a
-      // warp scan of the run counts and lengths places them in row order
-      int np = 0;
-      unsigned b0 = 0, l0 = 0, b1 = 0, l1 = 0;
-      if (lane < 9) {
-        const unsigned yy = (unsigned)wrapi(cyc + lane % 3 - 1, K.nx), zz = (unsigned)wrapi(czc + lane / 3 - 1, K.nx);
-        const unsigned long long base = (unsigned long long)K.nx * (yy + (unsigned long long)K.nx * zz);
-        const int x0 = cxc - 1, x1 = cxc + 1;
-        int pa0, pb0, pa1 = 0, pb1 = -1;
-        if (x0 < 0) { pa0 = x0 + K.nx; pb0 = K.nx - 1; pa1 = 0; pb1 = x1; np = 2; }
-        else if (x1 >= K.nx) { pa0 = x0; pb0 = K.nx - 1; pa1 = 0; pb1 = x1 - K.nx; np = 2; }
-        else { pa0 = x0; pb0 = x1; np = 1; }
-        b0 = B.cs[base + (unsigned)pa0];
-        l0 = B.cs[base + (unsigned)pb0 + 1] - b0;
-        if (np == 2) {
-          b1 = B.cs[base + (unsigned)pa1];
-          l1 = B.cs[base + (unsigned)pb1 + 1] - b1;
-        }
-      }
-      unsigned pc = (unsigned)np, len = l0 + l1;
-      for (int o = 1; o < 32; o <<= 1) {
-        const unsigned tp = __shfl_up_sync(0xffffffffu, pc, o), tl = __shfl_up_sync(0xffffffffu, len, o);
-        if (lane >= o) {
-          pc += tp;
-          len += tl;
-        }
-      }
-      if (lane < 9) {
-        const unsigned pf = pc - (unsigned)np, lf = len - (l0 + l1);
-        s_rb[w][pf] = b0;
-        s_rp[w][pf] = lf;
-        if (np == 2) {
-          s_rb[w][pf + 1] = b1;
-          s_rp[w][pf + 1] = lf + l0;
-        }
-      }
-      if (lane == 8) {
-        s_rp[w][pc] = len;
-        s_nr[w] = (int)pc;
-      }
-      if (lane == 0) {
-        // the 3-cell coordinate window of each axis stays clear of the box edge
-        auto clear = [&](int c, int a) {
-          double s0 = (double)(c - 1) + K.xs[a];
-          s0 -= K.tx * floor(s0 / K.tx);
-          return s0 >= 1.0 && s0 + 3.0 <= K.tx - 1.0;
-        };
-        s_wf[w] = clear(cxc, 0) && clear(cyc, 1) && clear(czc, 2);
-      }
-    }
-    __syncwarp();
-    const int nr = s_nr[w];
-    const unsigned total = s_rp[w][nr];
-    const bool wf = s_wf[w];
-    const bool active = have && !quirk, active1 = have1 && !quirk1;
-    // bounding box of the item's candidates: records farther than 1 from it
-    // in every direction meet no candidate (wrap-free items only)
-    float lox = active ? cx : 3e38f, hix = active ? cx : -3e38f, loy = active ? cy : 3e38f,
-          hiy = active ? cy : -3e38f, loz = active ? cz : 3e38f, hiz = active ? cz : -3e38f;
-    if (active1) {
-      lox = fminf(lox, bx);
-      hix = fmaxf(hix, bx);
-      loy = fminf(loy, by);
-      hiy = fmaxf(hiy, by);
-      loz = fminf(loz, bz);
-      hiz = fmaxf(hiz, bz);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-      lox = fminf(lox, __shfl_xor_sync(0xffffffffu, lox, o));
-      hix = fmaxf(hix, __shfl_xor_sync(0xffffffffu, hix, o));
-      loy = fminf(loy, __shfl_xor_sync(0xffffffffu, loy, o));
-      hiy = fmaxf(hiy, __shfl_xor_sync(0xffffffffu, hiy, o));
-      loz = fminf(loz, __shfl_xor_sync(0xffffffffu, loz, o));
-      hiz = fmaxf(hiz, __shfl_xor_sync(0xffffffffu, hiz, o));
-    }
-    const bool any_active = lox <= hix;
-    const unsigned r0 = nchunk * RN_CHUNK, r1 = any_active ? min(total, r0 + RN_CHUNK) : r0;
-    const unsigned lt = (1u << lane) - 1u;
-    double sum = 0.0, sum1 = 0.0;
-    unsigned visits = 0, slots = 0, loaded = 0;
-    // tile of 32 kept records: the pair tests of every candidate lane
-    float uf = 0.f;  // BOUND: this lane's far records
-    const float e2b = (float)K.eps2;
-    auto consume = [&](unsigned nt) {
-      // pad to a multiple of 8 with records far from every candidate
-      if ((unsigned)lane < ((8u - (nt & 7u)) & 7u)) {
-        s_tile[w].x[nt + lane] = 1e18f;
-        s_tile[w].y[nt + lane] = 1e18f;
-        s_tile[w].z[nt + lane] = 1e18f;
-      }
-      __syncwarp();
-      if (two) {
-        if (active || active1) {
-          if (wf) tile_terms2<true>(s_tile[w], nt, cx, cy, cz, bx, by, bz, K, sum, sum1);
-          else tile_terms2<false>(s_tile[w], nt, cx, cy, cz, bx, by, bz, K, sum, sum1);
-        }
-      } else if (active) {
-        sum += wf ? tile_terms<true>(s_tile[w], nt, cx, cy, cz, K) : tile_terms<false>(s_tile[w], nt, cx, cy, cz, K);
-      }
-      if (lane == 0) {
-        visits += min(64u, cnt - chunk * 64u) * nt;
-        slots += (two ? 64u : 32u) * ((nt + 7u) & ~7u);
-      }
-      __syncwarp();
-    };
-    // Stage the chunk's records run by run, lanes on consecutive records of
-    // one run.  Only alive records within reach of the candidates' box are
-    // kept (warp-wide compaction into a 64-entry buffer); each full tile of
-    // 32 is consumed at once and the overflow moves to the front, so no
-    // record is loaded twice.
-    unsigned fill = 0;
-    int r = 0;
-    while (r + 1 < nr && s_rp[w][r + 1] <= r0) r++;
-    // (items near the periodic edge have no box filter: their bound is
-    // infinite and they are not staged by the bound pass)
-    for (unsigned pos = (BOUND && !wf) ? r1 : r0; pos < r1; r++) {
-      const unsigned run_end = min(s_rp[w][r + 1], r1);
-      const unsigned base = s_rb[w][r] - s_rp[w][r];  // cube slot = base + record number
-      // SD steps of 32 records per pass: each lane issues its SD loads
-      // before the first is used.  Both passes run best with one (measured
-      // at 1024^3: with its exact near-field tiles the bound pass needs the
-      // registers more than the loads in flight; four took it from 325 to
-      // 603 ms through spills).
-      constexpr int SD = 1;
-      for (unsigned xs0 = pos; xs0 < run_end; xs0 += 32u * SD) {
-        float4 vs[SD];
-#pragma unroll
-        for (int u = 0; u < SD; u++) {
-          const unsigned x = xs0 + 32u * (unsigned)u + (unsigned)lane;
-          vs[u] = x < run_end ? B.cube[base + x] : make_float4(0.f, 0.f, 0.f, 0.f);
-        }
-#pragma unroll
-        for (int u = 0; u < SD; u++) {
-          const unsigned x0 = xs0 + 32u * (unsigned)u;
-          if (x0 >= run_end) break;  // warp-uniform
-          const unsigned x = x0 + (unsigned)lane;
-          bool keep = false;
-          float4 rec = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (x < run_end) {
-            const float4 v = vs[u];
-            rec = make_float4(to_grid(v.x, K.nxf), to_grid(v.y, K.nxf), to_grid(v.z, K.nxf), 0.f);
-            keep = !(__float_as_uint(v.w) & PSOD_DEAD_BIT);
-            if (wf) {
-              const float ex = fmaxf(fmaxf(lox - rec.x, rec.x - hix), 0.f), ey = fmaxf(fmaxf(loy - rec.y, rec.y - hiy), 0.f),
-                          ez = fmaxf(fmaxf(loz - rec.z, rec.z - hiz), 0.f);
-              const float db2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-              if (BOUND) {
-                // far records add k(d to the group's box) to every
-                // candidate here; near ones go to the tile for exact sums
-                if (keep && db2 >= NEAR2 && db2 <= 1.0001f) uf += rsqrt_pos(db2 + e2b);
-                keep = keep && db2 < NEAR2;
-              } else {
-                keep = keep && db2 <= 1.0001f;
-              }
-            }
-          }
-          const unsigned m = __ballot_sync(0xffffffffu, keep);
-          if (keep) {  // fill < 32: index < 64
-            const unsigned at = fill + __popc(m & lt);
-            s_tile[w].x[at] = rec.x;
-            s_tile[w].y[at] = rec.y;
-            s_tile[w].z[at] = rec.z;
-          }
-          fill += (unsigned)__popc(m);
-          if (!BOUND) loaded += min(32u, run_end - x0);
-          if (fill >= 32u) {
-            consume(32u);
-            if ((unsigned)lane < fill - 32u) {
-              s_tile[w].x[lane] = s_tile[w].x[32 + lane];
-              s_tile[w].y[lane] = s_tile[w].y[32 + lane];
-              s_tile[w].z[lane] = s_tile[w].z[32 + lane];
-            }
-            __syncwarp();
-            fill -= 32u;
-          }
-        }
-      }
-      pos = run_end;
-    }
-    if (fill > 0) consume(fill);
-    if (BOUND) {
-      for (int sh = 16; sh > 0; sh >>= 1) uf += __shfl_xor_sync(0xffffffffu, uf, sh);
-      // the particle the run scan files under another cell may add up to
-      // 1/eps = 64 to any candidate's sum outside these runs; a candidate
-      // that is the run scan's own quirk particle gets no bound (it always
-      // stays in the exact pass), nor do items near the periodic edge
-      const float extra = (K.has_quirk && nchunk == 0) ? 64.f : 0.f;
-      const float inf = __int_as_float(0x7f800000);
-      if (have) atomicAdd(&B.cand_u[q], (wf && !quirk) ? (float)((sum + (double)uf) * 1.001) + extra : inf);
-      if (have1) atomicAdd(&B.cand_u[q1], (wf && !quirk1) ? (float)((sum1 + (double)uf) * 1.001) + extra : inf);
-    }
-    if (lane == 0) {
-      s_count[w][0] += visits;
-      s_count[w][1] += slots;
-      s_count[w][2] += loaded;
-    }
-    if (BOUND) continue;
-    if (nchunk == 0 && K.has_quirk && (active || active1)) {
-      // the particle the run scan files under another cell: counted if that
-      // cell is in x_sel2 but outside this candidate cell's 27 neighbours
-      const int ax = (int)(K.quirk_listed % K.nx), ay = (int)((K.quirk_listed / K.nx) % K.nx),
-                az = (int)(K.quirk_listed / ((unsigned)K.nx * K.nx));
-      const bool listed_in_sel2 = in_sel2(K, ax, ay, az, g.ic, g.jc, g.kc);
-      const bool seen = abs(pdiff(ax, cxc, K.nx)) <= 1 && abs(pdiff(ay, cyc, K.nx)) <= 1 && abs(pdiff(az, czc, K.nx)) <= 1;
-      if (listed_in_sel2 && !seen) {
-        const float4 qv = B.cube[K.quirk_pos];
-        if (!(__float_as_uint(qv.w) & PSOD_DEAD_BIT)) {
-          const double qx = to_grid(qv.x, K.nxf), qy = to_grid(qv.y, K.nxf), qz = to_grid(qv.z, K.nxf);
-          if (active) {
-            const double d2 = min_image_d2(qx, qy, qz, (double)cx, (double)cy, (double)cz, K.tx);
-            if (d2 <= K.rmin2) sum += ddiv(1.0, dsqrt(dadd(d2, K.eps2)));
-          }
-          if (active1) {
-            const double d2 = min_image_d2(qx, qy, qz, (double)bx, (double)by, (double)bz, K.tx);
-            if (d2 <= K.rmin2) sum1 += ddiv(1.0, dsqrt(dadd(d2, K.eps2)));
-          }
-        }
-      }
-    }
-    if (active && sum != 0.0) atomicAdd(&B.cand_s[q], sum);
-    if (active1 && sum1 != 0.0) atomicAdd(&B.cand_s[q1], sum1);
+    refine_item<BOUND>(K, B, ci, rem, phase2, R);
   }
   if (lane == 0) {
-    if (s_count[w][0]) atomicAdd(B.pairs, s_count[w][0]);
-    if (s_count[w][1]) atomicAdd(B.pair_slots, s_count[w][1]);
-    if (s_count[w][2]) atomicAdd(B.pair_slots + 1, s_count[w][2]);
-    if (!BOUND && s_count[w][3]) atomicAdd(B.pair_slots + 6, s_count[w][3]);
+    if (R.count[0]) atomicAdd(B.pairs, R.count[0]);
+    if (R.count[1]) atomicAdd(B.pair_slots, R.count[1]);
+    if (R.count[2]) atomicAdd(B.pair_slots + 1, R.count[2]);
+    if (!BOUND && R.count[3]) atomicAdd(B.pair_slots + 6, R.count[3]);
   }
 }
 
@@ -3378,9 +3395,20 @@ __device__ __forceinline__ void small_seed(const SodConst &K, const SodBufs &B, 
   __syncthreads();
   const unsigned ncand = s_ncand;
   if (nlist > (unsigned)NB || ncand > B.max_cand) {
-    // more than shared memory holds (or the loop's limit): the host's rounds
-    put_back();
-    if (t == 0) atomicOr(B.deferred, 1u);
+    // more records than shared memory holds: the whole grid refines the seed
+    // after this step; more candidates than the loop takes: the host's rounds
+    if (t == 0) {
+      s_work = LOOP_BIG;
+      if (ncand <= B.max_cand) s_work = atomicAdd(B.nbigq, 1u);
+    }
+    __syncthreads();
+    if (s_work < LOOP_BIG) {
+      if (t == 0) B.bigq[s_work] = slot;
+      prep_seed(K, B, S, slot, rank);
+    } else {
+      put_back();
+      if (t == 0) atomicOr(B.deferred, 1u);
+    }
     return;
   }
   if (t == 0) atomicAdd(B.nprocessed, 1ull);
@@ -3582,15 +3610,19 @@ enum : unsigned { TAIL_RUNNING = 0, TAIL_DONE = 1, TAIL_DEFERRED = 2, TAIL_STALL
 
 struct TailState {
   unsigned nact[2];       // active-block count of list act[p]
-  unsigned nready[2];     // per round parity
-  unsigned work[2];       // work counter of the seed step
-  unsigned gmin[2];
+  unsigned gmin[2];       // per round parity
+  // this round's counters, reset in its heads step (the previous round's last
+  // barrier is behind every reader); the kernel's SodBufs point at them
+  unsigned nready;
+  unsigned work;          // work counter of the seed step
+  unsigned cand_used;     // candidate buffer of the grid-refined seeds
+  unsigned nbigq, bigq[LOOP_BIG];
+  unsigned long long xused;
   unsigned deferred;
   unsigned status;
   unsigned rounds;        // rounds completed by the launch
   unsigned parity;        // parity of the next round (its live list is act[parity])
   unsigned bar_count, bar_gen;
-  unsigned long long xused[2];
   // time spent by the launch in each step (ns, block 0's clock, each step
   // up to the barrier that ends it)
   unsigned long long t_heads, t_ready, t_seeds;
@@ -3642,7 +3674,70 @@ __device__ bool grid_barrier(TailState *ts) {
 // value written by another CTA before the last barrier
 __device__ __forceinline__ unsigned ld_shared_state(const unsigned *p) { return *(volatile const unsigned *)p; }
 
-__global__ void __launch_bounds__(LOOP_TPB, 1) k_tail_rounds(SodConst K, SodBufs B, TailState *ts, unsigned *act0,
+// The refinement items of the seeds whose records exceed a CTA's list, over
+// the grid's warps, then a CTA per seed from the exact sums on.  A function of
+// its own, so that its registers are not the one-CTA path's.
+__device__ __noinline__ bool big_seeds(const SodConst &K, const SodBufs &B, Smem &S, TailState *ts, unsigned nbig) {
+  const int lane = threadIdx.x & 31;
+  const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
+  const int w = threadIdx.x >> 5;
+  static_assert(27 * LOOP_BIG <= 4 * LOOP_TPB && 4 * LOOP_TPB <= NB, "item prefix: four cells a thread");
+  unsigned v[4], sum = 0;
+  for (int k = 0; k < 4; k++) {
+    const unsigned e = 4u * threadIdx.x + (unsigned)k;
+    v[k] = 0;
+    if (e < 27u * nbig) {
+      const unsigned slot = B.bigq[e / 27u];
+      if (B.st_active[slot]) v[k] = B.cell_chunks[slot * 27u + e % 27u];
+    }
+    sum += v[k];
+  }
+  unsigned inc = sum;
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += y;
+  }
+  if (lane == 31) S.red_u32[w] = inc;
+  __syncthreads();
+  unsigned at = inc - sum, nitem = 0;
+  for (int k = 0; k < nwarp(); k++) {
+    if (k < w) at += S.red_u32[k];
+    nitem += S.red_u32[k];
+  }
+  for (int k = 0; k < 4; k++) {
+    S.pref[4u * threadIdx.x + (unsigned)k] = at;
+    at += v[k];
+  }
+  static_assert(sizeof(WarpRef) * MAX_WARP <= sizeof(unsigned) * MAXLEV * NB, "staging over the histograms");
+  WarpRef &R = reinterpret_cast<WarpRef *>(S.hist)[w];
+  __syncthreads();
+  for (unsigned it = gtid >> 5; it < nitem; it += gthreads >> 5) {
+    unsigned lo = 0, hi = 27u * nbig;  // last cell whose prefix is <= it
+    while (hi - lo > 1) {
+      const unsigned mid = (lo + hi) >> 1;
+      if (S.pref[mid] <= it) lo = mid;
+      else hi = mid;
+    }
+    refine_item<false>(K, B, B.bigq[lo / 27u] * 27u + lo % 27u, it - S.pref[lo], false, R);
+    __syncwarp();
+  }
+  if (!grid_barrier(ts)) return false;
+  for (unsigned k = blockIdx.x; k < nbig; k += gridDim.x) {
+    __syncthreads();
+    const unsigned slot = B.bigq[k];
+    if (!B.st_active[slot]) continue;
+    const unsigned rank = B.ready[slot];
+    select_seed(K, B, S, slot, rank);
+    __syncthreads();
+    if (B.learn_collect) seed_features(K, B, S, slot, rank);
+    __syncthreads();
+    cross_seed(K, B, S, slot, rank, seed_geo(K, B, rank), B.st_na[slot], B.st_centre[slot]);
+  }
+  return grid_barrier(ts);
+}
+
+__global__ void __launch_bounds__(LOOP_TPB, 1) k_tail_rounds(const __grid_constant__ SodConst K,
+                                                                const __grid_constant__ SodBufs B, TailState *ts, unsigned *act0,
                                                     unsigned *act1, const unsigned *bbegin, unsigned *cursor,
                                                     const unsigned *blist, unsigned *head, int nb, int rb,
                                                     unsigned quirk_rank, unsigned *ready) {
@@ -3662,6 +3757,13 @@ __global__ void __launch_bounds__(LOOP_TPB, 1) k_tail_rounds(SodConst K, SodBufs
     const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
     unsigned long long tk = timer ? global_ns() : 0ull;
     unsigned *cur = q ? act1 : act0, *nxt = q ? act0 : act1;
+    if (timer) {
+      ts->nready = 0;
+      ts->work = 0;
+      ts->cand_used = 0;
+      ts->nbigq = 0;
+      ts->xused = 0;
+    }
     // heads (k_heads): warp-uniform strides over the active list
     for (unsigned base = gtid - (unsigned)lane; base < cnt; base += gthreads) {
       const unsigned i = base + (unsigned)lane;
@@ -3693,13 +3795,10 @@ __global__ void __launch_bounds__(LOOP_TPB, 1) k_tail_rounds(SodConst K, SodBufs
       ts->t_heads += now - tk;
       tk = now;
     }
-    // the next round's counters (parity q^1) are free now: reset them
+    // the next round's counts (parity q^1) are free now: reset them
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       ts->nact[q] = 0;
       ts->gmin[q ^ 1u] = PSOD_INF_RANK;
-      ts->nready[q ^ 1u] = 0;
-      ts->work[q ^ 1u] = 0;
-      ts->xused[q ^ 1u] = 0;
     }
     if (threadIdx.x == 0) s_next = ld_shared_state(&ts->nact[q ^ 1u]);
     __syncthreads();
@@ -3708,14 +3807,14 @@ __global__ void __launch_bounds__(LOOP_TPB, 1) k_tail_rounds(SodConst K, SodBufs
     // readiness: the direct window test (the launch is used only while few
     // blocks are active), a warp per active block
     for (unsigned wi = gtid >> 5; wi < next; wi += gthreads >> 5)
-      ready_test_warp(nxt[wi], head, nb, rb, quirk_rank, gmin, ready, &ts->nready[q], B.cap_ready);
+      ready_test_warp(nxt[wi], head, nb, rb, quirk_rank, gmin, ready, &ts->nready, B.cap_ready);
     if (!grid_barrier(ts)) return;
     if (timer) {
       const unsigned long long now = global_ns();
       ts->t_ready += now - tk;
       tk = now;
     }
-    if (threadIdx.x == 0) s_nready = ld_shared_state(&ts->nready[q]);
+    if (threadIdx.x == 0) s_nready = ld_shared_state(&ts->nready);
     __syncthreads();
     const unsigned nready = min(s_nready, B.cap_ready);
     if (nready == 0) {
@@ -3729,18 +3828,16 @@ __global__ void __launch_bounds__(LOOP_TPB, 1) k_tail_rounds(SodConst K, SodBufs
     }
     // the round's seeds, a CTA each from the preselect to the claims: ready
     // seeds share no particle, so nothing is waited for in between
-    SodBufs Br = B;
-    Br.nready = &ts->nready[q];
-    Br.xused = &ts->xused[q];
-    Br.deferred = &ts->deferred;
-    Br.maxcand = nullptr;
-    Br.learn_use = 0;
     while (true) {
-      const unsigned item = next_item(&ts->work[q]);
+      const unsigned item = next_item(&ts->work);
       if (item >= nready) break;
-      small_seed(K, Br, S, item, B.ready[item]);
+      small_seed(K, B, S, item, B.ready[item]);
     }
     if (!grid_barrier(ts)) return;
+    if (threadIdx.x == 0) s_cnt = ld_shared_state(&ts->nbigq);
+    __syncthreads();
+    const unsigned nbig = min(s_cnt, LOOP_BIG);
+    if (nbig > 0 && !big_seeds(K, B, S, ts, nbig)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       ts->rounds++;
       ts->parity = q ^ 1u;
@@ -3759,10 +3856,7 @@ __global__ void __launch_bounds__(LOOP_TPB, 1) k_tail_rounds(SodConst K, SodBufs
 __global__ void k_tail_init(TailState *ts, unsigned n_active) {
   ts->nact[0] = n_active;
   ts->nact[1] = 0;
-  ts->nready[0] = ts->nready[1] = 0;
-  ts->work[0] = ts->work[1] = 0;
   ts->gmin[0] = ts->gmin[1] = PSOD_INF_RANK;
-  ts->xused[0] = ts->xused[1] = 0;
   ts->deferred = 0;
   ts->status = TAIL_RUNNING;
   ts->rounds = 0;
@@ -4245,6 +4339,8 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
   B.maxcand = ctrs + 13;
   B.max_cand = ~0u;
   B.deferred = ctrs + 14;
+  B.rn_chunk = RN_CHUNK;
+  B.bigq = B.nbigq = nullptr;
   B.alive_cnt = nullptr;
   B.pairs = u64s + 5;
   B.touch = u64s + 7;
@@ -4489,6 +4585,15 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
       k_tail_init<<<1, 1, 0, c->stream>>>(tail, n_active);
       SodBufs Bt = B;
       Bt.max_cand = (unsigned)std::min<long long>(LOOP_CAND * c->tune.tail_max_cand, NB);
+      Bt.rn_chunk = LOOP_CHUNK;
+      Bt.nready = &tail->nready;
+      Bt.cand_used = &tail->cand_used;
+      Bt.nbigq = &tail->nbigq;
+      Bt.bigq = tail->bigq;
+      Bt.xused = &tail->xused;
+      Bt.deferred = &tail->deferred;
+      Bt.maxcand = nullptr;
+      Bt.learn_use = 0;
       Bt.st_big = nullptr;
       Bt.touch = u64s + 19;  // the tail's crossings counted apart from k_cross
       Bt.kept_members = u64s + 20;
