@@ -296,7 +296,7 @@ enum : int {
   SLOT_HOST_POS = 87,   // load: device copy of host positions
   SLOT_VEL = 88,        // load: velocities
   SLOT_SEED_IDX = 89,   // tri_cic: seed order (persistent)
-  SLOT_OUT_IDX = 90,    // psod_get_halos: member indices staged for a host copy
+  SLOT_OUT_IDX = 90,    // member indices (psod_get_halos), seed order (tri_cic) staged for a host copy
   SLOT_OUT_ID = 91,     // psod_get_halos: member IDs staged for a host copy
   SLOT_H_ID = 92,       // halo table (persistent until the next SOD call)
   SLOT_H_MASS,

@@ -430,18 +430,27 @@ __global__ void k_cic_interp(const float4 *cube, long long n, CicConst k, const 
   rho[idx] = r;
 }
 
-// Tile-fused CIC: one CTA owns CT^3 SOD cells.  It deposits the particles
-// of those cells and of a one-cell halo into a shared-memory window of
-// fixed-point nodes, then interpolates rho for its own particles.  Every
-// node the own particles read receives all its contributions inside the
-// window, so the integer node sums, and therefore rho, equal the global
-// grid's exactly.  Needs each particle's CIC cell to be one of the two fine
-// cells of its SOD cell (true when nx is a power of two); a particle that
-// breaks this sets *bad and the caller falls back to the global grid.
-constexpr int CT = 8;                 // SOD cells per tile side
-constexpr int CW = 2 * (CT + 2) + 1;  // window nodes per side
+// Tile-fused CIC: one CTA owns a tile of up to CT^3 SOD cells, its fine cells
+// [0, w) per axis (w = twice its cells).  It deposits into a shared-memory
+// window of nodes [0, w] every particle that touches them -- those of the
+// tile and of the adjacent fine cells, all filed in the tile's cells and a
+// one-cell halo -- then interpolates rho for the particles of its fine cells.
+// Every node they read receives all its contributions inside the window, so
+// the integer node sums, and therefore rho, equal the global grid's exactly.
+//
+// Bound: latency inside a tile (a tile of a mean-density box holds 512
+// particles: the range look-ups, the barriers and the shared atomics are its
+// time, not HBM and not FP64), so what counts is how many tiles an SM holds
+// and how few steps one takes.  A window of 17^3 nodes, not of the whole halo's
+// 21^3, lets five CTAs run instead of three and drops 27 % of the deposits; a
+// tile of at most SPLIT_MAX particles adds each weight as two 20-bit halves
+// with 32-bit atomics that return nothing; a tile without particles leaves at
+// once.  CIC_MS.
+constexpr int CT = 8;             // SOD cells per tile side
+constexpr int CW = 2 * CT + 1;    // window nodes per side
 constexpr int CW3 = CW * CW * CW;
-constexpr unsigned DEP_BATCH = 4;    // record loads in flight per thread in the deposit
+constexpr unsigned DEP_BATCH = 4;     // record loads in flight per thread in the deposit
+constexpr unsigned SPLIT_MAX = 4095;  // particles whose 20-bit halves a 32-bit sum holds
 
 constexpr int CRNG = 2 * (CT + 2) * (CT + 2);  // record ranges of a tile plus halo (two where x wraps)
 
@@ -465,52 +474,133 @@ __device__ __forceinline__ void range_prefix(const unsigned *s_len, unsigned *s_
 }
 
 // ZONE: particles outside the zone with buffer are skipped (zone contexts;
-// the test costs registers, so one-zone contexts run without it)
-template <bool ZONE>
-__global__ void __launch_bounds__(256) k_cic_tile(const float4 *cube, const unsigned *cs, int nx, double3 xs, CicConst k,
-                                                  double *rho, int *bad, unsigned quirk_pos) {
+// the test costs registers, so one-zone contexts run without it).
+// RAGGED: nx is not a power of two (or the zone's corner no multiple of the
+// cell), so a particle at a cell edge may be filed, by the rounding of its
+// grid coordinate, in the cell beside the one its CIC coordinate lies in.  The
+// tile holding its fine cell interpolates it, whatever cell lists it: every
+// loaded record is looked at, not only those of the tile's own cells.
+template <bool ZONE, bool RAGGED>
+__global__ void __launch_bounds__(256, 4) k_cic_tile(const float4 *cube, const unsigned *cs, int nx, CicConst k,
+                                                     double *rho, int *bad, unsigned quirk_pos) {
   extern __shared__ __align__(16) unsigned long long win[];
+  unsigned *win32 = reinterpret_cast<unsigned *>(win);  // split sums: [low 20 bits | high 20 bits] of CW3 each
   __shared__ unsigned s_rb[CRNG], s_len[CRNG], s_pre[CRNG + 1];
-  const int ntile = nx / CT;
-  const int tx = blockIdx.x % ntile, ty = (blockIdx.x / ntile) % ntile, tz = blockIdx.x / (ntile * ntile);
-  const int x0 = tx * CT, y0 = ty * CT, z0 = tz * CT;
-  const int nc = k.nc;  // 2*nx fine cells
-  const float nxf = (float)nx;
-  for (int i = threadIdx.x; i < CW3; i += blockDim.x) win[i] = 0ull;
-  auto widx = [&](int f, int o) {  // fine index -> window offset (periodic)
+  const int ntile = (nx + CT - 1) / CT;
+  const int x0 = (int)(blockIdx.x % (unsigned)ntile) * CT, y0 = (int)((blockIdx.x / (unsigned)ntile) % (unsigned)ntile) * CT,
+            z0 = (int)(blockIdx.x / (unsigned)(ntile * ntile)) * CT;
+  const int xe = min(x0 + CT, nx), ye = min(y0 + CT, nx), ze = min(z0 + CT, nx);
+  const int wx_ = 2 * (xe - x0), wy_ = 2 * (ye - y0), wz_ = 2 * (ze - z0);  // fine cells; nodes 0..w
+  const int nc = k.nc;
+  const int ox = 2 * x0, oy = 2 * y0, oz = 2 * z0;
+  auto rel = [&](int f, int o) {  // fine index from the tile's first, in [-1, nc - 2]
     int d = f - o;
-    if (d < 0) d += nc;
-    if (d >= nc) d -= nc;
+    if (d < -1) d += nc;
+    if (d > nc - 2) d -= nc;
     return d;
   };
-  const int ox = 2 * (x0 - 1), oy = 2 * (y0 - 1), oz = 2 * (z0 - 1);
+  struct Pt {
+    int fx, fy, fz;      // fine cell relative to the tile
+    double wx[2], wy[2], wz[2];
+  };
+  auto locate = [&](const float4 &v, Pt &q) {
+    int i0, i1;
+    cic_axis(v.x, k, 0, i0, i1, q.wx[1], q.wx[0]);
+    q.fx = rel(i0, ox);
+    cic_axis(v.y, k, 1, i0, i1, q.wy[1], q.wy[0]);
+    q.fy = rel(i0, oy);
+    cic_axis(v.z, k, 2, i0, i1, q.wz[1], q.wz[0]);
+    q.fz = rel(i0, oz);
+  };
+  const bool has_q = quirk_pos != 0xffffffffu;
+  // the tile's own records; without any (and without the quirk particle,
+  // which another cell's run may hold) there is nothing to do
+  unsigned own = 0;
+  for (int row = threadIdx.x; row < (ye - y0) * (ze - z0); row += blockDim.x) {
+    const int yy = y0 + row % (ye - y0), zz = z0 + row / (ye - y0);
+    const unsigned long long base = (unsigned long long)nx * ((unsigned)yy + (unsigned long long)nx * (unsigned)zz);
+    const unsigned rb = cs[base + (unsigned)x0];
+    unsigned len = cs[base + (unsigned)xe] - rb;
+    if (len && rb + len - 1u == quirk_pos) len--;  // handled below, by its own fine cell
+    own += len;
+  }
+  // (a ragged tile may interpolate records filed beside it: its halo counts)
+  if (!RAGGED && !has_q && !__syncthreads_or(own != 0)) return;
   // record ranges of the rows of the tile plus halo; the particles are then
   // dealt to all threads of the CTA evenly, whatever their spread over rows
-  for (int row = threadIdx.x; row < (CT + 2) * (CT + 2); row += blockDim.x) {
-    const int yy = (y0 - 1 + row % (CT + 2) + nx) % nx, zz = (z0 - 1 + row / (CT + 2) + nx) % nx;
-    const unsigned long long base = (unsigned long long)nx * ((unsigned)yy + (unsigned long long)nx * (unsigned)zz);
-    const int xa = x0 - 1, xb = x0 + CT;  // inclusive, may wrap
-    int pa[2] = {0, 0}, pb[2] = {-1, -1};
-    if (xa < 0) { pa[0] = xa + nx; pb[0] = nx - 1; pa[1] = 0; pb[1] = xb; }
-    else if (xb >= nx) { pa[0] = xa; pb[0] = nx - 1; pa[1] = 0; pb[1] = xb - nx; }
-    else { pa[0] = xa; pb[0] = xb; }
+  const int ny = ye - y0 + 2, nrow = ny * (ze - z0 + 2);
+  unsigned any = 0;
+  for (int row = threadIdx.x; row < CRNG / 2; row += blockDim.x) {
+    unsigned rb[2] = {0, 0}, len[2] = {0, 0};
+    if (row < nrow) {
+      const int yy = (y0 - 1 + row % ny + nx) % nx, zz = (z0 - 1 + row / ny + nx) % nx;
+      const unsigned long long base = (unsigned long long)nx * ((unsigned)yy + (unsigned long long)nx * (unsigned)zz);
+      const int xa = x0 - 1, xb = xe;  // inclusive, may wrap
+      int pa[2] = {0, 0}, pb[2] = {-1, -1};
+      if (xa < 0) { pa[0] = xa + nx; pb[0] = nx - 1; pa[1] = 0; pb[1] = xb; }
+      else if (xb >= nx) { pa[0] = xa; pb[0] = nx - 1; pa[1] = 0; pb[1] = xb - nx; }
+      else { pa[0] = xa; pb[0] = xb; }
+      for (int q = 0; q < 2; q++)
+        if (pb[q] >= pa[q]) {
+          rb[q] = cs[base + (unsigned)pa[q]];
+          len[q] = cs[base + (unsigned)pb[q] + 1] - rb[q];
+          // the quirk particle is the cube's last record, at the end of its listed cell's run
+          if (len[q] && rb[q] + len[q] - 1u == quirk_pos) len[q]--;
+        }
+    }
     for (int q = 0; q < 2; q++) {
-      unsigned rb = 0, len = 0;
-      if (pb[q] >= pa[q]) {
-        rb = cs[base + (unsigned)pa[q]];
-        len = cs[base + (unsigned)pb[q] + 1] - rb;
-        // the quirk particle (the cube's last record, at the end of its
-        // listed cell's run) is deposited below from its own cell
-        if (len && rb + len - 1u == quirk_pos) len--;
-      }
-      s_rb[2 * row + q] = rb;
-      s_len[2 * row + q] = len;
+      s_rb[2 * row + q] = rb[q];
+      s_len[2 * row + q] = len[q];
+      any |= len[q];
     }
   }
-  __syncthreads();
+  if (!__syncthreads_or(any != 0) && !has_q) return;
+  for (int i = threadIdx.x; i < CW3; i += blockDim.x) win[i] = 0ull;
   range_prefix(s_len, s_pre, CRNG);
   __syncthreads();
-  {
+  const unsigned total = s_pre[CRNG];
+  const bool split = total < SPLIT_MAX;  // the quirk particle makes one more
+  // quantised weight: (w 2^40) rounded to an integer; 2^40 goes into one axis
+  // weight (an exact scaling), and adding 1.5 2^52 leaves the rounded integer
+  // in the low bits
+  auto quant = [&](double w) {
+    return (unsigned long long)(__double_as_longlong(dadd(w, 6755399441055744.0)) - 0x4338000000000000ll);
+  };
+  auto node = [&](const Pt &q, int c) { return (q.fx + (c & 1)) + CW * ((q.fy + ((c >> 1) & 1)) + CW * (q.fz + (c >> 2))); };
+  auto touches = [&](const Pt &q, int c) {
+    const int a = q.fx + (c & 1), b = q.fy + ((c >> 1) & 1), e = q.fz + (c >> 2);
+    return a >= 0 && a <= wx_ && b >= 0 && b <= wy_ && e >= 0 && e <= wz_;
+  };
+  auto deposit_split = [&](const float4 &v) {
+    if (ZONE && !in_cic_zone(v, k)) return;
+    Pt q;
+    locate(v, q);
+    if (q.fx > wx_ || q.fy > wy_ || q.fz > wz_) return;
+    const double wx[2] = {dmul(q.wx[0], FIX_ONE), dmul(q.wx[1], FIX_ONE)};
+#pragma unroll
+    for (int c = 0; c < 8; c++) {
+      if (!touches(q, c)) continue;
+      const unsigned long long w = quant(dmul(dmul(wx[c & 1], q.wy[(c >> 1) & 1]), q.wz[c >> 2]));
+      const int at = node(q, c);
+      atomicAdd(&win32[at], (unsigned)w & 0xfffffu);
+      atomicAdd(&win32[CW3 + at], (unsigned)(w >> 20));
+    }
+  };
+  if (split) {
+    int r = 0;
+    for (unsigned f = threadIdx.x; f < total; f += 2 * blockDim.x) {
+      const unsigned g = f + blockDim.x;
+      while (s_pre[r + 1] <= f) r++;
+      const float4 va = cube[s_rb[r] + (f - s_pre[r])];
+      float4 vb = va;
+      if (g < total) {
+        while (s_pre[r + 1] <= g) r++;
+        vb = cube[s_rb[r] + (g - s_pre[r])];
+      }
+      deposit_split(va);
+      if (g < total) deposit_split(vb);
+    }
+  } else {
     // Each thread deposits one contiguous share of the tile's particles
     // (all threads busy, whatever the tile's count).  Dense cells are
     // sub-cell ordered, so consecutive particles mostly share a fine cell
@@ -518,7 +608,6 @@ __global__ void __launch_bounds__(256) k_cic_tile(const float4 *cube, const unsi
     // written with one atomic per node when the fine cell changes (integer
     // sums, so the grid is the same).  Records are loaded DEP_BATCH at a
     // time before any is used.
-    const unsigned total = s_pre[CRNG];
     const unsigned per = (total + blockDim.x - 1) / blockDim.x;
     const unsigned f0 = min(total, threadIdx.x * per), f1 = min(total, f0 + per);
     int r = 0;  // last range with s_pre[r] <= f0
@@ -531,17 +620,14 @@ __global__ void __launch_bounds__(256) k_cic_tile(const float4 *cube, const unsi
       }
     }
     unsigned long long acc[8];
-    int kx = -1, ky = -1, kz = -1;  // fine cell of the accumulated run
-    int ncx[2], ncy[2], ncz[2];     // its nodes' window offsets
+    Pt run;  // fine cell of the accumulated run
+    run.fx = -2;
     auto flush = [&]() {
-      if (kx < 0) return;
+      if (run.fx < -1) return;
 #pragma unroll
-      for (int c = 0; c < 8; c++) {
-        const int a = c & 1, bb = (c >> 1) & 1, ee = c >> 2;
-        if (ncx[a] < CW && ncy[bb] < CW && ncz[ee] < CW && acc[c])
-          atomicAdd(&win[ncx[a] + CW * (ncy[bb] + CW * ncz[ee])], acc[c]);
-      }
-      kx = -1;
+      for (int c = 0; c < 8; c++)
+        if (touches(run, c) && acc[c]) atomicAdd(&win[node(run, c)], acc[c]);
+      run.fx = -2;
     };
     for (unsigned fb = f0; fb < f1; fb += DEP_BATCH) {
       float4 vb[DEP_BATCH];
@@ -556,143 +642,113 @@ __global__ void __launch_bounds__(256) k_cic_tile(const float4 *cube, const unsi
 #pragma unroll
       for (unsigned u = 0; u < DEP_BATCH; u++) {
         if (fb + u >= f1) break;
-        const float4 v = vb[u];
-        int ix, ixp, iy, iyp, iz, izp;
-        double ddx, dex, ddy, dey, ddz, dez;
-        cic_axis(v.x, k, 0, ix, ixp, ddx, dex);
-        cic_axis(v.y, k, 1, iy, iyp, ddy, dey);
-        cic_axis(v.z, k, 2, iz, izp, ddz, dez);
-        if (ZONE && !in_cic_zone(v, k)) continue;
-        const int sx = sod_cell_axis(to_grid(v.x, nxf), xs.x, nx), sy = sod_cell_axis(to_grid(v.y, nxf), xs.y, nx),
-                  sz = sod_cell_axis(to_grid(v.z, nxf), xs.z, nx);
-        if ((ix >> 1) != sx || (iy >> 1) != sy || (iz >> 1) != sz) {
-          atomicOr(bad, 1);
-          continue;
-        }
-        if (ix != kx || iy != ky || iz != kz) {
+        if (ZONE && !in_cic_zone(vb[u], k)) continue;
+        Pt q;
+        locate(vb[u], q);
+        if (q.fx > wx_ || q.fy > wy_ || q.fz > wz_) continue;
+        if (q.fx != run.fx || q.fy != run.fy || q.fz != run.fz) {
           flush();
-          kx = ix;
-          ky = iy;
-          kz = iz;
-          ncx[0] = widx(ix, ox);
-          ncx[1] = widx(ixp, ox);
-          ncy[0] = widx(iy, oy);
-          ncy[1] = widx(iyp, oy);
-          ncz[0] = widx(iz, oz);
-          ncz[1] = widx(izp, oz);
+          run.fx = q.fx;
+          run.fy = q.fy;
+          run.fz = q.fz;
 #pragma unroll
           for (int c = 0; c < 8; c++) acc[c] = 0ull;
         }
-        const double wx[2] = {dex, ddx}, wy[2] = {dey, ddy}, wz[2] = {dez, ddz};
+        const double wx[2] = {dmul(q.wx[0], FIX_ONE), dmul(q.wx[1], FIX_ONE)};
 #pragma unroll
-        for (int c = 0; c < 8; c++) {
-          const int a = c & 1, bb = (c >> 1) & 1, ee = c >> 2;
-          const double wgt = dmul(dmul(wx[a], wy[bb]), wz[ee]);
-          acc[c] += (unsigned long long)__double2ll_rn(dmul(wgt, FIX_ONE));
-        }
+        for (int c = 0; c < 8; c++) acc[c] += quant(dmul(dmul(wx[c & 1], q.wy[(c >> 1) & 1]), q.wz[c >> 2]));
       }
     }
     flush();
   }
   // The run scan files a single particle of the last cell under the
   // previous cell's run (the linked-list quirk), which may lie in another
-  // tile.  Its CIC weights belong to its own cell: every tile whose cells
-  // with halo hold that cell deposits it, and the tile owning the cell
-  // interpolates it.
-  auto cell_rel = [&](int c, int c0) {  // periodic offset of cell c from c0 - 1
-    int d = c - (c0 - 1);
-    if (d < 0) d += nx;
-    if (d >= nx) d -= nx;
-    return d;
-  };
+  // tile.  Its CIC weights belong to its own cell: every tile it touches
+  // deposits it, and the tile holding its fine cell interpolates it.
   float4 vq = make_float4(0.f, 0.f, 0.f, 0.f);
-  int qx = 0, qy = 0, qz = 0;
-  const bool has_q = quirk_pos != 0xffffffffu;
-  if (has_q) {
+  Pt pq;
+  bool own_q = false;
+  if (has_q && threadIdx.x == 0) {
     vq = cube[quirk_pos];
-    qx = cell_rel(sod_cell_axis(to_grid(vq.x, nxf), xs.x, nx), x0);
-    qy = cell_rel(sod_cell_axis(to_grid(vq.y, nxf), xs.y, nx), y0);
-    qz = cell_rel(sod_cell_axis(to_grid(vq.z, nxf), xs.z, nx), z0);
-  }
-  if (threadIdx.x == 0 && has_q && qx <= CT + 1 && qy <= CT + 1 && qz <= CT + 1 &&
-      !(ZONE && !in_cic_zone(vq, k))) {
-    int ix, ixp, iy, iyp, iz, izp;
-    double ddx, dex, ddy, dey, ddz, dez;
-    cic_axis(vq.x, k, 0, ix, ixp, ddx, dex);
-    cic_axis(vq.y, k, 1, iy, iyp, ddy, dey);
-    cic_axis(vq.z, k, 2, iz, izp, ddz, dez);
-    const int cx[2] = {widx(ix, ox), widx(ixp, ox)}, cy[2] = {widx(iy, oy), widx(iyp, oy)},
-              cz[2] = {widx(iz, oz), widx(izp, oz)};
-    const double wx[2] = {dex, ddx}, wy[2] = {dey, ddy}, wz[2] = {dez, ddz};
+    locate(vq, pq);
+    const bool sel = !(ZONE && !in_cic_zone(vq, k));
+    own_q = pq.fx >= 0 && pq.fx < wx_ && pq.fy >= 0 && pq.fy < wy_ && pq.fz >= 0 && pq.fz < wz_;
+    if (sel && pq.fx <= wx_ && pq.fy <= wy_ && pq.fz <= wz_) {
 #pragma unroll
-    for (int c = 0; c < 8; c++) {
-      const int a = c & 1, bb = (c >> 1) & 1, ee = c >> 2;
-      if (cx[a] < CW && cy[bb] < CW && cz[ee] < CW) {
-        const double wgt = dmul(dmul(wx[a], wy[bb]), wz[ee]);
-        atomicAdd(&win[cx[a] + CW * (cy[bb] + CW * cz[ee])], (unsigned long long)__double2ll_rn(dmul(wgt, FIX_ONE)));
+      for (int c = 0; c < 8; c++) {
+        if (!touches(pq, c)) continue;
+        const unsigned long long w =
+            quant(dmul(dmul(dmul(pq.wx[c & 1], FIX_ONE), pq.wy[(c >> 1) & 1]), pq.wz[c >> 2]));
+        if (split) {
+          atomicAdd(&win32[node(pq, c)], (unsigned)w & 0xfffffu);
+          atomicAdd(&win32[CW3 + node(pq, c)], (unsigned)(w >> 20));
+        } else {
+          atomicAdd(&win[node(pq, c)], w);
+        }
       }
     }
   }
   __syncthreads();
-  // own particles: rho in the reference's term order (main:1368-1383)
-  for (int row = threadIdx.x; row < CT * CT; row += blockDim.x) {
-    const int yy = y0 + row % CT, zz = z0 + row / CT;
-    const unsigned long long base = (unsigned long long)nx * ((unsigned)yy + (unsigned long long)nx * (unsigned)zz);
-    const unsigned rb = cs[base + (unsigned)x0];
-    unsigned len = cs[base + (unsigned)(x0 + CT - 1) + 1] - rb;
-    if (len && rb + len - 1u == quirk_pos) len--;  // interpolated below, by its own cell's tile
-    s_rb[row] = rb;
-    s_len[row] = len;
-  }
-  __syncthreads();
-  range_prefix(s_len, s_pre, CT * CT);
-  __syncthreads();
-  const unsigned total = s_pre[CT * CT];
-  auto interp = [&](const float4 v) {
+  // the tile's particles: rho in the reference's term order (main:1368-1383)
+  auto interp = [&](const float4 &v) {
+    Pt q;
+    locate(v, q);
+    const bool mine = q.fx >= 0 && q.fx < wx_ && q.fy >= 0 && q.fy < wy_ && q.fz >= 0 && q.fz < wz_;
+    if (!mine) {
+      if (!RAGGED) atomicOr(bad, 1);
+      return;
+    }
     const unsigned idx = __float_as_uint(v.w) & PSOD_IDX_MASK;
     if (ZONE && !in_cic_zone(v, k)) {  // not selected by cicm1: rho stays 0
       rho[idx] = 0.0;
       return;
     }
-    int ix, ixp, iy, iyp, iz, izp;
-    double ddx, dex, ddy, dey, ddz, dez;
-    cic_axis(v.x, k, 0, ix, ixp, ddx, dex);
-    cic_axis(v.y, k, 1, iy, iyp, ddy, dey);
-    cic_axis(v.z, k, 2, iz, izp, ddz, dez);
-    const int cx[2] = {widx(ix, ox), widx(ixp, ox)}, cy[2] = {widx(iy, oy), widx(iyp, oy)},
-              cz[2] = {widx(iz, oz), widx(izp, oz)};
-    const double wx[2] = {dex, ddx}, wy[2] = {dey, ddy}, wz[2] = {dez, ddz};
     double rr = 0.0;
-    bool ok = true;
 #pragma unroll
     for (int c = 0; c < 8; c++) {
-      const int a = c & 1, bb = (c >> 1) & 1, ee = c >> 2;
-      if (cx[a] >= CW || cy[bb] >= CW || cz[ee] >= CW) {
-        ok = false;
-        continue;
-      }
-      const double gval = dmul((double)(long long)win[cx[a] + CW * (cy[bb] + CW * cz[ee])], k.kc);
-      rr = dadd(rr, dmul(dmul(dmul(gval, wx[a]), wy[bb]), wz[ee]));
+      const int at = node(q, c);
+      // a split sum is below 2^53: exact
+      const double sum = split ? dadd(dmul((double)win32[CW3 + at], 1048576.0), (double)win32[at]) : (double)(long long)win[at];
+      rr = dadd(rr, dmul(dmul(dmul(dmul(sum, k.kc), q.wx[c & 1]), q.wy[(c >> 1) & 1]), q.wz[c >> 2]));
     }
-    if (!ok) atomicOr(bad, 1);
     rho[idx] = rr;
   };
+  unsigned nown = total;
+  if (!RAGGED) {
+    // only the tile's own cells
+    __syncthreads();
+    for (int row = threadIdx.x; row < CT * CT; row += blockDim.x) {
+      unsigned rb = 0, len = 0;
+      if (row < (ye - y0) * (ze - z0)) {
+        const int yy = y0 + row % (ye - y0), zz = z0 + row / (ye - y0);
+        const unsigned long long base = (unsigned long long)nx * ((unsigned)yy + (unsigned long long)nx * (unsigned)zz);
+        rb = cs[base + (unsigned)x0];
+        len = cs[base + (unsigned)xe] - rb;
+        if (len && rb + len - 1u == quirk_pos) len--;
+      }
+      s_rb[row] = rb;
+      s_len[row] = len;
+    }
+    __syncthreads();
+    range_prefix(s_len, s_pre, CT * CT);
+    __syncthreads();
+    nown = s_pre[CT * CT];
+  }
   // two records per thread and step, both loaded before either is used
   int r = 0;
-  for (unsigned fa = threadIdx.x; fa < total; fa += 2 * blockDim.x) {
+  for (unsigned fa = threadIdx.x; fa < nown; fa += 2 * blockDim.x) {
     const unsigned fb = fa + blockDim.x;
     while (s_pre[r + 1] <= fa) r++;
     const float4 va = cube[s_rb[r] + (fa - s_pre[r])];
     float4 vb = va;
-    if (fb < total) {
+    if (fb < nown) {
       while (s_pre[r + 1] <= fb) r++;
       vb = cube[s_rb[r] + (fb - s_pre[r])];
     }
     interp(va);
-    if (fb < total) interp(vb);
+    if (fb < nown) interp(vb);
   }
-  // the quirk particle, by the tile that owns its cell
-  if (threadIdx.x == 0 && has_q && qx >= 1 && qx <= CT && qy >= 1 && qy <= CT && qz >= 1 && qz <= CT) interp(vq);
+  if (own_q) interp(vq);
 }
 
 __global__ void k_grid_to_double(const unsigned long long *grid, long long nnode, double kc, double *out) {
@@ -747,6 +803,11 @@ __global__ void k_seed_compact(const double *rho, long long n, const unsigned *f
   unsigned o = pos[i];
   keys[o] = dbits(ddiv(1.0, rho[i]));
   vals[o] = (unsigned)i;
+}
+
+__global__ void k_widen_seeds(const unsigned *in, long long n, long long *out) {
+  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = (long long)in[i];
 }
 
 inline unsigned nblk(long long n, int t) { return (unsigned)((n + t - 1) / t); }
@@ -875,24 +936,25 @@ int stage_cic(psod_ctx *c, double *grid_out) {
     if ((st = dalloc(c, &c->d_rho, (size_t)c->n))) return st;
     c->rho_cap = c->n;
   }
-  // fused tile path (no global grid) when the box tiles evenly
+  // fused tile path (no global grid); boxes of fewer than CT + 2 cells a side
+  // would meet their own halo
   bool tiled = false;
-  if (c->nx % CT == 0 && c->nx >= 2 * (CT + 2)) {
+  if (c->nx >= CT + 2) {
     int *bad = nullptr;
     if ((st = scratch(c, SLOT_CIC_FLAG, 1, &bad))) return st;
     PSOD_CUDA(c, cudaMemsetAsync(bad, 0, sizeof(int), c->stream));
     const int smem = CW3 * (int)sizeof(unsigned long long);
-    PSOD_CUDA(c, cudaFuncSetAttribute(k_cic_tile<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    PSOD_CUDA(c, cudaFuncSetAttribute(k_cic_tile<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    const long long ntiles = (long long)(c->nx / CT) * (c->nx / CT) * (c->nx / CT);
-    const double3 xs = make_double3(c->xxmin[0] * c->scale, c->xxmin[1] * c->scale, c->xxmin[2] * c->scale);
+    const int nt = (c->nx + CT - 1) / CT;
+    const unsigned ntiles = (unsigned)nt * (unsigned)nt * (unsigned)nt;
     const unsigned qpos = c->has_quirk ? c->quirk_pos : 0xffffffffu;
-    if (k.zone_test)
-      k_cic_tile<true><<<(unsigned)ntiles, 256, smem, c->stream>>>(c->d_cube, c->d_cell_start, c->nx, xs, k, c->d_rho,
-                                                                   bad, qpos);
-    else
-      k_cic_tile<false><<<(unsigned)ntiles, 256, smem, c->stream>>>(c->d_cube, c->d_cell_start, c->nx, xs, k, c->d_rho,
-                                                                    bad, qpos);
+    auto launch = [&](auto *kern) -> int {
+      PSOD_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      kern<<<ntiles, 256, smem, c->stream>>>(c->d_cube, c->d_cell_start, c->nx, k, c->d_rho, bad, qpos);
+      return PSOD_OK;
+    };
+    if ((st = k.zone_test ? launch(k_cic_tile<true, true>)
+                          : (k.inv_dx != 0.0 ? launch(k_cic_tile<false, false>) : launch(k_cic_tile<false, true>))))
+      return st;
     int hbad = 0;
     PSOD_CUDA(c, cudaMemcpyAsync(&hbad, bad, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     PSOD_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -973,13 +1035,17 @@ int stage_tri_cic(psod_ctx *c, int64_t *isort_out) {
   c->nseed_dense = nd;
   c->npart_new = nseed;  // main:1032 (clamped to n when every particle is dense)
   if (isort_out && nseed > 0) {
-    std::vector<unsigned> h((size_t)nseed);
-    PSOD_CUDA(c, cudaMemcpy(h.data(), c->d_seed_idx, sizeof(unsigned) * nseed, cudaMemcpyDeviceToHost));
-    if (is_device_ptr(isort_out)) {
-      std::vector<int64_t> hh(h.begin(), h.end());
-      PSOD_CUDA(c, cudaMemcpy(isort_out, hh.data(), sizeof(int64_t) * nseed, cudaMemcpyHostToDevice));
+    // widened on the device, in place for a device destination (through host
+    // vectors a 256^3 box took 13 ms of its 22; the kernel takes 20 us)
+    long long *d = reinterpret_cast<long long *>(isort_out);
+    const bool host = !is_device_ptr(isort_out);
+    if (host && (st = scratch(c, SLOT_OUT_IDX, (size_t)nseed, &d))) return st;
+    k_widen_seeds<<<nblk(nseed, 256), 256, 0, c->stream>>>(c->d_seed_idx, nseed, d);
+    PSOD_CUDA(c, cudaGetLastError());
+    if (host) {
+      if ((st = copy_out(c, isort_out, d, sizeof(int64_t) * nseed))) return st;
     } else {
-      for (long long i = 0; i < nseed; i++) isort_out[i] = (int64_t)h[(size_t)i];
+      PSOD_CUDA(c, cudaStreamSynchronize(c->stream));
     }
   }
   c->seeds_done = true;
