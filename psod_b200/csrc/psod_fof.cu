@@ -47,6 +47,7 @@ namespace {
 
 constexpr int FOF_TPB = 256;
 constexpr unsigned FOF_SMALL_CELL = 16;  // records a thread sorts itself
+constexpr unsigned LINK_BRUTE = 512;     // records of a cell linked record by record
 constexpr unsigned FOF_THREAD_RUN = 4;   // runs a thread links; longer ones go to a warp
 constexpr int FOF_MAX_OFF = 171;         // half of the 7^3 - 1 neighbour offsets
 constexpr unsigned FOF_WARP_HALO = 2048; // halos whose observables a warp computes; larger: a CTA
@@ -163,20 +164,25 @@ __global__ void k_fof_keys(const float4 *cube, long long n, FofGeo G, unsigned s
 
 // A thread per SOD cell: cells of at most FOF_SMALL_CELL records are sorted
 // here (insertion sort on (key, slot)); larger ones are listed for the CTA
-// sort.  Writes the FoF order (perm: cube slot), the sorted keys, each
-// position's run head (the union-find parent) and the inverse map.
+// sort.  Writes the FoF order (perm: cube slot), the sorted keys, the run-head
+// flags, the inverse map and the union-find parents.  The cell's own friend
+// pairs are joined at once, all of them, in the thread's registers: every
+// position starts with the root of its group inside the cell.
 __global__ void k_fof_sort_small(const unsigned *cs, unsigned long long ncell, const unsigned short *key,
-                                 const float4 *cube, unsigned *perm, unsigned short *skey, unsigned *par,
-                                 unsigned *finv, unsigned *big, unsigned *nbig) {
+                                 const float4 *cube, FofGeo G, unsigned *perm, unsigned short *skey, unsigned *par,
+                                 unsigned *finv, unsigned *flag, unsigned *big, unsigned *nbig, unsigned *dense,
+                                 unsigned *ndense) {
   const unsigned long long c = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncell) return;
   const unsigned b = cs[c], e = cs[c + 1], m = e - b;
   if (m == 0) return;
   if (m > FOF_SMALL_CELL) {
     big[atomicAdd(nbig, 1u)] = (unsigned)c;
+    if (m > LINK_BRUTE) dense[atomicAdd(ndense, 1u)] = (unsigned)c;
     return;
   }
   unsigned kk[FOF_SMALL_CELL], ss[FOF_SMALL_CELL];
+  unsigned char root[FOF_SMALL_CELL];
   for (unsigned j = 0; j < m; j++) {
     const unsigned kv = key[b + j];
     unsigned t = j;
@@ -188,64 +194,165 @@ __global__ void k_fof_sort_small(const unsigned *cs, unsigned long long ncell, c
     kk[t] = kv;
     ss[t] = b + j;
   }
-  unsigned head = b;
   for (unsigned j = 0; j < m; j++) {
-    if (j > 0 && kk[j] != kk[j - 1]) head = b + j;
+    const float4 v = cube[ss[j]];
+    const bool head = j == 0 || kk[j] != kk[j - 1];
+    unsigned rj = j;
+    if (!head) rj = root[j - 1];  // one linking cell: friends
+    // the lower root of every earlier group that holds a friend
+    for (unsigned i = 0; i < j; i++) {
+      if (root[i] == rj || !fof_friends(cube[ss[i]], v, G.r2, G.rT)) continue;
+      const unsigned lo = min((unsigned)root[i], rj), hi = max((unsigned)root[i], rj);
+      for (unsigned q = 0; q < j; q++)
+        if (root[q] == hi) root[q] = (unsigned char)lo;
+      if (rj == hi) rj = lo;
+    }
+    root[j] = (unsigned char)rj;
     perm[b + j] = ss[j];
     skey[b + j] = (unsigned short)kk[j];
-    par[b + j] = head;
-    finv[__float_as_uint(cube[ss[j]].w) & ~PSOD_DEAD_BIT] = b + j;
+    flag[b + j] = head ? 1u : 0u;
+    finv[__float_as_uint(v.w) & ~PSOD_DEAD_BIT] = b + j;
+  }
+  for (unsigned j = 0; j < m; j++) par[b + j] = b + root[j];
+}
+
+// union-find over the linking cells of one SOD cell, in shared memory
+__device__ __forceinline__ unsigned loc_find(volatile unsigned *par, unsigned x) {
+  unsigned p = par[x];
+  while (p != x) {
+    const unsigned g = par[p];
+    if (g == p) return p;
+    par[x] = g;
+    x = g;
+    p = par[x];
+  }
+  return x;
+}
+
+__device__ __forceinline__ void loc_union(unsigned *par, unsigned a, unsigned b) {
+  while (true) {
+    a = loc_find(par, a);
+    b = loc_find(par, b);
+    if (a == b) return;
+    if (a > b) {
+      const unsigned t = a;
+      a = b;
+      b = t;
+    }
+    const unsigned old = atomicCAS(par + b, b, a);
+    if (old == b) return;
+    b = old;
   }
 }
 
 // A CTA per large SOD cell: counting sort on the linking-cell key with the
-// k^3 bins in shared memory; a run head is its bin's start.
+// k^3 bins in shared memory.  With room for it (LOCAL) the bins are then
+// linked there: the first records of touching linking cells are tested and
+// friends joined, which already makes one group of most of a dense cell, so
+// that the linking passes meet a few groups per cell and not hundreds of runs
+// (their walks and retried hooks on one shared tree took most of their time).
+// Pairs it leaves are tested by the full pass.
+template <bool LOCAL>
 __global__ void __launch_bounds__(FOF_TPB) k_fof_sort_big(const unsigned *cs, const unsigned *big,
-                                                          const unsigned *nbig, int nbins,
+                                                          const unsigned *nbig, int nbins, FofGeo G,
                                                           const unsigned short *key, const float4 *cube,
                                                           unsigned *perm, unsigned short *skey, unsigned *par,
-                                                          unsigned *finv) {
+                                                          unsigned *finv, unsigned *flag) {
   extern __shared__ unsigned bins[];
+  unsigned *loc = bins + nbins;                                     // LOCAL: parents of the bins
+  float *rx = reinterpret_cast<float *>(loc + nbins), *ry = rx + nbins, *rz = ry + nbins;  // their first records
+  __shared__ unsigned s_w[FOF_TPB / 32];
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const unsigned nb = *nbig;
+  const int per = (nbins + FOF_TPB - 1) / FOF_TPB;
   for (unsigned q = blockIdx.x; q < nb; q += gridDim.x) {
     const unsigned c = big[q];
     const unsigned b = cs[c], e = cs[c + 1];
-    for (int i = threadIdx.x; i < nbins; i += blockDim.x) bins[i] = 0;
+    for (int i = tid; i < nbins; i += FOF_TPB) bins[i] = 0;
     __syncthreads();
-    for (unsigned s = b + threadIdx.x; s < e; s += blockDim.x) atomicAdd(&bins[key[s]], 1u);
+    for (unsigned s = b + tid; s < e; s += FOF_TPB) atomicAdd(&bins[key[s]], 1u);
     __syncthreads();
-    if (threadIdx.x == 0) {
-      unsigned run = 0;
-      for (int i = 0; i < nbins; i++) {
+    {  // exclusive scan, each thread over its own bins
+      const int lo = min(nbins, tid * per), hi = min(nbins, lo + per);
+      unsigned own = 0;
+      for (int i = lo; i < hi; i++) own += bins[i];
+      unsigned inc = own;
+      for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+      }
+      if (lane == 31) s_w[w] = inc;
+      __syncthreads();
+      unsigned run = inc - own;
+      for (int k = 0; k < w; k++) run += s_w[k];
+      for (int i = lo; i < hi; i++) {
         const unsigned v = bins[i];
         bins[i] = run;
+        if (LOCAL) loc[i] = v ? (unsigned)i : 0xffffffffu;
         run += v;
       }
     }
     __syncthreads();
     // bins[i] is the start of bin i and serves as its write cursor
-    for (unsigned s = b + threadIdx.x; s < e; s += blockDim.x) {
+    for (unsigned s = b + tid; s < e; s += FOF_TPB) {
       const unsigned kv = key[s];
+      const float4 v = cube[s];
       const unsigned at = b + atomicAdd(&bins[kv], 1u);
       perm[at] = s;
       skey[at] = (unsigned short)kv;
-      finv[__float_as_uint(cube[s].w) & ~PSOD_DEAD_BIT] = at;
+      finv[__float_as_uint(v.w) & ~PSOD_DEAD_BIT] = at;
     }
     __syncthreads();
     // bins[i] is now the end of bin i: a position's head is the first
     // position with its key (the end of the previous bin)
-    for (unsigned p = b + threadIdx.x; p < e; p += blockDim.x) {
+    if (LOCAL) {
+      const int k = G.k;
+      for (int i = tid; i < nbins; i += FOF_TPB) {
+        if (loc[i] == 0xffffffffu) continue;
+        const float4 v = cube[perm[b + (i == 0 ? 0u : bins[i - 1])]];
+        rx[i] = v.x;
+        ry[i] = v.y;
+        rz[i] = v.z;
+      }
+      __syncthreads();
+      for (int i = tid; i < nbins; i += FOF_TPB) {
+        if (loc[i] == 0xffffffffu) continue;
+        const int x = i % k, y = (i / k) % k, z = i / (k * k);
+        const float4 a = make_float4(rx[i], ry[i], rz[i], 0.f);
+        for (int o = 1; o <= 13; o++) {  // the half space of the 26 touching cells
+          const int ox = (o + 13) % 3 - 1, oy = ((o + 13) / 3) % 3 - 1, oz = (o + 13) / 9 - 1;
+          const int nx = x + ox, ny = y + oy, nz = z + oz;
+          if (nx < 0 || nx >= k || ny < 0 || ny >= k || nz >= k) continue;
+          const int j = nx + k * (ny + k * nz);
+          if (loc[j] == 0xffffffffu) continue;
+          if (fof_friends(a, make_float4(rx[j], ry[j], rz[j], 0.f), G.r2, G.rT))
+            loc_union(loc, (unsigned)i, (unsigned)j);
+        }
+      }
+      __syncthreads();
+    }
+    for (unsigned p = b + tid; p < e; p += FOF_TPB) {
       const unsigned kv = skey[p];
-      par[p] = b + (kv == 0 ? 0u : bins[kv - 1]);
+      const unsigned head = b + (kv == 0 ? 0u : bins[kv - 1]);
+      flag[p] = p == head ? 1u : 0u;
+      if (LOCAL) {
+        unsigned r = kv;
+        while (loc[r] != r) r = loc[r];
+        par[p] = b + (r == 0 ? 0u : bins[r - 1]);
+      } else {
+        par[p] = head;
+      }
     }
     __syncthreads();
   }
 }
 
-// run-head flags (a head is its own parent)
-__global__ void k_fof_head_flags(const unsigned *par, long long n, unsigned *flag) {
-  const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < n) flag[p] = par[p] == (unsigned)p ? 1u : 0u;
+__global__ void k_fof_count(const unsigned *flag, long long n, unsigned long long *out) {
+  unsigned long long s = 0;
+  for (long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x)
+    s += flag[p];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0 && s) atomicAdd(out, s);
 }
 
 __global__ void k_fof_head_list(const unsigned *flag, const unsigned *pos, long long n, unsigned *heads) {
@@ -273,7 +380,9 @@ __device__ __forceinline__ RunGeo run_geo(float4 v, const FofGeo &G, float lo[3]
   return r;
 }
 
-// the run of linking cell (run origin + offset o), or an empty range
+// the run of linking cell (run origin + offset o), or an empty range; false
+// too where the other run looks at this one: of two SOD cells the one with the
+// lower index, inside a cell the run that precedes in (z, y, x)
 __device__ __forceinline__ bool find_run(const RunGeo &u, int ox, int oy, int oz, const FofGeo &G, const unsigned *cs,
                                          const unsigned short *skey, unsigned &vlo, unsigned &vhi) {
   int tx = u.fx + ox, ty = u.fy + oy, tz = u.fz + oz;
@@ -288,6 +397,10 @@ __device__ __forceinline__ bool find_run(const RunGeo &u, int ox, int oy, int oz
   cz = cz < 0 ? cz + G.nx : (cz >= G.nx ? cz - G.nx : cz);
   const unsigned long long c =
       (unsigned long long)cx + (unsigned long long)G.nx * ((unsigned long long)cy + (unsigned long long)G.nx * cz);
+  const unsigned long long own =
+      (unsigned long long)u.cx + (unsigned long long)G.nx * ((unsigned long long)u.cy + (unsigned long long)G.nx * u.cz);
+  const bool after = oz > 0 || (oz == 0 && (oy > 0 || (oy == 0 && ox > 0)));
+  if (c == own ? !after : c < own) return false;
   const unsigned lo = __ldg(cs + c), hi = __ldg(cs + c + 1);
   if (lo == hi) return false;
   const unsigned short kv = (unsigned short)(tx + G.k * (ty + G.k * tz));
@@ -330,25 +443,28 @@ __device__ __forceinline__ float box_gap2(const RunGeo &u, int ox, int oy, int o
 }
 
 // Linking runs in two passes (the sampling scheme of Afforest, Sutton et
-// al. 2018).  The first pass joins each short run to at most FOF_SAMPLE
-// friends and each long run to the friends among FOF_SAMPLE_WARP
-// neighbouring runs, which already builds most of every large group (one
-// friend per run, or six, measured slower at 512^3 and 1024^3); after
-// a compression every position points at its root, so in the full pass a
-// neighbour run with the same parent is skipped with two loads instead of
-// two path walks.  Both passes test the same pairs' friendship, so the
-// components are the same as without sampling.
-constexpr int FOF_SAMPLE = 3;       // friends a thread's run joins in the first pass
+// al. 2018).  The sort has joined the runs inside each SOD cell (all of a small
+// cell's, most of a large one's).  The first pass joins each short run to at
+// most FOF_SAMPLE friends in neighbouring SOD cells and each long run to the
+// friends among FOF_SAMPLE_WARP neighbouring runs of other groups, which builds
+// most of every large group; after a compression every position points at its
+// root, so in the full pass a neighbour with the same parent is skipped with
+// two loads instead of two path walks.  All passes test the same pairs'
+// friendship, so the components are the same as without sampling.
+constexpr int FOF_SAMPLE = 1;       // friends a thread's run joins in the first pass
 constexpr int FOF_SAMPLE_WARP = 2;  // neighbour runs a warp's run examines in the first pass
 
 // A thread per run of up to FOF_THREAD_RUN records; longer runs are listed
-// (in the first pass) for k_fof_link_warp.  The neighbour cells are walked
-// row by row: for each (dy, dz) of the half space whose row of linking
-// cells comes within reach of the run's records, the cells of the row that
-// do form one key range inside each SOD cell the row crosses, found with
-// one search; every record of the range is then tested.  A friend joins the
-// two components; in the full pass a record whose parent is the run's
-// parent (both compressed) needs no test.
+// (in the first pass) for k_fof_link_warp.  The SOD cells within reach of the
+// run's records are visited, of each pair of cells the one with the lower
+// index visiting the other.  A cell of up to FOF_SMALL_CELL records is tested
+// record by record; in a larger one the linking cells within reach form one
+// key range per row, found with one search.  In the full pass a record whose
+// parent is the run's parent (both compressed) needs no test, and the run's
+// own cell is searched too when it is a large one (the half space of rows
+// after the run).  256^3 box: a thread walking the 13 rows of linking cells
+// around every run, with all joins on the global tree, took 18.7 + 8.1 ms for
+// the two passes; FOF_MS.
 template <bool FULL>
 __global__ void __launch_bounds__(FOF_TPB, 3) k_fof_link_thread(const unsigned *heads, long long nrun, FofGeo G,
                                                              const unsigned *cs, const unsigned short *skey,
@@ -357,7 +473,7 @@ __global__ void __launch_bounds__(FOF_TPB, 3) k_fof_link_thread(const unsigned *
                                                              unsigned long long *counters) {
   unsigned long long tests = 0, pairs = 0;
   const int R = G.R;
-  const float reach2 = (float)G.reach2;
+  const float reach2 = (float)G.reach2, kf = (float)G.k;
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nrun;
        q += (long long)gridDim.x * blockDim.x) {
     const unsigned h = heads[q], e = heads[q + 1];
@@ -389,69 +505,88 @@ __global__ void __launch_bounds__(FOF_TPB, 3) k_fof_link_thread(const unsigned *
     }
     const unsigned myroot = FULL ? __ldcg(par + h) : 0u;
     int found = 0;
-    for (int oz = 0; oz <= R && found < FOF_SAMPLE; oz++) {
-      const float bz = (float)(u.fz + oz);
-      const float gz = fmaxf(fmaxf(bz - hi[2], lo[2] - (bz + 1.f)), 0.f);
-      if (gz * gz > reach2) continue;
-      for (int oy = (oz == 0 ? 0 : -R); oy <= R && found < FOF_SAMPLE; oy++) {
-        const float by = (float)(u.fy + oy);
-        const float gy = fmaxf(fmaxf(by - hi[1], lo[1] - (by + 1.f)), 0.f);
-        const float left = reach2 - gz * gz - gy * gy;
-        if (left < 0.f) continue;
-        const float rx = sqrtf(left);
-        // cells of the row within reach, in the run's SOD-cell frame
-        int xa = (int)floorf(lo[0] - rx), xb = (int)floorf(hi[0] + rx);
-        xa = max(xa, u.fx - R);
-        xb = min(xb, u.fx + R);
-        if (oz == 0 && oy == 0) xa = max(xa, u.fx + 1);  // own row: cells after the run's
-        if (xa > xb) continue;
-        // the row's SOD cells in y and z
-        int ty = u.fy + oy, tz = u.fz + oz;
-        const int dcy = ty < 0 ? -1 : (ty >= G.k ? 1 : 0), dcz = tz < 0 ? -1 : (tz >= G.k ? 1 : 0);
-        ty -= dcy * G.k;
-        tz -= dcz * G.k;
-        int cy = u.cy + dcy, cz = u.cz + dcz;
-        cy = cy < 0 ? cy + G.nx : (cy >= G.nx ? cy - G.nx : cy);
-        cz = cz < 0 ? cz + G.nx : (cz >= G.nx ? cz - G.nx : cz);
-        // up to three SOD cells along x
-        for (int dcx = -1; dcx <= 1 && found < FOF_SAMPLE; dcx++) {
-          const int s0 = max(xa, dcx * G.k), s1 = min(xb, dcx * G.k + G.k - 1);
-          if (s0 > s1) continue;
-          int cx = u.cx + dcx;
-          cx = cx < 0 ? cx + G.nx : (cx >= G.nx ? cx - G.nx : cx);
-          const unsigned long long c = (unsigned long long)cx +
-                                       (unsigned long long)G.nx * ((unsigned long long)cy + (unsigned long long)G.nx * cz);
-          const unsigned clo = __ldg(cs + c), chi = __ldg(cs + c + 1);
-          if (clo == chi) continue;
-          const unsigned rowkey = (unsigned)(G.k * (ty + G.k * tz));
-          const unsigned k0 = rowkey + (unsigned)(s0 - dcx * G.k), k1 = rowkey + (unsigned)(s1 - dcx * G.k);
-          unsigned v = clo;
-          if (chi - clo <= 16) {
-            while (v < chi && __ldg(skey + v) < k0) v++;
-          } else {
-            unsigned b2 = chi;
-            while (v < b2) {
-              const unsigned mid = (v + b2) >> 1;
-              if (__ldg(skey + mid) < k0) v = mid + 1;
-              else b2 = mid;
-            }
+    // record v of another run: a friend joins the two groups
+    auto visit = [&](unsigned v) {
+      if (FULL && __ldcg(par + v) == myroot) return;
+      const float4 bv = cube[perm[v]];
+      bool hit = false;
+#pragma unroll
+      for (unsigned j = 0; j < FOF_THREAD_RUN; j++) {
+        if (j < m && !hit) {
+          tests++;
+          hit = fof_friends(ur[j], bv, G.r2, G.rT);
+        }
+      }
+      if (hit) {
+        uf_union(par, h, v);
+        if (!FULL) found++;
+      }
+    };
+    // linking cells of SOD cell offset (dx, dy, dz), records [clo, chi): the
+    // rows within reach, one key range each
+    auto rows = [&](int dx, int dy, int dz, unsigned clo, unsigned chi) {
+      const bool self = (dx | dy | dz) == 0;
+      const int z0 = max(u.fz - R, dz * G.k), z1 = min(u.fz + R, dz * G.k + G.k - 1);
+      for (int tz = self ? u.fz : z0; tz <= z1 && found < FOF_SAMPLE; tz++) {
+        const float gz = fmaxf(fmaxf((float)tz - hi[2], lo[2] - ((float)tz + 1.f)), 0.f);
+        if (gz * gz > reach2) continue;
+        const int y0 = max(u.fy - R, dy * G.k), y1 = min(u.fy + R, dy * G.k + G.k - 1);
+        for (int ty = (self && tz == u.fz) ? u.fy : y0; ty <= y1 && found < FOF_SAMPLE; ty++) {
+          const float gy = fmaxf(fmaxf((float)ty - hi[1], lo[1] - ((float)ty + 1.f)), 0.f);
+          const float left = reach2 - gz * gz - gy * gy;
+          if (left < 0.f) continue;
+          const float rx = sqrtf(left);
+          int xa = max(max((int)floorf(lo[0] - rx), u.fx - R), dx * G.k);
+          const int xb = min(min((int)floorf(hi[0] + rx), u.fx + R), dx * G.k + G.k - 1);
+          if (self && tz == u.fz && ty == u.fy) xa = max(xa, u.fx + 1);  // own row: cells after the run's
+          if (xa > xb) continue;
+          const unsigned rowkey = (unsigned)(G.k * ((ty - dy * G.k) + G.k * (tz - dz * G.k)));
+          const unsigned k0 = rowkey + (unsigned)(xa - dx * G.k), k1 = rowkey + (unsigned)(xb - dx * G.k);
+          unsigned v = clo, b2 = chi;
+          while (v < b2) {
+            const unsigned mid = (v + b2) >> 1;
+            if (__ldg(skey + mid) < k0) v = mid + 1;
+            else b2 = mid;
           }
           pairs++;
           for (; v < chi && __ldg(skey + v) <= k1; v++) {
-            if (FULL && __ldcg(par + v) == myroot) continue;
-            const float4 bv = cube[perm[v]];
-            bool hit = false;
-#pragma unroll
-            for (unsigned j = 0; j < FOF_THREAD_RUN; j++) {
-              if (j < m && !hit) {
-                tests++;
-                hit = fof_friends(ur[j], bv, G.r2, G.rT);
-              }
-            }
-            if (hit) {
-              uf_union(par, h, v);
-              if (!FULL && ++found >= FOF_SAMPLE) break;
-            }
+            visit(v);
+            if (found >= FOF_SAMPLE) break;
+          }
+        }
+      }
+    };
+    const unsigned long long own =
+        (unsigned long long)u.cx + (unsigned long long)G.nx * ((unsigned long long)u.cy + (unsigned long long)G.nx * u.cz);
+    if (FULL) {  // a small own cell was linked by the sort
+      const unsigned clo = __ldg(cs + own), chi = __ldg(cs + own + 1);
+      if (chi - clo > FOF_SMALL_CELL) rows(0, 0, 0, clo, chi);
+    }
+    for (int dz = -1; dz <= 1 && found < FOF_SAMPLE; dz++) {
+      const float gz = dz < 0 ? lo[2] : (dz > 0 ? kf - hi[2] : 0.f);
+      if (gz > 0.f && gz * gz > reach2) continue;
+      int cz = u.cz + dz;
+      cz = cz < 0 ? cz + G.nx : (cz >= G.nx ? cz - G.nx : cz);
+      for (int dy = -1; dy <= 1 && found < FOF_SAMPLE; dy++) {
+        const float gy = dy < 0 ? lo[1] : (dy > 0 ? kf - hi[1] : 0.f);
+        const float g2 = fmaxf(gz, 0.f) * fmaxf(gz, 0.f) + fmaxf(gy, 0.f) * fmaxf(gy, 0.f);
+        if (g2 > reach2) continue;
+        int cy = u.cy + dy;
+        cy = cy < 0 ? cy + G.nx : (cy >= G.nx ? cy - G.nx : cy);
+        for (int dx = -1; dx <= 1 && found < FOF_SAMPLE; dx++) {
+          const float gx = fmaxf(dx < 0 ? lo[0] : (dx > 0 ? kf - hi[0] : 0.f), 0.f);
+          if (g2 + gx * gx > reach2) continue;
+          int cx = u.cx + dx;
+          cx = cx < 0 ? cx + G.nx : (cx >= G.nx ? cx - G.nx : cx);
+          const unsigned long long c =
+              (unsigned long long)cx + (unsigned long long)G.nx * ((unsigned long long)cy + (unsigned long long)G.nx * cz);
+          if (c <= own) continue;  // that cell visits this one
+          const unsigned clo = __ldg(cs + c), chi = __ldg(cs + c + 1);
+          if (chi - clo > FOF_SMALL_CELL) {
+            rows(dx, dy, dz, clo, chi);
+          } else if (chi != clo) {
+            pairs++;
+            for (unsigned v = clo; v < chi && found < FOF_SAMPLE; v++) visit(v);
           }
         }
       }
@@ -493,15 +628,16 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_link_warp(const unsigned *heads
     lo[2] = (float)u.fz;
     hi[2] = (float)(u.fz + 1);
     int sampled = 0;  // neighbour runs examined (warp-uniform)
-    for (int o = 0; o < G.noff && (FULL || sampled < FOF_SAMPLE_WARP); o++) {
-      const int ox = c_fof_off[3 * o], oy = c_fof_off[3 * o + 1], oz = c_fof_off[3 * o + 2];
+    for (int o2 = 0; o2 < 2 * G.noff && (FULL || sampled < FOF_SAMPLE_WARP); o2++) {
+      const int o = o2 >> 1, sg = (o2 & 1) ? -1 : 1;  // both halves of the offsets
+      const int ox = sg * c_fof_off[3 * o], oy = sg * c_fof_off[3 * o + 1], oz = sg * c_fof_off[3 * o + 2];
       if (box_gap2(u, ox, oy, oz, lo, hi) > (float)G.reach2) continue;
       unsigned vlo, vhi;
       if (!find_run(u, ox, oy, oz, G, cs, skey, vlo, vhi)) continue;
       if (vlo == h) continue;
+      if (__ldcg(par + h) == __ldcg(par + vlo)) continue;
       sampled++;
       if (lane == 0) pairs++;
-      if (FULL && __ldcg(par + h) == __ldcg(par + vlo)) continue;
       bool hit = false;
       for (unsigned ub = h; ub < e && !hit; ub += 32) {
         const unsigned uu = ub + (unsigned)lane;
@@ -527,6 +663,276 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_link_warp(const unsigned *heads
     pairs += __shfl_down_sync(0xffffffffu, pairs, o);
   }
   if (lane == 0) {
+    atomicAdd(counters, tests);
+    atomicAdd(counters + 1, pairs);
+  }
+}
+
+// A CTA per SOD cell of more than LINK_BRUTE records: its runs against each other
+// (FULL) and against
+// the runs of the neighbouring cells.  The cell's linking cells are a table in
+// shared memory (first and last record, group), and a warp at a time takes a
+// neighbour, with a table of that cell's linking cells within reach (two
+// layers at the common face), so a neighbouring run is one look-up where a
+// thread alone would search the cell's sorted keys.  The large cell of a pair
+// does the pair, of two large ones the lower index.  The sampled pass (!FULL)
+// tests the first records of neighbouring linking cells and stops at
+// LINK_SAMPLE joins a neighbour; the full pass tests every pair of runs whose
+// groups differ until a friend pair is met, long products by the warp.  A
+// neighbour all of whose runs in reach are of the cell's one group is skipped.
+// FOF_MS.
+constexpr unsigned LINK_SAMPLE = 2;
+constexpr unsigned LINK_SERIAL = 64;  // record pairs a lane tests itself
+
+template <bool FULL>
+__global__ void __launch_bounds__(FOF_TPB) k_fof_cell_link(const unsigned *cs, const unsigned *big,
+                                                           const unsigned *nbig, int nbins, FofGeo G,
+                                                           const unsigned short *skey, const unsigned *perm,
+                                                           const float4 *cube, unsigned *par,
+                                                           unsigned long long *counters) {
+  constexpr unsigned NONE = 0xffffffffu;
+  extern __shared__ unsigned tab[];
+  unsigned *sa = tab, *ea = sa + nbins, *ra = ea + nbins;  // own cell: run start, end, group
+  const int k = G.k, R = G.R, nreg = R * k * k;
+  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  unsigned *sb = ra + nbins + 3 * nreg * w, *eb = sb + nreg, *rb = eb + nreg;  // the warp's neighbour region
+  __shared__ unsigned s_item, s_root, s_mixed;
+  const float reach2 = (float)G.reach2;
+  const unsigned nb = *nbig;
+  const unsigned nself = FULL ? (unsigned)(nbins + 31) / 32u : 0u;  // items of the cell itself, 32 linking cells each
+  unsigned long long tests = 0, pairs = 0;
+  for (unsigned qc = blockIdx.x; qc < nb; qc += gridDim.x) {
+    const unsigned c = big[qc];
+    const int cx = (int)(c % (unsigned)G.nx), cy = (int)((c / (unsigned)G.nx) % (unsigned)G.nx),
+              cz = (int)(c / ((unsigned)G.nx * (unsigned)G.nx));
+    const unsigned b1 = cs[c], e1c = cs[c + 1];
+    __syncthreads();
+    for (int i = tid; i < nbins; i += FOF_TPB) sa[i] = NONE;
+    if (tid == 0) {
+      s_item = 0;
+      s_mixed = 0;
+      s_root = __ldcg(par + b1);
+    }
+    __syncthreads();
+    for (unsigned p = b1 + tid; p < e1c; p += FOF_TPB) {
+      const unsigned kv = skey[p];
+      if (p == b1 || skey[p - 1] != kv) {
+        const unsigned r = __ldcg(par + p);
+        sa[kv] = p;
+        ra[kv] = r;
+        if (r != s_root) s_mixed = 1;
+      }
+      if (p + 1 == e1c || skey[p + 1] != kv) ea[kv] = p + 1;
+    }
+    __syncthreads();
+    const unsigned single = s_mixed ? NONE : s_root;  // the cell's group when it has one
+    while (true) {
+      unsigned it = 0;
+      if (lane == 0) it = atomicAdd(&s_item, 1u);
+      it = __shfl_sync(0xffffffffu, it, 0);
+      if (it >= nself + 26u) break;
+      const bool self = FULL && it < nself;
+      const int m = self ? 13 : ((int)(it - nself) < 13 ? (int)(it - nself) : (int)(it - nself) + 1);
+      const int dx = m % 3 - 1, dy = (m / 3) % 3 - 1, dz = m / 9 - 1;
+      // the linking cells of this cell, and of the neighbour, that can meet
+      const int qx = dx ? R : k, qy = dy ? R : k, qz = dz ? R : k;
+      const int ax0 = dx > 0 ? k - R : 0, ay0 = dy > 0 ? k - R : 0, az0 = dz > 0 ? k - R : 0;
+      const int bx0 = dx < 0 ? k - R : 0, by0 = dy < 0 ? k - R : 0, bz0 = dz < 0 ? k - R : 0;
+      const unsigned *st = sa, *et = ea, *rt = ra;
+      if (self) {
+        if (single != NONE) continue;
+      } else {
+        const int xx = (cx + dx + G.nx) % G.nx, yy = (cy + dy + G.nx) % G.nx, zz = (cz + dz + G.nx) % G.nx;
+        const unsigned c2 = (unsigned)xx + (unsigned)G.nx * ((unsigned)yy + (unsigned)G.nx * (unsigned)zz);
+        const unsigned b2 = cs[c2], e2 = cs[c2 + 1];
+        if (b2 == e2 || (e2 - b2 > LINK_BRUTE && c2 < c)) continue;
+        __syncwarp();
+        for (int i = lane; i < qx * qy * qz; i += 32) sb[i] = NONE;
+        __syncwarp();
+        bool other = false;
+        for (unsigned p = b2 + (unsigned)lane; p < e2; p += 32u) {
+          const unsigned kv = skey[p];
+          const int lx = (int)(kv % (unsigned)k) - bx0, ly = (int)((kv / (unsigned)k) % (unsigned)k) - by0,
+                    lz = (int)(kv / (unsigned)(k * k)) - bz0;
+          if (lx < 0 || lx >= qx || ly < 0 || ly >= qy || lz < 0 || lz >= qz) continue;
+          const int j = lx + qx * (ly + qy * lz);
+          if (p == b2 || skey[p - 1] != kv) {
+            const unsigned r = __ldcg(par + p);
+            sb[j] = p;
+            rb[j] = r;
+            if (r != single) other = true;
+          }
+          if (p + 1 == e2 || skey[p + 1] != kv) eb[j] = p + 1;
+        }
+        __syncwarp();
+        if (!__any_sync(0xffffffffu, other) && single != NONE) continue;
+        st = sb;
+        et = eb;
+        rt = rb;
+      }
+      unsigned joined = 0;
+      const int i_beg = self ? (int)it * 32 : 0, i_end = self ? min(nbins, i_beg + 32) : qx * qy * qz;
+      for (int i0 = i_beg; i0 < i_end && joined < LINK_SAMPLE; i0 += 32) {
+        const int i = i0 + lane;
+        const int x = ax0 + i % qx, y = ay0 + (i / qx) % qy, z = az0 + i / (qx * qy);
+        const int own = x + k * (y + k * z);
+        const bool have = i < i_end && sa[own] != NONE;
+        if (!__any_sync(0xffffffffu, have)) continue;
+        const unsigned s0 = have ? sa[own] : 0u, e0 = have ? ea[own] : 0u, r0 = have ? ra[own] : 0u;
+        float4 first = make_float4(0.f, 0.f, 0.f, 0.f);
+        bool loaded = false;
+        for (int oz = self ? 0 : (dz > 0 ? 1 : -R); oz <= (dz < 0 ? -1 : R); oz++)
+          for (int oy = dy > 0 ? 1 : -R; oy <= (dy < 0 ? -1 : R); oy++)
+            for (int ox = dx > 0 ? 1 : -R; ox <= (dx < 0 ? -1 : R); ox++) {
+              if (self && oz == 0 && (oy < 0 || (oy == 0 && ox <= 0))) continue;  // the half space after the run
+              const float gx = (float)max(abs(ox) - 1, 0), gy = (float)max(abs(oy) - 1, 0), gz = (float)max(abs(oz) - 1, 0);
+              if (gx * gx + gy * gy + gz * gz > reach2) continue;
+              const int lx = x + ox - dx * k - bx0, ly = y + oy - dy * k - by0, lz = z + oz - dz * k - bz0;
+              const bool in = have && lx >= 0 && lx < qx && ly >= 0 && ly < qy && lz >= 0 && lz < qz;
+              const int j = lx + qx * (ly + qy * lz);
+              const unsigned s1 = in ? st[j] : NONE;
+              const bool ok = s1 != NONE && rt[j] != r0;
+              if (!__any_sync(0xffffffffu, ok)) continue;
+              bool hit = false;
+              bool lng = false;
+              if (ok) {
+                pairs++;
+                if (!loaded) {
+                  first = cube[perm[s0]];
+                  loaded = true;
+                }
+                const unsigned t1 = FULL ? et[j] : s1 + 1u, t0 = FULL ? e0 : s0 + 1u;
+                lng = (unsigned long long)(t0 - s0) * (t1 - s1) > LINK_SERIAL;
+                for (unsigned u = s0; u < t0 && !hit && !lng; u++) {
+                  const float4 a = u == s0 ? first : cube[perm[u]];
+                  for (unsigned v = s1; v < t1 && !hit; v++) {
+                    tests++;
+                    hit = fof_friends(a, cube[perm[v]], G.r2, G.rT);
+                  }
+                }
+                if (hit) uf_union(par, s0, s1);
+              }
+              if (FULL) {
+                unsigned lm = __ballot_sync(0xffffffffu, lng);
+                while (lm) {
+                  const int src = __ffs(lm) - 1;
+                  lm &= lm - 1u;
+                  const unsigned u0 = __shfl_sync(0xffffffffu, s0, src), u1 = __shfl_sync(0xffffffffu, e0, src),
+                                 v0 = __shfl_sync(0xffffffffu, s1, src),
+                                 v1 = __shfl_sync(0xffffffffu, lng ? et[j] : 0u, src);
+                  unsigned same = 0;  // joined meanwhile?
+                  if (lane == 0) same = uf_root(par, u0) == uf_root(par, v0);
+                  if (__shfl_sync(0xffffffffu, same, 0)) continue;
+                  bool any = false;
+                  for (unsigned ub = u0; ub < u1 && !any; ub += 32u) {
+                    const unsigned u = ub + (unsigned)lane;
+                    const float4 a = cube[perm[min(u, u1 - 1u)]];
+                    bool mine = false;
+                    for (unsigned v = v0; v < v1; v++) {
+                      tests++;
+                      mine = mine || fof_friends(a, cube[perm[v]], G.r2, G.rT);
+                      if (((v - v0) & 7u) == 7u && __any_sync(0xffffffffu, mine)) break;
+                    }
+                    any = __any_sync(0xffffffffu, mine);
+                  }
+                  if (any && lane == 0) uf_union(par, u0, v0);
+                  __syncwarp();
+                }
+              } else {
+                joined += (unsigned)__popc(__ballot_sync(0xffffffffu, hit));
+                if (joined >= LINK_SAMPLE) {  // warp-uniform
+                  oz = oy = ox = R + 1;
+                }
+              }
+            }
+      }
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    tests += __shfl_down_sync(0xffffffffu, tests, o);
+    pairs += __shfl_down_sync(0xffffffffu, pairs, o);
+  }
+  if (lane == 0) {
+    atomicAdd(counters, tests);
+    atomicAdd(counters + 1, pairs);
+  }
+}
+
+// A thread per record of the cells of up to LINK_BRUTE records, against every
+// record of the neighbouring such cells of higher index within reach, and
+// (FULL, cells the sort has not linked whole) the later records of its own
+// cell.  Testing all of them costs less than finding the linking cells within
+// reach: a test is a dozen FP32 operations on a record that the warp's other
+// lanes read too, where a search is a chain of dependent loads.  The sampled
+// pass stops at the first friend.  The particle that the run scan files under a
+// foreign cell looks at all its neighbours itself, since they do not find it in
+// its own.
+template <bool FULL>
+__global__ void __launch_bounds__(FOF_TPB) k_fof_rec_link(const unsigned *cs, long long n, FofGeo G,
+                                                          const unsigned *finv, const float4 *cube, unsigned quirk_pos,
+                                                          unsigned *par, unsigned long long *counters) {
+  const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  unsigned long long tests = 0, pairs = 0;
+  const float reach2 = (float)G.reach2, kf = (float)G.k;
+  if (s < n) {
+    const float4 a = cube[s];
+    int cx, cy, cz, f;
+    float x, y, z;
+    fof_axis(a.x, G, cx, f, x);
+    fof_axis(a.y, G, cy, f, y);
+    fof_axis(a.z, G, cz, f, z);
+    const unsigned long long own =
+        (unsigned long long)cx + (unsigned long long)G.nx * ((unsigned long long)cy + (unsigned long long)G.nx * cz);
+    const unsigned b0 = __ldg(cs + own), e0 = __ldg(cs + own + 1);
+    const bool quirk = (unsigned)s == quirk_pos;
+    if (quirk || e0 - b0 <= LINK_BRUTE) {
+      const unsigned p = finv[__float_as_uint(a.w) & ~PSOD_DEAD_BIT];
+      const unsigned myroot = FULL ? __ldcg(par + p) : 0u;
+      bool done = false;
+      auto visit = [&](unsigned t) {
+        const float4 v = cube[t];
+        tests++;
+        if (!fof_friends(a, v, G.r2, G.rT)) return;
+        const unsigned q = finv[__float_as_uint(v.w) & ~PSOD_DEAD_BIT];
+        if (FULL && __ldcg(par + q) == myroot) return;
+        uf_union(par, p, q);
+        done = !FULL;
+      };
+      if (FULL && !quirk && e0 - b0 > FOF_SMALL_CELL)
+        for (unsigned t = (unsigned)s + 1u; t < e0; t++) visit(t);
+      for (int dz = -1; dz <= 1 && !done; dz++) {
+        const float gz = fmaxf(dz < 0 ? z : (dz > 0 ? kf - z : 0.f), 0.f);
+        if (gz * gz > reach2) continue;
+        int tz = cz + dz;
+        tz = tz < 0 ? tz + G.nx : (tz >= G.nx ? tz - G.nx : tz);
+        for (int dy = -1; dy <= 1 && !done; dy++) {
+          const float gy = fmaxf(dy < 0 ? y : (dy > 0 ? kf - y : 0.f), 0.f);
+          const float g2 = gz * gz + gy * gy;
+          if (g2 > reach2) continue;
+          int ty = cy + dy;
+          ty = ty < 0 ? ty + G.nx : (ty >= G.nx ? ty - G.nx : ty);
+          for (int dx = -1; dx <= 1 && !done; dx++) {
+            const float gx = fmaxf(dx < 0 ? x : (dx > 0 ? kf - x : 0.f), 0.f);
+            if (g2 + gx * gx > reach2) continue;
+            int tx = cx + dx;
+            tx = tx < 0 ? tx + G.nx : (tx >= G.nx ? tx - G.nx : tx);
+            const unsigned long long c =
+                (unsigned long long)tx + (unsigned long long)G.nx * ((unsigned long long)ty + (unsigned long long)G.nx * tz);
+            if (c <= own && !quirk) continue;  // that cell visits this one
+            const unsigned b = __ldg(cs + c), e = __ldg(cs + c + 1);
+            if (b == e || (e - b > LINK_BRUTE && !quirk)) continue;
+            pairs++;
+            for (unsigned t = b; t < e && !done; t++) visit(t);
+          }
+        }
+      }
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    tests += __shfl_down_sync(0xffffffffu, tests, o);
+    pairs += __shfl_down_sync(0xffffffffu, pairs, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
     atomicAdd(counters, tests);
     atomicAdd(counters + 1, pairs);
   }
@@ -911,42 +1317,69 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
   PSOD_CUDA(c, cudaMemsetAsync(cnt, 0, 8 * sizeof(unsigned), c->stream));
   PSOD_CUDA(c, cudaMemsetAsync(ctr, 0, 4 * sizeof(unsigned long long), c->stream));
 
-  // 1. keys and the per-cell sort (big cells listed in aux2)
+  // 1. keys and the per-cell sort (large cells listed; at most n / (FOF_SMALL_CELL + 1))
   k_fof_keys<<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cube, n, G, key);
-  big = aux2;
+  unsigned *dense = nullptr;
+  const size_t big_cap = (size_t)n / (FOF_SMALL_CELL + 1) + 1;
+  if ((st = scratch(c, SLOT_FOF_BIGCELL, big_cap + (size_t)n / (LINK_BRUTE + 1) + 1, &big))) return st;
+  dense = big + big_cap;
   k_fof_sort_small<<<grid_for((long long)c->ncell), FOF_TPB, 0, c->stream>>>(
-      c->d_cell_start, c->ncell, key, c->d_cube, perm, skey, par, finv, big, cnt);
+      c->d_cell_start, c->ncell, key, c->d_cube, G, perm, skey, par, finv, aux1, big, cnt, dense, cnt + 2);
   const int nbins = k * k * k;
-  PSOD_CUDA(c, cudaFuncSetAttribute(k_fof_sort_big, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)(nbins * sizeof(unsigned))));
-  k_fof_sort_big<<<1184, FOF_TPB, nbins * sizeof(unsigned), c->stream>>>(c->d_cell_start, big, cnt, nbins, key,
-                                                                         c->d_cube, perm, skey, par, finv);
+  {
+    // bins, their parents and first records; the linking inside the cell is
+    // left to the passes when they do not fit
+    const size_t local_bytes = (size_t)nbins * (2 * sizeof(unsigned) + 3 * sizeof(float));
+    const bool local = local_bytes <= 200u * 1024u;
+    const size_t smem = local ? local_bytes : (size_t)nbins * sizeof(unsigned);
+    auto launch = [&](auto *kern) -> int {
+      PSOD_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      kern<<<1184, FOF_TPB, smem, c->stream>>>(c->d_cell_start, big, cnt, nbins, G, key, c->d_cube, perm, skey, par,
+                                               finv, aux1);
+      return PSOD_OK;
+    };
+    if ((st = local ? launch(k_fof_sort_big<true>) : launch(k_fof_sort_big<false>))) return st;
+  }
   PSOD_CUDA(c, cudaGetLastError());
-  // run heads: flags in aux1, their exclusive scan in aux2, then the list
-  k_fof_head_flags<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n, aux1);
-  if ((st = scan_u32(c, aux1, aux2, n, true))) return st;
-  unsigned nrun_u = 0;
-  PSOD_CUDA(c, cudaMemcpyAsync(&nrun_u, aux2 + n, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
-  PSOD_CUDA(c, cudaStreamSynchronize(c->stream));
-  const long long nrun = nrun_u;
-  unsigned *heads = nullptr, *bigrun = nullptr;
-  if ((st = scratch(c, SLOT_FOF_HEADS, (size_t)nrun + 1, &heads))) return st;
-  if ((st = scratch(c, SLOT_FOF_BIGRUN, (size_t)nrun + 1, &bigrun))) return st;
-  k_fof_head_list<<<grid_for(n), FOF_TPB, 0, c->stream>>>(aux1, aux2, n, heads);
-  PSOD_CUDA(c, cudaGetLastError());
+  // 2. linking: sampled pass, compression, full pass, compression.  Tables of
+  // both cells' linking cells where they fit shared memory (k <= 20, linking
+  // lengths from 0.09 cells), else runs that search the sorted keys
+  k_fof_count<<<148 * 8, FOF_TPB, 0, c->stream>>>(aux1, n, ctr + 2);
+  unsigned long long nrun = 0;
+  PSOD_CUDA(c, cudaMemcpyAsync(&nrun, ctr + 2, sizeof(nrun), cudaMemcpyDeviceToHost, c->stream));
   S.ms_sort = tm.stop();
-  S.fine_cells = nrun;
-
-  // 2. linking: sampled pass, compression, full pass, compression
-  k_fof_link_thread<false><<<148 * 8, FOF_TPB, 0, c->stream>>>(heads, nrun, G, c->d_cell_start, skey, perm,
-                                                               c->d_cube, par, bigrun, cnt + 1, ctr);
-  k_fof_link_warp<false><<<148 * 8, FOF_TPB, 0, c->stream>>>(heads, bigrun, cnt + 1, G, c->d_cell_start, skey,
-                                                             perm, c->d_cube, par, ctr);
-  k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n);
-  k_fof_link_thread<true><<<148 * 8, FOF_TPB, 0, c->stream>>>(heads, nrun, G, c->d_cell_start, skey, perm,
-                                                              c->d_cube, par, bigrun, cnt + 1, ctr);
-  k_fof_link_warp<true><<<148 * 8, FOF_TPB, 0, c->stream>>>(heads, bigrun, cnt + 1, G, c->d_cell_start, skey,
-                                                            perm, c->d_cube, par, ctr);
+  S.fine_cells = (int64_t)nrun;
+  const size_t tab_bytes = 3 * sizeof(unsigned) * ((size_t)nbins + (FOF_TPB / 32) * (size_t)R * k * k);
+  if (tab_bytes <= 210u * 1024u) {
+    auto link = [&](auto *kern) -> int {
+      PSOD_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab_bytes));
+      kern<<<148 * 8, FOF_TPB, tab_bytes, c->stream>>>(c->d_cell_start, dense, cnt + 2, nbins, G, skey, perm,
+                                                       c->d_cube, par, ctr);
+      return PSOD_OK;
+    };
+    if ((st = link(k_fof_cell_link<false>))) return st;
+    const unsigned qpos = c->has_quirk ? c->quirk_pos : 0xffffffffu;
+    k_fof_rec_link<false><<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cell_start, n, G, finv, c->d_cube, qpos, par, ctr);
+    k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n);
+    if ((st = link(k_fof_cell_link<true>))) return st;
+    k_fof_rec_link<true><<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cell_start, n, G, finv, c->d_cube, qpos, par, ctr);
+  } else {
+    // run heads: flags in aux1, their exclusive scan in aux2, then the list
+    unsigned *heads = nullptr, *bigrun = nullptr;
+    if ((st = scan_u32(c, aux1, aux2, n, true))) return st;
+    if ((st = scratch(c, SLOT_FOF_HEADS, (size_t)nrun + 1, &heads))) return st;
+    if ((st = scratch(c, SLOT_FOF_BIGRUN, (size_t)nrun + 1, &bigrun))) return st;
+    k_fof_head_list<<<grid_for(n), FOF_TPB, 0, c->stream>>>(aux1, aux2, n, heads);
+    k_fof_link_thread<false><<<148 * 8, FOF_TPB, 0, c->stream>>>(heads, (long long)nrun, G, c->d_cell_start, skey, perm,
+                                                                 c->d_cube, par, bigrun, cnt + 1, ctr);
+    k_fof_link_warp<false><<<148 * 8, FOF_TPB, 0, c->stream>>>(heads, bigrun, cnt + 1, G, c->d_cell_start, skey,
+                                                               perm, c->d_cube, par, ctr);
+    k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n);
+    k_fof_link_thread<true><<<148 * 8, FOF_TPB, 0, c->stream>>>(heads, (long long)nrun, G, c->d_cell_start, skey, perm,
+                                                                c->d_cube, par, bigrun, cnt + 1, ctr);
+    k_fof_link_warp<true><<<148 * 8, FOF_TPB, 0, c->stream>>>(heads, bigrun, cnt + 1, G, c->d_cell_start, skey,
+                                                              perm, c->d_cube, par, ctr);
+  }
   k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n);
   PSOD_CUDA(c, cudaGetLastError());
   S.ms_link = tm.stop();
@@ -1053,7 +1486,7 @@ int psod_fof_release(psod_ctx *c) {
   if (!c) return PSOD_ERR_ARG;
   cudaSetDevice(c->device);
   for (int s : {SLOT_FOF_KEY, SLOT_FOF_SKEY, SLOT_FOF_PERM, SLOT_FOF_PAR, SLOT_FOF_INV, SLOT_FOF_AUX1, SLOT_FOF_AUX2,
-                SLOT_FOF_HEADS, SLOT_FOF_BIGRUN, SLOT_FOF_HPOS, SLOT_FOF_HKEY, SLOT_FOF_HROOT, SLOT_FOF_MKEY,
+                SLOT_FOF_HEADS, SLOT_FOF_BIGRUN, SLOT_FOF_BIGCELL, SLOT_FOF_HPOS, SLOT_FOF_HKEY, SLOT_FOF_HROOT, SLOT_FOF_MKEY,
                 SLOT_FOF_MCOUNT})
     free_scratch_slot(c, s);
   return PSOD_OK;

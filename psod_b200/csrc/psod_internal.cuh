@@ -323,6 +323,7 @@ enum : int {
   SLOT_FOF_AUX1,        // fof: head flags, then component sizes
   SLOT_FOF_AUX2,        // fof: large cells and head scan, then lowest index / halo rank
   SLOT_FOF_HEADS,       // fof: run heads (+ end)
+  SLOT_FOF_BIGCELL,     // fof: large SOD cells
   SLOT_FOF_BIGRUN,      // fof: runs linked by a warp
   SLOT_FOF_HPOS,        // fof: flag scans
   SLOT_FOF_HKEY,        // fof: halo labels (sort keys)
