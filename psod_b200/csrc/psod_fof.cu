@@ -858,19 +858,18 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_cell_link(const unsigned *cs, c
   }
 }
 
-// A thread per record of the cells of up to LINK_BRUTE records, against every
-// record of the neighbouring such cells of higher index within reach, and
-// (FULL, cells the sort has not linked whole) the later records of its own
-// cell.  Testing all of them costs less than finding the linking cells within
-// reach: a test is a dozen FP32 operations on a record that the warp's other
-// lanes read too, where a search is a chain of dependent loads.  The sampled
-// pass stops at the first friend.  The particle that the run scan files under a
-// foreign cell looks at all its neighbours itself, since they do not find it in
-// its own.
-template <bool FULL>
-__global__ void __launch_bounds__(FOF_TPB) k_fof_rec_link(const unsigned *cs, long long n, FofGeo G,
-                                                          const unsigned *finv, const float4 *cube, unsigned quirk_pos,
-                                                          unsigned *par, unsigned long long *counters) {
+// Cells of up to LINK_BRUTE records are linked record by record.  Testing all
+// records within reach costs less than finding their linking cells: a test is
+// a dozen FP32 operations, a search a chain of dependent loads.
+//
+// k_fof_small_link: a thread per record of the small cells (those the sort has
+// linked whole), against the records of the neighbouring small cells of higher
+// index within reach.  The particle that the run scan files under a foreign
+// cell looks at all its neighbours itself: they do not find it in its own.
+__global__ void __launch_bounds__(FOF_TPB) k_fof_small_link(const unsigned *cs, long long n, FofGeo G,
+                                                            const unsigned *finv, const float4 *cube,
+                                                            unsigned quirk_pos, unsigned *par,
+                                                            unsigned long long *counters) {
   const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long tests = 0, pairs = 0;
   const float reach2 = (float)G.reach2, kf = (float)G.k;
@@ -883,35 +882,21 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_rec_link(const unsigned *cs, lo
     fof_axis(a.z, G, cz, f, z);
     const unsigned long long own =
         (unsigned long long)cx + (unsigned long long)G.nx * ((unsigned long long)cy + (unsigned long long)G.nx * cz);
-    const unsigned b0 = __ldg(cs + own), e0 = __ldg(cs + own + 1);
     const bool quirk = (unsigned)s == quirk_pos;
-    if (quirk || e0 - b0 <= LINK_BRUTE) {
+    if (quirk || __ldg(cs + own + 1) - __ldg(cs + own) <= FOF_SMALL_CELL) {
       const unsigned p = finv[__float_as_uint(a.w) & ~PSOD_DEAD_BIT];
-      const unsigned myroot = FULL ? __ldcg(par + p) : 0u;
-      bool done = false;
-      auto visit = [&](unsigned t) {
-        const float4 v = cube[t];
-        tests++;
-        if (!fof_friends(a, v, G.r2, G.rT)) return;
-        const unsigned q = finv[__float_as_uint(v.w) & ~PSOD_DEAD_BIT];
-        if (FULL && __ldcg(par + q) == myroot) return;
-        uf_union(par, p, q);
-        done = !FULL;
-      };
-      if (FULL && !quirk && e0 - b0 > FOF_SMALL_CELL)
-        for (unsigned t = (unsigned)s + 1u; t < e0; t++) visit(t);
-      for (int dz = -1; dz <= 1 && !done; dz++) {
+      for (int dz = -1; dz <= 1; dz++) {
         const float gz = fmaxf(dz < 0 ? z : (dz > 0 ? kf - z : 0.f), 0.f);
         if (gz * gz > reach2) continue;
         int tz = cz + dz;
         tz = tz < 0 ? tz + G.nx : (tz >= G.nx ? tz - G.nx : tz);
-        for (int dy = -1; dy <= 1 && !done; dy++) {
+        for (int dy = -1; dy <= 1; dy++) {
           const float gy = fmaxf(dy < 0 ? y : (dy > 0 ? kf - y : 0.f), 0.f);
           const float g2 = gz * gz + gy * gy;
           if (g2 > reach2) continue;
           int ty = cy + dy;
           ty = ty < 0 ? ty + G.nx : (ty >= G.nx ? ty - G.nx : ty);
-          for (int dx = -1; dx <= 1 && !done; dx++) {
+          for (int dx = -1; dx <= 1; dx++) {
             const float gx = fmaxf(dx < 0 ? x : (dx > 0 ? kf - x : 0.f), 0.f);
             if (g2 + gx * gx > reach2) continue;
             int tx = cx + dx;
@@ -920,9 +905,13 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_rec_link(const unsigned *cs, lo
                 (unsigned long long)tx + (unsigned long long)G.nx * ((unsigned long long)ty + (unsigned long long)G.nx * tz);
             if (c <= own && !quirk) continue;  // that cell visits this one
             const unsigned b = __ldg(cs + c), e = __ldg(cs + c + 1);
-            if (b == e || (e - b > LINK_BRUTE && !quirk)) continue;
+            if (b == e || (e - b > FOF_SMALL_CELL && !quirk)) continue;
             pairs++;
-            for (unsigned t = b; t < e && !done; t++) visit(t);
+            for (unsigned t = b; t < e; t++) {
+              const float4 v = cube[t];
+              tests++;
+              if (fof_friends(a, v, G.r2, G.rT)) uf_union(par, p, finv[__float_as_uint(v.w) & ~PSOD_DEAD_BIT]);
+            }
           }
         }
       }
@@ -933,6 +922,108 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_rec_link(const unsigned *cs, lo
     pairs += __shfl_down_sync(0xffffffffu, pairs, o);
   }
   if ((threadIdx.x & 31) == 0) {
+    atomicAdd(counters, tests);
+    atomicAdd(counters + 1, pairs);
+  }
+}
+
+// k_fof_mid_link: a warp per cell of more than FOF_SMALL_CELL and up to LINK_BRUTE
+// records, against its small neighbours, the like of higher index and (FULL)
+// itself.  Of 32 of the cell's records a few lie within reach of a given
+// neighbour: the lanes hold 32 of the neighbour's records, and those few are
+// broadcast to them in turn (a lane per own record walked every neighbour with
+// a fifth of its lanes).  The sampled pass stops at the first friend of each 32
+// records and neighbour.
+template <bool FULL>
+__global__ void __launch_bounds__(FOF_TPB) k_fof_mid_link(const unsigned *cs, const unsigned *big, const unsigned *nbig,
+                                                          FofGeo G, const unsigned *finv, const float4 *cube,
+                                                          unsigned *par, unsigned *next, unsigned long long *counters) {
+  const int lane = threadIdx.x & 31;
+  const float reach2 = (float)G.reach2, kf = (float)G.k;
+  const unsigned nb = *nbig;
+  unsigned long long tests = 0, pairs = 0;
+  while (true) {
+    unsigned it = 0;
+    if (lane == 0) it = atomicAdd(next, 1u);
+    it = __shfl_sync(0xffffffffu, it, 0);
+    if (it >= nb) break;
+    const unsigned own = big[it];
+    const unsigned b0 = __ldg(cs + own), e0 = __ldg(cs + own + 1);
+    if (e0 - b0 > LINK_BRUTE) continue;
+    const int cx = (int)(own % (unsigned)G.nx), cy = (int)((own / (unsigned)G.nx) % (unsigned)G.nx),
+              cz = (int)(own / ((unsigned)G.nx * (unsigned)G.nx));
+    // lane m < 27: the records of neighbour m this cell visits
+    unsigned nbeg = 0, nend = 0;
+    if (lane < 27 && (lane != 13 || FULL)) {
+      int tx = cx + lane % 3 - 1, ty = cy + (lane / 3) % 3 - 1, tz = cz + lane / 9 - 1;
+      tx = tx < 0 ? tx + G.nx : (tx >= G.nx ? tx - G.nx : tx);
+      ty = ty < 0 ? ty + G.nx : (ty >= G.nx ? ty - G.nx : ty);
+      tz = tz < 0 ? tz + G.nx : (tz >= G.nx ? tz - G.nx : tz);
+      const unsigned c = (unsigned)tx + (unsigned)G.nx * ((unsigned)ty + (unsigned)G.nx * (unsigned)tz);
+      nbeg = __ldg(cs + c);
+      nend = __ldg(cs + c + 1);
+      const unsigned cnt = nend - nbeg;
+      if (cnt > LINK_BRUTE || (cnt > FOF_SMALL_CELL && c < own)) nend = nbeg;
+    }
+    for (unsigned s0 = b0; s0 < e0; s0 += 32u) {
+      const unsigned s = s0 + (unsigned)lane;
+      const bool have = s < e0;
+      const float4 a = cube[have ? s : e0 - 1u];
+      int c, f;
+      float x, y, z;
+      fof_axis(a.x, G, c, f, x);
+      fof_axis(a.y, G, c, f, y);
+      fof_axis(a.z, G, c, f, z);
+      const unsigned p = finv[__float_as_uint(a.w) & ~PSOD_DEAD_BIT];
+      const unsigned root = FULL ? __ldcg(par + p) : 0u;
+      for (int m = 0; m < 27; m++) {
+        const unsigned b = __shfl_sync(0xffffffffu, nbeg, m), e = __shfl_sync(0xffffffffu, nend, m);
+        if (b == e) continue;
+        const bool self = FULL && m == 13;
+        const int dx = m % 3 - 1, dy = (m / 3) % 3 - 1, dz = m / 9 - 1;
+        const float gx = fmaxf(dx < 0 ? x : (dx > 0 ? kf - x : 0.f), 0.f), gy = fmaxf(dy < 0 ? y : (dy > 0 ? kf - y : 0.f), 0.f),
+                    gz = fmaxf(dz < 0 ? z : (dz > 0 ? kf - z : 0.f), 0.f);
+        const unsigned act = __ballot_sync(0xffffffffu, have && gx * gx + gy * gy + gz * gz <= reach2);
+        if (!act) continue;
+        if (lane == 0) pairs += (unsigned)__popc(act);
+        bool met = false;
+        for (unsigned t0 = self ? s0 : b; t0 < e && !met; t0 += 32u) {
+          const unsigned t = t0 + (unsigned)lane;
+          const bool there = t < e;
+          const float4 v = cube[there ? t : e - 1u];
+          unsigned q = 0xffffffffu, rq = 0;  // the record's position and group, when first needed
+          for (unsigned left = act; left; left &= left - 1u) {
+            const int src = __ffs(left) - 1;
+            const float4 u = make_float4(__shfl_sync(0xffffffffu, a.x, src), __shfl_sync(0xffffffffu, a.y, src),
+                                         __shfl_sync(0xffffffffu, a.z, src), 0.f);
+            const unsigned pu = __shfl_sync(0xffffffffu, p, src), ru = __shfl_sync(0xffffffffu, root, src);
+            const bool hit = there && (!self || t > s0 + (unsigned)src) && fof_friends(u, v, G.r2, G.rT);
+            if (hit) {
+              if (q == 0xffffffffu) {
+                q = finv[__float_as_uint(v.w) & ~PSOD_DEAD_BIT];
+                if (FULL) rq = __ldcg(par + q);
+              }
+              if (!FULL) {
+                uf_union(par, pu, q);
+              } else if (rq != ru) {
+                uf_union(par, pu, q);
+              }
+            }
+            if (!FULL) {
+              met = __any_sync(0xffffffffu, hit);
+              if (met) break;
+            }
+          }
+          if (there) tests += (unsigned)__popc(act);
+        }
+      }
+    }
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    tests += __shfl_down_sync(0xffffffffu, tests, o);
+    pairs += __shfl_down_sync(0xffffffffu, pairs, o);
+  }
+  if (lane == 0) {
     atomicAdd(counters, tests);
     atomicAdd(counters + 1, pairs);
   }
@@ -1359,10 +1450,13 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
     };
     if ((st = link(k_fof_cell_link<false>))) return st;
     const unsigned qpos = c->has_quirk ? c->quirk_pos : 0xffffffffu;
-    k_fof_rec_link<false><<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cell_start, n, G, finv, c->d_cube, qpos, par, ctr);
+    k_fof_mid_link<false><<<148 * 8, FOF_TPB, 0, c->stream>>>(c->d_cell_start, big, cnt, G, finv, c->d_cube, par, cnt + 3,
+                                                              ctr);
+    k_fof_small_link<<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cell_start, n, G, finv, c->d_cube, qpos, par, ctr);
     k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n);
     if ((st = link(k_fof_cell_link<true>))) return st;
-    k_fof_rec_link<true><<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cell_start, n, G, finv, c->d_cube, qpos, par, ctr);
+    k_fof_mid_link<true><<<148 * 8, FOF_TPB, 0, c->stream>>>(c->d_cell_start, big, cnt, G, finv, c->d_cube, par, cnt + 4,
+                                                             ctr);
   } else {
     // run heads: flags in aux1, their exclusive scan in aux2, then the list
     unsigned *heads = nullptr, *bigrun = nullptr;
