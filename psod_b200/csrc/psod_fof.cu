@@ -48,6 +48,7 @@ namespace {
 constexpr int FOF_TPB = 256;
 constexpr unsigned FOF_SMALL_CELL = 16;  // records a thread sorts itself
 constexpr unsigned LINK_BRUTE = 512;     // records of a cell linked record by record
+constexpr unsigned LINK_SPLIT = 64;      // ... a warp each up to here, above a warp per 32 records
 constexpr unsigned FOF_THREAD_RUN = 4;   // runs a thread links; longer ones go to a warp
 constexpr int FOF_MAX_OFF = 171;         // half of the 7^3 - 1 neighbour offsets
 constexpr unsigned FOF_WARP_HALO = 2048; // halos whose observables a warp computes; larger: a CTA
@@ -170,8 +171,8 @@ __global__ void k_fof_keys(const float4 *cube, long long n, FofGeo G, unsigned s
 // position starts with the root of its group inside the cell.
 __global__ void k_fof_sort_small(const unsigned *cs, unsigned long long ncell, const unsigned short *key,
                                  const float4 *cube, FofGeo G, unsigned *perm, unsigned short *skey, unsigned *par,
-                                 unsigned *finv, unsigned *flag, unsigned *big, unsigned *nbig, unsigned *dense,
-                                 unsigned *ndense) {
+                                 unsigned *finv, unsigned *flag, unsigned *big, unsigned *nbig, unsigned *mid,
+                                 unsigned *nmid, unsigned *dense, unsigned *ndense) {
   const unsigned long long c = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (c >= ncell) return;
   const unsigned b = cs[c], e = cs[c + 1], m = e - b;
@@ -179,6 +180,7 @@ __global__ void k_fof_sort_small(const unsigned *cs, unsigned long long ncell, c
   if (m > FOF_SMALL_CELL) {
     big[atomicAdd(nbig, 1u)] = (unsigned)c;
     if (m > LINK_BRUTE) dense[atomicAdd(ndense, 1u)] = (unsigned)c;
+    else if (m > LINK_SPLIT) mid[atomicAdd(nmid, 1u)] = (unsigned)c;
     return;
   }
   unsigned kk[FOF_SMALL_CELL], ss[FOF_SMALL_CELL];
@@ -682,6 +684,7 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_link_warp(const unsigned *heads
 // neighbour all of whose runs in reach are of the cell's one group is skipped.
 // FOF_MS.
 constexpr unsigned LINK_SAMPLE = 2;
+constexpr unsigned LINK_SEARCH = 1024;  // records from which a neighbour's table is searched, not walked
 constexpr unsigned LINK_SERIAL = 64;  // record pairs a lane tests itself
 
 template <bool FULL>
@@ -750,7 +753,29 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_cell_link(const unsigned *cs, c
         for (int i = lane; i < qx * qy * qz; i += 32) sb[i] = NONE;
         __syncwarp();
         bool other = false;
-        for (unsigned p = b2 + (unsigned)lane; p < e2; p += 32u) {
+        if (e2 - b2 > LINK_SEARCH) {
+          // a search per linking cell of the region instead of a walk over all records
+          auto lower = [&](unsigned key) {
+            unsigned lo = b2, hi = e2;
+            while (lo < hi) {
+              const unsigned mid = (lo + hi) >> 1;
+              if (__ldg(skey + mid) < key) lo = mid + 1;
+              else hi = mid;
+            }
+            return lo;
+          };
+          for (int j = lane; j < qx * qy * qz; j += 32) {
+            const unsigned kv =
+                (unsigned)((bx0 + j % qx) + k * ((by0 + (j / qx) % qy) + k * (bz0 + j / (qx * qy))));
+            const unsigned p = lower(kv);
+            if (p >= e2 || __ldg(skey + p) != kv) continue;
+            sb[j] = p;
+            eb[j] = lower(kv + 1u);
+            const unsigned r = __ldcg(par + p);
+            rb[j] = r;
+            if (r != single) other = true;
+          }
+        } else for (unsigned p = b2 + (unsigned)lane; p < e2; p += 32u) {
           const unsigned kv = skey[p];
           const int lx = (int)(kv % (unsigned)k) - bx0, ly = (int)((kv / (unsigned)k) % (unsigned)k) - by0,
                     lz = (int)(kv / (unsigned)(k * k)) - bz0;
@@ -933,23 +958,38 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_small_link(const unsigned *cs, 
 // neighbour: the lanes hold 32 of the neighbour's records, and those few are
 // broadcast to them in turn (a lane per own record walked every neighbour with
 // a fifth of its lanes).  The sampled pass stops at the first friend of each 32
-// records and neighbour.
+// records and neighbour; the full pass skips 32 records of the same one group.
 template <bool FULL>
 __global__ void __launch_bounds__(FOF_TPB) k_fof_mid_link(const unsigned *cs, const unsigned *big, const unsigned *nbig,
-                                                          FofGeo G, const unsigned *finv, const float4 *cube,
-                                                          unsigned *par, unsigned *next, unsigned long long *counters) {
+                                                          const unsigned *mid, const unsigned *nmid, FofGeo G, const unsigned *finv, const float4 *cube,
+                                                          const unsigned *slot_root, unsigned *par, unsigned *next,
+                                                          unsigned long long *counters) {
   const int lane = threadIdx.x & 31;
   const float reach2 = (float)G.reach2, kf = (float)G.k;
-  const unsigned nb = *nbig;
+  // items: the cells of up to LINK_SPLIT records whole, the others 32 records each
+  constexpr unsigned PARTS = LINK_BRUTE / 32u, GRAB = 4u;
+  const unsigned nb = *nbig, nitem = nb + *nmid * PARTS;
   unsigned long long tests = 0, pairs = 0;
+  unsigned it = 0, left_items = 0;
   while (true) {
-    unsigned it = 0;
-    if (lane == 0) it = atomicAdd(next, 1u);
-    it = __shfl_sync(0xffffffffu, it, 0);
-    if (it >= nb) break;
-    const unsigned own = big[it];
-    const unsigned b0 = __ldg(cs + own), e0 = __ldg(cs + own + 1);
-    if (e0 - b0 > LINK_BRUTE) continue;
+    if (left_items == 0) {
+      if (lane == 0) it = atomicAdd(next, GRAB);
+      it = __shfl_sync(0xffffffffu, it, 0);
+      left_items = GRAB;
+    } else {
+      it++;
+    }
+    left_items--;
+    if (it >= nitem) break;
+    const unsigned own = it < nb ? big[it] : mid[(it - nb) / PARTS];
+    unsigned b0 = __ldg(cs + own), e0 = __ldg(cs + own + 1);
+    if (it < nb) {
+      if (e0 - b0 > LINK_SPLIT) continue;
+    } else {
+      b0 += 32u * ((it - nb) % PARTS);
+      if (b0 >= e0) continue;
+      e0 = min(e0, b0 + 32u);
+    }
     const int cx = (int)(own % (unsigned)G.nx), cy = (int)((own / (unsigned)G.nx) % (unsigned)G.nx),
               cz = (int)(own / ((unsigned)G.nx * (unsigned)G.nx));
     // lane m < 27: the records of neighbour m this cell visits
@@ -975,11 +1015,13 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_mid_link(const unsigned *cs, co
       fof_axis(a.y, G, c, f, y);
       fof_axis(a.z, G, c, f, z);
       const unsigned p = finv[__float_as_uint(a.w) & ~PSOD_DEAD_BIT];
-      const unsigned root = FULL ? __ldcg(par + p) : 0u;
+      const unsigned root = FULL ? slot_root[have ? s : e0 - 1u] : 0u;
+      const unsigned one = __shfl_sync(0xffffffffu, root, 0);  // these records' group, when they have one
+      const bool uniform = FULL && __all_sync(0xffffffffu, root == one);
       for (int m = 0; m < 27; m++) {
         const unsigned b = __shfl_sync(0xffffffffu, nbeg, m), e = __shfl_sync(0xffffffffu, nend, m);
         if (b == e) continue;
-        const bool self = FULL && m == 13;
+        const bool self = FULL && m == 13;  // e is the whole cell's end here
         const int dx = m % 3 - 1, dy = (m / 3) % 3 - 1, dz = m / 9 - 1;
         const float gx = fmaxf(dx < 0 ? x : (dx > 0 ? kf - x : 0.f), 0.f), gy = fmaxf(dy < 0 ? y : (dy > 0 ? kf - y : 0.f), 0.f),
                     gz = fmaxf(dz < 0 ? z : (dz > 0 ? kf - z : 0.f), 0.f);
@@ -990,25 +1032,16 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_mid_link(const unsigned *cs, co
         for (unsigned t0 = self ? s0 : b; t0 < e && !met; t0 += 32u) {
           const unsigned t = t0 + (unsigned)lane;
           const bool there = t < e;
+          const unsigned rq = FULL ? slot_root[there ? t : e - 1u] : 0u;
           const float4 v = cube[there ? t : e - 1u];
-          unsigned q = 0xffffffffu, rq = 0;  // the record's position and group, when first needed
+          if (uniform && !__any_sync(0xffffffffu, there && rq != one)) continue;  // all of one group
           for (unsigned left = act; left; left &= left - 1u) {
             const int src = __ffs(left) - 1;
             const float4 u = make_float4(__shfl_sync(0xffffffffu, a.x, src), __shfl_sync(0xffffffffu, a.y, src),
                                          __shfl_sync(0xffffffffu, a.z, src), 0.f);
             const unsigned pu = __shfl_sync(0xffffffffu, p, src), ru = __shfl_sync(0xffffffffu, root, src);
             const bool hit = there && (!self || t > s0 + (unsigned)src) && fof_friends(u, v, G.r2, G.rT);
-            if (hit) {
-              if (q == 0xffffffffu) {
-                q = finv[__float_as_uint(v.w) & ~PSOD_DEAD_BIT];
-                if (FULL) rq = __ldcg(par + q);
-              }
-              if (!FULL) {
-                uf_union(par, pu, q);
-              } else if (rq != ru) {
-                uf_union(par, pu, q);
-              }
-            }
+            if (hit && (!FULL || rq != ru)) uf_union(par, pu, finv[__float_as_uint(v.w) & ~PSOD_DEAD_BIT]);
             if (!FULL) {
               met = __any_sync(0xffffffffu, hit);
               if (met) break;
@@ -1031,9 +1064,13 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_mid_link(const unsigned *cs, co
 
 // every position points at its component's root (no unions run meanwhile;
 // each thread stores only its own position's entry)
-__global__ void k_fof_compress(unsigned *par, long long n) {
+// slot_root, when given, gets the roots by cube slot
+__global__ void k_fof_compress(unsigned *par, long long n, const unsigned *perm, unsigned *slot_root) {
   const long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < n) __stcg(par + p, uf_root(par, (unsigned)p));
+  if (p >= n) return;
+  const unsigned r = uf_root(par, (unsigned)p);
+  __stcg(par + p, r);
+  if (slot_root) slot_root[perm[p]] = r;
 }
 
 // ---------------------------------------------------------------------------
@@ -1410,12 +1447,11 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
 
   // 1. keys and the per-cell sort (large cells listed; at most n / (FOF_SMALL_CELL + 1))
   k_fof_keys<<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cube, n, G, key);
-  unsigned *dense = nullptr;
-  const size_t big_cap = (size_t)n / (FOF_SMALL_CELL + 1) + 1;
-  if ((st = scratch(c, SLOT_FOF_BIGCELL, big_cap + (size_t)n / (LINK_BRUTE + 1) + 1, &big))) return st;
-  dense = big + big_cap;
+  const size_t big_cap = (size_t)n / (FOF_SMALL_CELL + 1) + 1, mid_cap = (size_t)n / (LINK_SPLIT + 1) + 1;
+  if ((st = scratch(c, SLOT_FOF_BIGCELL, big_cap + mid_cap + (size_t)n / (LINK_BRUTE + 1) + 1, &big))) return st;
+  unsigned *mid = big + big_cap, *dense = mid + mid_cap;
   k_fof_sort_small<<<grid_for((long long)c->ncell), FOF_TPB, 0, c->stream>>>(
-      c->d_cell_start, c->ncell, key, c->d_cube, G, perm, skey, par, finv, aux1, big, cnt, dense, cnt + 2);
+      c->d_cell_start, c->ncell, key, c->d_cube, G, perm, skey, par, finv, aux1, big, cnt, mid, cnt + 5, dense, cnt + 2);
   const int nbins = k * k * k;
   {
     // bins, their parents and first records; the linking inside the cell is
@@ -1450,13 +1486,13 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
     };
     if ((st = link(k_fof_cell_link<false>))) return st;
     const unsigned qpos = c->has_quirk ? c->quirk_pos : 0xffffffffu;
-    k_fof_mid_link<false><<<148 * 8, FOF_TPB, 0, c->stream>>>(c->d_cell_start, big, cnt, G, finv, c->d_cube, par, cnt + 3,
-                                                              ctr);
+    k_fof_mid_link<false><<<148 * 8, FOF_TPB, 0, c->stream>>>(c->d_cell_start, big, cnt, mid, cnt + 5, G, finv, c->d_cube,
+                                                              nullptr, par, cnt + 3, ctr);
     k_fof_small_link<<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cell_start, n, G, finv, c->d_cube, qpos, par, ctr);
-    k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n);
+    k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n, perm, aux2);
     if ((st = link(k_fof_cell_link<true>))) return st;
-    k_fof_mid_link<true><<<148 * 8, FOF_TPB, 0, c->stream>>>(c->d_cell_start, big, cnt, G, finv, c->d_cube, par, cnt + 4,
-                                                             ctr);
+    k_fof_mid_link<true><<<148 * 8, FOF_TPB, 0, c->stream>>>(c->d_cell_start, big, cnt, mid, cnt + 5, G, finv, c->d_cube,
+                                                             aux2, par, cnt + 4, ctr);
   } else {
     // run heads: flags in aux1, their exclusive scan in aux2, then the list
     unsigned *heads = nullptr, *bigrun = nullptr;
@@ -1468,13 +1504,13 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
                                                                  c->d_cube, par, bigrun, cnt + 1, ctr);
     k_fof_link_warp<false><<<148 * 8, FOF_TPB, 0, c->stream>>>(heads, bigrun, cnt + 1, G, c->d_cell_start, skey,
                                                                perm, c->d_cube, par, ctr);
-    k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n);
+    k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n, perm, nullptr);
     k_fof_link_thread<true><<<148 * 8, FOF_TPB, 0, c->stream>>>(heads, (long long)nrun, G, c->d_cell_start, skey, perm,
                                                                 c->d_cube, par, bigrun, cnt + 1, ctr);
     k_fof_link_warp<true><<<148 * 8, FOF_TPB, 0, c->stream>>>(heads, bigrun, cnt + 1, G, c->d_cell_start, skey,
                                                               perm, c->d_cube, par, ctr);
   }
-  k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n);
+  k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n, perm, nullptr);
   PSOD_CUDA(c, cudaGetLastError());
   S.ms_link = tm.stop();
 
