@@ -48,6 +48,8 @@ namespace {
 constexpr int FOF_TPB = 256;
 constexpr unsigned FOF_SMALL_CELL = 16;  // records a thread sorts itself
 constexpr unsigned LINK_BRUTE = 512;     // records of a cell linked record by record
+constexpr int LINK_TABLE_K = 12;          // linking cells a SOD cell and axis up to which cells are linked by tables
+constexpr long long LINK_TABLE_N = 1 << 18;  // ... in boxes of at least this many particles
 constexpr unsigned LINK_SPLIT = 64;      // ... a warp each up to here, above a warp per 32 records
 constexpr unsigned FOF_THREAD_RUN = 4;   // runs a thread links; longer ones go to a warp
 constexpr int FOF_MAX_OFF = 171;         // half of the 7^3 - 1 neighbour offsets
@@ -382,9 +384,7 @@ __device__ __forceinline__ RunGeo run_geo(float4 v, const FofGeo &G, float lo[3]
   return r;
 }
 
-// the run of linking cell (run origin + offset o), or an empty range; false
-// too where the other run looks at this one: of two SOD cells the one with the
-// lower index, inside a cell the run that precedes in (z, y, x)
+// the run of linking cell (run origin + offset o), or an empty range
 __device__ __forceinline__ bool find_run(const RunGeo &u, int ox, int oy, int oz, const FofGeo &G, const unsigned *cs,
                                          const unsigned short *skey, unsigned &vlo, unsigned &vhi) {
   int tx = u.fx + ox, ty = u.fy + oy, tz = u.fz + oz;
@@ -399,10 +399,6 @@ __device__ __forceinline__ bool find_run(const RunGeo &u, int ox, int oy, int oz
   cz = cz < 0 ? cz + G.nx : (cz >= G.nx ? cz - G.nx : cz);
   const unsigned long long c =
       (unsigned long long)cx + (unsigned long long)G.nx * ((unsigned long long)cy + (unsigned long long)G.nx * cz);
-  const unsigned long long own =
-      (unsigned long long)u.cx + (unsigned long long)G.nx * ((unsigned long long)u.cy + (unsigned long long)G.nx * u.cz);
-  const bool after = oz > 0 || (oz == 0 && (oy > 0 || (oy == 0 && ox > 0)));
-  if (c == own ? !after : c < own) return false;
   const unsigned lo = __ldg(cs + c), hi = __ldg(cs + c + 1);
   if (lo == hi) return false;
   const unsigned short kv = (unsigned short)(tx + G.k * (ty + G.k * tz));
@@ -444,29 +440,27 @@ __device__ __forceinline__ float box_gap2(const RunGeo &u, int ox, int oy, int o
   return gx * gx + gy * gy + gz * gz;
 }
 
-// Linking runs in two passes (the sampling scheme of Afforest, Sutton et
-// al. 2018).  The sort has joined the runs inside each SOD cell (all of a small
-// cell's, most of a large one's).  The first pass joins each short run to at
-// most FOF_SAMPLE friends in neighbouring SOD cells and each long run to the
-// friends among FOF_SAMPLE_WARP neighbouring runs of other groups, which builds
-// most of every large group; after a compression every position points at its
-// root, so in the full pass a neighbour with the same parent is skipped with
-// two loads instead of two path walks.  All passes test the same pairs'
-// friendship, so the components are the same as without sampling.
-constexpr int FOF_SAMPLE = 1;       // friends a thread's run joins in the first pass
+// Fine linking cells (more than LINK_TABLE_K a SOD cell and axis): runs linked
+// through the sorted keys, in two passes (the sampling scheme of Afforest, Sutton et
+// al. 2018).  The first pass joins each short run to at most FOF_SAMPLE
+// friends and each long run to the friends among FOF_SAMPLE_WARP
+// neighbouring runs, which already builds most of every large group (one
+// friend per run, or six, measured slower at 512^3 and 1024^3); after
+// a compression every position points at its root, so in the full pass a
+// neighbour run with the same parent is skipped with two loads instead of
+// two path walks.  Both passes test the same pairs' friendship, so the
+// components are the same as without sampling.
+constexpr int FOF_SAMPLE = 3;       // friends a thread's run joins in the first pass
 constexpr int FOF_SAMPLE_WARP = 2;  // neighbour runs a warp's run examines in the first pass
 
 // A thread per run of up to FOF_THREAD_RUN records; longer runs are listed
-// (in the first pass) for k_fof_link_warp.  The SOD cells within reach of the
-// run's records are visited, of each pair of cells the one with the lower
-// index visiting the other.  A cell of up to FOF_SMALL_CELL records is tested
-// record by record; in a larger one the linking cells within reach form one
-// key range per row, found with one search.  In the full pass a record whose
-// parent is the run's parent (both compressed) needs no test, and the run's
-// own cell is searched too when it is a large one (the half space of rows
-// after the run).  256^3 box: a thread walking the 13 rows of linking cells
-// around every run, with all joins on the global tree, took 18.7 + 8.1 ms for
-// the two passes; FOF_MS.
+// (in the first pass) for k_fof_link_warp.  The neighbour cells are walked
+// row by row: for each (dy, dz) of the half space whose row of linking
+// cells comes within reach of the run's records, the cells of the row that
+// do form one key range inside each SOD cell the row crosses, found with
+// one search; every record of the range is then tested.  A friend joins the
+// two components; in the full pass a record whose parent is the run's
+// parent (both compressed) needs no test.
 template <bool FULL>
 __global__ void __launch_bounds__(FOF_TPB, 3) k_fof_link_thread(const unsigned *heads, long long nrun, FofGeo G,
                                                              const unsigned *cs, const unsigned short *skey,
@@ -475,7 +469,7 @@ __global__ void __launch_bounds__(FOF_TPB, 3) k_fof_link_thread(const unsigned *
                                                              unsigned long long *counters) {
   unsigned long long tests = 0, pairs = 0;
   const int R = G.R;
-  const float reach2 = (float)G.reach2, kf = (float)G.k;
+  const float reach2 = (float)G.reach2;
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nrun;
        q += (long long)gridDim.x * blockDim.x) {
     const unsigned h = heads[q], e = heads[q + 1];
@@ -507,88 +501,69 @@ __global__ void __launch_bounds__(FOF_TPB, 3) k_fof_link_thread(const unsigned *
     }
     const unsigned myroot = FULL ? __ldcg(par + h) : 0u;
     int found = 0;
-    // record v of another run: a friend joins the two groups
-    auto visit = [&](unsigned v) {
-      if (FULL && __ldcg(par + v) == myroot) return;
-      const float4 bv = cube[perm[v]];
-      bool hit = false;
-#pragma unroll
-      for (unsigned j = 0; j < FOF_THREAD_RUN; j++) {
-        if (j < m && !hit) {
-          tests++;
-          hit = fof_friends(ur[j], bv, G.r2, G.rT);
-        }
-      }
-      if (hit) {
-        uf_union(par, h, v);
-        if (!FULL) found++;
-      }
-    };
-    // linking cells of SOD cell offset (dx, dy, dz), records [clo, chi): the
-    // rows within reach, one key range each
-    auto rows = [&](int dx, int dy, int dz, unsigned clo, unsigned chi) {
-      const bool self = (dx | dy | dz) == 0;
-      const int z0 = max(u.fz - R, dz * G.k), z1 = min(u.fz + R, dz * G.k + G.k - 1);
-      for (int tz = self ? u.fz : z0; tz <= z1 && found < FOF_SAMPLE; tz++) {
-        const float gz = fmaxf(fmaxf((float)tz - hi[2], lo[2] - ((float)tz + 1.f)), 0.f);
-        if (gz * gz > reach2) continue;
-        const int y0 = max(u.fy - R, dy * G.k), y1 = min(u.fy + R, dy * G.k + G.k - 1);
-        for (int ty = (self && tz == u.fz) ? u.fy : y0; ty <= y1 && found < FOF_SAMPLE; ty++) {
-          const float gy = fmaxf(fmaxf((float)ty - hi[1], lo[1] - ((float)ty + 1.f)), 0.f);
-          const float left = reach2 - gz * gz - gy * gy;
-          if (left < 0.f) continue;
-          const float rx = sqrtf(left);
-          int xa = max(max((int)floorf(lo[0] - rx), u.fx - R), dx * G.k);
-          const int xb = min(min((int)floorf(hi[0] + rx), u.fx + R), dx * G.k + G.k - 1);
-          if (self && tz == u.fz && ty == u.fy) xa = max(xa, u.fx + 1);  // own row: cells after the run's
-          if (xa > xb) continue;
-          const unsigned rowkey = (unsigned)(G.k * ((ty - dy * G.k) + G.k * (tz - dz * G.k)));
-          const unsigned k0 = rowkey + (unsigned)(xa - dx * G.k), k1 = rowkey + (unsigned)(xb - dx * G.k);
-          unsigned v = clo, b2 = chi;
-          while (v < b2) {
-            const unsigned mid = (v + b2) >> 1;
-            if (__ldg(skey + mid) < k0) v = mid + 1;
-            else b2 = mid;
+    for (int oz = 0; oz <= R && found < FOF_SAMPLE; oz++) {
+      const float bz = (float)(u.fz + oz);
+      const float gz = fmaxf(fmaxf(bz - hi[2], lo[2] - (bz + 1.f)), 0.f);
+      if (gz * gz > reach2) continue;
+      for (int oy = (oz == 0 ? 0 : -R); oy <= R && found < FOF_SAMPLE; oy++) {
+        const float by = (float)(u.fy + oy);
+        const float gy = fmaxf(fmaxf(by - hi[1], lo[1] - (by + 1.f)), 0.f);
+        const float left = reach2 - gz * gz - gy * gy;
+        if (left < 0.f) continue;
+        const float rx = sqrtf(left);
+        // cells of the row within reach, in the run's SOD-cell frame
+        int xa = (int)floorf(lo[0] - rx), xb = (int)floorf(hi[0] + rx);
+        xa = max(xa, u.fx - R);
+        xb = min(xb, u.fx + R);
+        if (oz == 0 && oy == 0) xa = max(xa, u.fx + 1);  // own row: cells after the run's
+        if (xa > xb) continue;
+        // the row's SOD cells in y and z
+        int ty = u.fy + oy, tz = u.fz + oz;
+        const int dcy = ty < 0 ? -1 : (ty >= G.k ? 1 : 0), dcz = tz < 0 ? -1 : (tz >= G.k ? 1 : 0);
+        ty -= dcy * G.k;
+        tz -= dcz * G.k;
+        int cy = u.cy + dcy, cz = u.cz + dcz;
+        cy = cy < 0 ? cy + G.nx : (cy >= G.nx ? cy - G.nx : cy);
+        cz = cz < 0 ? cz + G.nx : (cz >= G.nx ? cz - G.nx : cz);
+        // up to three SOD cells along x
+        for (int dcx = -1; dcx <= 1 && found < FOF_SAMPLE; dcx++) {
+          const int s0 = max(xa, dcx * G.k), s1 = min(xb, dcx * G.k + G.k - 1);
+          if (s0 > s1) continue;
+          int cx = u.cx + dcx;
+          cx = cx < 0 ? cx + G.nx : (cx >= G.nx ? cx - G.nx : cx);
+          const unsigned long long c = (unsigned long long)cx +
+                                       (unsigned long long)G.nx * ((unsigned long long)cy + (unsigned long long)G.nx * cz);
+          const unsigned clo = __ldg(cs + c), chi = __ldg(cs + c + 1);
+          if (clo == chi) continue;
+          const unsigned rowkey = (unsigned)(G.k * (ty + G.k * tz));
+          const unsigned k0 = rowkey + (unsigned)(s0 - dcx * G.k), k1 = rowkey + (unsigned)(s1 - dcx * G.k);
+          unsigned v = clo;
+          if (chi - clo <= 16) {
+            while (v < chi && __ldg(skey + v) < k0) v++;
+          } else {
+            unsigned b2 = chi;
+            while (v < b2) {
+              const unsigned mid = (v + b2) >> 1;
+              if (__ldg(skey + mid) < k0) v = mid + 1;
+              else b2 = mid;
+            }
           }
           pairs++;
           for (; v < chi && __ldg(skey + v) <= k1; v++) {
-            visit(v);
-            if (found >= FOF_SAMPLE) break;
-          }
-        }
-      }
-    };
-    const unsigned long long own =
-        (unsigned long long)u.cx + (unsigned long long)G.nx * ((unsigned long long)u.cy + (unsigned long long)G.nx * u.cz);
-    if (FULL) {  // a small own cell was linked by the sort
-      const unsigned clo = __ldg(cs + own), chi = __ldg(cs + own + 1);
-      if (chi - clo > FOF_SMALL_CELL) rows(0, 0, 0, clo, chi);
-    }
-    for (int dz = -1; dz <= 1 && found < FOF_SAMPLE; dz++) {
-      const float gz = dz < 0 ? lo[2] : (dz > 0 ? kf - hi[2] : 0.f);
-      if (gz > 0.f && gz * gz > reach2) continue;
-      int cz = u.cz + dz;
-      cz = cz < 0 ? cz + G.nx : (cz >= G.nx ? cz - G.nx : cz);
-      for (int dy = -1; dy <= 1 && found < FOF_SAMPLE; dy++) {
-        const float gy = dy < 0 ? lo[1] : (dy > 0 ? kf - hi[1] : 0.f);
-        const float g2 = fmaxf(gz, 0.f) * fmaxf(gz, 0.f) + fmaxf(gy, 0.f) * fmaxf(gy, 0.f);
-        if (g2 > reach2) continue;
-        int cy = u.cy + dy;
-        cy = cy < 0 ? cy + G.nx : (cy >= G.nx ? cy - G.nx : cy);
-        for (int dx = -1; dx <= 1 && found < FOF_SAMPLE; dx++) {
-          const float gx = fmaxf(dx < 0 ? lo[0] : (dx > 0 ? kf - hi[0] : 0.f), 0.f);
-          if (g2 + gx * gx > reach2) continue;
-          int cx = u.cx + dx;
-          cx = cx < 0 ? cx + G.nx : (cx >= G.nx ? cx - G.nx : cx);
-          const unsigned long long c =
-              (unsigned long long)cx + (unsigned long long)G.nx * ((unsigned long long)cy + (unsigned long long)G.nx * cz);
-          if (c <= own) continue;  // that cell visits this one
-          const unsigned clo = __ldg(cs + c), chi = __ldg(cs + c + 1);
-          if (chi - clo > FOF_SMALL_CELL) {
-            rows(dx, dy, dz, clo, chi);
-          } else if (chi != clo) {
-            pairs++;
-            for (unsigned v = clo; v < chi && found < FOF_SAMPLE; v++) visit(v);
+            if (FULL && __ldcg(par + v) == myroot) continue;
+            const float4 bv = cube[perm[v]];
+            bool hit = false;
+#pragma unroll
+            for (unsigned j = 0; j < FOF_THREAD_RUN; j++) {
+              if (j < m && !hit) {
+                tests++;
+                hit = fof_friends(ur[j], bv, G.r2, G.rT);
+              }
+            }
+            if (hit) {
+              uf_union(par, h, v);
+              if (!FULL && ++found >= FOF_SAMPLE) break;
+            }
           }
         }
       }
@@ -630,16 +605,15 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_link_warp(const unsigned *heads
     lo[2] = (float)u.fz;
     hi[2] = (float)(u.fz + 1);
     int sampled = 0;  // neighbour runs examined (warp-uniform)
-    for (int o2 = 0; o2 < 2 * G.noff && (FULL || sampled < FOF_SAMPLE_WARP); o2++) {
-      const int o = o2 >> 1, sg = (o2 & 1) ? -1 : 1;  // both halves of the offsets
-      const int ox = sg * c_fof_off[3 * o], oy = sg * c_fof_off[3 * o + 1], oz = sg * c_fof_off[3 * o + 2];
+    for (int o = 0; o < G.noff && (FULL || sampled < FOF_SAMPLE_WARP); o++) {
+      const int ox = c_fof_off[3 * o], oy = c_fof_off[3 * o + 1], oz = c_fof_off[3 * o + 2];
       if (box_gap2(u, ox, oy, oz, lo, hi) > (float)G.reach2) continue;
       unsigned vlo, vhi;
       if (!find_run(u, ox, oy, oz, G, cs, skey, vlo, vhi)) continue;
       if (vlo == h) continue;
-      if (__ldcg(par + h) == __ldcg(par + vlo)) continue;
       sampled++;
       if (lane == 0) pairs++;
+      if (FULL && __ldcg(par + h) == __ldcg(par + vlo)) continue;
       bool hit = false;
       for (unsigned ub = h; ub < e && !hit; ub += 32) {
         const unsigned uu = ub + (unsigned)lane;
@@ -682,7 +656,12 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_link_warp(const unsigned *heads
 // LINK_SAMPLE joins a neighbour; the full pass tests every pair of runs whose
 // groups differ until a friend pair is met, long products by the warp.  A
 // neighbour all of whose runs in reach are of the cell's one group is skipped.
-// FOF_MS.
+//
+// 256^3 box (16.8 M particles, b = 0.2): a thread walking the 13 rows of linking
+// cells around every run, all joins on one global tree, took 18.7 + 8.1 ms for
+// its two passes and the long runs' warps 4.0 ms (30.8 in all); by cells: the
+// sort's linking 2.4, small cells 1.0, medium ones 0.7 + 2.0, dense ones 0.2 +
+// 0.8 ms (7.1 in all).  Bound: dependent loads of records and groups.
 constexpr unsigned LINK_SAMPLE = 2;
 constexpr unsigned LINK_SEARCH = 1024;  // records from which a neighbour's table is searched, not walked
 constexpr unsigned LINK_SERIAL = 64;  // record pairs a lane tests itself
@@ -1453,31 +1432,34 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
   k_fof_sort_small<<<grid_for((long long)c->ncell), FOF_TPB, 0, c->stream>>>(
       c->d_cell_start, c->ncell, key, c->d_cube, G, perm, skey, par, finv, aux1, big, cnt, mid, cnt + 5, dense, cnt + 2);
   const int nbins = k * k * k;
+  // How the runs are linked.  By SOD cells (tables and record by record) where
+  // the linking cells are coarse, k <= 12 or linking lengths from 0.15 cells,
+  // and the box has enough cells to fill the chip; finer linking cells hold one
+  // record each and their runs search the sorted keys (k = 18, a 96^3 box: 2.1
+  // ms, the tables of 18^3 cells 2.8 ms and their sort 2.4 ms more), and so do
+  // boxes of a few large halos (50^3 with a halo of 5e4: linking 0.63 against
+  // 0.84 ms; 96^3: 1.7 against 1.2 ms)
+  const bool tables = k <= LINK_TABLE_K && n >= LINK_TABLE_N;
   {
-    // bins, their parents and first records; the linking inside the cell is
-    // left to the passes when they do not fit
-    const size_t local_bytes = (size_t)nbins * (2 * sizeof(unsigned) + 3 * sizeof(float));
-    const bool local = local_bytes <= 200u * 1024u;
-    const size_t smem = local ? local_bytes : (size_t)nbins * sizeof(unsigned);
+    // bins, their parents and first records
+    const size_t smem = (size_t)nbins * (tables ? 2 * sizeof(unsigned) + 3 * sizeof(float) : sizeof(unsigned));
     auto launch = [&](auto *kern) -> int {
       PSOD_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       kern<<<1184, FOF_TPB, smem, c->stream>>>(c->d_cell_start, big, cnt, nbins, G, key, c->d_cube, perm, skey, par,
                                                finv, aux1);
       return PSOD_OK;
     };
-    if ((st = local ? launch(k_fof_sort_big<true>) : launch(k_fof_sort_big<false>))) return st;
+    if ((st = tables ? launch(k_fof_sort_big<true>) : launch(k_fof_sort_big<false>))) return st;
   }
   PSOD_CUDA(c, cudaGetLastError());
-  // 2. linking: sampled pass, compression, full pass, compression.  Tables of
-  // both cells' linking cells where they fit shared memory (k <= 20, linking
-  // lengths from 0.09 cells), else runs that search the sorted keys
+  // 2. linking: sampled pass, compression, full pass, compression
   k_fof_count<<<148 * 8, FOF_TPB, 0, c->stream>>>(aux1, n, ctr + 2);
   unsigned long long nrun = 0;
   PSOD_CUDA(c, cudaMemcpyAsync(&nrun, ctr + 2, sizeof(nrun), cudaMemcpyDeviceToHost, c->stream));
   S.ms_sort = tm.stop();
   S.fine_cells = (int64_t)nrun;
   const size_t tab_bytes = 3 * sizeof(unsigned) * ((size_t)nbins + (FOF_TPB / 32) * (size_t)R * k * k);
-  if (tab_bytes <= 210u * 1024u) {
+  if (tables) {
     auto link = [&](auto *kern) -> int {
       PSOD_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab_bytes));
       kern<<<148 * 8, FOF_TPB, tab_bytes, c->stream>>>(c->d_cell_start, dense, cnt + 2, nbins, G, skey, perm,
