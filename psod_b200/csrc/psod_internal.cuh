@@ -284,15 +284,15 @@ enum : int {
   SLOT_BIG_TAB = 3,     // cell sort: sub-cell slot tables of dense cells
   SLOT_BIG_CELL = 4,    // cell sort: the dense cells
   SLOT_LOAD_FLAGS = 5,  // cell sort: bad-position flag, dense-cell count
-  SLOT_PART_U32 = 6,    // n u32: cell ids (load), seed flags (tri_cic), member pool indices (SOD)
-  SLOT_PART_U64 = 7,    // n u64: seed prefix sums (tri_cic), member pool keys (SOD)
+  SLOT_PART_U32 = 6,    // n u32: cell ids (load), seed tile counts (tri_cic), member pool indices (SOD)
+  SLOT_PART_U64 = 7,    // n u64: member pool keys (SOD)
   SLOT_CELL_U32 = 80,   // ncell+1 u32: cell counts (load), alive counts per cell (SOD)
   SLOT_SORT_KEYS = 81,  // radix sort: key ping-pong buffer
   SLOT_SORT_VALS = 82,  // radix sort: value ping-pong buffer
   SLOT_SORT_HIST = 83,  // radix sort: per-tile digit counts
   SLOT_SORT_RNG = 84,   // radix sort: key range
   SLOT_TRI_KEYS = 85,   // tri_cic: seed sort keys
-  SLOT_TRI_MIN = 86,    // tri_cic: densest-non-seed key and index
+  SLOT_TRI_MIN = 86,    // tri_cic: extreme keys, densest non-seed's index, tie flag
   SLOT_HOST_POS = 87,   // load: device copy of host positions
   SLOT_VEL = 88,        // load: velocities
   SLOT_SEED_IDX = 89,   // tri_cic: seed order (persistent)

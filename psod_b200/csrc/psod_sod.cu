@@ -2842,15 +2842,26 @@ __global__ void __launch_bounds__(TPB) k_cross(SodConst K, SodBufs B) {
 
 // Lower bound of each ready seed's best refinement sum: the seed is one of
 // its own candidates, so its sum (FP32 terms, relative error below 2e-6),
-// deflated by 1e-3, is at most the maximum.  Warp per seed.
-__global__ void k_seed_lower(SodConst K, SodBufs B) {
-  const unsigned slot = (unsigned)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+// deflated by 1e-3, is at most the maximum.  CTA per seed, each warp a share of
+// the records (a warp alone walked the 1e5 records of a cluster's 27 cells in
+// 2.9 ms; the kernel took SEED_LOWER at 512^3).
+constexpr int LOWER_TPB = 512;
+
+__global__ void __launch_bounds__(LOWER_TPB) k_seed_lower(SodConst K, SodBufs B) {
+  __shared__ double s_sum[LOWER_TPB / 32];
+  const unsigned slot = blockIdx.x;
   if (slot >= min(*B.nready, B.cap_ready) || !B.st_active[slot] || B.st_cn[slot] < B.bound_min) return;
   const SeedGeo g = seed_geo(K, B, B.ready[slot]);
   unsigned long long sq = 0;
   double sf = 0.0;
-  refine_sum<false>(K, B, g.sp, g.ic, g.jc, g.kc, sq, sf);
-  if ((threadIdx.x & 31) == 0) atomicMax(&B.s_lmax[slot], __float_as_uint((float)(sf * 0.999)));
+  const int w = threadIdx.x >> 5;
+  refine_sum<false>(K, B, g.sp, g.ic, g.jc, g.kc, sq, sf, nullptr, (unsigned)w, LOWER_TPB / 32);
+  if ((threadIdx.x & 31) == 0) s_sum[w] = sf;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int q = 1; q < LOWER_TPB / 32; q++) sf += s_sum[q];
+    atomicMax(&B.s_lmax[slot], __float_as_uint((float)(sf * 0.999)));
+  }
 }
 
 // The group holding the candidate with the largest finite upper bound, per
@@ -4512,7 +4523,7 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
       t_bound.start(c->stream);
       k_zero_bounds<<<ref_grid, 256, 0, c->stream>>>(cand_used, (unsigned long long)cand_cap, cand_u);
       PSOD_CUDA(c, cudaMemsetAsync(s_lmax, 0, sizeof(unsigned) * nready, c->stream));
-      k_seed_lower<<<nblk((long long)nready * 32, 256), 256, 0, c->stream>>>(K, B);
+      k_seed_lower<<<nready, LOWER_TPB, 0, c->stream>>>(K, B);
       k_refine_warp<true><<<ref_grid, 256, 0, c->stream>>>(K, B);
       k_top_group<<<nblk((long long)nready * 32, 256), 256, 0, c->stream>>>(K, B);
       if ((rc = scan_u32(c, B.top_n, B.top_pref, (long long)nready, true))) return rc;

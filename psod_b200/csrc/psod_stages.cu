@@ -13,6 +13,7 @@
 //                  stable radix sort of the seeds, ties by input index.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 
 #include "psod_internal.cuh"
 
@@ -175,9 +176,10 @@ __device__ __forceinline__ unsigned sub_key(const float4 &p, float nxf, double3 
 // count[c] becomes BIG_FLAG | table index for cells of SUB_MIN or more
 // particles, else the cell's first slot start[c] (the fill cursor of the
 // scatter, so that one atomic gives the slot; start < n < 2^31 keeps the
-// flag bit clear).  With assign false it only counts them.
-__global__ void k_mark_big(unsigned *count, unsigned long long ncell, unsigned *nbig, bool assign,
-                           unsigned *bigcell, const unsigned *start) {
+// flag bit clear).  The tables have room for every cell that can be dense, so
+// no pass counts them first (a zone of a 512^3 grid: 1.05 -> 0.64 ms).
+__global__ void k_mark_big(unsigned *count, unsigned long long ncell, unsigned *nbig, unsigned *bigcell,
+                           const unsigned *start) {
   const unsigned long long c = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
   const bool big = c < ncell && count[c] >= SUB_MIN;
   const unsigned m = __ballot_sync(0xffffffffu, big);
@@ -185,7 +187,7 @@ __global__ void k_mark_big(unsigned *count, unsigned long long ncell, unsigned *
   unsigned base = 0;
   if (lane == 0 && m) base = atomicAdd(nbig, (unsigned)__popc(m));
   base = __shfl_sync(0xffffffffu, base, 0);
-  if (!assign || c >= ncell) return;
+  if (c >= ncell) return;
   if (big) {
     const unsigned idx = base + __popc(m & ((1u << lane) - 1u));
     bigcell[idx] = (unsigned)c;
@@ -782,50 +784,136 @@ __global__ void k_grid_to_double(const unsigned long long *grid, long long nnode
 // ---------------------------------------------------------------------------
 // seeds
 // ---------------------------------------------------------------------------
-// Seed flags (1/rho < 0.01) and the smallest key of the others.  Fixed
-// grid, each thread over a strided range; one atomic per CTA (a per-warp
-// atomic on the single minimum serialises tens of millions of updates).
-__global__ void __launch_bounds__(256) k_seed_flags(const double *rho, long long n, unsigned *flag,
-                                                    unsigned long long *minbits) {
-  __shared__ unsigned long long s_min[8];
-  unsigned long long mb = ~0ull;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const double pd = ddiv(1.0, rho[i]);  // main:1022
-    unsigned f = 0;
-    if (pd < 0.01) {
-      f = 1;  // main:1029: 1/rho < 1/100
+// Seeds are the particles with 1/rho < 0.01 (main:1029), i.e. rho >= rho_seed,
+// the smallest double whose quotient is below (the rounded quotient falls as
+// rho grows).  Two passes over rho: the counts per tile of SEED_TILE particles
+// with the extreme keys, then the compaction in input order.  (Flags, their
+// scan over all particles and separate passes for the extremes moved 44 bytes a
+// particle; these move 16.  256^3: 0.32 -> 0.10 ms.)
+constexpr int SEED_TILE = 2048, SEED_PER = SEED_TILE / 256;
+
+__global__ void __launch_bounds__(256) k_seed_count(const double *rho, long long n, double rho_seed, unsigned *count,
+                                                    unsigned long long *seed_min, unsigned long long *other_min) {
+  __shared__ unsigned s_cnt[8];
+  __shared__ unsigned long long s_seed[8], s_other[8];
+  const long long base = (long long)blockIdx.x * SEED_TILE;
+  unsigned cnt = 0;
+  double top = 0.0, below = 0.0;  // largest rho among the seeds and among the others
+  bool any = false;
+#pragma unroll
+  for (int u = 0; u < SEED_PER; u++) {
+    const long long i = base + u * 256 + threadIdx.x;
+    if (i >= n) break;
+    const double r = rho[i];
+    if (r >= rho_seed) {
+      cnt++;
+      top = fmax(top, r);
     } else {
-      const unsigned long long b = dbits(pd);
-      mb = b < mb ? b : mb;
+      below = any ? fmax(below, r) : r;
+      any = true;
     }
-    flag[i] = f;
   }
+  // keys: bits of 1/rho, which falls as rho grows
+  unsigned long long ks = cnt ? dbits(ddiv(1.0, top)) : ~0ull, ko = any ? dbits(ddiv(1.0, below)) : ~0ull;
   for (int o = 16; o > 0; o >>= 1) {
-    const unsigned long long t = __shfl_down_sync(0xffffffffu, mb, o);
-    mb = t < mb ? t : mb;
+    cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+    const unsigned long long a = __shfl_down_sync(0xffffffffu, ks, o), b = __shfl_down_sync(0xffffffffu, ko, o);
+    ks = a < ks ? a : ks;
+    ko = b < ko ? b : ko;
   }
-  if ((threadIdx.x & 31) == 0) s_min[threadIdx.x >> 5] = mb;
+  const int w = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) {
+    s_cnt[w] = cnt;
+    s_seed[w] = ks;
+    s_other[w] = ko;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int q = 1; q < (int)(blockDim.x >> 5); q++) mb = s_min[q] < mb ? s_min[q] : mb;
-    if (mb != ~0ull) atomicMin(minbits, mb);
+    for (int q = 1; q < 8; q++) {
+      cnt += s_cnt[q];
+      ks = s_seed[q] < ks ? s_seed[q] : ks;
+      ko = s_other[q] < ko ? s_other[q] : ko;
+    }
+    count[blockIdx.x] = cnt;
+    // the running minima only fall: a tile that does not lower them writes nothing
+    if (ks < *(volatile unsigned long long *)seed_min) atomicMin(seed_min, ks);
+    if (ko < *(volatile unsigned long long *)other_min) atomicMin(other_min, ko);
   }
 }
 
-__global__ void k_seed_extra_idx(const double *rho, long long n, unsigned long long minbits, unsigned *minidx) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double pd = ddiv(1.0, rho[i]);
-  if (!(pd < 0.01) && dbits(pd) == minbits) atomicMin(minidx, (unsigned)i);
+// the seeds in input order with their keys: K = unsigned, the 32 bits of (bits
+// - kmin) from bit `shift` up, or the full bits (shift 0, kmin 0); and the
+// lowest index of a particle with the others' smallest key
+template <typename K>
+__global__ void __launch_bounds__(256) k_seed_compact(const double *rho, long long n, double rho_seed,
+                                                      const unsigned *tile_pos, unsigned long long kmin, int shift,
+                                                      double rho_other, unsigned long long other_min, unsigned *minidx,
+                                                      K *keys, unsigned *vals) {
+  __shared__ unsigned s_cnt[SEED_PER][8];
+  const long long base = (long long)blockIdx.x * SEED_TILE;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  double r[SEED_PER];
+  unsigned m[SEED_PER];
+#pragma unroll
+  for (int u = 0; u < SEED_PER; u++) {
+    const long long i = base + u * 256 + threadIdx.x;
+    r[u] = i < n ? rho[i] : -1.0;
+  }
+#pragma unroll
+  for (int u = 0; u < SEED_PER; u++) {
+    m[u] = __ballot_sync(0xffffffffu, r[u] >= rho_seed);
+    if (lane == 0) s_cnt[u][w] = (unsigned)__popc(m[u]);
+    const long long i = base + u * 256 + threadIdx.x;
+    if (i < n && !(r[u] >= rho_seed) && r[u] >= rho_other && dbits(ddiv(1.0, r[u])) == other_min)
+      atomicMin(minidx, (unsigned)i);
+  }
+  __syncthreads();
+  unsigned at = tile_pos[blockIdx.x];
+#pragma unroll
+  for (int u = 0; u < SEED_PER; u++) {
+    unsigned mine = at;
+    for (int q = 0; q < 8; q++) {
+      if (q < w) mine += s_cnt[u][q];
+      at += s_cnt[u][q];
+    }
+    if (r[u] >= rho_seed) {
+      const unsigned o = mine + __popc(m[u] & ((1u << lane) - 1u));
+      keys[o] = (K)((dbits(ddiv(1.0, r[u])) - kmin) >> shift);
+      vals[o] = (unsigned)(base + u * 256 + threadIdx.x);
+    }
+  }
 }
 
-__global__ void k_seed_compact(const double *rho, long long n, const unsigned *flag, const unsigned *pos,
-                               unsigned long long *keys, unsigned *vals) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !flag[i]) return;
-  unsigned o = pos[i];
-  keys[o] = dbits(ddiv(1.0, rho[i]));
-  vals[o] = (unsigned)i;
+// After the sort on the truncated keys: each run of equal ones is put in (full
+// key, input index) order by the thread at its start.  A run longer than
+// TIE_MAX sets *redo (the caller sorts the full keys instead).
+constexpr unsigned TIE_MAX = 64;
+
+__global__ void k_seed_ties(const unsigned *key, unsigned *val, unsigned n, const double *rho, unsigned *redo) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i + 1 >= n) return;
+  const unsigned k = key[i];
+  if (key[i + 1] != k || (i > 0 && key[i - 1] == k)) return;
+  unsigned e = i + 2;
+  while (e < n && e - i <= TIE_MAX && key[e] == k) e++;
+  if (e - i > TIE_MAX) {
+    *redo = 1;
+    return;
+  }
+  auto full = [&](unsigned v) { return dbits(ddiv(1.0, rho[v])); };
+  for (unsigned a = i + 1; a < e; a++) {
+    const unsigned v = val[a];
+    const unsigned long long fk = full(v);
+    unsigned b = a;
+    while (b > i) {
+      const unsigned u = val[b - 1];
+      const unsigned long long fu = full(u);
+      if (fu < fk || (fu == fk && u < v)) break;
+      val[b] = u;
+      b--;
+    }
+    val[b] = v;
+  }
 }
 
 __global__ void k_widen_seeds(const unsigned *in, long long n, long long *out) {
@@ -872,19 +960,18 @@ int stage_cellsort(psod_ctx *c, const float *dpos) {
   if ((st = scan_u32(c, count, c->d_cell_start, (long long)c->ncell, true))) return st;
   unsigned *nbig = reinterpret_cast<unsigned *>(bad + 1);
   const long long ncell = (long long)c->ncell;
-  k_mark_big<<<nblk(ncell, 256), 256, 0, c->stream>>>(count, c->ncell, nbig, false, nullptr, nullptr);
+  unsigned *tab = nullptr, *bigcell = nullptr;
+  const size_t big_cap = (size_t)n / SUB_MIN + 1;
+  if ((st = scratch(c, SLOT_BIG_TAB, big_cap * SUB_N, &tab))) return st;
+  if ((st = scratch(c, SLOT_BIG_CELL, big_cap, &bigcell))) return st;
+  k_mark_big<<<nblk(ncell, 256), 256, 0, c->stream>>>(count, c->ncell, nbig, bigcell, c->d_cell_start);
   int hflags[2] = {0, 0};
   PSOD_CUDA(c, cudaMemcpyAsync(hflags, bad, sizeof(hflags), cudaMemcpyDeviceToHost, c->stream));
   PSOD_CUDA(c, cudaStreamSynchronize(c->stream));
   const int hbad = hflags[0];
   const unsigned hnbig = (unsigned)hflags[1];
-  unsigned *tab = nullptr, *bigcell = nullptr;
   if (!hbad) {
-    if ((st = scratch(c, SLOT_BIG_TAB, (size_t)hnbig * SUB_N + 1, &tab))) return st;
-    if ((st = scratch(c, SLOT_BIG_CELL, (size_t)hnbig + 1, &bigcell))) return st;
-    PSOD_CUDA(c, cudaMemsetAsync(nbig, 0, sizeof(unsigned), c->stream));
-    PSOD_CUDA(c, cudaMemsetAsync(tab, 0, sizeof(unsigned) * ((size_t)hnbig * SUB_N + 1), c->stream));
-    k_mark_big<<<nblk(ncell, 256), 256, 0, c->stream>>>(count, c->ncell, nbig, true, bigcell, c->d_cell_start);
+    PSOD_CUDA(c, cudaMemsetAsync(tab, 0, sizeof(unsigned) * (size_t)hnbig * SUB_N, c->stream));
     if (hnbig) {
       k_sub_count<<<nblk(n, 256), 256, 0, c->stream>>>(rec, n, cell, count, (float)nx, xs, tab);
       k_sub_scan<<<nblk((long long)hnbig * 32, 256), 256, 0, c->stream>>>(tab, bigcell, hnbig, c->d_cell_start);
@@ -1022,35 +1109,61 @@ int stage_tri_cic(psod_ctx *c, int64_t *isort_out) {
   if (!c->rho_done) return set_err(c, PSOD_ERR_STATE, "psod_tri_cic needs psod_cic first");
   const long long n = c->n;
   int st;
-  unsigned *flag = nullptr, *posn = nullptr, *minidx = nullptr;
-  unsigned long long *minbits = nullptr, *keys = nullptr;
-  if ((st = scratch(c, SLOT_PART_U32, (size_t)n, &flag))) return st;
-  if ((st = scratch(c, SLOT_PART_U64, (size_t)n + 1, &posn))) return st;
-  if ((st = scratch(c, SLOT_TRI_MIN, 2, &minbits))) return st;
-  minidx = reinterpret_cast<unsigned *>(minbits + 1);
-  PSOD_CUDA(c, cudaMemsetAsync(minbits, 0xff, sizeof(unsigned long long), c->stream));
-  PSOD_CUDA(c, cudaMemsetAsync(minidx, 0xff, sizeof(unsigned), c->stream));
-  {
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    const unsigned grid = (unsigned)std::max<long long>(1, std::min<long long>(nblk(n, 256), (long long)sms * 8));
-    k_seed_flags<<<grid, 256, 0, c->stream>>>(c->d_rho, n, flag, minbits);
-  }
-  if ((st = scan_u32(c, flag, posn, n, true))) return st;
+  // the smallest rho whose 1/rho rounds below 0.01
+  double rho_seed = 100.0;
+  while (!(1.0 / rho_seed < 0.01)) rho_seed = std::nextafter(rho_seed, 1e300);
+  while (1.0 / std::nextafter(rho_seed, 0.0) < 0.01) rho_seed = std::nextafter(rho_seed, 0.0);
+  unsigned *tiles = nullptr;
+  unsigned long long *mins = nullptr;  // smallest key of the seeds, of the others; index of the latter, tie flag
+  const long long ntile = nblk(n, SEED_TILE);
+  if ((st = scratch(c, SLOT_PART_U32, (size_t)std::max<long long>(n, ntile + 1), &tiles))) return st;
+  if ((st = scratch(c, SLOT_TRI_MIN, 3, &mins))) return st;
+  unsigned *minidx = reinterpret_cast<unsigned *>(mins + 2), *redo = minidx + 1;
+  PSOD_CUDA(c, cudaMemsetAsync(mins, 0xff, 3 * sizeof(unsigned long long), c->stream));
+  k_seed_count<<<(unsigned)ntile, 256, 0, c->stream>>>(c->d_rho, n, rho_seed, tiles, mins, mins + 1);
+  if ((st = scan_u32(c, tiles, tiles, ntile, true))) return st;
   unsigned nd = 0;
-  unsigned long long hmin = 0;
-  PSOD_CUDA(c, cudaMemcpyAsync(&nd, posn + n, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
-  PSOD_CUDA(c, cudaMemcpyAsync(&hmin, minbits, sizeof(hmin), cudaMemcpyDeviceToHost, c->stream));
+  unsigned long long hm[2] = {0, 0};
+  PSOD_CUDA(c, cudaMemcpyAsync(&nd, tiles + ntile, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  PSOD_CUDA(c, cudaMemcpyAsync(hm, mins, sizeof(hm), cudaMemcpyDeviceToHost, c->stream));
   PSOD_CUDA(c, cudaStreamSynchronize(c->stream));
-  const bool has_extra = hmin != ~0ull;
-  if (has_extra) k_seed_extra_idx<<<nblk(n, 256), 256, 0, c->stream>>>(c->d_rho, n, hmin, minidx);
+  const bool has_extra = hm[1] != ~0ull;
   const long long nseed = (long long)nd + (has_extra ? 1 : 0);
-  if ((st = scratch(c, SLOT_TRI_KEYS, (size_t)nd + 1, &keys))) return st;
+  // densities that can have the others' smallest key
+  double rho_other = 0.0;
+  if (has_extra) {
+    double pd;
+    memcpy(&pd, &hm[1], sizeof(pd));
+    rho_other = (1.0 / pd) * (1.0 - 1e-14);
+  }
   if ((st = scratch(c, SLOT_SEED_IDX, (size_t)nseed + 1, &c->d_seed_idx))) return st;
-  k_seed_compact<<<nblk(n, 256), 256, 0, c->stream>>>(c->d_rho, n, flag, posn, keys, c->d_seed_idx);
-  // seeds arrive in input order; a stable sort on 1/rho leaves ties in
-  // input order
-  if ((st = radix_sort_u64(c, keys, c->d_seed_idx, (long long)nd, 64))) return st;
+  // Seeds arrive in input order; a stable sort on 1/rho leaves ties in input
+  // order.  The keys are sorted by their top 32 varying bits (four digit passes
+  // of 8 bytes a seed instead of seven of 12), then the few equal ones are put
+  // in full order.
+  const double edge = 0.01;
+  unsigned long long kmax;
+  memcpy(&kmax, &edge, sizeof(kmax));
+  int shift = 0;
+  while (nd && ((kmax - hm[0]) >> shift) > 0xffffffffull) shift++;
+  unsigned *keys = nullptr;
+  if ((st = scratch(c, SLOT_TRI_KEYS, (size_t)nd + 1, &keys))) return st;
+  k_seed_compact<unsigned><<<(unsigned)ntile, 256, 0, c->stream>>>(c->d_rho, n, rho_seed, tiles, nd ? hm[0] : 0ull, shift,
+                                                                   rho_other, hm[1], minidx, keys, c->d_seed_idx);
+  if ((st = radix_sort_u32(c, keys, c->d_seed_idx, (long long)nd, 32))) return st;
+  PSOD_CUDA(c, cudaMemsetAsync(redo, 0, sizeof(unsigned), c->stream));
+  if (nd > 1 && shift > 0) k_seed_ties<<<nblk(nd, 256), 256, 0, c->stream>>>(keys, c->d_seed_idx, nd, c->d_rho, redo);
+  unsigned hredo = 0;
+  PSOD_CUDA(c, cudaMemcpyAsync(&hredo, redo, sizeof(unsigned), cudaMemcpyDeviceToHost, c->stream));
+  PSOD_CUDA(c, cudaStreamSynchronize(c->stream));
+  if (hredo) {
+    // long runs of nearly equal densities: sort the full keys
+    unsigned long long *keys64 = nullptr;
+    if ((st = scratch(c, SLOT_TRI_KEYS, (size_t)nd + 1, &keys64))) return st;
+    k_seed_compact<unsigned long long><<<(unsigned)ntile, 256, 0, c->stream>>>(
+        c->d_rho, n, rho_seed, tiles, 0ull, 0, rho_other, hm[1], minidx, keys64, c->d_seed_idx);
+    if ((st = radix_sort_u64(c, keys64, c->d_seed_idx, (long long)nd, 64))) return st;
+  }
   if (has_extra)
     PSOD_CUDA(c, cudaMemcpyAsync(c->d_seed_idx + nd, minidx, sizeof(unsigned), cudaMemcpyDeviceToDevice, c->stream));
   PSOD_CUDA(c, cudaGetLastError());
