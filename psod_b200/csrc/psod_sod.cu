@@ -36,7 +36,8 @@ constexpr int TPB = 256;          // threads per seed CTA of the host rounds' ke
 constexpr int LOOP_TPB = 512;     // threads per seed CTA of the device round loop
 constexpr unsigned RN_CHUNK = 2048;  // neighbour records per refinement work item
 constexpr unsigned LOOP_CHUNK = 512;  // in the device round loop: few seeds, all SMs for each
-constexpr unsigned LOOP_BIG = 64;     // seeds of a loop round whose refinement the whole grid shares
+constexpr unsigned LOOP_BIG = 8;      // seeds whose refinement the idle CTAs of the loop can share at one time
+constexpr int LOOP_MAX_CTA = 256;     // CTAs of the device seed loop at most
 constexpr int MAX_WARP = LOOP_TPB / 32;
 // the seed steps run in CTAs of either size
 __device__ __forceinline__ int tpb() { return (int)blockDim.x; }
@@ -95,10 +96,11 @@ struct SodBufs {
   unsigned *nbig;       // seeds of this round with bound_min candidates or more
   unsigned bound_min;   // seeds with this many candidates or more get the bound pass
   unsigned *maxcand;    // largest candidate count of a seed this round (or null)
-  unsigned max_cand;    // seeds with more candidates wait (device tail loop), else ~0u
-  unsigned *deferred;   // set when a seed waited for that reason
   unsigned rn_chunk;    // neighbour records per refinement work item
-  unsigned *bigq, *nbigq;  // device round loop: slots of the seeds refined by the whole grid
+  // device seed loop (0 in host rounds): seeds with more candidates are left
+  // to a host round; candidate and crossing buffer entries that a CTA owns
+  unsigned max_cand, loop_cand;
+  unsigned long long loop_x, *cused;
   unsigned *alive_cnt;  // alive records per cell (batched modes)
   unsigned long long *pairs;       // candidate-neighbour records visited
   unsigned long long *touch;       // records of the balls out to each stop
@@ -208,6 +210,8 @@ struct Smem {
   unsigned nsorted;
   unsigned long long pool_base;
   unsigned long long xbase;  // the seed's slice of the crossing buffer (bucketed ball)
+  unsigned xshared, cshared;  // device seed loop: slices held of the shared part, also of the candidate buffer's
+  unsigned cbase;             // and the seed's candidate slice
   unsigned claim_cnt;
   // last radial_search hit: sorted-buffer index and bucket lower bound
   int res_k;
@@ -988,20 +992,17 @@ __device__ __forceinline__ void prep_seed(const SodConst &K, const SodBufs &B, S
       s_coff[o] = tot;
       tot += s_cnt[o];
     }
-    const bool too_many = tot > B.max_cand;
-    s_base = too_many ? 0u : atomicAdd(B.cand_used, tot);
+    s_base = B.loop_cand ? S.cbase : atomicAdd(B.cand_used, tot);
     if (B.maxcand) atomicMax(B.maxcand, tot);
-    if (too_many || (unsigned long long)s_base + tot > B.cand_cap) {
-      // candidate buffer full this round, or more candidates than the
-      // device tail loop takes: the seed waits for the next round
+    if ((unsigned long long)s_base + tot > B.cand_cap) {
+      // candidate buffer full this round: the seed waits for the next
       s_base = 0xffffffffu;
       B.processed[rank] = 0;
       {
         const unsigned bi = B.bidx_of_rank[rank];
         atomicAnd(&B.resolved[bi >> 5], ~(1u << (bi & 31)));
       }
-      if (too_many) atomicOr(B.deferred, 1u);
-      else if (tot > B.cand_cap) record_error(B, rank, PSOD_ERR_STATE);
+      if (tot > B.cand_cap) record_error(B, rank, PSOD_ERR_STATE);
     } else {
       B.st_na[slot] = na;  // 0 when unknown (batched modes)
       B.st_coff[slot] = s_base;
@@ -2061,6 +2062,9 @@ __device__ __forceinline__ bool stop_may_lie_inside(const SodConst &K, Smem &S, 
   return block_max_i(S, any) > 0;
 }
 
+// device seed loop: *xused counts the holders of shared slices from this bit up
+constexpr unsigned long long XHOLD = 1ull << 40;
+
 // Bucketed ball: grow the ball (one histogram walk per size) until every
 // threshold's stop may lie inside it, then scatter its entries into a slice
 // of the crossing buffer in level-0 bucket order (one more walk).  Returns
@@ -2087,8 +2091,17 @@ __device__ __forceinline__ long long bucket_ball(const SodConst &K, const SodBuf
     rb *= 2.0;
   }
   if (threadIdx.x == 0) {
-    const unsigned long long at = atomicAdd(B.xused, (unsigned long long)nball);
-    S.xbase = (at + nball <= B.xcap) ? at : ~0ull;
+    if (!B.loop_x) {
+      const unsigned long long at = atomicAdd(B.xused, (unsigned long long)nball);
+      S.xbase = (at + nball <= B.xcap) ? at : ~0ull;
+    } else if (nball <= B.loop_x) {
+      S.xbase = blockIdx.x * B.loop_x;
+    } else {  // the part shared by the loop's CTAs, holders counted above XHOLD
+      const unsigned long long at =
+          (atomicAdd(B.xused, XHOLD + nball) & (XHOLD - 1)) + (unsigned long long)gridDim.x * B.loop_x;
+      S.xbase = (at + nball <= B.xcap) ? at : ~0ull;
+      S.xshared++;
+    }
   }
   __syncthreads();
   if (S.xbase == ~0ull) return -1;
@@ -3171,21 +3184,6 @@ __global__ void k_ready_direct(const unsigned *active, const unsigned *nactive, 
 }
 
 // ---------------------------------------------------------------------------
-// Device tail loop.  Late rounds hold few, small seeds; run as separate
-// launches with a host read per round they cost more in launch and
-// synchronisation latency than in work.  One cooperative launch (all CTAs
-// resident) runs round after round on the device: the heads of the active
-// blocks, their readiness (the direct window test, or the separable min
-// filter when many blocks are active) and every ready seed's preselect,
-// refinement (FP32 approximate sums, a warp per candidate, then the exact
-// sums of the contenders and the argmax, as k_select does) and crossing by
-// one CTA, with a grid-wide barrier between the steps.  A seed with more
-// than max_cand candidates waits; the launch ends after its round and the
-// host runs the next rounds with the batched kernels.  The learned first
-// ball is not used here (the crossing starts from BALL0; the halo table does
-// not depend on it).  Every barrier wait is bounded: a wait that runs out
-// records PSOD_ERR_TIMEOUT and every CTA leaves at its next barrier.
-// ---------------------------------------------------------------------------
 // One seed from the preselect to the claims in one CTA (the device round
 // loop).  The alive records filed under the 125 cells within +-2 of the seed
 // cell (the reference's x_sel2) are gathered once into shared memory, cell
@@ -3199,6 +3197,7 @@ __global__ void k_ready_direct(const unsigned *active, const unsigned *nactive, 
 // separate steps 200 us (preselect 20, refinement a warp per candidate cell
 // 120, select 12, crossing 30, seven grid barriers); one CTA ROUND_US.
 constexpr int SL_CELLS = 125;
+enum : int { SEED_DONE = 0, SEED_BIG = 1, SEED_DEFERRED = 2 };
 
 // the inner cell (listed offset o of the 27, x outer and z inner as the
 // reference scans) as an index of the 125
@@ -3264,7 +3263,7 @@ __device__ __forceinline__ void list_terms(const SmallList &L, unsigned j0, unsi
   }
 }
 
-__device__ __forceinline__ void small_seed(const SodConst &K, const SodBufs &B, Smem &S, unsigned slot, unsigned rank) {
+__device__ __forceinline__ int small_seed(const SodConst &K, const SodBufs &B, Smem &S, unsigned slot, unsigned rank) {
   // per cell: first record, first flat record number, alive records, first
   // list entry, fill cursor
   __shared__ unsigned c_beg[SL_CELLS], c_flat[SL_CELLS + 1], c_al[SL_CELLS], c_off[SL_CELLS + 1], c_cur[SL_CELLS];
@@ -3281,15 +3280,10 @@ __device__ __forceinline__ void small_seed(const SodConst &K, const SodBufs &B, 
   }
   const SeedGeo g = seed_geo(K, B, rank);
   const float4 sv = B.cube[g.sp];
-  if (__float_as_uint(sv.w) & PSOD_DEAD_BIT) return;  // claimed (main:1628)
-  auto put_back = [&]() {  // the seed waits: it is unresolved again
-    if (t == 0) {
-      B.processed[rank] = 0;
-      atomicAnd(&B.resolved[bi >> 5], ~(1u << (bi & 31)));
-    }
-  };
+  if (__float_as_uint(sv.w) & PSOD_DEAD_BIT) return SEED_DONE;  // claimed (main:1628)
   // ---- preselect (as prep_seed) and the cells' alive counts ----
   unsigned na = 0;
+  unsigned long long nrec = 0;
   if (B.mode == PSOD_MODE_PLAIN) {
     unsigned cnt = 0, recs = 0;
     for_cube(K, B, g.ic, g.jc, g.kc, K.ncut, [&](unsigned, float4 v) {
@@ -3297,20 +3291,20 @@ __device__ __forceinline__ void small_seed(const SodConst &K, const SodBufs &B, 
       if (!(__float_as_uint(v.w) & PSOD_DEAD_BIT)) cnt++;
     });
     na = block_sum_u32(S, cnt);
-    const unsigned nrec = block_sum_u32(S, recs);
-    if (t == 0) atomicAdd(B.touched, (unsigned long long)nrec);
+    nrec = block_sum_u32(S, recs);
+    if (t == 0) atomicAdd(B.touched, nrec);
     if ((long long)na > K.nsel) {
       if (t == 0) record_error(B, rank, PSOD_ERR_NSEL);
-      return;
+      return SEED_DONE;
     }
-    if (!(dmul((double)na, K.munit) >= K.mmin)) return;  // main:1759
+    if (!(dmul((double)na, K.munit) >= K.mmin)) return SEED_DONE;  // main:1759
   } else if (K.n_total > K.nsel) {
     const unsigned recs = cube_records(K, B, S, g.ic, g.jc, g.kc);
     if ((long long)recs > K.nsel) {
       const unsigned exact = alive_rows(K, B, S, g.ic, g.jc, g.kc, ~0u);
       if ((long long)exact > K.nsel) {
         if (t == 0) record_error(B, rank, PSOD_ERR_NSEL);
-        return;
+        return SEED_DONE;
       }
     }
   }
@@ -3386,7 +3380,7 @@ __device__ __forceinline__ void small_seed(const SodConst &K, const SodBufs &B, 
   if (B.mode != PSOD_MODE_PLAIN) {
     // Mmin: the cells at hand usually reach it
     const unsigned need = K.mmin_count;
-    if (near < need && alive_rows(K, B, S, g.ic, g.jc, g.kc, need) < need) return;  // main:1759
+    if (near < need && alive_rows(K, B, S, g.ic, g.jc, g.kc, need) < need) return SEED_DONE;  // main:1759
   }
   if (w == 0) {
     const int o = lane;
@@ -3406,21 +3400,25 @@ __device__ __forceinline__ void small_seed(const SodConst &K, const SodBufs &B, 
   __syncthreads();
   const unsigned ncand = s_ncand;
   if (nlist > (unsigned)NB || ncand > B.max_cand) {
-    // more records than shared memory holds: the whole grid refines the seed
-    // after this step; more candidates than the loop takes: the host's rounds
+    // more records than shared memory holds: idle CTAs share the refinement
     if (t == 0) {
-      s_work = LOOP_BIG;
-      if (ncand <= B.max_cand) s_work = atomicAdd(B.nbigq, 1u);
+      if (B.mode == PSOD_MODE_PLAIN) atomicAdd(B.touched, 0ull - nrec);  // counted again
+      s_work = ncand <= B.max_cand ? SEED_BIG : SEED_DEFERRED;
+      S.cbase = blockIdx.x * B.loop_cand;
+      if (s_work == SEED_BIG && ncand > B.loop_cand) {
+        const unsigned long long at =
+            (atomicAdd(B.cused, XHOLD + ncand) & (XHOLD - 1)) + (unsigned long long)gridDim.x * B.loop_cand;
+        S.cbase = (unsigned)at;
+        S.cshared = 1;
+        if (at + ncand > B.cand_cap) s_work = SEED_DEFERRED;
+      }
+      if (s_work == SEED_DEFERRED) {  // unresolved again
+        B.processed[rank] = 0;
+        atomicAnd(&B.resolved[bi >> 5], ~(1u << (bi & 31)));
+      }
     }
     __syncthreads();
-    if (s_work < LOOP_BIG) {
-      if (t == 0) B.bigq[s_work] = slot;
-      prep_seed(K, B, S, slot, rank);
-    } else {
-      put_back();
-      if (t == 0) atomicOr(B.deferred, 1u);
-    }
-    return;
+    return (int)s_work;
   }
   if (t == 0) atomicAdd(B.nprocessed, 1ull);
   // ---- gather: coordinates in grid units, padding far from every candidate.
@@ -3615,266 +3613,495 @@ __device__ __forceinline__ void small_seed(const SodConst &K, const SodBufs &B, 
       abs(pdiff((int)(K.quirk_listed / ((unsigned)K.nx * K.nx)), g.kc, K.nx)) <= 4)
     use_list = false;
   cross_seed(K, B, S, slot, rank, g, na, cpos, use_list ? nlist : 0u, lq);
+  return SEED_DONE;
 }
 
-enum : unsigned { TAIL_RUNNING = 0, TAIL_DONE = 1, TAIL_DEFERRED = 2, TAIL_STALLED = 3, TAIL_TIMEOUT = 4 };
+// ---------------------------------------------------------------------------
+// Device seed loop.  Late rounds hold few, small seeds; run as separate
+// launches with a host read per round they cost more in launch and
+// synchronisation latency than in work.  One cooperative launch (all CTAs
+// resident) runs the seeds that are left without rounds: a seed starts as
+// soon as the last head below it in its window has been resolved.
+//
+// The state is a word per scheduler block: the rank of its head, with BUSY
+// set from the moment the head is found ready until it has been finished, so
+// that nothing moves past a seed in flight.  The CTA that finishes a seed
+//  1. moves the other heads of the window past seeds it has claimed,
+//  2. moves its own block's head,
+//  3. tests the heads whose window holds a moved head, as k_ready_direct does;
+//     the one that sets BUSY queues the block, and keeps the first for itself.
+// Heads only grow, and two seeds in flight are never in each other's window,
+// so the order is the rounds' order: every seed after all lower ones of its
+// window.  Of two CTAs that move heads of one window at the same time at
+// least one sees both (a fence between the moves and the tests).  The
+// particle filed under a foreign cell waits until nothing is queued or in
+// flight: then every head left is above it.
+//
+// A seed whose records exceed a CTA's list is refined with the help of the
+// idle CTAs (share_refine); one with more than max_cand candidates ends the
+// loop, and a host round takes it.  The learned first ball is not used here
+// (the crossing starts from BALL0; the halo table does not depend on it).
+// Every wait is bounded: one that runs out without any seed being finished
+// records TAIL_TIMEOUT and every CTA leaves.
+//
+// Bound: the longest chain of seeds, each waiting for the one before.
+// Measured against rounds with three grid barriers each, which wait for the
+// slowest seed (grid-wide): 512^3 LOOP_512, heavy 256^3 LOOP_HEAVY.
+// ---------------------------------------------------------------------------
+enum : unsigned { TAIL_RUNNING = 0, TAIL_DONE = 1, TAIL_DEFERRED = 2, TAIL_TIMEOUT = 3 };
+constexpr unsigned HEAD_BUSY = 0x80000000u, RING_EMPTY = 0xffffffffu, NO_BLOCK = 0xffffffffu;
+static_assert((PSOD_INF_RANK & HEAD_BUSY) != 0u && PSOD_IDX_MASK < HEAD_BUSY, "ranks below the busy bit");
+
+// a seed's refinement items: exclusive prefix over its 27 candidate cells
+struct SharedRefine {
+  unsigned nitem, work, done, pad;
+  unsigned pref[28];
+};
+constexpr unsigned REFINE_CLOSED = 1u << 30;  // no item left to take
 
 struct TailState {
-  unsigned nact[2];       // active-block count of list act[p]
-  unsigned gmin[2];       // per round parity
-  // this round's counters, reset in its heads step (the previous round's last
-  // barrier is behind every reader); the kernel's SodBufs point at them
-  unsigned nready;
-  unsigned work;          // work counter of the seed step
-  unsigned cand_used;     // candidate buffer of the grid-refined seeds
-  unsigned nbigq, bigq[LOOP_BIG];
-  unsigned long long xused;
-  unsigned deferred;
+  // the words an idle CTA polls (one 64-byte read): queue head and tail,
+  // leave, seeds finished, and the slots + 1 of the shared refinements
+  unsigned qhead, qtail, leave, finished;
+  unsigned pad[4];
+  unsigned help[LOOP_BIG];
+  unsigned nact;          // active blocks at the launch
+  unsigned inflight;      // blocks queued or running, and CTAs in the first tests
+  unsigned quirk_wait;    // block + 1 whose head is the foreign-filed particle
   unsigned status;
-  unsigned rounds;        // rounds completed by the launch
-  unsigned parity;        // parity of the next round (its live list is act[parity])
-  unsigned bar_count, bar_gen;
-  // time spent by the launch in each step (ns, block 0's clock, each step
-  // up to the barrier that ends it)
-  unsigned long long t_heads, t_ready, t_seeds;
+  unsigned rounds;        // longest chain of seeds
+  unsigned long long xused, cused;  // shared parts of the crossing and candidate buffers
+  SharedRefine refine[LOOP_MAX_CTA];
+};
+static_assert(offsetof(TailState, help) == 32 && LOOP_BIG == 8, "polled words");
+
+constexpr unsigned LOOP_POLLS = 1u << 24;  // a few seconds without a finished seed
+
+__device__ __forceinline__ unsigned ld_state(const unsigned *p) { return *(volatile const unsigned *)p; }
+
+__device__ __forceinline__ void loop_timeout(TailState *ts) {
+  atomicExch(&ts->status, TAIL_TIMEOUT);
+  atomicExch(&ts->leave, 1u);
+}
+
+struct Flow {
+  TailState *ts;
+  const unsigned *bbegin, *blist;
+  unsigned *cursor, *head, *chain, *ring;
+  unsigned nblk;
+  int nb, rb;
+  unsigned quirk_rank;
 };
 
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
+__device__ __forceinline__ int wrap_block(int v, int nb) {
+  v %= nb;
+  return v < 0 ? v + nb : v;
 }
 
-constexpr unsigned long long BARRIER_POLLS = 1ull << 25;  // a few seconds of polling
-
-// Grid-wide barrier of the cooperative launch (generation counting).  The
-// fences make every write before the barrier visible to every read after
-// it.  Returns false when the wait ran out or another CTA's did.
-__device__ bool grid_barrier(TailState *ts) {
-  __shared__ int s_ok;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    volatile unsigned *gen = &ts->bar_gen;
-    volatile unsigned *status = &ts->status;
-    const unsigned g0 = *gen;
-    __threadfence();
-    if (atomicAdd(&ts->bar_count, 1u) == gridDim.x - 1) {
-      ts->bar_count = 0;
-      __threadfence();
-      atomicAdd(&ts->bar_gen, 1u);
-    } else {
-      unsigned long long polls = 0;
-      while (*gen == g0) {
-        if (*status == TAIL_TIMEOUT || ++polls > BARRIER_POLLS) {
-          ok = 0;
-          break;
-        }
-        __nanosleep(32);
-      }
-      if (!ok) atomicExch(&ts->status, TAIL_TIMEOUT);
+// first unresolved seed of block b at or after its cursor, and its list place
+__device__ __forceinline__ unsigned next_head(const Flow &F, const SodBufs &B, unsigned b, unsigned &cu) {
+  const unsigned end = F.bbegin[b + 1];
+  unsigned cur = ld_state(&F.cursor[b]);
+  while (cur < end) {
+    const unsigned zero = ~(ld_state(&B.resolved[cur >> 5]) >> (cur & 31u)) & (0xffffffffu >> (cur & 31u));
+    if (zero) {
+      cur = min(end, cur + (unsigned)(__ffs(zero) - 1));
+      break;
     }
-    __threadfence();
-    if (*status == TAIL_TIMEOUT) ok = 0;
-    s_ok = ok;
+    cur = (cur | 31u) + 1u;
   }
-  __syncthreads();
-  return s_ok != 0;
+  cu = min(cur, end);
+  return cu < end ? F.blist[cu] : PSOD_INF_RANK;
 }
 
-// value written by another CTA before the last barrier
-__device__ __forceinline__ unsigned ld_shared_state(const unsigned *p) { return *(volatile const unsigned *)p; }
-
-// The refinement items of the seeds whose records exceed a CTA's list, over
-// the grid's warps, then a CTA per seed from the exact sums on.  A function of
-// its own, so that its registers are not the one-CTA path's.
-__device__ __noinline__ bool big_seeds(const SodConst &K, const SodBufs &B, Smem &S, TailState *ts, unsigned nbig) {
+// Readiness of block c's head h (as ready_test_warp, over the live words).
+// A ready block is marked busy and queued, or kept in *keep.
+__device__ __forceinline__ void queue_if_ready(const Flow &F, unsigned c, unsigned h, unsigned chain, unsigned *keep) {
   const int lane = threadIdx.x & 31;
-  const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
-  const int w = threadIdx.x >> 5;
-  static_assert(27 * LOOP_BIG <= 4 * LOOP_TPB && 4 * LOOP_TPB <= NB, "item prefix: four cells a thread");
-  unsigned v[4], sum = 0;
-  for (int k = 0; k < 4; k++) {
-    const unsigned e = 4u * threadIdx.x + (unsigned)k;
-    v[k] = 0;
-    if (e < 27u * nbig) {
-      const unsigned slot = B.bigq[e / 27u];
-      if (B.st_active[slot]) v[k] = B.cell_chunks[slot * 27u + e % 27u];
+  const int nb = F.nb, rb = F.rb;
+  const int bx = (int)(c % (unsigned)nb), by = (int)((c / (unsigned)nb) % (unsigned)nb),
+            bz = (int)(c / ((unsigned)nb * nb));
+  const bool full = 2 * rb + 1 >= nb;
+  const int side = full ? nb : 2 * rb + 1, lo = full ? 0 : -rb;
+  const int nwin = side * side * side;
+  for (int e0 = 0; e0 < nwin; e0 += 128) {
+    bool lower = false;
+#pragma unroll
+    for (int u = 0; u < 4; u++) {
+      const int e = e0 + u * 32 + lane;
+      if (e < nwin) {
+        const int dx = e % side + lo, dy = (e / side) % side + lo, dz = e / (side * side) + lo;
+        int x = full ? dx : bx + dx, y = full ? dy : by + dy, z = full ? dz : bz + dz;
+        if (x < 0) x += nb;
+        if (x >= nb) x -= nb;
+        if (y < 0) y += nb;
+        if (y >= nb) y -= nb;
+        if (z < 0) z += nb;
+        if (z >= nb) z -= nb;
+        lower |= (ld_state(&F.head[(unsigned)x + (unsigned)nb * ((unsigned)y + (unsigned)nb * (unsigned)z)]) &
+                  ~HEAD_BUSY) < h;
+      }
     }
-    sum += v[k];
+    if (__any_sync(0xffffffffu, lower)) return;
   }
-  unsigned inc = sum;
-  for (int o = 1; o < 32; o <<= 1) {
-    const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
-    if (lane >= o) inc += y;
+  if (lane != 0) return;
+  TailState *ts = F.ts;
+  if (h == F.quirk_rank) {
+    atomicExch(&ts->quirk_wait, c + 1u);
+    return;
   }
-  if (lane == 31) S.red_u32[w] = inc;
+  if (atomicCAS(&F.head[c], h, h | HEAD_BUSY) != h) return;  // moved or queued by another CTA
+  F.chain[c] = chain;
+  if (atomicCAS(keep, NO_BLOCK, c) == NO_BLOCK) return;
+  atomicAdd(&ts->inflight, 1u);
+  __threadfence();
+  const unsigned at = atomicAdd(&ts->qtail, 1u);
+  for (unsigned p = 0; p < LOOP_POLLS; p++)  // the entry a lap before is being emptied at most
+    if (atomicCAS(&F.ring[at % F.nblk], RING_EMPTY, c) == RING_EMPTY) return;
+  loop_timeout(ts);
+}
+
+// Thread 0: the CTA's turn ends without a block of its own.  The last one out
+// ends the loop, or starts the foreign-filed particle's seed.
+__device__ __forceinline__ void leave_turn(const Flow &F, unsigned *keep) {
+  TailState *ts = F.ts;
+  __threadfence();
+  if (atomicSub(&ts->inflight, 1u) != 1u) return;
+  __threadfence();
+  const unsigned q = atomicExch(&ts->quirk_wait, 0u);
+  if (q != 0u && atomicCAS(&F.head[q - 1u], F.quirk_rank, F.quirk_rank | HEAD_BUSY) == F.quirk_rank) {
+    atomicAdd(&ts->inflight, 1u);
+    F.chain[q - 1u] = ld_state(&ts->rounds) + 1u;
+    *keep = q - 1u;
+    return;
+  }
+  atomicCAS(&ts->status, TAIL_RUNNING, TAIL_DONE);
+  __threadfence();
+  atomicExch(&ts->leave, 1u);
+}
+
+// After the seed of block b (rank r): the window's heads, the block's own,
+// and the blocks that this made ready.
+__device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Smem &S, unsigned b, unsigned r,
+                                             unsigned *keep) {
+  constexpr unsigned MOVED = 512, TESTS = 4096;
+  __shared__ unsigned s_moved, s_tests, s_own;
+  unsigned *mv_b = S.hist[0], *mv_h = S.hist[0] + MOVED, *test = S.hist[1];
+  static_assert(TESTS <= NB && 2 * MOVED <= NB && TESTS % LOOP_TPB == 0, "lists over the histograms");
+  const int t = threadIdx.x, w = t >> 5;
+  const int nb = F.nb, rb = F.rb;
+  const int bx = (int)(b % (unsigned)nb), by = (int)((b / (unsigned)nb) % (unsigned)nb),
+            bz = (int)(b / ((unsigned)nb * nb));
+  auto block_at = [&](int e, int rad, int side) {
+    return (unsigned)wrap_block(bx + e % side - rad, nb) +
+           (unsigned)nb * ((unsigned)wrap_block(by + (e / side) % side - rad, nb) +
+                           (unsigned)nb * (unsigned)wrap_block(bz + e / (side * side) - rad, nb));
+  };
+  __threadfence();  // the claims, before anything that follows from them
   __syncthreads();
-  unsigned at = inc - sum, nitem = 0;
-  for (int k = 0; k < nwarp(); k++) {
-    if (k < w) at += S.red_u32[k];
-    nitem += S.red_u32[k];
+  if (t == 0) s_moved = 1;
+  __syncthreads();
+  const int side1 = min(2 * rb + 1, nb), n1 = side1 * side1 * side1;
+  for (int e = t; e < n1; e += tpb()) {
+    const unsigned x = block_at(e, rb, side1);
+    if (x == b) {
+      unsigned cu;
+      unsigned h = next_head(F, B, b, cu);
+      if (h <= r) {  // the finished seed is not marked: never run it again
+        record_error(B, r, PSOD_ERR_STATE);
+        h = PSOD_INF_RANK;
+      }
+      *(volatile unsigned *)&F.cursor[b] = cu;
+      s_own = h;
+      mv_b[0] = b;
+      continue;
+    }
+    const unsigned h = ld_state(&F.head[x]);
+    if (h & HEAD_BUSY) continue;  // in flight, or no seed left
+    unsigned cu;
+    const unsigned h2 = next_head(F, B, x, cu);
+    if (h2 > h && atomicCAS(&F.head[x], h, h2) == h) {
+      *(volatile unsigned *)&F.cursor[x] = cu;  // a hint: any earlier place would do
+      const unsigned k = atomicAdd(&s_moved, 1u);
+      if (k < MOVED) {
+        mv_b[k] = x;
+      }
+    }
   }
-  for (int k = 0; k < 4; k++) {
-    S.pref[4u * threadIdx.x + (unsigned)k] = at;
-    at += v[k];
+  __syncthreads();
+  if (t == 0) atomicExch(&F.head[b], s_own);
+  __threadfence();
+  __syncthreads();
+  __threadfence();
+  // the moved heads as they are now: another CTA may have moved them on
+  for (unsigned k = t; k < min(s_moved, MOVED); k += tpb()) mv_h[k] = ld_state(&F.head[mv_b[k]]) & ~HEAD_BUSY;
+  __syncthreads();
+  // the heads whose window holds a moved one, and none moved that is still
+  // below them
+  const unsigned nmoved = min(s_moved, MOVED);
+  const bool all = s_moved > MOVED;
+  const unsigned chain = F.chain[b] + 1u;
+  const int rad2 = nmoved > 1u ? 2 * rb : rb;
+  const int side2 = min(2 * rad2 + 1, nb);
+  const long long n2 = (long long)side2 * side2 * side2;
+  for (long long e0 = 0; e0 < n2; e0 += TESTS) {
+    if (t == 0) s_tests = 0;
+    __syncthreads();
+    for (long long e = e0 + t; e < min(n2, e0 + (long long)TESTS); e += tpb()) {
+      const unsigned x = block_at((int)e, rad2, side2);
+      const unsigned h = ld_state(&F.head[x]);
+      if (h & HEAD_BUSY) continue;
+      const int cx = (int)(x % (unsigned)nb), cy = (int)((x / (unsigned)nb) % (unsigned)nb),
+                cz = (int)(x / ((unsigned)nb * nb));
+      bool near = all, below = false;
+      for (unsigned k = 0; k < nmoved && !below; k++) {
+        const unsigned m = mv_b[k];
+        int dx = abs((int)(m % (unsigned)nb) - cx), dy = abs((int)((m / (unsigned)nb) % (unsigned)nb) - cy),
+            dz = abs((int)(m / ((unsigned)nb * nb)) - cz);
+        dx = min(dx, nb - dx);
+        dy = min(dy, nb - dy);
+        dz = min(dz, nb - dz);
+        if (max(dx, max(dy, dz)) <= rb) {
+          near = true;
+          below = mv_h[k] < h;
+        }
+      }
+      if (near && !below) test[atomicAdd(&s_tests, 1u)] = x;
+    }
+    __syncthreads();
+    const unsigned nt = s_tests;
+    for (unsigned k = w; k < nt; k += nwarp()) {
+      const unsigned h = ld_state(&F.head[test[k]]);
+      if (!__any_sync(0xffffffffu, (h & HEAD_BUSY) != 0u)) queue_if_ready(F, test[k], __shfl_sync(0xffffffffu, h, 0), chain, keep);
+      __syncwarp();
+    }
+    __syncthreads();
   }
+}
+
+// Warps of any CTA take refinement items of the seed in `slot` until none is
+// left.  The item's data are read after it was taken, and the owner closes the
+// counter before it writes another seed's, so that a late warp takes nothing.
+__device__ __noinline__ void share_refine(const SodConst &K, const SodBufs &B, Smem &S, TailState *ts, unsigned slot) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   static_assert(sizeof(WarpRef) * MAX_WARP <= sizeof(unsigned) * MAXLEV * NB, "staging over the histograms");
   WarpRef &R = reinterpret_cast<WarpRef *>(S.hist)[w];
-  __syncthreads();
-  for (unsigned it = gtid >> 5; it < nitem; it += gthreads >> 5) {
-    unsigned lo = 0, hi = 27u * nbig;  // last cell whose prefix is <= it
-    while (hi - lo > 1) {
-      const unsigned mid = (lo + hi) >> 1;
-      if (S.pref[mid] <= it) lo = mid;
-      else hi = mid;
-    }
-    refine_item<false>(K, B, B.bigq[lo / 27u] * 27u + lo % 27u, it - S.pref[lo], false, R);
+  SharedRefine &H = ts->refine[slot];
+  while (true) {
+    unsigned it = 0;
+    if (lane == 0) it = atomicAdd(&H.work, 1u);
+    it = __shfl_sync(0xffffffffu, it, 0);
+    __threadfence();
+    if (it >= __shfl_sync(0xffffffffu, ld_state(&H.nitem), 0)) break;
+    const unsigned p = lane < 27 ? ld_state(&H.pref[lane]) : ~0u;
+    const unsigned le = __ballot_sync(0xffffffffu, p <= it);  // lane 0's prefix is 0
+    const int cell = 31 - __clz((int)le);
+    refine_item<false>(K, B, slot * 27u + (unsigned)cell, it - __shfl_sync(0xffffffffu, p, cell), false, R);
+    __threadfence();
     __syncwarp();
+    if (lane == 0) atomicAdd(&H.done, 1u);
   }
-  if (!grid_barrier(ts)) return false;
-  for (unsigned k = blockIdx.x; k < nbig; k += gridDim.x) {
-    __syncthreads();
-    const unsigned slot = B.bigq[k];
-    if (!B.st_active[slot]) continue;
-    const unsigned rank = B.ready[slot];
-    select_seed(K, B, S, slot, rank);
-    __syncthreads();
-    if (B.learn_collect) seed_features(K, B, S, slot, rank);
-    __syncthreads();
-    cross_seed(K, B, S, slot, rank, seed_geo(K, B, rank), B.st_na[slot], B.st_centre[slot]);
-  }
-  return grid_barrier(ts);
+  if (lane < (int)LOOP_BIG && ld_state(&ts->help[lane]) == slot + 1u) atomicCAS(&ts->help[lane], slot + 1u, 0u);
 }
 
-__global__ void __launch_bounds__(LOOP_TPB, 1) k_tail_rounds(const __grid_constant__ SodConst K,
-                                                                const __grid_constant__ SodBufs B, TailState *ts, unsigned *act0,
-                                                    unsigned *act1, const unsigned *bbegin, unsigned *cursor,
-                                                    const unsigned *blist, unsigned *head, int nb, int rb,
-                                                    unsigned quirk_rank, unsigned *ready) {
+// A seed whose records exceed a CTA's list.  A function of its own, so that
+// its registers are not the one-CTA path's.
+__device__ __noinline__ void big_seed(const SodConst &K, const SodBufs &B, Smem &S, TailState *ts, unsigned slot,
+                                      unsigned rank) {
+  const int t = threadIdx.x;
+  __shared__ int s_ok;
+  __syncthreads();
+  prep_seed(K, B, S, slot, rank);
+  __threadfence();
+  __syncthreads();
+  if (!ld_state(&B.st_active[slot])) return;
+  SharedRefine &H = ts->refine[slot];
+  if (t < 32) {
+    unsigned v = t < 27 ? B.cell_chunks[slot * 27u + (unsigned)t] : 0u, inc = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
+      if (t >= o) inc += y;
+    }
+    if (t < 28) *(volatile unsigned *)&H.pref[t] = inc - v;
+    if (t == 31) *(volatile unsigned *)&H.nitem = inc;
+    if (t == 0) *(volatile unsigned *)&H.done = 0u;
+    __threadfence();
+    __syncwarp();
+    if (t == 0) {
+      atomicExch(&H.work, 0u);
+      __threadfence();
+      for (unsigned k = 0; k < LOOP_BIG; k++)
+        if (atomicCAS(&ts->help[(slot + k) % LOOP_BIG], 0u, slot + 1u) == 0u) break;
+    }
+  }
+  __syncthreads();
+  share_refine(K, B, S, ts, slot);
+  __syncthreads();
+  if (t == 0) {
+    const unsigned n = ld_state(&H.nitem);
+    unsigned polls = 0;
+    s_ok = 1;
+    while (ld_state(&H.done) != n) {
+      if (++polls > LOOP_POLLS || ld_state(&ts->status) == TAIL_TIMEOUT) {
+        loop_timeout(ts);
+        s_ok = 0;
+        break;
+      }
+      __nanosleep(32);
+    }
+    atomicExch(&H.work, REFINE_CLOSED);
+    __threadfence();
+  }
+  __syncthreads();
+  __threadfence();
+  if (!s_ok) return;
+  select_seed(K, B, S, slot, rank);
+  __syncthreads();
+  if (B.learn_collect) seed_features(K, B, S, slot, rank);
+  __syncthreads();
+  cross_seed(K, B, S, slot, rank, seed_geo(K, B, rank), B.st_na[slot], B.st_centre[slot]);
+}
+
+// the last holder empties the shared part of a buffer
+__device__ __forceinline__ void release_shared(unsigned long long *used, unsigned n) {
+  if (n == 0) return;
+  const unsigned long long held = XHOLD * n, old = atomicAdd(used, 0ull - held);
+  if (old / XHOLD == n) atomicCAS(used, old - held, 0ull);
+}
+
+enum : unsigned { IDLE_SEED = 0, IDLE_HELP = 1, IDLE_LEAVE = 2 };
+
+// Warp 0 of an idle CTA: the next queued block, a refinement to share, or the
+// end.  Returned in *kind and *arg.
+__device__ __forceinline__ void idle_wait(const Flow &F, unsigned *kind, unsigned *arg) {
+  TailState *ts = F.ts;
+  const int lane = threadIdx.x & 31;
+  unsigned polls = 0, seen = 0xffffffffu, k = IDLE_LEAVE, a = 0;
+  while (true) {
+    const unsigned v = lane < 16 ? ld_state(&ts->qhead + lane) : 0u;
+    const unsigned qh = __shfl_sync(0xffffffffu, v, 0), qt = __shfl_sync(0xffffffffu, v, 1),
+                   leave = __shfl_sync(0xffffffffu, v, 2), fin = __shfl_sync(0xffffffffu, v, 3);
+    const unsigned hm = __ballot_sync(0xffffffffu, lane >= 8 && lane < 16 && v != 0u);
+    if (leave) break;
+    if ((int)(qt - qh) > 0) {
+      unsigned got = NO_BLOCK;
+      if (lane == 0 && atomicCAS(&ts->qhead, qh, qh + 1u) == qh) {
+        // the entry is written right after the tail was moved
+        for (unsigned p = 0; p < LOOP_POLLS && got == NO_BLOCK; p++) got = ld_state(&F.ring[qh % F.nblk]);
+        if (got == NO_BLOCK) loop_timeout(ts);
+        else atomicExch(&F.ring[qh % F.nblk], RING_EMPTY);
+      }
+      got = __shfl_sync(0xffffffffu, got, 0);
+      if (got != NO_BLOCK) {
+        k = IDLE_SEED;
+        a = got;
+        break;
+      }
+      continue;
+    }
+    if (hm) {
+      const unsigned m = hm >> 8, r = blockIdx.x & 7u;  // CTAs start at different entries
+      const unsigned e = (unsigned)(__ffs((int)(m >> r | m << (8u - r))) - 1) + r;
+      k = IDLE_HELP;
+      a = __shfl_sync(0xffffffffu, v, 8 + (int)(e & 7u)) - 1u;
+      break;
+    }
+    if (fin != seen) {
+      seen = fin;
+      polls = 0;
+    } else if (++polls > LOOP_POLLS) {
+      if (lane == 0) loop_timeout(ts);
+      break;
+    }
+    __nanosleep(40);
+  }
+  __threadfence();
+  if (lane == 0) {
+    *kind = k;
+    *arg = a;
+  }
+}
+
+__global__ void __launch_bounds__(LOOP_TPB, 1) k_seed_loop(const __grid_constant__ SodConst K,
+                                                           const __grid_constant__ SodBufs B,
+                                                           const __grid_constant__ Flow F, const unsigned *active,
+                                                           unsigned *ready) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Smem &S = *reinterpret_cast<Smem *>(smem_raw);
-  __shared__ unsigned s_cnt, s_next, s_nready;
-  const unsigned gtid = blockIdx.x * blockDim.x + threadIdx.x, gthreads = gridDim.x * blockDim.x;
-  const int lane = threadIdx.x & 31;
-  // the round parity: every CTA flips its own copy once per round
-  unsigned q = ts->parity;
+  __shared__ unsigned s_keep, s_kind, s_arg;
+  TailState *ts = F.ts;
+  const int t = threadIdx.x;
+  const unsigned slot = blockIdx.x;
+  const unsigned gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, gwarps = (gridDim.x * blockDim.x) >> 5;
+  if (t == 0) s_keep = NO_BLOCK;
+  __syncthreads();
+  // the first ready blocks; other CTAs may already be finishing theirs
+  const unsigned cnt = ts->nact;
+  for (unsigned wi = gwarp; wi < cnt; wi += gwarps) {
+    const unsigned b = active[wi];
+    const unsigned h = __shfl_sync(0xffffffffu, ld_state(&F.head[b]), 0);
+    if (!(h & HEAD_BUSY)) queue_if_ready(F, b, h, 1u, &s_keep);
+    __syncwarp();
+  }
   while (true) {
-    // this round's active count was written (heads of the previous round,
-    // or the host) before the last barrier
-    if (threadIdx.x == 0) s_cnt = ld_shared_state(&ts->nact[q]);
     __syncthreads();
-    const unsigned cnt = s_cnt;
-    const bool timer = blockIdx.x == 0 && threadIdx.x == 0;
-    unsigned long long tk = timer ? global_ns() : 0ull;
-    unsigned *cur = q ? act1 : act0, *nxt = q ? act0 : act1;
-    if (timer) {
-      ts->nready = 0;
-      ts->work = 0;
-      ts->cand_used = 0;
-      ts->nbigq = 0;
-      ts->xused = 0;
+    if (t == 0 && s_keep == NO_BLOCK) leave_turn(F, &s_keep);
+    __syncthreads();
+    unsigned b = s_keep;
+    while (b == NO_BLOCK) {
+      if (t < 32) idle_wait(F, &s_kind, &s_arg);
+      __syncthreads();
+      const unsigned kind = s_kind, arg = s_arg;
+      __threadfence();
+      if (kind == IDLE_LEAVE) return;
+      if (kind == IDLE_SEED) b = arg;
+      else share_refine(K, B, S, ts, arg);
+      __syncthreads();
     }
-    // heads (k_heads): warp-uniform strides over the active list
-    for (unsigned base = gtid - (unsigned)lane; base < cnt; base += gthreads) {
-      const unsigned i = base + (unsigned)lane;
-      const bool have = i < cnt;
-      unsigned b = 0, h = PSOD_INF_RANK, cu = 0;
-      if (have) {
-        b = cur[i];
-        const unsigned end = bbegin[b + 1];
-        cu = first_unresolved(B.resolved, cursor[b], end);
-        if (cu < end) h = blist[cu];
+    const unsigned rank = ld_state(&F.head[b]) & ~HEAD_BUSY;
+    __syncthreads();  // every thread has read s_keep
+    if (t == 0) {
+      ready[slot] = rank;
+      S.xshared = S.cshared = 0;
+      s_keep = NO_BLOCK;
+    }
+    __syncthreads();
+    const int how = small_seed(K, B, S, slot, rank);
+    if (how == SEED_BIG) big_seed(K, B, S, ts, slot, rank);
+    __syncthreads();
+    if (t == 0) {
+      release_shared(B.xused, S.xshared);
+      release_shared(B.cused, S.cshared);
+      atomicAdd(&ts->finished, 1u);
+      atomicMax(&ts->rounds, F.chain[b]);
+      if (how == SEED_DEFERRED) {
+        atomicCAS(&ts->status, TAIL_RUNNING, TAIL_DEFERRED);
+        atomicExch(&ts->leave, 1u);
       }
-      const bool live = have && h != PSOD_INF_RANK;
-      const unsigned lm = __ballot_sync(0xffffffffu, live);
-      unsigned at = 0;
-      if (lane == 0 && lm) at = atomicAdd(&ts->nact[q ^ 1u], (unsigned)__popc(lm));
-      at = __shfl_sync(0xffffffffu, at, 0);
-      unsigned hmin = live ? h : PSOD_INF_RANK;
-      for (int o = 16; o > 0; o >>= 1) hmin = min(hmin, __shfl_xor_sync(0xffffffffu, hmin, o));
-      if (lane == 0 && hmin != PSOD_INF_RANK) atomicMin(&ts->gmin[q], hmin);
-      if (have) {
-        cursor[b] = cu;
-        head[b] = h;
-        if (live) nxt[at + __popc(lm & ((1u << lane) - 1u))] = b;
-      }
+      s_kind = ld_state(&ts->leave);
     }
-    if (!grid_barrier(ts)) return;
-    if (timer) {
-      const unsigned long long now = global_ns();
-      ts->t_heads += now - tk;
-      tk = now;
-    }
-    // the next round's counts (parity q^1) are free now: reset them
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      ts->nact[q] = 0;
-      ts->gmin[q ^ 1u] = PSOD_INF_RANK;
-    }
-    if (threadIdx.x == 0) s_next = ld_shared_state(&ts->nact[q ^ 1u]);
     __syncthreads();
-    const unsigned next = s_next;
-    const unsigned gmin = ld_shared_state(&ts->gmin[q]);
-    // readiness: the direct window test (the launch is used only while few
-    // blocks are active), a warp per active block
-    for (unsigned wi = gtid >> 5; wi < next; wi += gthreads >> 5)
-      ready_test_warp(nxt[wi], head, nb, rb, quirk_rank, gmin, ready, &ts->nready, B.cap_ready);
-    if (!grid_barrier(ts)) return;
-    if (timer) {
-      const unsigned long long now = global_ns();
-      ts->t_ready += now - tk;
-      tk = now;
-    }
-    if (threadIdx.x == 0) s_nready = ld_shared_state(&ts->nready);
-    __syncthreads();
-    const unsigned nready = min(s_nready, B.cap_ready);
-    if (nready == 0) {
-      // the lowest-ranked unresolved seed is always ready: an empty round
-      // with active blocks left is a scheduler fault
-      if (blockIdx.x == 0 && threadIdx.x == 0) {
-        ts->status = next > 0 ? TAIL_STALLED : TAIL_DONE;
-        ts->parity = q ^ 1u;
-      }
-      return;
-    }
-    // the round's seeds, a CTA each from the preselect to the claims: ready
-    // seeds share no particle, so nothing is waited for in between
-    while (true) {
-      const unsigned item = next_item(&ts->work);
-      if (item >= nready) break;
-      small_seed(K, B, S, item, B.ready[item]);
-    }
-    if (!grid_barrier(ts)) return;
-    if (threadIdx.x == 0) s_cnt = ld_shared_state(&ts->nbigq);
-    __syncthreads();
-    const unsigned nbig = min(s_cnt, LOOP_BIG);
-    if (nbig > 0 && !big_seeds(K, B, S, ts, nbig)) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-      ts->rounds++;
-      ts->parity = q ^ 1u;
-      ts->t_seeds += global_ns() - tk;
-    }
-    if (threadIdx.x == 0) s_nready = ld_shared_state(&ts->deferred);
-    __syncthreads();
-    if (s_nready) {
-      if (blockIdx.x == 0 && threadIdx.x == 0) ts->status = TAIL_DEFERRED;
-      return;
-    }
-    q ^= 1u;
+    // the loop ends: the block stays as it is, the host finds its head anew
+    if (s_kind) return;
+    finish_block(F, B, S, b, rank, &s_keep);
   }
 }
 
-__global__ void k_tail_init(TailState *ts, unsigned n_active) {
-  ts->nact[0] = n_active;
-  ts->nact[1] = 0;
-  ts->gmin[0] = ts->gmin[1] = PSOD_INF_RANK;
-  ts->deferred = 0;
-  ts->status = TAIL_RUNNING;
-  ts->rounds = 0;
-  ts->parity = 0;
-  ts->bar_count = 0;
-  ts->bar_gen = 0;
-  ts->t_heads = ts->t_ready = ts->t_seeds = 0;
+// one launch before the loop: its state, an empty ring, the live count
+__global__ void k_tail_init(TailState *ts, const unsigned *n_active, unsigned grid, unsigned *ring, unsigned nblk) {
+  const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
+  for (unsigned k = i; k < nblk; k += gridDim.x * blockDim.x) ring[k] = RING_EMPTY;
+  if (i < LOOP_MAX_CTA) ts->refine[i].work = REFINE_CLOSED;
+  if (i < LOOP_BIG) ts->help[i] = 0;
+  if (i == 0) {
+    ts->qhead = ts->qtail = ts->leave = ts->finished = 0;
+    ts->nact = *n_active;
+    ts->inflight = grid;
+    ts->quirk_wait = 0;
+    ts->status = TAIL_RUNNING;
+    ts->rounds = 0;
+    ts->xused = ts->cused = 0;
+  }
 }
 
 __global__ void k_find_rank(const unsigned *seed_idx, long long nseed, unsigned idx, unsigned *out) {
@@ -4349,9 +4576,10 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
   B.bound_min = (unsigned)c->tune.bound_min_cand;
   B.maxcand = ctrs + 13;
   B.max_cand = ~0u;
-  B.deferred = ctrs + 14;
+  B.loop_cand = 0;
+  B.loop_x = 0;
+  B.cused = nullptr;
   B.rn_chunk = RN_CHUNK;
-  B.bigq = B.nbigq = nullptr;
   B.alive_cnt = nullptr;
   B.pairs = u64s + 5;
   B.touch = u64s + 7;
@@ -4455,10 +4683,10 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, c->device);
     int per_sm_tail = 0;
     if (coop && (rc = scratch(c, SC_TAIL, 1, &tail)) == PSOD_OK &&
-        cudaFuncSetAttribute(k_tail_rounds, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_tail, k_tail_rounds, LOOP_TPB, smem) == cudaSuccess &&
+        cudaFuncSetAttribute(k_seed_loop, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm_tail, k_seed_loop, LOOP_TPB, smem) == cudaSuccess &&
         per_sm_tail > 0)
-      tail_grid = dev_sms * per_sm_tail;
+      tail_grid = (int)std::min<long long>(std::min(dev_sms * per_sm_tail, LOOP_MAX_CTA), cap_ready);
     if (rc) return rc;
     cudaGetLastError();
   }
@@ -4593,48 +4821,49 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
         (long long)nready <= LOOP_READY * c->tune.tail_max_ready && rest >= rest_need && n_active > 0 &&
         (long long)n_active * direct_cost_per_block <= LOOP_TESTS) {
       // the following rounds on the device, until a larger seed or the end
-      k_tail_init<<<1, 1, 0, c->stream>>>(tail, n_active);
+      k_round_reset<<<1, 32, 0, c->stream>>>(ctrs, u64s + 17);
+      k_heads<<<nblk((long long)n_active, 256), 256, 0, c->stream>>>(act_a, n_active, bbegin, cursor, blist, resolved,
+                                                                     head, nullptr, act_b, ctrs + 9);
+      std::swap(act_a, act_b);
+      k_tail_init<<<64, 256, 0, c->stream>>>(tail, ctrs + 9, (unsigned)tail_grid, filt_b, (unsigned)nblocks);
       SodBufs Bt = B;
       Bt.max_cand = (unsigned)std::min<long long>(LOOP_CAND * c->tune.tail_max_cand, NB);
-      Bt.rn_chunk = LOOP_CHUNK;
-      Bt.nready = &tail->nready;
-      Bt.cand_used = &tail->cand_used;
-      Bt.nbigq = &tail->nbigq;
-      Bt.bigq = tail->bigq;
+      // half of the candidate and crossing buffers in equal parts for the
+      // CTAs, the rest shared by the seeds that need more
+      Bt.loop_cand = (unsigned)std::max<long long>(1, cand_cap / 2 / tail_grid);
+      Bt.loop_x = (unsigned long long)std::max<long long>(1, xcap / 2 / tail_grid);
       Bt.xused = &tail->xused;
-      Bt.deferred = &tail->deferred;
+      Bt.cused = &tail->cused;
+      Bt.rn_chunk = LOOP_CHUNK;
       Bt.maxcand = nullptr;
       Bt.learn_use = 0;
       Bt.st_big = nullptr;
       Bt.touch = u64s + 19;  // the tail's crossings counted apart from k_cross
       Bt.kept_members = u64s + 20;
-      void *args[] = {(void *)&K,     (void *)&Bt,   (void *)&tail, (void *)&act_a,      (void *)&act_b,
-                      (void *)&bbegin, (void *)&cursor, (void *)&blist, (void *)&head, (void *)&nb,
-                      (void *)&rb,    (void *)&quirk_rank, (void *)&ready};
+      Flow F{tail, bbegin, blist, cursor, head, filt_a, filt_b, (unsigned)nblocks, nb, rb, quirk_rank};
+      void *args[] = {(void *)&K, (void *)&Bt, (void *)&F, (void *)&act_a, (void *)&ready};
       t_tail.start(c->stream);
-      PSOD_CUDA(c, cudaLaunchCooperativeKernel((const void *)k_tail_rounds, dim3(tail_grid), dim3(LOOP_TPB), args, smem,
+      PSOD_CUDA(c, cudaLaunchCooperativeKernel((const void *)k_seed_loop, dim3(tail_grid), dim3(LOOP_TPB), args, smem,
                                                c->stream));
       t_tail.stop(c->stream);
-      kernels += 2;
+      kernels += 4;
       TailState ts;
-      PSOD_CUDA(c, cudaMemcpyAsync(&ts, tail, sizeof(ts), cudaMemcpyDeviceToHost, c->stream));
+      PSOD_CUDA(c, cudaMemcpyAsync(&ts, tail, offsetof(TailState, refine), cudaMemcpyDeviceToHost, c->stream));
       PSOD_CUDA(c, cudaStreamSynchronize(c->stream));
       t_tail.collect();
       collect_pending();
       rounds += ts.rounds;
       tail_rounds += ts.rounds;
 #ifdef PSOD_TRACE_ROUNDS
-      fprintf(stderr, "psod tail launch rounds %u status %u heads %.3f ready %.3f seeds %.3f ms total %.3f ms grid %d\n",
-              ts.rounds, ts.status, ts.t_heads * 1e-6, ts.t_ready * 1e-6, ts.t_seeds * 1e-6, t_tail.last, tail_grid);
+      fprintf(stderr, "psod tail launch: chain %u seeds %u status %u total %.3f ms grid %d\n", ts.rounds, ts.finished,
+              ts.status, t_tail.last, tail_grid);
 #endif
       if (ts.status == TAIL_TIMEOUT)
-        return set_err(c, PSOD_ERR_TIMEOUT, "device tail loop: a grid barrier wait ran out");
-      if (ts.status == TAIL_STALLED) return set_err(c, PSOD_ERR_STATE, "scheduler stalled with unresolved seeds");
+        return set_err(c, PSOD_ERR_TIMEOUT, "device seed loop: a wait ran out");
       if (ts.status != TAIL_DONE && ts.status != TAIL_DEFERRED)
-        return set_err(c, PSOD_ERR_STATE, "device tail loop ended in an unknown state");
-      // the live list and its count for the host's next round
-      if (ts.parity) std::swap(act_a, act_b);
-      n_active = ts.status == TAIL_DONE ? 0u : ts.nact[ts.parity];
+        return set_err(c, PSOD_ERR_STATE, "device seed loop ended in an unknown state");
+      // the list at the launch holds every block still active
+      n_active = ts.status == TAIL_DONE ? 0u : ts.nact;
       rest = 0;
       rest_need = (int)ts.rounds < LOOP_SHORT ? LOOP_REST : 1;
     }
