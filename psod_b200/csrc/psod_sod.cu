@@ -2857,7 +2857,7 @@ __global__ void __launch_bounds__(TPB) k_cross(SodConst K, SodBufs B) {
 // its own candidates, so its sum (FP32 terms, relative error below 2e-6),
 // deflated by 1e-3, is at most the maximum.  CTA per seed, each warp a share of
 // the records (a warp alone walked the 1e5 records of a cluster's 27 cells in
-// 2.9 ms; the kernel took SEED_LOWER at 512^3).
+// 2.9 ms; the kernel took 2.75 ms at 512^3, under 0.3 with a CTA a seed).
 constexpr int LOWER_TPB = 512;
 
 __global__ void __launch_bounds__(LOWER_TPB) k_seed_lower(SodConst K, SodBufs B) {
@@ -3195,7 +3195,8 @@ __global__ void k_ready_direct(const unsigned *active, const unsigned *nactive, 
 // Bound: latency of one CTA (late rounds hold a few seeds, each waiting for
 // the one before it).  Measured per round at 512^3 (1-50 seeds a round):
 // separate steps 200 us (preselect 20, refinement a warp per candidate cell
-// 120, select 12, crossing 30, seven grid barriers); one CTA ROUND_US.
+// 120, select 12, crossing 30, seven grid barriers); one CTA about 70 a seed
+// (list 11, approximate sums 24, exact sums 5, ball 6, the rest).
 constexpr int SL_CELLS = 125;
 enum : int { SEED_DONE = 0, SEED_BIG = 1, SEED_DEFERRED = 2 };
 
@@ -3646,7 +3647,7 @@ __device__ __forceinline__ int small_seed(const SodConst &K, const SodBufs &B, S
 //
 // Bound: the longest chain of seeds, each waiting for the one before.
 // Measured against rounds with three grid barriers each, which wait for the
-// slowest seed (grid-wide): 512^3 LOOP_512, heavy 256^3 LOOP_HEAVY.
+// slowest seed (grid-wide): loop of 512^3 90 -> 74 ms, heavy 256^3 65 -> 39.
 // ---------------------------------------------------------------------------
 enum : unsigned { TAIL_RUNNING = 0, TAIL_DONE = 1, TAIL_DEFERRED = 2, TAIL_TIMEOUT = 3 };
 constexpr unsigned HEAD_BUSY = 0x80000000u, RING_EMPTY = 0xffffffffu, NO_BLOCK = 0xffffffffu;
@@ -3673,7 +3674,8 @@ struct TailState {
   unsigned long long xused, cused;  // shared parts of the crossing and candidate buffers
   SharedRefine refine[LOOP_MAX_CTA];
 };
-static_assert(offsetof(TailState, help) == 32 && LOOP_BIG == 8, "polled words");
+constexpr int BOARD_HELP = 8, BOARD_END = BOARD_HELP + (int)LOOP_BIG;
+static_assert(offsetof(TailState, help) == 4 * BOARD_HELP && LOOP_BIG == 8, "polled words");
 
 constexpr unsigned LOOP_POLLS = 1u << 24;  // a few seconds without a finished seed
 
@@ -3688,35 +3690,34 @@ struct Flow {
   TailState *ts;
   const unsigned *bbegin, *blist;
   unsigned *cursor, *head, *chain, *ring;
-  unsigned nblk;
+  unsigned cap;  // entries of the queue, ring: the active blocks at the launch
   int nb, rb;
   unsigned quirk_rank;
 };
 
-__device__ __forceinline__ int wrap_block(int v, int nb) {
-  v %= nb;
-  return v < 0 ? v + nb : v;
-}
-
-// first unresolved seed of block b at or after its cursor, and its list place
-__device__ __forceinline__ unsigned next_head(const Flow &F, const SodBufs &B, unsigned b, unsigned &cu) {
-  const unsigned end = F.bbegin[b + 1];
-  unsigned cur = ld_state(&F.cursor[b]);
+// first_unresolved on words that other CTAs are writing
+__device__ __forceinline__ unsigned next_unresolved(const SodBufs &B, unsigned cur, unsigned end) {
   while (cur < end) {
     const unsigned zero = ~(ld_state(&B.resolved[cur >> 5]) >> (cur & 31u)) & (0xffffffffu >> (cur & 31u));
-    if (zero) {
-      cur = min(end, cur + (unsigned)(__ffs(zero) - 1));
-      break;
-    }
+    if (zero) return min(end, cur + (unsigned)(__ffs(zero) - 1));
     cur = (cur | 31u) + 1u;
   }
-  cu = min(cur, end);
-  return cu < end ? F.blist[cu] : PSOD_INF_RANK;
+  return end;
 }
 
 // Readiness of block c's head h (as ready_test_warp, over the live words).
-// A ready block is marked busy and queued, or kept in *keep.
-__device__ __forceinline__ void queue_if_ready(const Flow &F, unsigned c, unsigned h, unsigned chain, unsigned *keep) {
+// True in lane 0 when this warp marked the block busy.
+__device__ __forceinline__ bool mark_ready(const Flow &F, unsigned c, unsigned h, unsigned chain) {
+  if (h == F.quirk_rank) {
+    atomicExch(&F.ts->quirk_wait, c + 1u);
+    return false;
+  }
+  if (atomicCAS(&F.head[c], h, h | HEAD_BUSY) != h) return false;  // moved or queued by another CTA
+  F.chain[c] = chain;
+  return true;
+}
+
+__device__ __forceinline__ bool mark_if_ready_warp(const Flow &F, unsigned c, unsigned h, unsigned chain) {
   const int lane = threadIdx.x & 31;
   const int nb = F.nb, rb = F.rb;
   const int bx = (int)(c % (unsigned)nb), by = (int)((c / (unsigned)nb) % (unsigned)nb),
@@ -3742,22 +3743,21 @@ __device__ __forceinline__ void queue_if_ready(const Flow &F, unsigned c, unsign
                   ~HEAD_BUSY) < h;
       }
     }
-    if (__any_sync(0xffffffffu, lower)) return;
+    if (__any_sync(0xffffffffu, lower)) return false;
   }
-  if (lane != 0) return;
+  return lane == 0 && mark_ready(F, c, h, chain);
+}
+
+// One more block in flight, first come first served.  (Queues by rank or by
+// the seeds left around the block, tried at 512^3, did not shorten the loop:
+// a CTA that keeps a block it made ready already follows the long chains.)
+__device__ __forceinline__ void push_block(const Flow &F, unsigned c) {
   TailState *ts = F.ts;
-  if (h == F.quirk_rank) {
-    atomicExch(&ts->quirk_wait, c + 1u);
-    return;
-  }
-  if (atomicCAS(&F.head[c], h, h | HEAD_BUSY) != h) return;  // moved or queued by another CTA
-  F.chain[c] = chain;
-  if (atomicCAS(keep, NO_BLOCK, c) == NO_BLOCK) return;
   atomicAdd(&ts->inflight, 1u);
   __threadfence();
-  const unsigned at = atomicAdd(&ts->qtail, 1u);
+  const unsigned at = atomicAdd(&ts->qtail, 1u) % F.cap;
   for (unsigned p = 0; p < LOOP_POLLS; p++)  // the entry a lap before is being emptied at most
-    if (atomicCAS(&F.ring[at % F.nblk], RING_EMPTY, c) == RING_EMPTY) return;
+    if (atomicCAS(&F.ring[at], RING_EMPTY, c) == RING_EMPTY) return;
   loop_timeout(ts);
 }
 
@@ -3781,50 +3781,69 @@ __device__ __forceinline__ void leave_turn(const Flow &F, unsigned *keep) {
 }
 
 // After the seed of block b (rank r): the window's heads, the block's own,
-// and the blocks that this made ready.
+// and the blocks that this made ready, one of them kept in *keep.  Only blocks
+// whose window holds a moved head can be: those within rb of the moved heads'
+// box.  The heads of all their windows are staged in shared memory, a slab of
+// planes at a time, and a separable minimum over them tells the ready ones
+// (windows too large for one plane of it are tested a warp per block).
+// Bound: eight or so dependent L2 reads; tests a warp per block took
+// 25 us a seed at 512^3 (rb 4), staged 16.
 __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Smem &S, unsigned b, unsigned r,
                                              unsigned *keep) {
-  constexpr unsigned MOVED = 512, TESTS = 4096;
-  __shared__ unsigned s_moved, s_tests, s_own;
-  unsigned *mv_b = S.hist[0], *mv_h = S.hist[0] + MOVED, *test = S.hist[1];
-  static_assert(TESTS <= NB && 2 * MOVED <= NB && TESTS % LOOP_TPB == 0, "lists over the histograms");
+  constexpr long long STAGE = (long long)MAXLEV * NB;
+  __shared__ unsigned s_own;
+  __shared__ int s_lo[3], s_hi[3];  // box of the moved heads, from b
   const int t = threadIdx.x, w = t >> 5;
   const int nb = F.nb, rb = F.rb;
   const int bx = (int)(b % (unsigned)nb), by = (int)((b / (unsigned)nb) % (unsigned)nb),
             bz = (int)(b / ((unsigned)nb * nb));
-  auto block_at = [&](int e, int rad, int side) {
-    return (unsigned)wrap_block(bx + e % side - rad, nb) +
-           (unsigned)nb * ((unsigned)wrap_block(by + (e / side) % side - rad, nb) +
-                           (unsigned)nb * (unsigned)wrap_block(bz + e / (side * side) - rad, nb));
+  // the block (dx, dy, dz) from b, and place e of a box as its offsets
+  auto wrap = [&](int v) {
+    while (v < 0) v += nb;
+    while (v >= nb) v -= nb;
+    return (unsigned)v;
+  };
+  auto block_at = [&](int dx, int dy, int dz) {
+    return wrap(bx + dx) + (unsigned)nb * (wrap(by + dy) + (unsigned)nb * wrap(bz + dz));
+  };
+  auto split = [](int e, int sx, int sy, int &x, int &y, int &z) {  // e < 2^22: exact
+    const int q = (int)(((float)e + 0.5f) * (1.0f / (float)sx));
+    z = (int)(((float)q + 0.5f) * (1.0f / (float)sy));
+    x = e - q * sx;
+    y = q - z * sy;
   };
   __threadfence();  // the claims, before anything that follows from them
   __syncthreads();
-  if (t == 0) s_moved = 1;
+  if (t == 0) {
+    for (int k = 0; k < 3; k++) s_lo[k] = s_hi[k] = 0;
+  }
   __syncthreads();
   const int side1 = min(2 * rb + 1, nb), n1 = side1 * side1 * side1;
   for (int e = t; e < n1; e += tpb()) {
-    const unsigned x = block_at(e, rb, side1);
+    int d[3];
+    split(e, side1, side1, d[0], d[1], d[2]);
+    for (int k = 0; k < 3; k++) d[k] -= side1 / 2;
+    const unsigned x = block_at(d[0], d[1], d[2]);
+    const unsigned h = ld_state(&F.head[x]), end = F.bbegin[x + 1];
+    unsigned cu = ld_state(&F.cursor[x]);
+    if (x != b && (h & HEAD_BUSY)) continue;  // in flight, or no seed left
+    cu = next_unresolved(B, cu, end);
     if (x == b) {
-      unsigned cu;
-      unsigned h = next_head(F, B, b, cu);
-      if (h <= r) {  // the finished seed is not marked: never run it again
+      unsigned own = cu < end ? F.blist[cu] : PSOD_INF_RANK;
+      if (own <= r) {  // the finished seed is not marked: never run it again
         record_error(B, r, PSOD_ERR_STATE);
-        h = PSOD_INF_RANK;
+        own = PSOD_INF_RANK;
       }
       *(volatile unsigned *)&F.cursor[b] = cu;
-      s_own = h;
-      mv_b[0] = b;
+      s_own = own;
       continue;
     }
-    const unsigned h = ld_state(&F.head[x]);
-    if (h & HEAD_BUSY) continue;  // in flight, or no seed left
-    unsigned cu;
-    const unsigned h2 = next_head(F, B, x, cu);
+    const unsigned h2 = cu < end ? F.blist[cu] : PSOD_INF_RANK;
     if (h2 > h && atomicCAS(&F.head[x], h, h2) == h) {
       *(volatile unsigned *)&F.cursor[x] = cu;  // a hint: any earlier place would do
-      const unsigned k = atomicAdd(&s_moved, 1u);
-      if (k < MOVED) {
-        mv_b[k] = x;
+      for (int k = 0; k < 3; k++) {
+        if (d[k] < 0) atomicMin(&s_lo[k], d[k]);
+        if (d[k] > 0) atomicMax(&s_hi[k], d[k]);
       }
     }
   }
@@ -3833,49 +3852,65 @@ __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Sm
   __threadfence();
   __syncthreads();
   __threadfence();
-  // the moved heads as they are now: another CTA may have moved them on
-  for (unsigned k = t; k < min(s_moved, MOVED); k += tpb()) mv_h[k] = ld_state(&F.head[mv_b[k]]) & ~HEAD_BUSY;
-  __syncthreads();
-  // the heads whose window holds a moved one, and none moved that is still
-  // below them
-  const unsigned nmoved = min(s_moved, MOVED);
-  const bool all = s_moved > MOVED;
   const unsigned chain = F.chain[b] + 1u;
-  const int rad2 = nmoved > 1u ? 2 * rb : rb;
-  const int side2 = min(2 * rad2 + 1, nb);
-  const long long n2 = (long long)side2 * side2 * side2;
-  for (long long e0 = 0; e0 < n2; e0 += TESTS) {
-    if (t == 0) s_tests = 0;
-    __syncthreads();
-    for (long long e = e0 + t; e < min(n2, e0 + (long long)TESTS); e += tpb()) {
-      const unsigned x = block_at((int)e, rad2, side2);
-      const unsigned h = ld_state(&F.head[x]);
-      if (h & HEAD_BUSY) continue;
-      const int cx = (int)(x % (unsigned)nb), cy = (int)((x / (unsigned)nb) % (unsigned)nb),
-                cz = (int)(x / ((unsigned)nb * nb));
-      bool near = all, below = false;
-      for (unsigned k = 0; k < nmoved && !below; k++) {
-        const unsigned m = mv_b[k];
-        int dx = abs((int)(m % (unsigned)nb) - cx), dy = abs((int)((m / (unsigned)nb) % (unsigned)nb) - cy),
-            dz = abs((int)(m / ((unsigned)nb * nb)) - cz);
-        dx = min(dx, nb - dx);
-        dy = min(dy, nb - dy);
-        dz = min(dz, nb - dz);
-        if (max(dx, max(dy, dz)) <= rb) {
-          near = true;
-          below = mv_h[k] < h;
-        }
+  // candidates: from (x0, y0, z0), C on a side; their windows: L on a side
+  const int x0 = s_lo[0] - rb, y0 = s_lo[1] - rb, z0 = s_lo[2] - rb;
+  const int Cx = s_hi[0] + rb + 1 - x0, Cy = s_hi[1] + rb + 1 - y0, Cz = s_hi[2] + rb + 1 - z0;
+  const int Lx = Cx + 2 * rb, Ly = Cy + 2 * rb;
+  auto add_new = [&](unsigned x) {  // the first stays with this CTA
+    if (atomicCAS(keep, NO_BLOCK, x) != NO_BLOCK) push_block(F, x);
+  };
+  const long long plane = (long long)Lx * Ly + (long long)Cx * Ly + (long long)Cx * Cy;
+  const int slab = (int)min((long long)Cz, STAGE / plane - 2 * rb);  // candidate planes staged at a time
+  if (slab > 0) {
+    for (int zs = 0; zs < Cz; zs += slab) {
+      const int T = min(slab, Cz - zs), Lz = T + 2 * rb;
+      unsigned *raw = S.hist[0], *mx = raw + Lx * Ly * Lz, *my = mx + Cx * Ly * Lz;
+      int x, y, z;
+      for (int e = t; e < Lx * Ly * Lz; e += tpb()) {
+        split(e, Lx, Ly, x, y, z);
+        raw[e] = ld_state(&F.head[block_at(x0 - rb + x, y0 - rb + y, z0 - rb + zs + z)]);
       }
-      if (near && !below) test[atomicAdd(&s_tests, 1u)] = x;
+      __syncthreads();
+      for (int e = t; e < Cx * Ly * Lz; e += tpb()) {
+        split(e, Cx, Ly, x, y, z);
+        const unsigned *p = raw + x + Lx * (y + Ly * z);
+        unsigned m = ~0u;
+        for (int d = 0; d <= 2 * rb; d++) m = min(m, p[d] & ~HEAD_BUSY);
+        mx[e] = m;
+      }
+      __syncthreads();
+      for (int e = t; e < Cx * Cy * Lz; e += tpb()) {
+        split(e, Cx, Cy, x, y, z);
+        const unsigned *p = mx + x + Cx * (y + Ly * z);
+        unsigned m = ~0u;
+        for (int d = 0; d <= 2 * rb; d++) m = min(m, p[d * Cx]);
+        my[e] = m;
+      }
+      __syncthreads();
+      for (int e = t; e < Cx * Cy * T; e += tpb()) {
+        split(e, Cx, Cy, x, y, z);
+        const unsigned h = raw[x + rb + Lx * (y + rb + Ly * (z + rb))];
+        if (h & HEAD_BUSY) continue;
+        unsigned m = ~0u;
+        for (int d = 0; d <= 2 * rb; d++) m = min(m, my[e + d * Cx * Cy]);
+        if (m != h) continue;
+        const unsigned c = block_at(x0 + x, y0 + y, z0 + zs + z);
+        if (mark_ready(F, c, h, chain)) add_new(c);
+      }
+      __syncthreads();
     }
-    __syncthreads();
-    const unsigned nt = s_tests;
-    for (unsigned k = w; k < nt; k += nwarp()) {
-      const unsigned h = ld_state(&F.head[test[k]]);
-      if (!__any_sync(0xffffffffu, (h & HEAD_BUSY) != 0u)) queue_if_ready(F, test[k], __shfl_sync(0xffffffffu, h, 0), chain, keep);
+  } else {
+    const int sx = min(Cx, nb), sy = min(Cy, nb), sz = min(Cz, nb);
+    for (int e = w; e < sx * sy * sz; e += nwarp()) {
+      int x, y, z;
+      split(e, sx, sy, x, y, z);
+      const unsigned c = block_at(x0 + x, y0 + y, z0 + z);
+      const unsigned h = __shfl_sync(0xffffffffu, ld_state(&F.head[c]), 0);
+      if (h & HEAD_BUSY) continue;
+      if (mark_if_ready_warp(F, c, h, chain)) add_new(c);
       __syncwarp();
     }
-    __syncthreads();
   }
 }
 
@@ -3978,18 +4013,19 @@ __device__ __forceinline__ void idle_wait(const Flow &F, unsigned *kind, unsigne
   const int lane = threadIdx.x & 31;
   unsigned polls = 0, seen = 0xffffffffu, k = IDLE_LEAVE, a = 0;
   while (true) {
-    const unsigned v = lane < 16 ? ld_state(&ts->qhead + lane) : 0u;
+    const unsigned v = lane < BOARD_END ? ld_state(&ts->qhead + lane) : 0u;
     const unsigned qh = __shfl_sync(0xffffffffu, v, 0), qt = __shfl_sync(0xffffffffu, v, 1),
                    leave = __shfl_sync(0xffffffffu, v, 2), fin = __shfl_sync(0xffffffffu, v, 3);
-    const unsigned hm = __ballot_sync(0xffffffffu, lane >= 8 && lane < 16 && v != 0u);
+    const unsigned m = __ballot_sync(0xffffffffu, lane >= BOARD_HELP && v != 0u) >> BOARD_HELP;
     if (leave) break;
     if ((int)(qt - qh) > 0) {
       unsigned got = NO_BLOCK;
       if (lane == 0 && atomicCAS(&ts->qhead, qh, qh + 1u) == qh) {
         // the entry is written right after the tail was moved
-        for (unsigned p = 0; p < LOOP_POLLS && got == NO_BLOCK; p++) got = ld_state(&F.ring[qh % F.nblk]);
+        unsigned *entry = &F.ring[qh % F.cap];
+        for (unsigned p = 0; p < LOOP_POLLS && got == NO_BLOCK; p++) got = ld_state(entry);
         if (got == NO_BLOCK) loop_timeout(ts);
-        else atomicExch(&F.ring[qh % F.nblk], RING_EMPTY);
+        else atomicExch(entry, RING_EMPTY);
       }
       got = __shfl_sync(0xffffffffu, got, 0);
       if (got != NO_BLOCK) {
@@ -3999,11 +4035,11 @@ __device__ __forceinline__ void idle_wait(const Flow &F, unsigned *kind, unsigne
       }
       continue;
     }
-    if (hm) {
-      const unsigned m = hm >> 8, r = blockIdx.x & 7u;  // CTAs start at different entries
+    if (m) {
+      const unsigned r = blockIdx.x & 7u;  // CTAs start at different entries
       const unsigned e = (unsigned)(__ffs((int)(m >> r | m << (8u - r))) - 1) + r;
       k = IDLE_HELP;
-      a = __shfl_sync(0xffffffffu, v, 8 + (int)(e & 7u)) - 1u;
+      a = __shfl_sync(0xffffffffu, v, BOARD_HELP + (int)(e & 7u)) - 1u;
       break;
     }
     if (fin != seen) {
@@ -4040,7 +4076,8 @@ __global__ void __launch_bounds__(LOOP_TPB, 1) k_seed_loop(const __grid_constant
   for (unsigned wi = gwarp; wi < cnt; wi += gwarps) {
     const unsigned b = active[wi];
     const unsigned h = __shfl_sync(0xffffffffu, ld_state(&F.head[b]), 0);
-    if (!(h & HEAD_BUSY)) queue_if_ready(F, b, h, 1u, &s_keep);
+    if (h & HEAD_BUSY) continue;
+    if (mark_if_ready_warp(F, b, h, 1u)) push_block(F, b);
     __syncwarp();
   }
   while (true) {
@@ -4088,9 +4125,9 @@ __global__ void __launch_bounds__(LOOP_TPB, 1) k_seed_loop(const __grid_constant
 }
 
 // one launch before the loop: its state, an empty ring, the live count
-__global__ void k_tail_init(TailState *ts, const unsigned *n_active, unsigned grid, unsigned *ring, unsigned nblk) {
+__global__ void k_tail_init(TailState *ts, const unsigned *n_active, unsigned grid, unsigned *ring, unsigned nring) {
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
-  for (unsigned k = i; k < nblk; k += gridDim.x * blockDim.x) ring[k] = RING_EMPTY;
+  for (unsigned k = i; k < nring; k += gridDim.x * blockDim.x) ring[k] = RING_EMPTY;
   if (i < LOOP_MAX_CTA) ts->refine[i].work = REFINE_CLOSED;
   if (i < LOOP_BIG) ts->help[i] = 0;
   if (i == 0) {
@@ -4825,7 +4862,8 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
       k_heads<<<nblk((long long)n_active, 256), 256, 0, c->stream>>>(act_a, n_active, bbegin, cursor, blist, resolved,
                                                                      head, nullptr, act_b, ctrs + 9);
       std::swap(act_a, act_b);
-      k_tail_init<<<64, 256, 0, c->stream>>>(tail, ctrs + 9, (unsigned)tail_grid, filt_b, (unsigned)nblocks);
+      const unsigned qcap = (unsigned)n_active;
+      k_tail_init<<<64, 256, 0, c->stream>>>(tail, ctrs + 9, (unsigned)tail_grid, filt_b, qcap);
       SodBufs Bt = B;
       Bt.max_cand = (unsigned)std::min<long long>(LOOP_CAND * c->tune.tail_max_cand, NB);
       // half of the candidate and crossing buffers in equal parts for the
@@ -4840,7 +4878,7 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
       Bt.st_big = nullptr;
       Bt.touch = u64s + 19;  // the tail's crossings counted apart from k_cross
       Bt.kept_members = u64s + 20;
-      Flow F{tail, bbegin, blist, cursor, head, filt_a, filt_b, (unsigned)nblocks, nb, rb, quirk_rank};
+      Flow F{tail, bbegin, blist, cursor, head, filt_a, filt_b, qcap, nb, rb, quirk_rank};
       void *args[] = {(void *)&K, (void *)&Bt, (void *)&F, (void *)&act_a, (void *)&ready};
       t_tail.start(c->stream);
       PSOD_CUDA(c, cudaLaunchCooperativeKernel((const void *)k_seed_loop, dim3(tail_grid), dim3(LOOP_TPB), args, smem,
