@@ -88,8 +88,9 @@ __global__ void k_slab_scan(const unsigned *hist, int nslab, unsigned *cursor) {
 // records (x, y, z, input index) grouped by slab; the order inside a slab
 // carries no meaning
 __global__ void __launch_bounds__(SLAB_THREADS) k_slab_scatter(const float *pos, long long n, float nxf, double xs,
-                                                               int nx, int nslab, unsigned *cursor, float4 *rec) {
-  __shared__ unsigned cnt[SLAB_MAX], start[SLAB_MAX], gbase[SLAB_MAX];
+                                                               int nx, int nslab, unsigned *cursor, float4 *rec,
+                                                               unsigned *at_of) {
+  __shared__ unsigned cnt[SLAB_MAX], start[SLAB_MAX], gbase[SLAB_MAX], wsum[SLAB_THREADS / 32];
   extern __shared__ __align__(16) unsigned char slab_smem[];
   float4 *stage = reinterpret_cast<float4 *>(slab_smem);                                // SLAB_TILE records
   unsigned short *sdig = reinterpret_cast<unsigned short *>(stage + SLAB_TILE);          // their slabs
@@ -107,16 +108,27 @@ __global__ void __launch_bounds__(SLAB_THREADS) k_slab_scatter(const float *pos,
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned run = 0;
-    for (int k = 0; k < nslab; k++) {
-      start[k] = run;
-      run += cnt[k];
+  // exclusive scan of the slab counts, two slabs a thread (one thread in turn
+  // over all of them: the pass took 298 us at 256^3, 276 now with inv written too)
+  static_assert(SLAB_MAX == 2 * SLAB_THREADS, "two slabs a thread");
+  {
+    const int k = 2 * threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const unsigned a = k < nslab ? cnt[k] : 0u, b = k + 1 < nslab ? cnt[k + 1] : 0u;
+    if (a) gbase[k] = atomicAdd(&cursor[k], a);
+    if (b) gbase[k + 1] = atomicAdd(&cursor[k + 1], b);
+    unsigned x = a + b;
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
     }
+    if (lane == 31) wsum[w] = x;
+    __syncthreads();
+    x -= a + b;
+    for (int q = 0; q < w; q++) x += wsum[q];
+    start[k] = x;
+    start[k + 1] = x + a;
   }
   __syncthreads();
-  for (int k = threadIdx.x; k < nslab; k += SLAB_THREADS)
-    if (cnt[k]) gbase[k] = atomicAdd(&cursor[k], cnt[k]);
 #pragma unroll
   for (int u = 0; u < SLAB_PER; u++) {
     const int j = u * SLAB_THREADS + threadIdx.x;
@@ -125,6 +137,7 @@ __global__ void __launch_bounds__(SLAB_THREADS) k_slab_scatter(const float *pos,
       const unsigned at = start[d[u]] + r[u];
       stage[at] = make_float4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], __uint_as_float((unsigned)i));
       sdig[at] = (unsigned short)d[u];
+      at_of[i] = gbase[d[u]] + r[u];
     }
   }
   __syncthreads();
@@ -135,21 +148,38 @@ __global__ void __launch_bounds__(SLAB_THREADS) k_slab_scatter(const float *pos,
   }
 }
 
-__global__ void k_cell_count(const float4 *rec, long long n, float nxf, double3 xs, int nx, unsigned *cell,
-                             unsigned *count) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  unsigned c = 0xffffffffu;
-  if (i < n) {
-    const float4 v = rec[i];
-    const int ci = sod_cell_axis(to_grid(v.x, nxf), xs.x, nx);
-    const int cj = sod_cell_axis(to_grid(v.y, nxf), xs.y, nx);
-    const int ck = sod_cell_axis(to_grid(v.z, nxf), xs.z, nx);
-    c = (unsigned)ci + (unsigned)nx * ((unsigned)cj + (unsigned)nx * (unsigned)ck);
-    cell[i] = c;
+// The count, the sub-cell count and the scatter below wait for chains of
+// dependent L2 reads and atomics at scattered addresses, so each thread
+// carries CELL_PER records, the loads of all before the use of any
+// (256^3, us a pass: count 215 -> 180, sub-cell count 147 -> 103, scatter
+// with its own writes alone 300 with one record a thread, 270 with four).
+constexpr int CELL_PER = 4;
+constexpr int CELL_TILE = 256 * CELL_PER;
+
+__global__ void __launch_bounds__(256) k_cell_count(const float4 *rec, long long n, float nxf, double3 xs, int nx,
+                                                    unsigned *cell, unsigned *count) {
+  const long long i0 = (long long)blockIdx.x * CELL_TILE + threadIdx.x;
+  float4 v[CELL_PER];
+#pragma unroll
+  for (int u = 0; u < CELL_PER; u++) {
+    const long long i = i0 + u * 256;
+    v[u] = i < n ? rec[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  // one atomic per distinct cell in the warp
-  const unsigned peers = __match_any_sync(0xffffffffu, c);
-  if (c != 0xffffffffu && __ffs(peers) - 1 == (int)(threadIdx.x & 31)) atomicAdd(&count[c], __popc(peers));
+#pragma unroll
+  for (int u = 0; u < CELL_PER; u++) {
+    const long long i = i0 + u * 256;
+    unsigned c = 0xffffffffu;
+    if (i < n) {
+      const int ci = sod_cell_axis(to_grid(v[u].x, nxf), xs.x, nx);
+      const int cj = sod_cell_axis(to_grid(v[u].y, nxf), xs.y, nx);
+      const int ck = sod_cell_axis(to_grid(v[u].z, nxf), xs.z, nx);
+      c = (unsigned)ci + (unsigned)nx * ((unsigned)cj + (unsigned)nx * (unsigned)ck);
+      cell[i] = c;
+    }
+    // one atomic per distinct cell in the warp
+    const unsigned peers = __match_any_sync(0xffffffffu, c);
+    if (c != 0xffffffffu && __ffs(peers) - 1 == (int)(threadIdx.x & 31)) atomicAdd(&count[c], __popc(peers));
+  }
 }
 
 // Cells holding at least SUB_MIN particles are ordered inside by a 4x4x4
@@ -197,12 +227,25 @@ __global__ void k_mark_big(unsigned *count, unsigned long long ncell, unsigned *
   }
 }
 
-__global__ void k_sub_count(const float4 *rec, long long n, const unsigned *cell, const unsigned *count, float nxf,
-                            double3 xs, unsigned *tab) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const unsigned v = count[cell[i]];
-  if (v & BIG_FLAG) atomicAdd(&tab[(unsigned long long)(v & ~BIG_FLAG) * SUB_N + sub_key(rec[i], nxf, xs)], 1u);
+__global__ void __launch_bounds__(256) k_sub_count(const float4 *rec, long long n, const unsigned *cell,
+                                                   const unsigned *count, float nxf, double3 xs, unsigned *tab) {
+  const long long i0 = (long long)blockIdx.x * CELL_TILE + threadIdx.x;
+  unsigned v[CELL_PER];
+  float4 r[CELL_PER];
+#pragma unroll
+  for (int u = 0; u < CELL_PER; u++) {
+    const long long i = i0 + u * 256;
+    v[u] = i < n ? cell[i] : 0xffffffffu;
+  }
+#pragma unroll
+  for (int u = 0; u < CELL_PER; u++) v[u] = i0 + u * 256 < n ? count[v[u]] : 0u;
+#pragma unroll
+  for (int u = 0; u < CELL_PER; u++)
+    if (v[u] & BIG_FLAG) r[u] = rec[i0 + u * 256];
+#pragma unroll
+  for (int u = 0; u < CELL_PER; u++)
+    if (v[u] & BIG_FLAG)
+      atomicAdd(&tab[(unsigned long long)(v[u] & ~BIG_FLAG) * SUB_N + sub_key(r[u], nxf, xs)], 1u);
 }
 
 // one warp per dense cell: sub-cell counts -> absolute start slots
@@ -222,27 +265,66 @@ __global__ void k_sub_scan(unsigned *tab, const unsigned *bigcell, unsigned nbig
   t[2 * lane + 1] = excl + a0;
 }
 
-__global__ void k_cell_scatter(const float4 *rec, long long n, const unsigned *cell, unsigned *fill, unsigned *tab,
-                               float nxf, double3 xs, float4 *cube, unsigned *inv) {
-  const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  const unsigned c = i < n ? cell[i] : 0xffffffffu;
-  const unsigned v = i < n ? fill[c] : 0u;  // the flag bit never changes under the atomics below
-  const bool big = (v & BIG_FLAG) != 0;
-  const float4 r = i < n ? rec[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const unsigned long long key =
-      i >= n ? ~0ull
-      : big  ? (1ull << 63) | ((unsigned long long)(v & ~BIG_FLAG) * SUB_N + sub_key(r, nxf, xs))
-             : (unsigned long long)c;
-  const unsigned peers = __match_any_sync(0xffffffffu, key);
-  const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
-  unsigned base = 0;
-  if (i < n && lane == leader)
-    base = big ? atomicAdd(&tab[key & ~(1ull << 63)], __popc(peers)) : atomicAdd(&fill[c], __popc(peers));
-  base = __shfl_sync(0xffffffffu, base, leader);
-  if (i >= n) return;
-  const unsigned slot = base + __popc(peers & ((1u << lane) - 1u));
-  cube[slot] = r;
-  inv[__float_as_uint(r.w)] = slot;
+__global__ void __launch_bounds__(256) k_cell_scatter(const float4 *rec, long long n, unsigned *cell,
+                                                      unsigned *fill, unsigned *tab, float nxf, double3 xs,
+                                                      float4 *cube) {
+  const long long i0 = (long long)blockIdx.x * CELL_TILE + threadIdx.x;
+  const int lane = threadIdx.x & 31;
+  unsigned c[CELL_PER], v[CELL_PER], base[CELL_PER], peers[CELL_PER];
+  float4 r[CELL_PER];
+#pragma unroll
+  for (int u = 0; u < CELL_PER; u++) {
+    const long long i = i0 + u * 256;
+    c[u] = i < n ? cell[i] : 0xffffffffu;
+    r[u] = i < n ? rec[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  // the flag bit never changes under the atomics below
+#pragma unroll
+  for (int u = 0; u < CELL_PER; u++) v[u] = i0 + u * 256 < n ? fill[c[u]] : 0u;
+#pragma unroll
+  for (int u = 0; u < CELL_PER; u++) {
+    const bool in = i0 + u * 256 < n, big = (v[u] & BIG_FLAG) != 0;
+    const unsigned sub = big ? sub_key(r[u], nxf, xs) : 0u;
+    // records of one cell, and of one sub-cell where the cell is dense
+    peers[u] = __match_any_sync(0xffffffffu, in ? c[u] : 0xffffffffu);
+    if (__any_sync(0xffffffffu, big)) peers[u] &= __match_any_sync(0xffffffffu, sub);
+    base[u] = 0;
+    if (in && lane == __ffs(peers[u]) - 1)
+      base[u] = big ? atomicAdd(&tab[(unsigned long long)(v[u] & ~BIG_FLAG) * SUB_N + sub], __popc(peers[u]))
+                    : atomicAdd(&fill[c[u]], __popc(peers[u]));
+  }
+#pragma unroll
+  for (int u = 0; u < CELL_PER; u++) {
+    const unsigned slot =
+        __shfl_sync(0xffffffffu, base[u], __ffs(peers[u]) - 1) + __popc(peers[u] & ((1u << lane) - 1u));
+    if (i0 + u * 256 < n) {
+      cube[slot] = r[u];
+      cell[i0 + u * 256] = slot;
+    }
+  }
+}
+
+// Slot of each input record: inv holds its place among the slab records
+// (written by the partition in input order), slot the cube slot of each of
+// those.  A tile's records lie in one short run per slab, so the sectors that
+// a CTA gathers from are read whole; writing inv from the scatter instead
+// takes a sector per record, spread over all of inv (256^3: scatter 565 us,
+// now 270 and 53 here; 512^3: 7.6 ms, now 2.7 and 1.0).
+__global__ void __launch_bounds__(SLAB_THREADS) k_slot_of_input(unsigned *inv, long long n, const unsigned *slot) {
+  const long long i0 = (long long)blockIdx.x * SLAB_TILE + threadIdx.x;
+  unsigned v[SLAB_PER];
+#pragma unroll
+  for (int u = 0; u < SLAB_PER; u++) {
+    const long long i = i0 + u * SLAB_THREADS;
+    v[u] = i < n ? inv[i] : 0u;
+  }
+#pragma unroll
+  for (int u = 0; u < SLAB_PER; u++) v[u] = slot[v[u]];
+#pragma unroll
+  for (int u = 0; u < SLAB_PER; u++) {
+    const long long i = i0 + u * SLAB_THREADS;
+    if (i < n) inv[i] = v[u];
+  }
 }
 
 // Dense sub-cells are then ordered by a finer Morton key inside the
@@ -955,8 +1037,8 @@ int stage_cellsort(psod_ctx *c, const float *dpos) {
   const int slab_smem = SLAB_TILE * (int)(sizeof(float4) + sizeof(unsigned short));
   PSOD_CUDA(c, cudaFuncSetAttribute(k_slab_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, slab_smem));
   k_slab_scatter<<<ntile, SLAB_THREADS, slab_smem, c->stream>>>(dpos, n, (float)nx, xs.z, nx, nslab, slabs + SLAB_MAX,
-                                                                rec);
-  k_cell_count<<<nblk(n, 256), 256, 0, c->stream>>>(rec, n, (float)nx, xs, nx, cell, count);
+                                                                rec, c->d_inv);
+  k_cell_count<<<nblk(n, CELL_TILE), 256, 0, c->stream>>>(rec, n, (float)nx, xs, nx, cell, count);
   if ((st = scan_u32(c, count, c->d_cell_start, (long long)c->ncell, true))) return st;
   unsigned *nbig = reinterpret_cast<unsigned *>(bad + 1);
   const long long ncell = (long long)c->ncell;
@@ -973,11 +1055,11 @@ int stage_cellsort(psod_ctx *c, const float *dpos) {
   if (!hbad) {
     PSOD_CUDA(c, cudaMemsetAsync(tab, 0, sizeof(unsigned) * (size_t)hnbig * SUB_N, c->stream));
     if (hnbig) {
-      k_sub_count<<<nblk(n, 256), 256, 0, c->stream>>>(rec, n, cell, count, (float)nx, xs, tab);
+      k_sub_count<<<nblk(n, CELL_TILE), 256, 0, c->stream>>>(rec, n, cell, count, (float)nx, xs, tab);
       k_sub_scan<<<nblk((long long)hnbig * 32, 256), 256, 0, c->stream>>>(tab, bigcell, hnbig, c->d_cell_start);
     }
-    k_cell_scatter<<<nblk(n, 256), 256, 0, c->stream>>>(rec, n, cell, count, tab, (float)nx, xs, c->d_cube,
-                                                        c->d_inv);
+    k_cell_scatter<<<nblk(n, CELL_TILE), 256, 0, c->stream>>>(rec, n, cell, count, tab, (float)nx, xs, c->d_cube);
+    k_slot_of_input<<<ntile, SLAB_THREADS, 0, c->stream>>>(c->d_inv, n, cell);
     // rec is free once the scatter has read it
     if (hnbig)
       k_sub_fine<<<hnbig, 256, 0, c->stream>>>(c->d_cube, c->d_inv, rec, tab, bigcell, c->d_cell_start, (float)nx, xs);
