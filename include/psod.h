@@ -152,8 +152,8 @@ typedef struct psod_run_stats {
   double ms_refine_bound; /* refinement bound pass (part of ms_refine) */
   int64_t refine_items;   /* refinement work items summed (64 candidates x one record chunk) */
   int64_t refine_pruned;  /* refinement candidates not summed: their bound is below the best lower bound */
-  double ms_tail;         /* device tail loop (late rounds run by one cooperative launch) */
-  int64_t tail_rounds;    /* rounds run by the device tail loop (part of rounds) */
+  double ms_tail;         /* device seed loop (the seeds after the host rounds, one cooperative launch) */
+  int64_t tail_rounds;    /* its longest chain of seeds, each made ready by the one before (part of rounds) */
   int64_t tail_touch;     /* part of cross_touch from the tail loop's crossings */
   int64_t cross_members;  /* members of kept halos written by the crossing kernels (k_cross, k_cross_warp) */
   int64_t tail_members;   /* members of kept halos written by the tail loop */
@@ -359,8 +359,10 @@ int psod_learn_gradient(psod_ctx *ctx, int64_t n, const float *x, const float *t
 typedef struct psod_tuning {
   int32_t warp_cross_min_ready; /* rounds with at least this many ready seeds cross small balls a warp per seed */
   int32_t bound_min_cand;       /* seeds with at least this many candidates get the refinement bound pass */
-  int32_t tail_max_ready;       /* the device tail loop takes rounds of at most this many ready seeds (0: never) */
-  int32_t tail_max_cand;        /* ... whose seeds have at most this many candidates (<= bound_min_cand) */
+  int32_t tail_max_ready;       /* the device seed loop starts after a round of at most 16 times this many ready
+                                   seeds (0: never) */
+  int32_t tail_max_cand;        /* ... and takes seeds of up to 4 times this many candidates, 4096 at most
+                                   (<= bound_min_cand) */
 } psod_tuning;
 
 int psod_get_tuning(psod_ctx *ctx, psod_tuning *t);

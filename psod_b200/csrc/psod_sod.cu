@@ -33,9 +33,9 @@ namespace psod {
 namespace {
 
 constexpr int TPB = 256;          // threads per seed CTA of the host rounds' kernels
-constexpr int LOOP_TPB = 512;     // threads per seed CTA of the device round loop
+constexpr int LOOP_TPB = 512;     // threads per seed CTA of the device seed loop
 constexpr unsigned RN_CHUNK = 2048;  // neighbour records per refinement work item
-constexpr unsigned LOOP_CHUNK = 512;  // in the device round loop: few seeds, all SMs for each
+constexpr unsigned LOOP_CHUNK = 512;  // in the device seed loop, which spreads a big seed over the idle CTAs
 constexpr unsigned LOOP_BIG = 8;      // seeds whose refinement the idle CTAs of the loop can share at one time
 constexpr int LOOP_MAX_CTA = 256;     // CTAs of the device seed loop at most
 constexpr int MAX_WARP = LOOP_TPB / 32;
@@ -2121,7 +2121,7 @@ __device__ __forceinline__ long long bucket_ball(const SodConst &K, const SodBuf
   return (long long)nball;
 }
 
-// Alive records of the cells around a seed, gathered by the device round loop
+// Alive records of the cells around a seed, gathered by the device seed loop
 // (small_seed): coordinates in one frame, cube slots, in the histograms' place
 struct SmallList {
   float x[NB], y[NB], z[NB];
@@ -4368,11 +4368,11 @@ enum {
 };
 static_assert((int)SC_BIGSEG < (int)SLOT_CELL_U32, "SOD scratch slots overlap the shared ones");
 
-// Rounds go to the device round loop once the last host round had no seed for
+// Rounds go to the device seed loop once the last host round had no seed for
 // the bound pass, none with more than LOOP_CAND x tail_max_cand candidates and
 // at most LOOP_READY x tail_max_ready ready seeds (psod_tuning), and few
-// enough active blocks for the direct readiness test inside the loop
-// (LOOP_TESTS heads read a round).  A launch that ended on a larger seed within
+// enough active blocks for the loop's first readiness tests (LOOP_TESTS heads
+// read).  A launch that ended on a larger seed within
 // LOOP_SHORT rounds is followed by LOOP_REST host rounds before the next.
 constexpr long long LOOP_READY = 16, LOOP_CAND = 4, LOOP_TESTS = 1ll << 27;
 constexpr int LOOP_SHORT = 4, LOOP_REST = 8;
@@ -4711,7 +4711,7 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
   const long long window = (long long)std::min(2 * rb + 1, nb);
   const long long direct_cost_per_block = window * window * window, filter_cost = 3 * nblocks * window;
   bool pending = false, pend_learn = false, pend_bound = false;
-  // device tail loop: one CTA per seed slot resident on every SM
+  // device seed loop: one CTA per seed slot resident on every SM
   int tail_grid = 0, rest = 0, rest_need = 1;
   long long tail_rounds = 0;
   TailState *tail = nullptr;
