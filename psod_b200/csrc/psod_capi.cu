@@ -298,7 +298,8 @@ int psod_load_particles(psod_ctx *c, int64_t n, const float *pos, const float *v
     if ((st = copy_in(c, c->d_ids, id, sizeof(int64_t) * n))) return st;
     if (vel && (st = copy_in(c, c->d_vel, vel, sizeof(float) * 3 * n))) return st;
   }
-  return stage_cellsort(c, dpos);
+  if ((st = stage_cellsort(c, dpos))) c->n = 0;  // nothing is loaded
+  return st;
 }
 
 int psod_cic(psod_ctx *c, double *grid_out) {

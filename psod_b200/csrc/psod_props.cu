@@ -612,6 +612,7 @@ int psod_halo_properties(psod_ctx *c, const psod_props_params *p, psod_props_sta
   if (!c || !p) return PSOD_ERR_ARG;
   cudaSetDevice(c->device);
   c->props_done = false;
+  if (c->n <= 0) return set_err(c, PSOD_ERR_STATE, "no particles: call psod_load_particles first");
   const long long *off = nullptr;
   const unsigned *mem = nullptr;
   long long nh = 0;

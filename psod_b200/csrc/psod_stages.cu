@@ -43,8 +43,10 @@ __device__ __forceinline__ bool in_unit_box(float x, float y, float z) {
   return x >= 0.f && x <= 1.f && y >= 0.f && y <= 1.f && z >= 0.f && z <= 1.f;
 }
 
-// slab of a position: its z cell scaled to the slab count (slabs are runs of
-// whole z-planes, so runs of cell indices)
+// slab of a position in the unit box: its z cell scaled to the slab count
+// (slabs are runs of whole z-planes, so runs of cell indices).  A position
+// outside the box has no cell (sod_cell_axis wraps once): k_slab_count sets
+// *bad for one, and no pass computes a slab or a cell once it is set.
 __device__ __forceinline__ unsigned slab_of(float z, float nxf, double xs, int nx, int nslab) {
   const int k = sod_cell_axis(to_grid(z, nxf), xs, nx);
   return (unsigned)(((long long)k * nslab) / nx);
@@ -61,7 +63,10 @@ __global__ void __launch_bounds__(SLAB_THREADS) k_slab_count(const float *pos, l
     const long long i = base + (long long)u * SLAB_THREADS + threadIdx.x;
     if (i >= n) break;
     const float x = pos[3 * i], y = pos[3 * i + 1], z = pos[3 * i + 2];
-    if (!in_unit_box(x, y, z)) badl = 1;
+    if (!in_unit_box(x, y, z)) {
+      badl = 1;
+      continue;
+    }
     atomicAdd(&h[slab_of(z, nxf, xs, nx, nslab)], 1u);
   }
   if (badl) atomicOr(bad, 1);
@@ -88,8 +93,9 @@ __global__ void k_slab_scan(const unsigned *hist, int nslab, unsigned *cursor) {
 // records (x, y, z, input index) grouped by slab; the order inside a slab
 // carries no meaning
 __global__ void __launch_bounds__(SLAB_THREADS) k_slab_scatter(const float *pos, long long n, float nxf, double xs,
-                                                               int nx, int nslab, unsigned *cursor, float4 *rec,
-                                                               unsigned *at_of) {
+                                                               int nx, int nslab, const int *bad, unsigned *cursor,
+                                                               float4 *rec, unsigned *at_of) {
+  if (*bad) return;
   __shared__ unsigned cnt[SLAB_MAX], start[SLAB_MAX], gbase[SLAB_MAX], wsum[SLAB_THREADS / 32];
   extern __shared__ __align__(16) unsigned char slab_smem[];
   float4 *stage = reinterpret_cast<float4 *>(slab_smem);                                // SLAB_TILE records
@@ -157,7 +163,8 @@ constexpr int CELL_PER = 4;
 constexpr int CELL_TILE = 256 * CELL_PER;
 
 __global__ void __launch_bounds__(256) k_cell_count(const float4 *rec, long long n, float nxf, double3 xs, int nx,
-                                                    unsigned *cell, unsigned *count) {
+                                                    const int *bad, unsigned *cell, unsigned *count) {
+  if (*bad) return;
   const long long i0 = (long long)blockIdx.x * CELL_TILE + threadIdx.x;
   float4 v[CELL_PER];
 #pragma unroll
@@ -1036,9 +1043,9 @@ int stage_cellsort(psod_ctx *c, const float *dpos) {
   k_slab_scan<<<1, 32, 0, c->stream>>>(slabs, nslab, slabs + SLAB_MAX);
   const int slab_smem = SLAB_TILE * (int)(sizeof(float4) + sizeof(unsigned short));
   PSOD_CUDA(c, cudaFuncSetAttribute(k_slab_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, slab_smem));
-  k_slab_scatter<<<ntile, SLAB_THREADS, slab_smem, c->stream>>>(dpos, n, (float)nx, xs.z, nx, nslab, slabs + SLAB_MAX,
-                                                                rec, c->d_inv);
-  k_cell_count<<<nblk(n, CELL_TILE), 256, 0, c->stream>>>(rec, n, (float)nx, xs, nx, cell, count);
+  k_slab_scatter<<<ntile, SLAB_THREADS, slab_smem, c->stream>>>(dpos, n, (float)nx, xs.z, nx, nslab, bad,
+                                                                slabs + SLAB_MAX, rec, c->d_inv);
+  k_cell_count<<<nblk(n, CELL_TILE), 256, 0, c->stream>>>(rec, n, (float)nx, xs, nx, bad, cell, count);
   if ((st = scan_u32(c, count, c->d_cell_start, (long long)c->ncell, true))) return st;
   unsigned *nbig = reinterpret_cast<unsigned *>(bad + 1);
   const long long ncell = (long long)c->ncell;
