@@ -12,7 +12,7 @@ OUT_DIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(OUT_DIR, "libpsod.so")
 SOURCES = ["psod_capi.cu", "psod_stages.cu", "psod_sod.cu", "psod_sort.cu", "psod_static.cu", "psod_learn.cu",
            "psod_output.cu", "psod_input.cu", "psod_fof.cu", "psod_props.cu"]
-HEADERS = ["psod_internal.cuh"]
+HEADERS = ["psod_internal.cuh", "psod_loop.cuh"]
 # the halo-properties arithmetic follows the reference statement by
 # statement: no multiply-add contraction in that file
 FILE_FLAGS = {"psod_props.cu": ["--fmad=false"]}

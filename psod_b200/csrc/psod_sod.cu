@@ -27,6 +27,7 @@
 #include <cstdlib>
 
 #include "psod_internal.cuh"
+#include "psod_loop.cuh"
 
 namespace psod {
 
@@ -3653,12 +3654,13 @@ enum : unsigned { TAIL_RUNNING = 0, TAIL_DONE = 1, TAIL_DEFERRED = 2, TAIL_TIMEO
 constexpr unsigned HEAD_BUSY = 0x80000000u, RING_EMPTY = 0xffffffffu, NO_BLOCK = 0xffffffffu;
 static_assert((PSOD_INF_RANK & HEAD_BUSY) != 0u && PSOD_IDX_MASK < HEAD_BUSY, "ranks below the busy bit");
 
-// a seed's refinement items: exclusive prefix over its 27 candidate cells
+// a seed's refinement: its items to draw (refine_open), the finished ones, and
+// the exclusive prefix of the items over the 27 candidate cells
 struct SharedRefine {
-  unsigned nitem, work, done, pad;
+  unsigned long long work;
+  unsigned done, pad;
   unsigned pref[28];
 };
-constexpr unsigned REFINE_CLOSED = 1u << 30;  // no item left to take
 
 struct TailState {
   // the words an idle CTA polls (one 64-byte read): queue head and tail,
@@ -3915,19 +3917,22 @@ __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Sm
 }
 
 // Warps of any CTA take refinement items of the seed in `slot` until none is
-// left.  The item's data are read after it was taken, and the owner closes the
-// counter before it writes another seed's, so that a late warp takes nothing.
+// left.  One draw returns the item and the count it is measured by (refine_take),
+// so a warp that is late by any time takes nothing or a whole item of the seed
+// now published; the owner waits for every item that was accepted before it
+// writes another seed's data, which are read after the draw.
 __device__ __noinline__ void share_refine(const SodConst &K, const SodBufs &B, Smem &S, TailState *ts, unsigned slot) {
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   static_assert(sizeof(WarpRef) * MAX_WARP <= sizeof(unsigned) * MAXLEV * NB, "staging over the histograms");
   WarpRef &R = reinterpret_cast<WarpRef *>(S.hist)[w];
   SharedRefine &H = ts->refine[slot];
   while (true) {
-    unsigned it = 0;
-    if (lane == 0) it = atomicAdd(&H.work, 1u);
-    it = __shfl_sync(0xffffffffu, it, 0);
+    unsigned long long drawn = 0;
+    if (lane == 0) drawn = atomicAdd(&H.work, 1ull);
+    drawn = __shfl_sync(0xffffffffu, drawn, 0);
+    unsigned it;
+    if (!refine_take(drawn, it)) break;
     __threadfence();
-    if (it >= __shfl_sync(0xffffffffu, ld_state(&H.nitem), 0)) break;
     const unsigned p = lane < 27 ? ld_state(&H.pref[lane]) : ~0u;
     const unsigned le = __ballot_sync(0xffffffffu, p <= it);  // lane 0's prefix is 0
     const int cell = 31 - __clz((int)le);
@@ -3951,19 +3956,20 @@ __device__ __noinline__ void big_seed(const SodConst &K, const SodBufs &B, Smem 
   __syncthreads();
   if (!ld_state(&B.st_active[slot])) return;
   SharedRefine &H = ts->refine[slot];
+  unsigned nitem = 0;
   if (t < 32) {
     unsigned v = t < 27 ? B.cell_chunks[slot * 27u + (unsigned)t] : 0u, inc = v;
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned y = __shfl_up_sync(0xffffffffu, inc, o);
       if (t >= o) inc += y;
     }
+    nitem = __shfl_sync(0xffffffffu, inc, 31);
     if (t < 28) *(volatile unsigned *)&H.pref[t] = inc - v;
-    if (t == 31) *(volatile unsigned *)&H.nitem = inc;
     if (t == 0) *(volatile unsigned *)&H.done = 0u;
     __threadfence();
     __syncwarp();
     if (t == 0) {
-      atomicExch(&H.work, 0u);
+      atomicExch(&H.work, refine_open(nitem));
       __threadfence();
       for (unsigned k = 0; k < LOOP_BIG; k++)
         if (atomicCAS(&ts->help[(slot + k) % LOOP_BIG], 0u, slot + 1u) == 0u) break;
@@ -3973,10 +3979,9 @@ __device__ __noinline__ void big_seed(const SodConst &K, const SodBufs &B, Smem 
   share_refine(K, B, S, ts, slot);
   __syncthreads();
   if (t == 0) {
-    const unsigned n = ld_state(&H.nitem);
     unsigned polls = 0;
     s_ok = 1;
-    while (ld_state(&H.done) != n) {
+    while (ld_state(&H.done) < nitem) {
       if (++polls > LOOP_POLLS || ld_state(&ts->status) == TAIL_TIMEOUT) {
         loop_timeout(ts);
         s_ok = 0;
@@ -3984,7 +3989,7 @@ __device__ __noinline__ void big_seed(const SodConst &K, const SodBufs &B, Smem 
       }
       __nanosleep(32);
     }
-    atomicExch(&H.work, REFINE_CLOSED);
+    atomicExch(&H.work, refine_open(0u));
     __threadfence();
   }
   __syncthreads();
@@ -4128,7 +4133,7 @@ __global__ void __launch_bounds__(LOOP_TPB, 1) k_seed_loop(const __grid_constant
 __global__ void k_tail_init(TailState *ts, const unsigned *n_active, unsigned grid, unsigned *ring, unsigned nring) {
   const unsigned i = blockIdx.x * blockDim.x + threadIdx.x;
   for (unsigned k = i; k < nring; k += gridDim.x * blockDim.x) ring[k] = RING_EMPTY;
-  if (i < LOOP_MAX_CTA) ts->refine[i].work = REFINE_CLOSED;
+  if (i < LOOP_MAX_CTA) ts->refine[i].work = refine_open(0u);
   if (i < LOOP_BIG) ts->help[i] = 0;
   if (i == 0) {
     ts->qhead = ts->qtail = ts->leave = ts->finished = 0;

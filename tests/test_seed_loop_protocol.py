@@ -1,0 +1,101 @@
+"""The words that the CTAs of the device seed loop exchange
+(psod_b200/csrc/psod_loop.cuh), compiled for the host and walked through every
+interleaving of small cases."""
+
+import ctypes as C
+import os
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "psod_b200", "csrc")
+
+SHIM = r"""
+#include "psod_loop.cuh"
+extern "C" {
+unsigned long long open_word(unsigned n) { return psod::refine_open(n); }
+int take(unsigned long long drawn, unsigned *item) { return psod::refine_take(drawn, *item); }
+}
+"""
+
+
+@pytest.fixture(scope="module")
+def loop(tmp_path_factory):
+    d = tmp_path_factory.mktemp("loop")
+    (d / "shim.cpp").write_text(SHIM)
+    subprocess.run(["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-I", CSRC, str(d / "shim.cpp"), "-o",
+                    str(d / "shim.so")], check=True)
+    lib = C.CDLL(str(d / "shim.so"))
+    lib.open_word.restype = C.c_ulonglong
+    lib.take.argtypes = [C.c_ulonglong, C.POINTER(C.c_uint)]
+    return lib
+
+
+def refine_runs(open_word, take, two_step, items=(1, 2), helpers=2, draws=3):
+    """Every interleaving of an owner that publishes seeds of `items` items in
+    one slot (publish, take items itself, wait for all, close) with helper warps
+    of `draws` draws each.  A step is one access to shared memory.  Yields the
+    multiset of (seed whose data were read, item) of each complete run, or None
+    for one in which the owner went on with items unfinished."""
+    # shared: word, count (read apart in the two-step form), done, seed published
+    # owner: (seed, phase, drawn); helper: (draws left, drawn or None)
+    start = ((0, 0, 0, -1), ("publish", 0, None), ((draws, None),) * helpers, ())
+    stack, seen = [start], set()
+    while stack:
+        state = stack.pop()
+        if state in seen:
+            continue
+        seen.add(state)
+        (word, count, done, seed), owner, help_, ran = state
+        phase, k, drawn = owner
+        if phase == "end" and all(h == (0, None) for h in help_):
+            yield ran
+            continue
+        # the owner's next step
+        if phase == "publish":
+            stack.append(((open_word(items[k]), items[k], 0, k), ("draw", k, None), help_, ran))
+        elif phase == "draw":
+            stack.append(((word + 1, count, done, seed), ("check", k, word), help_, ran))
+        elif phase == "check":
+            item = take(drawn, count)
+            if item is None:
+                stack.append(((word, count, done, seed), ("wait", k, None), help_, ran))
+            else:
+                stack.append(((word, count, done + 1, seed), ("draw", k, None), help_,
+                              tuple(sorted(ran + ((seed, item),)))))
+        elif phase == "wait" and done >= items[k]:
+            if sum(1 for s, _ in ran if s == k) != items[k] or len(set(ran)) != len(ran):
+                yield None
+                continue
+            nxt = ("publish", k + 1, None) if k + 1 < len(items) else ("end", k, None)
+            stack.append(((open_word(0), 0 if not two_step else count, done, seed), nxt, help_, ran))
+        # a helper's next step
+        for i, (left, d) in enumerate(help_):
+            if d is None and left:
+                h = help_[:i] + ((left, word),) + help_[i + 1 :]
+                stack.append(((word + 1, count, done, seed), owner, h, ran))
+            elif d is not None:
+                item = take(d, count)
+                if item is None:  # it leaves
+                    h = help_[:i] + ((0, None),) + help_[i + 1 :]
+                    stack.append(((word, count, done, seed), owner, h, ran))
+                else:
+                    h = help_[:i] + ((left - 1, None),) + help_[i + 1 :]
+                    stack.append(((word, count, done + 1, seed), owner, h, tuple(sorted(ran + ((seed, item),)))))
+
+
+def test_every_item_runs_once_for_its_own_seed(loop):
+    def take(drawn, _count):
+        item = C.c_uint()
+        return item.value if loop.take(drawn, C.byref(item)) else None
+
+    runs = list(refine_runs(loop.open_word, take, False))
+    assert runs and set(runs) == {((0, 0), (1, 0), (1, 1))}
+
+
+def test_the_walk_sees_a_late_ticket():
+    """The item and its bound read in two steps: a warp that drew past the end
+    of one seed accepts the number as an item of the next."""
+    closed = 1 << 30
+    runs = list(refine_runs(lambda n: 0 if n else closed, lambda d, count: d if d < count else None, True))
+    assert None in runs or any(r != ((0, 0), (1, 0), (1, 1)) for r in runs)
