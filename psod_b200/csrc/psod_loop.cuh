@@ -25,4 +25,26 @@ PSOD_LOOP_FN bool refine_take(unsigned long long drawn, unsigned &item) {
   return item < (unsigned)(drawn >> 32);
 }
 
+// The queue of ready blocks is a ring of as many places as blocks were active
+// at the launch, which may be a handful, so that places are reused while
+// consumers of the lap before are still at them.  A value is put into an empty
+// place and taken out by an exchange: whichever consumer of a place exchanges
+// first has the value, no other one sees it, and each of them gets one, as many
+// values being put into a place as consumers were sent to it.  (Read first and
+// emptied afterwards, a value could be seen by the consumer a lap later too.)
+// Mem: load, exchange and compare-and-swap of a word shared by the CTAs.
+constexpr unsigned RING_EMPTY = 0xffffffffu;
+
+template <class Mem>
+PSOD_LOOP_FN bool ring_put(Mem &m, unsigned *place, unsigned block) {
+  return m.cas(place, RING_EMPTY, block) == RING_EMPTY;
+}
+
+template <class Mem>
+PSOD_LOOP_FN bool ring_take(Mem &m, unsigned *place, unsigned &block) {
+  if (m.load(place) == RING_EMPTY) return false;
+  block = m.exchange(place, RING_EMPTY);
+  return block != RING_EMPTY;
+}
+
 }  // namespace psod

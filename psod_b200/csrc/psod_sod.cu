@@ -3651,7 +3651,7 @@ __device__ __forceinline__ int small_seed(const SodConst &K, const SodBufs &B, S
 // slowest seed (grid-wide): loop of 512^3 90 -> 74 ms, heavy 256^3 65 -> 39.
 // ---------------------------------------------------------------------------
 enum : unsigned { TAIL_RUNNING = 0, TAIL_DONE = 1, TAIL_DEFERRED = 2, TAIL_TIMEOUT = 3 };
-constexpr unsigned HEAD_BUSY = 0x80000000u, RING_EMPTY = 0xffffffffu, NO_BLOCK = 0xffffffffu;
+constexpr unsigned HEAD_BUSY = 0x80000000u, NO_BLOCK = RING_EMPTY;
 static_assert((PSOD_INF_RANK & HEAD_BUSY) != 0u && PSOD_IDX_MASK < HEAD_BUSY, "ranks below the busy bit");
 
 // a seed's refinement: its items to draw (refine_open), the finished ones, and
@@ -3682,6 +3682,12 @@ static_assert(offsetof(TailState, help) == 4 * BOARD_HELP && LOOP_BIG == 8, "pol
 constexpr unsigned LOOP_POLLS = 1u << 24;  // a few seconds without a finished seed
 
 __device__ __forceinline__ unsigned ld_state(const unsigned *p) { return *(volatile const unsigned *)p; }
+
+struct LoopMem {  // of psod_loop.cuh
+  __device__ __forceinline__ unsigned load(const unsigned *p) { return ld_state(p); }
+  __device__ __forceinline__ unsigned exchange(unsigned *p, unsigned v) { return atomicExch(p, v); }
+  __device__ __forceinline__ unsigned cas(unsigned *p, unsigned was, unsigned v) { return atomicCAS(p, was, v); }
+};
 
 __device__ __forceinline__ void loop_timeout(TailState *ts) {
   atomicExch(&ts->status, TAIL_TIMEOUT);
@@ -3758,8 +3764,9 @@ __device__ __forceinline__ void push_block(const Flow &F, unsigned c) {
   atomicAdd(&ts->inflight, 1u);
   __threadfence();
   const unsigned at = atomicAdd(&ts->qtail, 1u) % F.cap;
-  for (unsigned p = 0; p < LOOP_POLLS; p++)  // the entry a lap before is being emptied at most
-    if (atomicCAS(&F.ring[at], RING_EMPTY, c) == RING_EMPTY) return;
+  LoopMem mem;
+  for (unsigned p = 0; p < LOOP_POLLS; p++)  // the value a lap before is being taken at most
+    if (ring_put(mem, &F.ring[at], c)) return;
   loop_timeout(ts);
 }
 
@@ -4026,11 +4033,12 @@ __device__ __forceinline__ void idle_wait(const Flow &F, unsigned *kind, unsigne
     if ((int)(qt - qh) > 0) {
       unsigned got = NO_BLOCK;
       if (lane == 0 && atomicCAS(&ts->qhead, qh, qh + 1u) == qh) {
-        // the entry is written right after the tail was moved
-        unsigned *entry = &F.ring[qh % F.cap];
-        for (unsigned p = 0; p < LOOP_POLLS && got == NO_BLOCK; p++) got = ld_state(entry);
+        // the value is put right after the tail was moved
+        LoopMem mem;
+        unsigned p = 0;
+        while (!ring_take(mem, &F.ring[qh % F.cap], got) && ++p < LOOP_POLLS) {
+        }
         if (got == NO_BLOCK) loop_timeout(ts);
-        else atomicExch(entry, RING_EMPTY);
       }
       got = __shfl_sync(0xffffffffu, got, 0);
       if (got != NO_BLOCK) {

@@ -12,7 +12,17 @@ CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))),
 
 SHIM = r"""
 #include "psod_loop.cuh"
+typedef void (*hook_fn)();
+struct HookMem {  // what other CTAs do between two accesses
+  hook_fn hook;
+  void between() { if (hook) { hook_fn h = hook; hook = nullptr; h(); } }
+  unsigned load(const unsigned *p) { const unsigned v = *p; between(); return v; }
+  unsigned exchange(unsigned *p, unsigned v) { const unsigned old = *p; *p = v; return old; }
+  unsigned cas(unsigned *p, unsigned was, unsigned v) { const unsigned old = *p; if (old == was) *p = v; return old; }
+};
 extern "C" {
+int ring_take(unsigned *place, unsigned *block, hook_fn hook) { HookMem m{hook}; return psod::ring_take(m, place, *block); }
+int ring_put(unsigned *place, unsigned block) { HookMem m{nullptr}; return psod::ring_put(m, place, block); }
 unsigned long long open_word(unsigned n) { return psod::refine_open(n); }
 int take(unsigned long long drawn, unsigned *item) { return psod::refine_take(drawn, *item); }
 }
@@ -99,3 +109,36 @@ def test_the_walk_sees_a_late_ticket():
     closed = 1 << 30
     runs = list(refine_runs(lambda n: 0 if n else closed, lambda d, count: d if d < count else None, True))
     assert None in runs or any(r != ((0, 0), (1, 0), (1, 1)) for r in runs)
+
+
+HOOK = C.CFUNCTYPE(None)
+EMPTY = 0xFFFFFFFF
+
+
+def test_a_ring_value_is_taken_once(loop):
+    """Consumers of three laps at one place, each with what the others can do
+    between its look at the place and its exchange."""
+    place = C.c_uint(EMPTY)
+    taken = []
+
+    def put(v):
+        return loop.ring_put(C.byref(place), C.c_uint(v))
+
+    def take(hook=None):
+        got = C.c_uint(EMPTY)
+        ok = loop.ring_take(C.byref(place), C.byref(got), HOOK(hook) if hook else C.cast(None, HOOK))
+        if ok:
+            taken.append(got.value)
+        return ok
+
+    assert not take()  # nothing was put yet
+    assert put(7) and not put(8)  # the place is full until 7 is taken
+    # the consumer a lap later takes 7 after this one saw it: this one waits
+    assert not take(lambda: take())
+    assert taken == [7]
+    # ... and gets the value put for the other
+    assert put(8) and take()
+    # between look and exchange the other takes the value and the next is put:
+    # the exchange has the new value, each value went out once
+    assert put(9) and take(lambda: (take(), put(10)))
+    assert taken == [7, 8, 9, 10] and place.value == EMPTY
