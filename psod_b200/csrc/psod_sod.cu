@@ -3635,7 +3635,10 @@ __device__ __forceinline__ int small_seed(const SodConst &K, const SodBufs &B, S
 // Heads only grow, and two seeds in flight are never in each other's window,
 // so the order is the rounds' order: every seed after all lower ones of its
 // window.  Of two CTAs that move heads of one window at the same time at
-// least one sees both (a fence between the moves and the tests).  The
+// least one sees both (a fence between the moves and the tests).  A CTA that
+// finds a block ready from the heads that others moved reads their claims only
+// after a fence of every thread that read a head: the block that it keeps
+// starts without passing through the queue and its fences.  The
 // particle filed under a foreign cell waits until nothing is queued or in
 // flight: then every head left is above it.
 //
@@ -3753,6 +3756,8 @@ __device__ __forceinline__ bool mark_if_ready_warp(const Flow &F, unsigned c, un
     }
     if (__any_sync(0xffffffffu, lower)) return false;
   }
+  __threadfence();  // the claims of the CTAs that moved these heads
+  __syncwarp();
   return lane == 0 && mark_ready(F, c, h, chain);
 }
 
@@ -3880,6 +3885,7 @@ __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Sm
         split(e, Lx, Ly, x, y, z);
         raw[e] = ld_state(&F.head[block_at(x0 - rb + x, y0 - rb + y, z0 - rb + zs + z)]);
       }
+      __threadfence();  // the claims of the CTAs that moved these heads
       __syncthreads();
       for (int e = t; e < Cx * Ly * Lz; e += tpb()) {
         split(e, Cx, Ly, x, y, z);

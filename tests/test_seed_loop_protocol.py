@@ -4,6 +4,7 @@ interleaving of small cases."""
 
 import ctypes as C
 import os
+import re
 import subprocess
 
 import pytest
@@ -142,3 +143,18 @@ def test_a_ring_value_is_taken_once(loop):
     # the exchange has the new value, each value went out once
     assert put(9) and take(lambda: (take(), put(10)))
     assert taken == [7, 8, 9, 10] and place.value == EMPTY
+
+
+def test_heads_are_acquired_before_a_block_is_marked():
+    """A block found ready from heads that other CTAs moved is kept by its
+    finder: between the reads of the heads and the mark stands a fence of the
+    threads that read them (no test on one GPU can show a stale line, so this
+    reads the source)."""
+    src = open(os.path.join(CSRC, "psod_sod.cu")).read()
+    for fn, read, mark in (("bool mark_if_ready_warp(", "ld_state(&F.head[", "mark_ready("),
+                           ("void finish_block(", "raw[e] = ld_state(&F.head[", "mark_ready(")):
+        body = src[src.index(fn) :]
+        body = body[: re.search(r"^}", body, re.M).end()]
+        i = body.index(read)
+        j = body.index(mark, i)
+        assert "__threadfence()" in body[i:j], fn
