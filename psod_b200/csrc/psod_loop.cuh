@@ -47,4 +47,22 @@ PSOD_LOOP_FN bool ring_take(Mem &m, unsigned *place, unsigned &block) {
   return block != RING_EMPTY;
 }
 
+// Place e of a box of sx by sy by any planes, total places in all, as (x, y, z).
+// Below 2^22 places the quotient through FP32 is exact: e + 1/2 is, the rounded
+// reciprocal and product are off by less than e / s * 2^-23 < 1 / (2 s), and the
+// quotient lies at least that far from a whole number.  Larger boxes divide
+// (blocks of one cell and ncut from 21: windows up to (4 ncut + 1)^3 places).
+PSOD_LOOP_FN void box_split(int e, int sx, int sy, int total, int &x, int &y, int &z) {
+  int q;
+  if (total <= (1 << 22)) {
+    q = (int)(((float)e + 0.5f) * (1.0f / (float)sx));
+    z = (int)(((float)q + 0.5f) * (1.0f / (float)sy));
+  } else {
+    q = e / sx;
+    z = q / sy;
+  }
+  x = e - q * sx;
+  y = q - z * sy;
+}
+
 }  // namespace psod

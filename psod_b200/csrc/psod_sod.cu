@@ -3811,7 +3811,7 @@ __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Sm
   const int nb = F.nb, rb = F.rb;
   const int bx = (int)(b % (unsigned)nb), by = (int)((b / (unsigned)nb) % (unsigned)nb),
             bz = (int)(b / ((unsigned)nb * nb));
-  // the block (dx, dy, dz) from b, and place e of a box as its offsets
+  // the block (dx, dy, dz) from b
   auto wrap = [&](int v) {
     while (v < 0) v += nb;
     while (v >= nb) v -= nb;
@@ -3819,12 +3819,6 @@ __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Sm
   };
   auto block_at = [&](int dx, int dy, int dz) {
     return wrap(bx + dx) + (unsigned)nb * (wrap(by + dy) + (unsigned)nb * wrap(bz + dz));
-  };
-  auto split = [](int e, int sx, int sy, int &x, int &y, int &z) {  // e < 2^22: exact
-    const int q = (int)(((float)e + 0.5f) * (1.0f / (float)sx));
-    z = (int)(((float)q + 0.5f) * (1.0f / (float)sy));
-    x = e - q * sx;
-    y = q - z * sy;
   };
   __threadfence();  // the claims, before anything that follows from them
   __syncthreads();
@@ -3835,7 +3829,7 @@ __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Sm
   const int side1 = min(2 * rb + 1, nb), n1 = side1 * side1 * side1;
   for (int e = t; e < n1; e += tpb()) {
     int d[3];
-    split(e, side1, side1, d[0], d[1], d[2]);
+    box_split(e, side1, side1, n1, d[0], d[1], d[2]);
     for (int k = 0; k < 3; k++) d[k] -= side1 / 2;
     const unsigned x = block_at(d[0], d[1], d[2]);
     const unsigned h = ld_state(&F.head[x]), end = F.bbegin[x + 1];
@@ -3882,13 +3876,13 @@ __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Sm
       unsigned *raw = S.hist[0], *mx = raw + Lx * Ly * Lz, *my = mx + Cx * Ly * Lz;
       int x, y, z;
       for (int e = t; e < Lx * Ly * Lz; e += tpb()) {
-        split(e, Lx, Ly, x, y, z);
+        box_split(e, Lx, Ly, Lx * Ly * Lz, x, y, z);
         raw[e] = ld_state(&F.head[block_at(x0 - rb + x, y0 - rb + y, z0 - rb + zs + z)]);
       }
       __threadfence();  // the claims of the CTAs that moved these heads
       __syncthreads();
       for (int e = t; e < Cx * Ly * Lz; e += tpb()) {
-        split(e, Cx, Ly, x, y, z);
+        box_split(e, Cx, Ly, Cx * Ly * Lz, x, y, z);
         const unsigned *p = raw + x + Lx * (y + Ly * z);
         unsigned m = ~0u;
         for (int d = 0; d <= 2 * rb; d++) m = min(m, p[d] & ~HEAD_BUSY);
@@ -3896,7 +3890,7 @@ __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Sm
       }
       __syncthreads();
       for (int e = t; e < Cx * Cy * Lz; e += tpb()) {
-        split(e, Cx, Cy, x, y, z);
+        box_split(e, Cx, Cy, Cx * Cy * Lz, x, y, z);
         const unsigned *p = mx + x + Cx * (y + Ly * z);
         unsigned m = ~0u;
         for (int d = 0; d <= 2 * rb; d++) m = min(m, p[d * Cx]);
@@ -3904,7 +3898,7 @@ __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Sm
       }
       __syncthreads();
       for (int e = t; e < Cx * Cy * T; e += tpb()) {
-        split(e, Cx, Cy, x, y, z);
+        box_split(e, Cx, Cy, Cx * Cy * T, x, y, z);
         const unsigned h = raw[x + rb + Lx * (y + rb + Ly * (z + rb))];
         if (h & HEAD_BUSY) continue;
         unsigned m = ~0u;
@@ -3919,7 +3913,7 @@ __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Sm
     const int sx = min(Cx, nb), sy = min(Cy, nb), sz = min(Cz, nb);
     for (int e = w; e < sx * sy * sz; e += nwarp()) {
       int x, y, z;
-      split(e, sx, sy, x, y, z);
+      box_split(e, sx, sy, sx * sy * sz, x, y, z);
       const unsigned c = block_at(x0 + x, y0 + y, z0 + z);
       const unsigned h = __shfl_sync(0xffffffffu, ld_state(&F.head[c]), 0);
       if (h & HEAD_BUSY) continue;

@@ -25,6 +25,18 @@ extern "C" {
 int ring_take(unsigned *place, unsigned *block, hook_fn hook) { HookMem m{hook}; return psod::ring_take(m, place, *block); }
 int ring_put(unsigned *place, unsigned block) { HookMem m{nullptr}; return psod::ring_put(m, place, block); }
 unsigned long long open_word(unsigned n) { return psod::refine_open(n); }
+long wrong_splits(int sx, int sy, int sz) {
+  long bad = 0;
+  const int total = sx * sy * sz;
+  for (int z = 0, e = 0; z < sz; z++)
+    for (int y = 0; y < sy; y++)
+      for (int x = 0; x < sx; x++, e++) {
+        int a, b, c;
+        psod::box_split(e, sx, sy, total, a, b, c);
+        bad += a != x || b != y || c != z;
+      }
+  return bad;
+}
 int take(unsigned long long drawn, unsigned *item) { return psod::refine_take(drawn, *item); }
 }
 """
@@ -158,3 +170,10 @@ def test_heads_are_acquired_before_a_block_is_marked():
         i = body.index(read)
         j = body.index(mark, i)
         assert "__threadfence()" in body[i:j], fn
+
+
+@pytest.mark.parametrize("sides", [(1, 1, 1), (9, 9, 9), (33, 17, 25), (161, 161, 161), (161, 161, 162), (163, 163, 163),
+                                   (4, 1024, 1024), (1023, 1, 4100), (1, 2047, 2049), (329, 329, 329), (401, 165, 401)])
+def test_places_of_a_box(loop, sides):
+    """Both sides of the 2^22 places up to which the FP32 quotient is exact."""
+    assert loop.wrong_splits(*sides) == 0
