@@ -3401,8 +3401,14 @@ __device__ __forceinline__ int small_seed(const SodConst &K, const SodBufs &B, S
   }
   __syncthreads();
   const unsigned ncand = s_ncand;
-  if (nlist > (unsigned)NB || ncand > B.max_cand) {
-    // more records than shared memory holds: idle CTAs share the refinement
+  // The particle filed under a foreign cell lies elsewhere than its cell says:
+  // its distance-1 neighbours are not those of the cells around it, and it
+  // counts for candidates whose cells do not touch the one that lists it.
+  const bool foreign = K.has_quirk && in_sel2(K, (int)(K.quirk_listed % K.nx), (int)((K.quirk_listed / K.nx) % K.nx),
+                                              (int)(K.quirk_listed / ((unsigned)K.nx * K.nx)), g.ic, g.jc, g.kc);
+  if (foreign || nlist > (unsigned)NB || ncand > B.max_cand) {
+    // that particle among the records, or more of them than shared memory
+    // holds: the batched kernels' steps, idle CTAs sharing the refinement
     if (t == 0) {
       if (B.mode == PSOD_MODE_PLAIN) atomicAdd(B.touched, 0ull - nrec);  // counted again
       s_work = ncand <= B.max_cand ? SEED_BIG : SEED_DEFERRED;
@@ -3426,12 +3432,9 @@ __device__ __forceinline__ int small_seed(const SodConst &K, const SodBufs &B, S
   // ---- gather: coordinates in grid units, padding far from every candidate.
   // The cells reach at most 3 from the seed; where that crosses the box edge,
   // the records beyond it are moved down by nx (exact, their coordinates are
-  // above nx/2), so plain differences are minimum-image ones.  Small boxes,
-  // and a list that may hold the particle filed under a foreign cell, keep
-  // their coordinates and take the minimum image pair by pair. ----
-  const bool wrap =
-      K.nx < 16 || (K.has_quirk && in_sel2(K, (int)(K.quirk_listed % K.nx), (int)((K.quirk_listed / K.nx) % K.nx),
-                                           (int)(K.quirk_listed / ((unsigned)K.nx * K.nx)), g.ic, g.jc, g.kc));
+  // above nx/2), so plain differences are minimum-image ones.  Small boxes
+  // keep their coordinates and take the minimum image pair by pair. ----
+  const bool wrap = K.nx < 16;
   auto beyond = [&](float x) {  // coordinates above this move down
     const float h = 0.5f * K.nxf;
     return wrap ? 3e38f : (x < 3.5f ? x + h : (x > K.nxf - 3.5f ? x - h : 3e38f));
