@@ -301,20 +301,35 @@ __device__ __forceinline__ void ball_rows(const SodConst &K, double ty, double t
   khi = min(R, (int)ceil(tz + rm + 0.5));
 }
 
+// no cube row that meets such a ball lies across the periodic boundary
+__device__ __forceinline__ bool ball_rows_direct(const SodConst &K, double ty, double tz, double rm) {
+  return (double)(K.nx - K.ncut) - 0.5 - rm > fmax(fabs(ty), fabs(tz));
+}
+
 // The rows a region walk visits: the ball's window, or every row of the cube
-// where the cube nearly spans the box and a row can be near across the
-// periodic boundary.  At ncut = 11 a first ball of 1.5 cells meets about 25
-// of the cube's 529 rows, each a few FP64 operations to test.
+// where the cube nearly spans the box (or the centre lies far from the seed)
+// and a row can be near across the periodic boundary.  At ncut = 11 a first
+// ball of 1.5 cells meets about 25 of the cube's 529 rows, each a few FP64
+// operations to test.
 struct RowWin {
   int jlo, klo, ny, nrow;
   __device__ __forceinline__ RowWin(const SodConst &K, double ty, double tz, double rm) {
     int jhi = K.ncut, khi = K.ncut;
     jlo = klo = -K.ncut;
-    if (K.nx >= 2 * K.ncut + 4) ball_rows(K, ty, tz, rm, jlo, jhi, klo, khi);
+    if (ball_rows_direct(K, ty, tz, rm)) ball_rows(K, ty, tz, rm, jlo, jhi, klo, khi);
     ny = jhi - jlo + 1;
     nrow = ny * (khi - klo + 1);
   }
 };
+
+// Does the preselect cube around cell (ic, jc, kc) list the particle that the
+// run scan files under a foreign cell?  That cell need not meet a ball which
+// the particle itself lies in.
+__device__ __forceinline__ bool cube_lists_foreign(const SodConst &K, int ic, int jc, int kc) {
+  return K.has_quirk && abs(pdiff((int)(K.quirk_listed % K.nx), ic, K.nx)) <= K.ncut &&
+         abs(pdiff((int)((K.quirk_listed / K.nx) % K.nx), jc, K.nx)) <= K.ncut &&
+         abs(pdiff((int)(K.quirk_listed / ((unsigned)K.nx * K.nx)), kc, K.nx)) <= K.ncut;
+}
 
 template <typename F>
 __device__ __forceinline__ void for_region(const SodConst &K, const SodBufs &B, const Region &G, F f) {
@@ -336,6 +351,8 @@ __device__ __forceinline__ void for_region(const SodConst &K, const SodBufs &B, 
   const double rm = G.rb + 1e-3;  // margin for rounding at cell edges
   const double rm2 = rm * rm;
   const RowWin W(K, ty, tz, rm);
+  // the foreign-filed particle, the cube's last record, is visited by itself
+  const unsigned lone_end = K.has_quirk ? K.quirk_pos + 1u : 0xffffffffu;
   for (int row = w; row < W.nrow; row += nwarp()) {
     const int dj = W.jlo + row % W.ny, dk = W.klo + row / W.ny;
     const double gy = cell_gap(ty, dj, nxd), gz = cell_gap(tz, dk, nxd);
@@ -359,8 +376,13 @@ __device__ __forceinline__ void for_region(const SodConst &K, const SodBufs &B, 
     } else {
       pa[0] = x0; pb[0] = x1; np = 1;
     }
-    for (int q = 0; q < np; q++) run_records(B, B.cs[base + (unsigned)pa[q]], B.cs[base + (unsigned)pb[q] + 1], f);
+    for (int q = 0; q < np; q++) {
+      unsigned e = B.cs[base + (unsigned)pb[q] + 1];
+      if (e == lone_end) e--;
+      run_records(B, B.cs[base + (unsigned)pa[q]], e, f);
+    }
   }
+  if (threadIdx.x == 0 && cube_lists_foreign(K, G.ic, G.jc, G.kc)) f(K.quirk_pos, B.cube[K.quirk_pos]);
 }
 
 // Records filed under the region's cells (alive or not), from the cell
@@ -2699,6 +2721,10 @@ __global__ void __launch_bounds__(256) k_cross_warp(SodConst K, SodBufs B) {
   auto to_cta = [&]() {
     if (lane == 0) B.st_big[slot] = 1;
   };
+  if (cube_lists_foreign(K, G.ic, G.jc, G.kc)) {  // for_region visits that particle
+    to_cta();
+    return;
+  }
   // 3. crossing (main:2040-2100) in growing partial balls
   unsigned passes = 0;
   unsigned long long records = 0;
@@ -3610,13 +3636,9 @@ __device__ __forceinline__ int small_seed(const SodConst &K, const SodBufs &B, S
     __syncthreads();
   }
   // The list holds the preselect cube's records around the centre when the
-  // cube has the list's cells.  The particle filed under a foreign cell may
-  // lie near the centre without being in them: then the region walk finds it.
-  bool use_list = lq != ~0u && K.ncut >= 2;
-  if (K.has_quirk && abs(pdiff((int)(K.quirk_listed % K.nx), g.ic, K.nx)) <= 4 &&
-      abs(pdiff((int)((K.quirk_listed / K.nx) % K.nx), g.jc, K.nx)) <= 4 &&
-      abs(pdiff((int)(K.quirk_listed / ((unsigned)K.nx * K.nx)), g.kc, K.nx)) <= 4)
-    use_list = false;
+  // cube has the list's cells, but not a foreign-filed particle that the cube
+  // lists in another cell: then the region walk finds it.
+  const bool use_list = lq != ~0u && K.ncut >= 2 && !cube_lists_foreign(K, g.ic, g.jc, g.kc);
   cross_seed(K, B, S, slot, rank, g, na, cpos, use_list ? nlist : 0u, lq);
   return SEED_DONE;
 }

@@ -93,3 +93,19 @@ def test_plain_mode_matches_oracle(oracle, nx, gap, kind):
     assert st["nprocessed"] == r.nprocessed
     for f in FIELDS:
         assert np.array_equal(getattr(t, f), getattr(r, f)), f
+
+
+@pytest.mark.parametrize("tuning", [{}, dict(tail_max_ready=0), dict(warp_cross_min_ready=1, tail_max_ready=0)])
+@pytest.mark.parametrize("nx,gap,kind", CASES)
+def test_batched_crossing_matches_oracle(oracle, nx, gap, kind, tuning):
+    """Balls that the particle lies in although the cell that lists it does not
+    meet them: by the CTA walk of the loop and of the host rounds, and by the
+    warp walk."""
+    pos, ids = foreign_box(nx, gap, kind, 11)
+    for ncut in (3, 5):
+        kw = dict(nmin=10, nbins=6, ncut=ncut, delta=100.0)
+        r = oracle.run(oracle.Params(nx=nx, **kw), pos, ids, oracle.CANONICAL)
+        t, st, _ = table(nx, pos, ids, tuning, mode=1, **kw)
+        assert st["nprocessed"] == r.nprocessed and st["cross_touch"] == r.cross_touch
+        for f in FIELDS:
+            assert np.array_equal(getattr(t, f), getattr(r, f)), f
