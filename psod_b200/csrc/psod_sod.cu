@@ -2721,7 +2721,9 @@ __global__ void __launch_bounds__(256) k_cross_warp(SodConst K, SodBufs B) {
   auto to_cta = [&]() {
     if (lane == 0) B.st_big[slot] = 1;
   };
-  if (cube_lists_foreign(K, G.ic, G.jc, G.kc)) {  // for_region visits that particle
+  // for_region visits a foreign-filed particle, and rows of a cube that nearly
+  // spans the box which meet the ball across the periodic boundary
+  if (cube_lists_foreign(K, G.ic, G.jc, G.kc) || K.nx < 2 * K.ncut + 4) {
     to_cta();
     return;
   }
