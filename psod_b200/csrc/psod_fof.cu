@@ -67,6 +67,7 @@ struct FofGeo {
   int noff;    // neighbour offsets in c_fof_off
   float r2, rT;
   unsigned long long ncell;
+  unsigned lone;  // cube slot of the particle filed under a foreign cell, or ~0
 };
 
 // SOD cell and linking cell of one axis: the same cell as the cube's sort
@@ -160,9 +161,41 @@ __device__ __forceinline__ void uf_union(unsigned *par, unsigned a, unsigned b) 
 // ---------------------------------------------------------------------------
 // 1. linking-cell keys and the per-cell sort
 // ---------------------------------------------------------------------------
+// The particle that the run scan files under a foreign cell (the cube's last
+// record) is of none of that cell's linking cells: its key is one above them,
+// so it is a run of its own, the last of the cell, that no linking cell's
+// search finds.  k_fof_lone_link joins it to its friends.
 __global__ void k_fof_keys(const float4 *cube, long long n, FofGeo G, unsigned short *key) {
   const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (s < n) key[s] = (unsigned short)fof_key(cube[s], G);
+  if (s < n) key[s] = (unsigned short)((unsigned)s == G.lone ? (unsigned)(G.k * G.k * G.k) : fof_key(cube[s], G));
+}
+
+// The foreign-filed particle against the records of the 27 cells around its own
+// place, a CTA per cell.
+__global__ void __launch_bounds__(FOF_TPB) k_fof_lone_link(const unsigned *cs, FofGeo G, const unsigned *finv,
+                                                           const float4 *cube, unsigned *par,
+                                                           unsigned long long *counters) {
+  const float4 a = cube[G.lone];
+  const unsigned p = finv[__float_as_uint(a.w) & ~PSOD_DEAD_BIT];
+  int cx, cy, cz, f;
+  float x;
+  fof_axis(a.x, G, cx, f, x);
+  fof_axis(a.y, G, cy, f, x);
+  fof_axis(a.z, G, cz, f, x);
+  const int m = (int)blockIdx.x;
+  const int tx = (cx + m % 3 - 1 + G.nx) % G.nx, ty = (cy + (m / 3) % 3 - 1 + G.nx) % G.nx,
+            tz = (cz + m / 9 - 1 + G.nx) % G.nx;
+  const unsigned long long c =
+      (unsigned long long)tx + (unsigned long long)G.nx * ((unsigned long long)ty + (unsigned long long)G.nx * tz);
+  const unsigned b = cs[c], e = cs[c + 1];
+  unsigned tests = 0;
+  for (unsigned t = b + threadIdx.x; t < e; t += FOF_TPB) {
+    const float4 v = cube[t];
+    tests++;
+    if (t != G.lone && fof_friends(a, v, G.r2, G.rT)) uf_union(par, p, finv[__float_as_uint(v.w) & ~PSOD_DEAD_BIT]);
+  }
+  if (tests) atomicAdd(counters, (unsigned long long)tests);
+  if (threadIdx.x == 0 && b < e) atomicAdd(counters + 1, 1ull);
 }
 
 // A thread per SOD cell: cells of at most FOF_SMALL_CELL records are sorted
@@ -263,21 +296,22 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_sort_big(const unsigned *cs, co
                                                           unsigned *perm, unsigned short *skey, unsigned *par,
                                                           unsigned *finv, unsigned *flag) {
   extern __shared__ unsigned bins[];
-  unsigned *loc = bins + nbins;                                     // LOCAL: parents of the bins
-  float *rx = reinterpret_cast<float *>(loc + nbins), *ry = rx + nbins, *rz = ry + nbins;  // their first records
+  const int nall = nbins + 1;                                       // and the foreign-filed particle's
+  unsigned *loc = bins + nall;                                      // LOCAL: parents of the bins
+  float *rx = reinterpret_cast<float *>(loc + nall), *ry = rx + nall, *rz = ry + nall;  // their first records
   __shared__ unsigned s_w[FOF_TPB / 32];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
   const unsigned nb = *nbig;
-  const int per = (nbins + FOF_TPB - 1) / FOF_TPB;
+  const int per = (nall + FOF_TPB - 1) / FOF_TPB;
   for (unsigned q = blockIdx.x; q < nb; q += gridDim.x) {
     const unsigned c = big[q];
     const unsigned b = cs[c], e = cs[c + 1];
-    for (int i = tid; i < nbins; i += FOF_TPB) bins[i] = 0;
+    for (int i = tid; i < nall; i += FOF_TPB) bins[i] = 0;
     __syncthreads();
     for (unsigned s = b + tid; s < e; s += FOF_TPB) atomicAdd(&bins[key[s]], 1u);
     __syncthreads();
     {  // exclusive scan, each thread over its own bins
-      const int lo = min(nbins, tid * per), hi = min(nbins, lo + per);
+      const int lo = min(nall, tid * per), hi = min(nall, lo + per);
       unsigned own = 0;
       for (int i = lo; i < hi; i++) own += bins[i];
       unsigned inc = own;
@@ -473,6 +507,7 @@ __global__ void __launch_bounds__(FOF_TPB, 3) k_fof_link_thread(const unsigned *
   for (long long q = (long long)blockIdx.x * blockDim.x + threadIdx.x; q < nrun;
        q += (long long)gridDim.x * blockDim.x) {
     const unsigned h = heads[q], e = heads[q + 1];
+    if (perm[h] == G.lone) continue;  // linked by k_fof_lone_link
     if (e - h > FOF_THREAD_RUN) {
       if (!FULL) bigrun[atomicAdd(nbigrun, 1u)] = (unsigned)q;
       continue;
@@ -698,6 +733,7 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_cell_link(const unsigned *cs, c
     __syncthreads();
     for (unsigned p = b1 + tid; p < e1c; p += FOF_TPB) {
       const unsigned kv = skey[p];
+      if (kv >= (unsigned)nbins) continue;  // the foreign-filed particle
       if (p == b1 || skey[p - 1] != kv) {
         const unsigned r = __ldcg(par + p);
         sa[kv] = p;
@@ -868,16 +904,14 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_cell_link(const unsigned *cs, c
 //
 // k_fof_small_link: a thread per record of the small cells (those the sort has
 // linked whole), against the records of the neighbouring small cells of higher
-// index within reach.  The particle that the run scan files under a foreign
-// cell looks at all its neighbours itself: they do not find it in its own.
+// index within reach.
 __global__ void __launch_bounds__(FOF_TPB) k_fof_small_link(const unsigned *cs, long long n, FofGeo G,
                                                             const unsigned *finv, const float4 *cube,
-                                                            unsigned quirk_pos, unsigned *par,
-                                                            unsigned long long *counters) {
+                                                            unsigned *par, unsigned long long *counters) {
   const long long s = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long tests = 0, pairs = 0;
   const float reach2 = (float)G.reach2, kf = (float)G.k;
-  if (s < n) {
+  if (s < n && (unsigned)s != G.lone) {
     const float4 a = cube[s];
     int cx, cy, cz, f;
     float x, y, z;
@@ -886,8 +920,7 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_small_link(const unsigned *cs, 
     fof_axis(a.z, G, cz, f, z);
     const unsigned long long own =
         (unsigned long long)cx + (unsigned long long)G.nx * ((unsigned long long)cy + (unsigned long long)G.nx * cz);
-    const bool quirk = (unsigned)s == quirk_pos;
-    if (quirk || __ldg(cs + own + 1) - __ldg(cs + own) <= FOF_SMALL_CELL) {
+    if (__ldg(cs + own + 1) - __ldg(cs + own) <= FOF_SMALL_CELL) {
       const unsigned p = finv[__float_as_uint(a.w) & ~PSOD_DEAD_BIT];
       for (int dz = -1; dz <= 1; dz++) {
         const float gz = fmaxf(dz < 0 ? z : (dz > 0 ? kf - z : 0.f), 0.f);
@@ -907,9 +940,9 @@ __global__ void __launch_bounds__(FOF_TPB) k_fof_small_link(const unsigned *cs, 
             tx = tx < 0 ? tx + G.nx : (tx >= G.nx ? tx - G.nx : tx);
             const unsigned long long c =
                 (unsigned long long)tx + (unsigned long long)G.nx * ((unsigned long long)ty + (unsigned long long)G.nx * tz);
-            if (c <= own && !quirk) continue;  // that cell visits this one
+            if (c <= own) continue;  // that cell visits this one
             const unsigned b = __ldg(cs + c), e = __ldg(cs + c + 1);
-            if (b == e || (e - b > FOF_SMALL_CELL && !quirk)) continue;
+            if (b == e || e - b > FOF_SMALL_CELL) continue;
             pairs++;
             for (unsigned t = b; t < e; t++) {
               const float4 v = cube[t];
@@ -1404,6 +1437,7 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
   G.rT = p->percolation / (float)nres;  // FP32, as rT = r / size
   G.r2 = G.rT * G.rT;
   G.ncell = c->ncell;
+  G.lone = c->has_quirk ? c->quirk_pos : 0xffffffffu;
   PSOD_CUDA(c, cudaMemcpyToSymbolAsync(c_fof_off, offs.data(), offs.size(), 0, cudaMemcpyHostToDevice, c->stream));
 
   psod_fof_stats S{};
@@ -1442,7 +1476,7 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
   const bool tables = k <= LINK_TABLE_K && n >= LINK_TABLE_N;
   {
     // bins, their parents and first records
-    const size_t smem = (size_t)nbins * (tables ? 2 * sizeof(unsigned) + 3 * sizeof(float) : sizeof(unsigned));
+    const size_t smem = (size_t)(nbins + 1) * (tables ? 2 * sizeof(unsigned) + 3 * sizeof(float) : sizeof(unsigned));
     auto launch = [&](auto *kern) -> int {
       PSOD_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
       kern<<<1184, FOF_TPB, smem, c->stream>>>(c->d_cell_start, big, cnt, nbins, G, key, c->d_cube, perm, skey, par,
@@ -1459,6 +1493,7 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
   S.ms_sort = tm.stop();
   S.fine_cells = (int64_t)nrun;
   const size_t tab_bytes = 3 * sizeof(unsigned) * ((size_t)nbins + (FOF_TPB / 32) * (size_t)R * k * k);
+  if (c->has_quirk) k_fof_lone_link<<<27, FOF_TPB, 0, c->stream>>>(c->d_cell_start, G, finv, c->d_cube, par, ctr);
   if (tables) {
     auto link = [&](auto *kern) -> int {
       PSOD_CUDA(c, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tab_bytes));
@@ -1467,10 +1502,9 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
       return PSOD_OK;
     };
     if ((st = link(k_fof_cell_link<false>))) return st;
-    const unsigned qpos = c->has_quirk ? c->quirk_pos : 0xffffffffu;
     k_fof_mid_link<false><<<148 * 8, FOF_TPB, 0, c->stream>>>(c->d_cell_start, big, cnt, mid, cnt + 5, G, finv, c->d_cube,
                                                               nullptr, par, cnt + 3, ctr);
-    k_fof_small_link<<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cell_start, n, G, finv, c->d_cube, qpos, par, ctr);
+    k_fof_small_link<<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cell_start, n, G, finv, c->d_cube, par, ctr);
     k_fof_compress<<<grid_for(n), FOF_TPB, 0, c->stream>>>(par, n, perm, aux2);
     if ((st = link(k_fof_cell_link<true>))) return st;
     k_fof_mid_link<true><<<148 * 8, FOF_TPB, 0, c->stream>>>(c->d_cell_start, big, cnt, mid, cnt + 5, G, finv, c->d_cube,
