@@ -213,8 +213,8 @@ __device__ __forceinline__ unsigned sub_key(const float4 &p, float nxf, double3 
 // count[c] becomes BIG_FLAG | table index for cells of SUB_MIN or more
 // particles, else the cell's first slot start[c] (the fill cursor of the
 // scatter, so that one atomic gives the slot; start < n < 2^31 keeps the
-// flag bit clear).  The tables have room for every cell that can be dense, so
-// no pass counts them first (a zone of a 512^3 grid: 1.05 -> 0.64 ms).
+// flag bit clear).  bigcell has room for every cell that can be dense, so no
+// pass counts them first (a zone of a 512^3 grid: 1.05 -> 0.64 ms).
 __global__ void k_mark_big(unsigned *count, unsigned long long ncell, unsigned *nbig, unsigned *bigcell,
                            const unsigned *start) {
   const unsigned long long c = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1049,17 +1049,20 @@ int stage_cellsort(psod_ctx *c, const float *dpos) {
   if ((st = scan_u32(c, count, c->d_cell_start, (long long)c->ncell, true))) return st;
   unsigned *nbig = reinterpret_cast<unsigned *>(bad + 1);
   const long long ncell = (long long)c->ncell;
-  unsigned *tab = nullptr, *bigcell = nullptr;
-  const size_t big_cap = (size_t)n / SUB_MIN + 1;
-  if ((st = scratch(c, SLOT_BIG_TAB, big_cap * SUB_N, &tab))) return st;
-  if ((st = scratch(c, SLOT_BIG_CELL, big_cap, &bigcell))) return st;
-  k_mark_big<<<nblk(ncell, 256), 256, 0, c->stream>>>(count, c->ncell, nbig, bigcell, c->d_cell_start);
+  // the dense cells are listed in the cube's memory, which the scatter fills
+  // later, so that their tables are allocated for as many as there are
+  unsigned *tab = nullptr, *bigcell = nullptr, *found = reinterpret_cast<unsigned *>(c->d_cube);
+  static_assert(SUB_MIN * sizeof(float4) >= sizeof(unsigned), "room in the cube for the dense cells");
+  k_mark_big<<<nblk(ncell, 256), 256, 0, c->stream>>>(count, c->ncell, nbig, found, c->d_cell_start);
   int hflags[2] = {0, 0};
   PSOD_CUDA(c, cudaMemcpyAsync(hflags, bad, sizeof(hflags), cudaMemcpyDeviceToHost, c->stream));
   PSOD_CUDA(c, cudaStreamSynchronize(c->stream));
   const int hbad = hflags[0];
   const unsigned hnbig = (unsigned)hflags[1];
   if (!hbad) {
+    if ((st = scratch(c, SLOT_BIG_TAB, (size_t)hnbig * SUB_N + 1, &tab))) return st;
+    if ((st = scratch(c, SLOT_BIG_CELL, (size_t)hnbig + 1, &bigcell))) return st;
+    PSOD_CUDA(c, cudaMemcpyAsync(bigcell, found, sizeof(unsigned) * hnbig, cudaMemcpyDeviceToDevice, c->stream));
     PSOD_CUDA(c, cudaMemsetAsync(tab, 0, sizeof(unsigned) * (size_t)hnbig * SUB_N, c->stream));
     if (hnbig) {
       k_sub_count<<<nblk(n, CELL_TILE), 256, 0, c->stream>>>(rec, n, cell, count, (float)nx, xs, tab);
