@@ -284,7 +284,7 @@ enum : int {
   SLOT_BIG_TAB = 3,     // cell sort: sub-cell slot tables of dense cells
   SLOT_BIG_CELL = 4,    // cell sort: the dense cells
   SLOT_LOAD_FLAGS = 5,  // cell sort: bad-position flag, dense-cell count
-  SLOT_PART_U32 = 6,    // n u32: cell ids (load), seed tile counts (tri_cic), member pool indices (SOD)
+  SLOT_PART_U32 = 6,    // n u32: cell ids (load), seed tile counts, staged seed order (tri_cic), member pool indices (SOD)
   SLOT_PART_U64 = 7,    // n u64: member pool keys (SOD)
   SLOT_CELL_U32 = 80,   // ncell+1 u32: cell counts (load), alive counts per cell (SOD)
   SLOT_SORT_KEYS = 81,  // radix sort: key ping-pong buffer
@@ -296,7 +296,7 @@ enum : int {
   SLOT_HOST_POS = 87,   // load: device copy of host positions
   SLOT_VEL = 88,        // load: velocities
   SLOT_SEED_IDX = 89,   // tri_cic: seed order (persistent)
-  SLOT_OUT_IDX = 90,    // member indices (psod_get_halos), seed order (tri_cic) staged for a host copy
+  SLOT_OUT_IDX = 90,    // psod_get_halos: member indices staged for a host copy
   SLOT_OUT_ID = 91,     // psod_get_halos: member IDs staged for a host copy
   SLOT_H_ID = 92,       // halo table (persistent until the next SOD call)
   SLOT_H_MASS,

@@ -13,6 +13,7 @@
 //                  stable radix sort of the seeds, ties by input index.
 #include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 
 #include "psod_internal.cuh"
@@ -1263,18 +1264,24 @@ int stage_tri_cic(psod_ctx *c, int64_t *isort_out) {
   c->nseed_dense = nd;
   c->npart_new = nseed;  // main:1032 (clamped to n when every particle is dense)
   if (isort_out && nseed > 0) {
-    // widened on the device, in place for a device destination (through host
-    // vectors a 256^3 box took 13 ms of its 22; the kernel takes 20 us)
-    long long *d = reinterpret_cast<long long *>(isort_out);
-    const bool host = !is_device_ptr(isort_out);
-    if (host && (st = scratch(c, SLOT_OUT_IDX, (size_t)nseed, &d))) return st;
-    k_widen_seeds<<<nblk(nseed, 256), 256, 0, c->stream>>>(c->d_seed_idx, nseed, d);
-    PSOD_CUDA(c, cudaGetLastError());
-    if (host) {
-      if ((st = copy_out(c, isort_out, d, sizeof(int64_t) * nseed))) return st;
-    } else {
-      PSOD_CUDA(c, cudaStreamSynchronize(c->stream));
+    // widened on the device (through host vectors a 256^3 box took 13 ms of its
+    // 22; the kernel takes 20 us): in place where the destination is this
+    // device's memory, else in pieces through the tile counts' slot, which are
+    // read by now
+    cudaPointerAttributes at{};
+    const bool known = cudaPointerGetAttributes(&at, isort_out) == cudaSuccess;
+    if (!known) cudaGetLastError();
+    const bool here = known && reinterpret_cast<uintptr_t>(isort_out) % sizeof(int64_t) == 0 &&
+                      (at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == c->device));
+    long long *stage = here ? reinterpret_cast<long long *>(isort_out) : reinterpret_cast<long long *>(tiles);
+    const long long piece = here ? nseed : std::max<long long>(n, ntile + 1) / 2;
+    for (long long i = 0; i < nseed; i += piece) {
+      const long long m = std::min(piece, nseed - i);
+      k_widen_seeds<<<nblk(m, 256), 256, 0, c->stream>>>(c->d_seed_idx + i, m, stage);
+      PSOD_CUDA(c, cudaGetLastError());
+      if (!here && (st = copy_out(c, isort_out + i, stage, sizeof(int64_t) * m))) return st;
     }
+    PSOD_CUDA(c, cudaStreamSynchronize(c->stream));
   }
   c->seeds_done = true;
   return PSOD_OK;
