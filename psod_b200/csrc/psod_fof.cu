@@ -1458,14 +1458,6 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
   PSOD_CUDA(c, cudaMemsetAsync(cnt, 0, 8 * sizeof(unsigned), c->stream));
   PSOD_CUDA(c, cudaMemsetAsync(ctr, 0, 4 * sizeof(unsigned long long), c->stream));
 
-  // 1. keys and the per-cell sort (large cells listed; at most n / (FOF_SMALL_CELL + 1))
-  k_fof_keys<<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cube, n, G, key);
-  const size_t big_cap = (size_t)n / (FOF_SMALL_CELL + 1) + 1, mid_cap = (size_t)n / (LINK_SPLIT + 1) + 1;
-  if ((st = scratch(c, SLOT_FOF_BIGCELL, big_cap + mid_cap + (size_t)n / (LINK_BRUTE + 1) + 1, &big))) return st;
-  unsigned *mid = big + big_cap, *dense = mid + mid_cap;
-  k_fof_sort_small<<<grid_for((long long)c->ncell), FOF_TPB, 0, c->stream>>>(
-      c->d_cell_start, c->ncell, key, c->d_cube, G, perm, skey, par, finv, aux1, big, cnt, mid, cnt + 5, dense, cnt + 2);
-  const int nbins = k * k * k;
   // How the runs are linked.  By SOD cells (tables and record by record) where
   // the linking cells are coarse, k <= 12 or linking lengths from 0.15 cells,
   // and the box has enough cells to fill the chip; finer linking cells hold one
@@ -1474,6 +1466,19 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
   // boxes of a few large halos (50^3 with a halo of 5e4: linking 0.63 against
   // 0.84 ms; 96^3: 1.7 against 1.2 ms)
   const bool tables = k <= LINK_TABLE_K && n >= LINK_TABLE_N;
+
+  // 1. keys and the per-cell sort (large cells listed; at most n / (FOF_SMALL_CELL + 1))
+  k_fof_keys<<<grid_for(n), FOF_TPB, 0, c->stream>>>(c->d_cube, n, G, key);
+  const size_t big_cap = (size_t)n / (FOF_SMALL_CELL + 1) + 1, mid_cap = (size_t)n / (LINK_SPLIT + 1) + 1;
+  // (the linking by runs has aux2 free for the lists until its head scan)
+  big = aux2;
+  if (tables &&
+      (st = scratch(c, SLOT_FOF_BIGCELL, big_cap + mid_cap + (size_t)n / (LINK_BRUTE + 1) + 1, &big)))
+    return st;
+  unsigned *mid = big + big_cap, *dense = mid + mid_cap;
+  k_fof_sort_small<<<grid_for((long long)c->ncell), FOF_TPB, 0, c->stream>>>(
+      c->d_cell_start, c->ncell, key, c->d_cube, G, perm, skey, par, finv, aux1, big, cnt, mid, cnt + 5, dense, cnt + 2);
+  const int nbins = k * k * k;
   {
     // bins, their parents and first records
     const size_t smem = (size_t)(nbins + 1) * (tables ? 2 * sizeof(unsigned) + 3 * sizeof(float) : sizeof(unsigned));

@@ -25,8 +25,8 @@ def used():
     return total - free
 
 
-def lattice():
-    g = (torch.arange(SIDE, device="cuda", dtype=torch.float32) + 0.5) / SIDE
+def lattice(side=SIDE):
+    g = (torch.arange(side, device="cuda", dtype=torch.float32) + 0.5) / side
     z, y, x = torch.meshgrid(g, g, g, indexing="ij")
     return torch.stack([x, y, z], -1).reshape(-1, 3).contiguous()
 
@@ -68,3 +68,20 @@ def test_seed_order_to_the_host():
     assert np.array_equal(np.sort(host), np.sort(np.unique(host))) and len(host) == nn
     for g in got:
         assert np.array_equal(g, host)
+
+
+def test_linking_by_runs():
+    """Fine linking cells: the lists of large cells need no memory of their own."""
+    pos = lattice(384)
+    n = len(pos)
+    ids = torch.arange(n, device="cuda")
+    with SphericalOverdensity(2 * NX) as s:
+        s.load(pos, ids)
+        before = used()
+        st = s.fof(percolation=0.14, mmin=2, nres=2 * NX)  # 13 linking cells a cell and axis
+        assert st["fine_cells"] == n  # one record each
+        # keys (2 + 2 bytes a particle), order, parents, inverse, two work arrays,
+        # the runs' heads and list, halo scan, group codes (4 each); memory comes
+        # in pieces of 2 MiB, which n fills and the five arrays of n + 1 do not;
+        # the rest is small (the lists took 17 MB)
+        assert used() - before <= 40 * n + (16 << 20)
