@@ -3825,14 +3825,17 @@ __device__ __forceinline__ void leave_turn(const Flow &F, unsigned *keep) {
 // and the blocks that this made ready, one of them kept in *keep.  Only blocks
 // whose window holds a moved head can be: those within rb of the moved heads'
 // box.  The heads of all their windows are staged in shared memory, a slab of
-// planes at a time, and a separable minimum over them tells the ready ones
-// (windows too large for one plane of it are tested a warp per block).
+// planes at a time, and a separable minimum over them tells the ready ones.
+// Where the planes of one window do not fit (rb from 7), the threads list the
+// blocks that have a head, and each of those is tested by a warp (a warp for
+// every block, its head's read exposed, before: loop of 125^3 in one-cell
+// blocks, rb 8, 4.3 ms, now 1.9; 149^3, rb 14, 44 ms, now 24.5).
 // Bound: eight or so dependent L2 reads; tests a warp per block took
 // 25 us a seed at 512^3 (rb 4), staged 16.
 __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Smem &S, unsigned b, unsigned r,
                                              unsigned *keep) {
   constexpr long long STAGE = (long long)MAXLEV * NB;
-  __shared__ unsigned s_own;
+  __shared__ unsigned s_own, s_nlist;
   __shared__ int s_lo[3], s_hi[3];  // box of the moved heads, from b
   const int t = threadIdx.x, w = t >> 5;
   const int nb = F.nb, rb = F.rb;
@@ -3937,15 +3940,39 @@ __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Sm
       __syncthreads();
     }
   } else {
-    const int sx = min(Cx, nb), sy = min(Cy, nb), sz = min(Cz, nb);
-    for (int e = w; e < sx * sy * sz; e += nwarp()) {
-      int x, y, z;
-      box_split(e, sx, sy, sx * sy * sz, x, y, z);
-      const unsigned c = block_at(x0 + x, y0 + y, z0 + z);
-      const unsigned h = __shfl_sync(0xffffffffu, ld_state(&F.head[c]), 0);
-      if (h & HEAD_BUSY) continue;
-      if (mark_if_ready_warp(F, c, h, chain)) add_new(c);
-      __syncwarp();
+    const int sx = min(Cx, nb), sy = min(Cy, nb), sz = min(Cz, nb), nc = sx * sy * sz;
+    // the blocks with a head to test, listed a part of the box at a time
+    constexpr int PART = MAXLEV * NB, IN_FLIGHT = 8;
+    unsigned *list = S.hist[0];
+    for (int e0 = 0; e0 < nc; e0 += PART) {
+      __syncthreads();
+      if (t == 0) s_nlist = 0;
+      __syncthreads();
+      const int e1 = min(nc, e0 + PART);
+      for (int eb = e0 + t; eb < e1; eb += IN_FLIGHT * tpb()) {
+        unsigned c[IN_FLIGHT], h[IN_FLIGHT];
+#pragma unroll
+        for (int u = 0; u < IN_FLIGHT; u++) {
+          const int e = eb + u * tpb();
+          int x, y, z;
+          box_split(min(e, e1 - 1), sx, sy, nc, x, y, z);
+          c[u] = block_at(x0 + x, y0 + y, z0 + z);
+          h[u] = ld_state(&F.head[c[u]]);
+          if (e >= e1) h[u] = HEAD_BUSY;
+        }
+#pragma unroll
+        for (int u = 0; u < IN_FLIGHT; u++)
+          if (!(h[u] & HEAD_BUSY)) list[atomicAdd(&s_nlist, 1u)] = c[u];
+      }
+      __syncthreads();
+      const unsigned n = s_nlist;
+      for (unsigned k = (unsigned)w; k < n; k += (unsigned)nwarp()) {
+        const unsigned c = list[k];
+        const unsigned h = __shfl_sync(0xffffffffu, ld_state(&F.head[c]), 0);
+        if (h & HEAD_BUSY) continue;
+        if (mark_if_ready_warp(F, c, h, chain)) add_new(c);
+        __syncwarp();
+      }
     }
   }
 }
