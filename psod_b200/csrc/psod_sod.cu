@@ -3032,9 +3032,9 @@ __global__ void k_seed_blocks(const unsigned *seed_idx, const unsigned *inv, con
   long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= nseed) return;
   const float4 v = cube[inv[seed_idx[r]]];
-  const int ci = sod_cell_axis(to_grid(v.x, K.nxf), K.xs[0], K.nx) / bs;
-  const int cj = sod_cell_axis(to_grid(v.y, K.nxf), K.xs[1], K.nx) / bs;
-  const int ck = sod_cell_axis(to_grid(v.z, K.nxf), K.xs[2], K.nx) / bs;
+  const int ci = min(sod_cell_axis(to_grid(v.x, K.nxf), K.xs[0], K.nx) / bs, nb - 1);
+  const int cj = min(sod_cell_axis(to_grid(v.y, K.nxf), K.xs[1], K.nx) / bs, nb - 1);
+  const int ck = min(sod_cell_axis(to_grid(v.z, K.nxf), K.xs[2], K.nx) / bs, nb - 1);
   block_of[r] = (unsigned)ci + (unsigned)nb * ((unsigned)cj + (unsigned)nb * (unsigned)ck);
   rank[r] = (unsigned)r;
 }
@@ -3828,8 +3828,8 @@ __device__ __forceinline__ void leave_turn(const Flow &F, unsigned *keep) {
 // planes at a time, and a separable minimum over them tells the ready ones.
 // Where the planes of one window do not fit (rb from 7), the threads list the
 // blocks that have a head, and each of those is tested by a warp (a warp for
-// every block, its head's read exposed, before: loop of 125^3 in one-cell
-// blocks, rb 8, 4.3 ms, now 1.9; 149^3, rb 14, 44 ms, now 24.5).
+// every block, its head's read exposed, before: loop of 250^3 at ncut 13, rb 7,
+// 24.5 ms, now 12.5).
 // Bound: eight or so dependent L2 reads; tests a warp per block took
 // 25 us a seed at 512^3 (rb 4), staged 16.
 __device__ __forceinline__ void finish_block(const Flow &F, const SodBufs &B, Smem &S, unsigned b, unsigned r,
@@ -4488,16 +4488,18 @@ int stage_spherover(psod_ctx *c, psod_run_stats *out_stats) {
   kernels++;
 
   // block grid of the scheduler
-  // block side: the largest power of two dividing nx and at most half the
-  // dependency radius, so the window spans 2-4 blocks each way
+  // Block side: the largest power of two dividing nx and at most half the
+  // dependency radius, so the window spans 2-4 blocks each way.  An odd nx gets
+  // blocks of 2 as well, the last of an axis 3 wide: no block is narrower than
+  // bs, so cells within rdep of each other, across the periodic boundary too,
+  // still lie at most ceil(rdep / bs) blocks apart.  (Sides that had to divide
+  // nx made blocks of one cell of odd boxes: a 225^3 step 17.0 -> 11.4 ms, at
+  // ncut 13 78 -> 17; a short last block, and so a window one block wider, took
+  // 13.3 and 22; blocks of 4 for every side lengthened the chain of seeds, 150^3
+  // 5.4 -> 7.2 ms.)
   const int rdep = c->ncut + std::max(c->ncut, 2);
-  int bs = 1;
-  for (int cand = 16; cand >= 2; cand >>= 1) {
-    if (c->nx % cand == 0 && cand <= std::max(1, rdep / 2)) {
-      bs = cand;
-      break;
-    }
-  }
+  int bs = rdep / 2 >= 2 ? 2 : 1;
+  while (bs < 16 && 2 * bs <= rdep / 2 && c->nx % (2 * bs) == 0) bs *= 2;
   const int nb = c->nx / bs;
   const long long nblocks = (long long)nb * nb * nb;
   const int rb = (rdep + bs - 1) / bs;
