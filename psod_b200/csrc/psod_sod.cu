@@ -2152,6 +2152,12 @@ struct SmallList {
 };
 static_assert(sizeof(SmallList) == sizeof(unsigned) * MAXLEV * NB, "the list takes the histograms' place");
 
+// a list coordinate as the box has it: those moved down by nx carry the sign
+// (moving them is exact, and so is this; the reference's minimum image rounds
+// |x - xc| and nx - |x - xc|, which a plain difference of moved coordinates
+// does not where one of them is tiny)
+__device__ __forceinline__ float unmoved(float x, float nxf) { return __float_as_int(x) < 0 ? __fadd_rn(x, nxf) : x; }
+
 // The list's entries within LIST_R of list entry q (the refined centre), sorted
 // as load_ball_sorted sorts a region's records; the list's cells hold every
 // record within one cell of a centre in the 27 inner cells.
@@ -2162,10 +2168,11 @@ __device__ __forceinline__ unsigned load_ball_list(const SodConst &K, const SodB
   const SmallList &L = *reinterpret_cast<const SmallList *>(S.hist);
   if (threadIdx.x == 0) S.nsorted = 0;
   __syncthreads();
-  const double xc = (double)L.x[q], yc = (double)L.y[q], zc = (double)L.z[q];
+  const double xc = (double)unmoved(L.x[q], K.nxf), yc = (double)unmoved(L.y[q], K.nxf), zc = (double)unmoved(L.z[q], K.nxf);
   for (unsigned j = threadIdx.x; j < nlist; j += tpb()) {
     if (L.x[j] > 1e17f) continue;  // padding
-    const double d2 = min_image_d2((double)L.x[j], (double)L.y[j], (double)L.z[j], xc, yc, zc, K.tx);
+    const double d2 = min_image_d2((double)unmoved(L.x[j], K.nxf), (double)unmoved(L.y[j], K.nxf),
+                                   (double)unmoved(L.z[j], K.nxf), xc, yc, zc, K.tx);
     if (!(d2 <= LIST_R * LIST_R)) continue;
     const unsigned s = atomicAdd(&S.nsorted, 1u);
     if (s < CAP) {
@@ -3255,7 +3262,9 @@ __device__ __forceinline__ void list_terms(const SmallList &L, unsigned j0, unsi
       const float dx = WRAP ? mi_dx(rx, cx, K.nxf) : __fsub_rn(rx, cx), dy = WRAP ? mi_dx(ry, cy, K.nxf) : __fsub_rn(ry, cy),
                   dz = WRAP ? mi_dx(rz, cz, K.nxf) : __fsub_rn(rz, cz);
       const float d2e = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, __fmaf_rn(dz, dz, e2f)));
-      if (min_image_d2((double)rx, (double)ry, (double)rz, (double)cx, (double)cy, (double)cz, K.tx) <= K.rmin2)
+      if (min_image_d2((double)unmoved(rx, K.nxf), (double)unmoved(ry, K.nxf), (double)unmoved(rz, K.nxf),
+                       (double)unmoved(cx, K.nxf), (double)unmoved(cy, K.nxf), (double)unmoved(cz, K.nxf),
+                       K.tx) <= K.rmin2)
         sum += (double)rsqrt_pos(d2e);
     }
     return sum;
@@ -3460,8 +3469,9 @@ __device__ __forceinline__ int small_seed(const SodConst &K, const SodBufs &B, S
   // ---- gather: coordinates in grid units, padding far from every candidate.
   // The cells reach at most 3 from the seed; where that crosses the box edge,
   // the records beyond it are moved down by nx (exact, their coordinates are
-  // above nx/2), so plain differences are minimum-image ones.  Small boxes
-  // keep their coordinates and take the minimum image pair by pair. ----
+  // above nx/2), so plain differences are minimum-image ones for the FP32
+  // sums; exact distances are taken from the unmoved ones.  Small boxes keep
+  // their coordinates and take the minimum image pair by pair. ----
   const bool wrap = K.nx < 16;
   auto beyond = [&](float x) {  // coordinates above this move down
     const float h = 0.5f * K.nxf;
@@ -3492,9 +3502,10 @@ __device__ __forceinline__ int small_seed(const SodConst &K, const SodBufs &B, S
       }
       const unsigned at = c_off[c] + k;
       const float x = to_grid(v.x, K.nxf), y = to_grid(v.y, K.nxf), z = to_grid(v.z, K.nxf);
-      L.x[at] = x > ox ? x - K.nxf : x;
-      L.y[at] = y > oy ? y - K.nxf : y;
-      L.z[at] = z > oz ? z - K.nxf : z;
+      // moved: negative, -0 for nx itself; others: never -0 (unmoved)
+      L.x[at] = x > ox ? -(K.nxf - x) : fabsf(x);
+      L.y[at] = y > oy ? -(K.nxf - y) : fabsf(y);
+      L.z[at] = z > oz ? -(K.nxf - z) : fabsf(z);
       L.pos[at] = c_beg[c] + (f0 + (unsigned)(u * tpb()) - c_flat[c]);
     }
   }
@@ -3554,14 +3565,16 @@ __device__ __forceinline__ int small_seed(const SodConst &K, const SodBufs &B, S
     // exact sum of candidate q of inner cell c over this warp's share of the
     // neighbour rows (part of nparts)
     auto exact = [&](int c, unsigned q, int part, int nparts) {
-      const double cx = (double)L.x[q], cy = (double)L.y[q], cz = (double)L.z[q];
+      const double cx = (double)unmoved(L.x[q], K.nxf), cy = (double)unmoved(L.y[q], K.nxf),
+                   cz = (double)unmoved(L.z[q], K.nxf);
       unsigned long long sq = 0;
       for (int r = part; r < 9; r += nparts) {
         const int row = c + 5 * (r % 3 - 1) + 25 * (r / 3 - 1);
         for (unsigned j = c_off[row - 1] + lane; j < c_off[row + 2]; j += 32u) {
           const float rx = L.x[j];
           if (rx > 1e17f) continue;
-          const double d2 = min_image_d2((double)rx, (double)L.y[j], (double)L.z[j], cx, cy, cz, K.tx);
+          const double d2 = min_image_d2((double)unmoved(rx, K.nxf), (double)unmoved(L.y[j], K.nxf),
+                                         (double)unmoved(L.z[j], K.nxf), cx, cy, cz, K.tx);
           if (d2 <= K.rmin2) {
             const double tt = ddiv(1.0, dsqrt(dadd(d2, K.eps2)));
             sq += (unsigned long long)__double2ll_rn(dmul(tt, 1099511627776.0));
