@@ -17,12 +17,17 @@
 //      linking cells at most R = floor(l*k)+1 cells away per axis.  Each SOD
 //      cell's records are sorted by linking cell (a thread per small cell, a
 //      CTA counting sort per large one), so a linking cell is a run.
-//   2. union-find over runs.  A run starts as one component.  For every pair
-//      of neighbouring runs (each unordered pair once: offsets in a half
-//      space) the particle pairs are tested until one pair are friends, and
-//      then the two components are joined (lock-free: the larger root is
-//      hooked under the smaller with atomicCAS).  Runs of up to 4 records are
-//      handled by a thread, larger ones by a warp.
+//   2. union-find (lock-free: the larger root is hooked under the smaller with
+//      atomicCAS), in one of two forms.  By cells, for coarse linking cells in
+//      large boxes: the sort joins the groups inside each SOD cell, and what
+//      is left are friends in neighbouring SOD cells, found record by record
+//      (a thread or a warp at a time) or, for dense cells, through tables of
+//      their linking cells.  By runs otherwise: for every pair of neighbouring
+//      runs (each unordered pair once: offsets in a half space) the particle
+//      pairs are tested until one pair are friends; runs of up to 4 records
+//      are handled by a thread, larger ones by a warp.  The particle that the
+//      cell sort files under a foreign cell is a run of its own, tested against
+//      the cells around its own place.
 //   3. labels, masses, members, centres and radii as the reference computes
 //      them, per halo.
 // The friendship test is the reference's FP32 arithmetic, bit for bit: two
@@ -1461,10 +1466,15 @@ int psod_fof(psod_ctx *c, const psod_fof_params *p, psod_fof_stats *stats) {
   // How the runs are linked.  By SOD cells (tables and record by record) where
   // the linking cells are coarse, k <= 12 or linking lengths from 0.15 cells,
   // and the box has enough cells to fill the chip; finer linking cells hold one
-  // record each and their runs search the sorted keys (k = 18, a 96^3 box: 2.1
-  // ms, the tables of 18^3 cells 2.8 ms and their sort 2.4 ms more), and so do
-  // boxes of a few large halos (50^3 with a halo of 5e4: linking 0.63 against
-  // 0.84 ms; 96^3: 1.7 against 1.2 ms)
+  // record each and their runs search the sorted keys, and so do boxes of a few
+  // large halos (50^3 with a halo of 5e4: linking 0.63 against 0.84 ms; 96^3:
+  // 1.7 against 1.2 ms).  Whole call by cells / by runs, ms:
+  //   k        9           12          13          15          16          18
+  //   96^3     1.8 / 2.4   2.2 / 2.3   2.1 / 2.3   2.6 / 2.1   4.0 / 2.1   4.3 / 2.0
+  //   160^3    3.6 / 8.8   4.4 / 8.3   5.2 / 7.9   5.5 / 7.4   7.4 / 7.4   9.4 / 6.9
+  //   256^3   10.9 / 34   13.0 / 30   13.9 / 30   16.7 / 30   22.5 / 28   31.3 / 27
+  // so the line holds on either side in small boxes; larger ones would gain by
+  // cells up to k = 15.
   const bool tables = k <= LINK_TABLE_K && n >= LINK_TABLE_N;
 
   // 1. keys and the per-cell sort (large cells listed; at most n / (FOF_SMALL_CELL + 1))

@@ -245,8 +245,10 @@ __device__ __forceinline__ double widen_pos(float x) {
 
 // 1/sqrt(x) in FP64 from the FP32 estimate y0 (relative error below 2^-21):
 // Halley's third-order step y0 + y0 e (1/2 + 3/8 e), e = 1 - x y0^2, whose
-// truncation error 5/16 e^3 is below 2^-61; with its roundings the result is
-// within one ulp, as the rounded square root and quotient it replaces.
+// truncation error 5/16 e^3 is below 2^-61.  Of its roundings two count: that of
+// x y0, which moves e by at most 2^-53 and the result by half of that, and the
+// last one, half an ulp; so the result is within one ulp (the rounded square
+// root and quotient that it replaces: one and a half at worst).
 __device__ __forceinline__ double rsqrt_halley(double x, float y0f) {
   const double y0 = widen_pos(y0f);
   const double t = x * y0;

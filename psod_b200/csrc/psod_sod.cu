@@ -3220,7 +3220,7 @@ __global__ void k_ready_direct(const unsigned *active, const unsigned *nactive, 
 }
 
 // ---------------------------------------------------------------------------
-// One seed from the preselect to the claims in one CTA (the device round
+// One seed from the preselect to the claims in one CTA (the device seed
 // loop).  The alive records filed under the 125 cells within +-2 of the seed
 // cell (the reference's x_sel2) are gathered once into shared memory, cell
 // after cell, so that the three cells of a neighbour row are one contiguous
@@ -3231,8 +3231,9 @@ __global__ void k_ready_direct(const unsigned *active, const unsigned *nactive, 
 // Bound: latency of one CTA (late rounds hold a few seeds, each waiting for
 // the one before it).  Measured per round at 512^3 (1-50 seeds a round):
 // separate steps 200 us (preselect 20, refinement a warp per candidate cell
-// 120, select 12, crossing 30, seven grid barriers); one CTA about 70 a seed
-// (list 11, approximate sums 24, exact sums 5, ball 6, the rest).
+// 120, select 12, crossing 30, seven grid barriers); one CTA 41 a seed on
+// average and about 50 late in the loop (cells and counts 5, gather 4-6,
+// approximate sums 19-24, exact sums 5, ball 6, masses and claims 10).
 constexpr int SL_CELLS = 125;
 enum : int { SEED_DONE = 0, SEED_BIG = 1, SEED_DEFERRED = 2 };
 
@@ -4453,7 +4454,10 @@ static_assert((int)SC_BIGSEG < (int)SLOT_CELL_U32, "SOD scratch slots overlap th
 // at most LOOP_READY x tail_max_ready ready seeds (psod_tuning), and few
 // enough active blocks for the loop's first readiness tests (LOOP_TESTS heads
 // read).  A launch that ended on a larger seed within
-// LOOP_SHORT rounds is followed by LOOP_REST host rounds before the next.
+// LOOP_SHORT rounds is followed by LOOP_REST host rounds before the next, so
+// that a box of such seeds does not alternate launches and rounds one by one
+// (plain 256^3, learned 512^3, heavy 256^3 with LOOP_SHORT 0, 4 and 16: 20-21,
+// 146-153, 68-77 ms, no difference beyond the runs' own).
 constexpr long long LOOP_READY = 16, LOOP_CAND = 4, LOOP_TESTS = 1ll << 27;
 constexpr int LOOP_SHORT = 4, LOOP_REST = 8;
 

@@ -534,12 +534,15 @@ __global__ void k_cic_interp(const float4 *cube, long long n, CicConst k, const 
 // particles: the range look-ups, the barriers and the shared atomics are its
 // time, not HBM and not FP64), so what counts is how many tiles an SM holds
 // and how few steps one takes.  A window of 17^3 nodes, not of the whole halo's
-// 21^3, lets five CTAs run instead of three and drops 27 % of the deposits; a
+// 21^3, lets four CTAs run instead of three (64 registers a thread, 39 KB; five
+// would fit by shared memory) and drops 27 % of the deposits; a
 // tile of at most SPLIT_MAX particles adds each weight as two 20-bit halves
 // with 32-bit atomics that return nothing; a tile without particles leaves at
-// once; a record number finds its range from a table (walking the ranges took
+// once, unless the load has a foreign-filed particle, which any tile may hold;
+// a record number finds its range from a table (walking the ranges took
 // 40 % of the instructions).  512^3 box: 17.0 -> 10.4 ms; one 4^3 zone of it,
-// mostly empty tiles, 4.3 -> 2.1 ms; 150^3 (was the global grid) 0.44 -> 0.39 ms.
+// mostly empty tiles, without that particle 4.3 -> 2.1 ms; 150^3 (was the global
+// grid) 0.44 -> 0.39 ms.
 constexpr int CT = 8;             // SOD cells per tile side
 constexpr int CW = 2 * CT + 1;    // window nodes per side
 constexpr int CW3 = CW * CW * CW;
