@@ -534,8 +534,8 @@ __global__ void k_cic_interp(const float4 *cube, long long n, CicConst k, const 
 // particles: the range look-ups, the barriers and the shared atomics are its
 // time, not HBM and not FP64), so what counts is how many tiles an SM holds
 // and how few steps one takes.  A window of 17^3 nodes, not of the whole halo's
-// 21^3, lets four CTAs run instead of three (64 registers a thread, 39 KB; five
-// would fit by shared memory) and drops 27 % of the deposits; a
+// 21^3, lets four CTAs run instead of three (64 registers a thread and 42 KB:
+// both limits are four) and drops 27 % of the deposits; a
 // tile of at most SPLIT_MAX particles adds each weight as two 20-bit halves
 // with 32-bit atomics that return nothing; a tile without particles leaves at
 // once, unless the load has a foreign-filed particle, which any tile may hold;
