@@ -181,7 +181,8 @@ int psod_set_stream(psod_ctx *ctx, void *stream);
  * Builds the cell-sorted cube (the linked list of main:1564-1604).
  * Device arrays are read on the context's stream: data written on another
  * stream must be complete first (synchronise, or run the context on the
- * producer's stream with psod_set_stream). */
+ * producer's stream with psod_set_stream).  Positions outside [0,1] are
+ * refused (PSOD_ERR_ARG); a load that fails leaves no particles loaded. */
 int psod_load_particles(psod_ctx *ctx, int64_t n, const float *pos,
                         const float *vel, const int64_t *id,
                         int64_t npart_total);
